@@ -41,7 +41,6 @@ namespace {
 
 struct AdjLayout {
   int state0, ang0, der0, pop0, stack0;  // offsets (in slots) of the per-thread regions
-  int trig0;                             // the block's sin/cos table (8 slots)
   int fr0;                               // friend visits: the rotation axis, 3 per visit
   int nv, npops, depth;                  // visits, pop frames and stack depth the regions hold
 };
@@ -198,9 +197,6 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  double2 *trig = reinterpret_cast<double2 *>(sm + (size_t)lay.trig0 * PHS_ADJ_BLOCK);
-  fill_trig_table(trig);
-  __syncthreads();
 
   for (int64_t tile = warp0; tile < a.n_tiles; tile += n_warps) {
     const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
@@ -270,7 +266,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
           const double xm = xrow_at(xe, C.x_msq, seg.x_stride);
           map_msq(C.map_id, xm, s, C.m, C.w, C.msq_min, C.msq_max, C.a0, C.a1, C.a2, cmsq[j], f,
                   aux);
-          cm[j] = sqrt(cmsq[j]);
+          cm[j] = fx_sqrt(cmsq[j]);
           cmax[j] = C.m_max;
           double dd[6];
           map_derivs(C, ad.visit[v].child[j], xm, aux, dd[0], dd[1], dd[2], dd[3], dd[4], dd[5]);
@@ -281,14 +277,11 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
           }
         }
       }
-      const double d = dsub(dsub(msq_b, cmsq[0]), cmsq[1]);
-      const double lda = dsub(dmul(d, d), dmul(dmul(4.0, cmsq[0]), cmsq[1]));
-      ok = ok && (lda > 0.0) && (m_b > dadd(cm[0], cm[1])) && (m_b <= mmax_b);
-      const double sl = sqrt(lda);
-      const double rm = m_b > 0.0 ? __drcp_rn(m_b) : 0.0;
+      double sl, rm, hm;
+      ok = kallen_ok(V.massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
+      mass_reciprocals(m_b, rm, hm);
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 4) = sl;
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 5) = rm;
-      const double hm = 0.5 * rm;
       const double pc = sl * hm;
       const double ce0 = (msq_b + cmsq[0] - cmsq[1]) * hm;
       const double ce1 = (msq_b + cmsq[1] - cmsq[0]) * hm;
@@ -297,7 +290,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
       double sphi, cphi, ct, st, fct;
       const double x_phi = xrow_at(xe, V.x_phi, seg.x_stride);
       const double x_ct = xrow_at(xe, V.x_ct, seg.x_stride);
-      sincos2pi_tab(x_phi, trig, sphi, cphi);
+      sincos2pi(x_phi, sphi, cphi);
       map_ct(V.ct_class, x_ct, V.b0, V.b1, ct, st, fct);
       {
         double dct, dst, dlf;
@@ -784,17 +777,14 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
 }  // namespace
 
 void phs_adjoint_sizes(int max_visits, int max_pops, int stack_depth, bool friends, int *state0,
-                       int *ang0, int *der0, int *pop0, int *stack0, int *trig0, int *fr0,
+                       int *ang0, int *der0, int *pop0, int *stack0, int *fr0,
                        size_t *smem) {
   *state0 = 0;
   *ang0 = PHS_ADJ_STATE * max_visits;
   *der0 = *ang0 + PHS_ADJ_ANG * max_visits;
   *pop0 = *der0 + PHS_ADJ_DER * max_visits;
   *stack0 = *pop0 + 16 * max_pops;
-  *trig0 = *stack0 + PHS_STATE * (stack_depth > 0 ? stack_depth : 0);
-  static_assert(PHS_TRIG_N * sizeof(double2) % (PHS_ADJ_BLOCK * sizeof(double)) == 0,
-                "the sin/cos table fills whole slots");
-  *fr0 = *trig0 + (int)(PHS_TRIG_N * sizeof(double2) / (PHS_ADJ_BLOCK * sizeof(double)));
+  *fr0 = *stack0 + PHS_STATE * (stack_depth > 0 ? stack_depth : 0);
   const int slots = *fr0 + (friends ? 3 * max_visits : 0);
   *smem = (size_t)slots * PHS_ADJ_BLOCK * sizeof(double);
 }
@@ -817,7 +807,7 @@ cudaError_t phs_launch_adjoint(const PhsLaunch &a, const PhsAdjChannel *adj, con
   AdjLayout lay;
   size_t smem;
   phs_adjoint_sizes(max_visits, max_pops, a.stack_depth, friends, &lay.state0, &lay.ang0,
-                    &lay.der0, &lay.pop0, &lay.stack0, &lay.trig0, &lay.fr0, &smem);
+                    &lay.der0, &lay.pop0, &lay.stack0, &lay.fr0, &smem);
   lay.nv = max_visits;
   lay.npops = max_pops;
   lay.depth = a.stack_depth;
@@ -842,9 +832,9 @@ cudaError_t phs_launch_adjoint(const PhsLaunch &a, const PhsAdjChannel *adj, con
 
 int phs_adjoint_blocks_per_sm(int max_visits, int max_pops, int stack_depth, bool friends,
                               bool stored) {
-  int s0, a0, d0, p0, k0, t0, f0;
+  int s0, a0, d0, p0, k0, f0;
   size_t smem;
-  phs_adjoint_sizes(max_visits, max_pops, stack_depth, friends, &s0, &a0, &d0, &p0, &k0, &t0, &f0,
+  phs_adjoint_sizes(max_visits, max_pops, stack_depth, friends, &s0, &a0, &d0, &p0, &k0, &f0,
                     &smem);
   const void *k = adjoint_kernel(friends, stored);
   if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -250,6 +250,9 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
     }
     const bool i0 = internal(kid(cur, 0)), i1 = internal(kid(cur, 1));
     V.both_leaves = !i0 && !i1;
+    V.massless = 0;
+    for (int j = 0; j < 2; j++)
+      if (!V.child[j].internal && V.child[j].msq_leaf == 0.0) V.massless |= 1 << j;
     V.push = V.carry = -1;
     if (i0 && i1) {
       int n0 = __builtin_popcount(kid(cur, 0)), n1 = __builtin_popcount(kid(cur, 1));

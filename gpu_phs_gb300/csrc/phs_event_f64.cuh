@@ -5,12 +5,19 @@
 // with explicit round-to-nearest intrinsics wherever a value feeds the kinematic ok test
 // (msq mappings, the Kallen function and the mass sums), so ok flags match the reference
 // bit for bit whenever the transcendental functions agree; factors and boosts use FMA.
+//
+// The FP64 pipe bounds this code (two lanes a cycle and SM).  What can run beside it does:
+// the elementary functions, square roots and reciprocals (phs_fix.h), the comparisons of the
+// kinematic test (as integers), and with a massless daughter the Kallen function needs
+// neither its product nor its square root.  1e7 tt events: 13.82 -> 8.28 ms; 3e6 events of
+// the 13 TeV caterpillar (split form) 0.346 -> 0.278 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "phs_device.h"
+#include "phs_fix.h"
 #include "phs_math.h"
 #include "phs_program.h"
 
@@ -41,8 +48,9 @@ __device__ __forceinline__ void map_msq(int t, double x, double s, double m, dou
       break;
     case PHS_MAP_SCHANNEL: {
       double z = dadd(dmul(dsub(1.0, x), a0), dmul(x, a1));
-      if (-PHS_PI / 2 < z && z < PHS_PI / 2) {
-        double tz = tan(z);
+      // |z| < pi / 2, as integers (NaN is not)
+      if ((fx_bits(z) & 0x7fffffffffffffffull) < 0x3ff921fb54442d18ull) {
+        double tz = fx_tan(z);
         msq = dmul(m, dadd(m, dmul(w, tz)));
         f = a2 * (1.0 + tz * tz);
         aux = tz;
@@ -55,7 +63,7 @@ __device__ __forceinline__ void map_msq(int t, double x, double s, double m, dou
     case PHS_MAP_COLLINEAR:
     case PHS_MAP_INFRARED:
     case PHS_MAP_RADIATION: {
-      double msq1 = dmul(a0, exp(dmul(x, a1)));
+      double msq1 = dmul(a0, fx_exp(dmul(x, a1)));
       msq = dadd(dsub(msq1, a0), msq_min);
       f = a2 * msq1;
       aux = msq1;
@@ -65,7 +73,7 @@ __device__ __forceinline__ void map_msq(int t, double x, double s, double m, dou
     case PHS_MAP_UCHANNEL: {
       // one exponential per lane: the side of x = 0.5 selects its argument and the sum
       const bool lower = x < 0.5;
-      const double msq1 = dmul(a0, exp(dmul(lower ? x : dsub(1.0, x), a1)));
+      const double msq1 = dmul(a0, fx_exp(dmul(lower ? x : dsub(1.0, x), a1)));
       msq = lower ? dadd(dsub(msq1, a0), msq_min) : dadd(-dsub(msq1, a0), msq_max);
       f = a2 * msq1;
       aux = msq1;
@@ -105,10 +113,10 @@ __device__ __forceinline__ void map_ct(int ct_class, double x, double b0, double
                                        double &st, double &f) {
   if (ct_class == PHS_CT_COLLINEAR) {
     const bool lower = x < 0.5;
-    const double tmp = dmul(b0, exp(dmul(dmul(2.0, lower ? x : dsub(1.0, x)), b1)));
+    const double tmp = dmul(b0, fx_exp(dmul(dmul(2.0, lower ? x : dsub(1.0, x)), b1)));
     ct = lower ? dsub(dsub(tmp, b0), 1.0) : dadd(-dsub(tmp, b0), 1.0);
     if (ct >= -1.0 && ct <= 1.0) {
-      st = sqrt(dsub(1.0, dmul(ct, ct)));
+      st = fx_sqrt(dsub(1.0, dmul(ct, ct)));
       f = tmp * b1;
     } else {
       ct = 1.0;
@@ -118,7 +126,7 @@ __device__ __forceinline__ void map_ct(int ct_class, double x, double b0, double
   } else {
     double tmp = 2.0 * (1.0 - x);
     ct = 1.0 - tmp;
-    st = sqrt(tmp * (2.0 - tmp));
+    st = fx_sqrt(tmp * (2.0 - tmp));
     f = 1.0;
   }
 }
@@ -229,60 +237,44 @@ __device__ void child_constants(const PhsChild &C, double sqrts, double m_tot, d
   }
 }
 
-#define PHS_TRIG_N 256   // entries of the sin/cos table: (sin, cos)(2 pi k / 256)
-
-// sin and cos of 2 pi x: the nearest multiple k/256 of x, tab[k] = (sin, cos)(2 pi k / 256)
-// from a table, and the Taylor series of sine and cosine of the remainder angle
-// t = 2 pi (x - k/256), |t| <= pi/256 (terms through t^7 and t^6: the next ones are below
-// 2e-20 of the result), joined by the angle-addition formulas.  Within 2 ulp of
-// sincospi(2x).  x - k/256 is exact (Sterbenz); for 0 <= x < 2 (every x a phi mapping
-// reads) k and the remainder come from the bits of x with integer operations, which keeps
-// the reduction off the FP64 pipe (two FP64 operations: the remainder's conversion and its
-// product with 2 pi), otherwise from rint.
-__device__ __forceinline__ void sincos2pi_tab(double x, const double2 *tab, double &s, double &c) {
-  const long long b = __double_as_longlong(x);
-  const int bexp = (int)(b >> 52);   // biased exponent (b >= 0: the sign bit is clear)
-  double t;
-  int k;
-  if (b >= 0 && bexp <= 1023) {
-    // x = M 2^(e - 52) with the 53-bit significand M; 256 x = M 2^-sh, sh = 44 - e
-    const bool small = bexp < 1023 - 9;   // x < 2^-9: k = 0, t = 2 pi x
-    const int e = small ? -9 : bexp - 1023;
-    const long long M = (b & ((1ll << 52) - 1)) | (1ll << 52);
-    const int sh = 44 - e;                                   // 44 .. 53
-    const int kk = (int)((M + (1ll << (sh - 1))) >> sh);     // round(256 x)
-    const long long r = M - ((long long)kk << sh);           // x - k/256 = r 2^(e - 52)
-    // 2 pi 2^(e - 52): 2 pi with its exponent lowered (a normal number, exact)
-    const double c2 = __longlong_as_double(__double_as_longlong(6.283185307179586) +
-                                           ((long long)(e - 52) << 52));
-    k = small ? 0 : kk;
-    t = (small ? x : (double)r) * (small ? 6.283185307179586 : c2);
+// sin and cos of 2 pi x for a phi mapping's x: in fixed point for 0 <= x < 1 (absolute
+// error 2^-60), else the library's.
+__device__ __forceinline__ void sincos2pi(double x, double &s, double &c) {
+  if (fx_hi(x) < 0x3ff00000u) {
+    int64_t si, ci;
+    fx_sincos2pi_q62(fx_q64(x), si, ci);
+    s = fx_from_q62(si);
+    c = fx_from_q62(ci);
   } else {
-    const double kd = rint(x * (double)PHS_TRIG_N);
-    k = (int)((long long)kd & (PHS_TRIG_N - 1));
-    t = (x - kd * (1.0 / PHS_TRIG_N)) * 6.283185307179586;
+    sincospi(2.0 * x, &s, &c);
   }
-  const double t2 = t * t;
-  const double sr = t + t * t2 * (-1.0 / 6 + t2 * (1.0 / 120 + t2 * (-1.0 / 5040)));
-  const double cr = 1.0 + t2 * (-0.5 + t2 * (1.0 / 24 + t2 * (-1.0 / 720)));
-  const double2 v = tab[k & (PHS_TRIG_N - 1)];
-  s = v.x * cr + v.y * sr;
-  c = v.y * cr - v.x * sr;
 }
 
-// Fills the PHS_TRIG_N-entry table of sincos2pi_tab (the block's threads in turn; the
-// caller synchronises).  Multiples of pi/2 are exact.
-__device__ __forceinline__ void fill_trig_table(double2 *tab) {
-  for (int k = threadIdx.x; k < PHS_TRIG_N; k += blockDim.x) {
-    double sv, cv;
-    sincospi(k / (PHS_TRIG_N / 2.0), &sv, &cv);
-    if (k % (PHS_TRIG_N / 4) == 0) {
-      const int q = k / (PHS_TRIG_N / 4);
-      sv = q == 1 ? 1.0 : (q == 3 ? -1.0 : 0.0);
-      cv = q == 0 ? 1.0 : (q == 2 ? -1.0 : 0.0);
-    }
-    tab[k] = make_double2(sv, cv);
+// 1 / m and 1 / (2 m) of the visited branch's mass; 0 where m is not positive (its event
+// fails the kinematic test).
+__device__ __forceinline__ void mass_reciprocals(double m, double &rm, double &hm) {
+  rm = fx_hi(m) - 1u < 0x7fefffffu ? fx_rcp(m) : 0.0;
+  hm = fx_hi(m) - 0x04000000u < 0x78000000u ? fx_from_bits(fx_bits(rm) - (1ull << 52)) : 0.5 * rm;
+}
+
+// The Kallen function of the visited branch with the kinematic test, in the reference's
+// rounding: sl = sqrt(lambda); V.massless has bit j set for a massless outgoing daughter j.
+// With one of them lambda is d^2 and its rounded square root |d| itself (no over- or
+// underflow for 2^-500 < |d| < 2^500; other d take the general form).
+__device__ __forceinline__ bool kallen_ok(int massless, double msq_b, double m_b, double mmax_b,
+                                          const double cmsq[2], const double cm[2], double &sl) {
+  const double d = massless == 3 ? msq_b : dsub(dsub(msq_b, cmsq[0]), cmsq[1]);
+  bool positive;
+  if (massless != 0 && (fx_hi(d) & 0x7fffffffu) - 0x20b00000u < 0x3e800000u) {
+    sl = fx_from_bits(fx_bits(d) & 0x7fffffffffffffffull);
+    positive = true;
+  } else {
+    const double lda = dsub(dmul(d, d), dmul(dmul(4.0, cmsq[0]), cmsq[1]));
+    sl = fx_sqrt(lda);
+    positive = fx_gt(lda, 0.0);
   }
+  const double msum = massless & 1 ? cm[1] : (massless & 2 ? cm[0] : dadd(cm[0], cm[1]));
+  return positive && fx_gt(m_b, msum) && !fx_gt(m_b, mmax_b);
 }
 
 // Frame stack slot k of depth `depth`: one column per thread of a BLOCK-thread block.
@@ -296,8 +288,7 @@ __device__ __forceinline__ double stack_load(const double *smem, int depth, int 
 }
 
 // One event: segment `seg`, local index `local` (< seg.ev_count).  smem is this block's
-// frame stack, PHS_STATE * stack_depth doubles per thread of a BLOCK-thread block; trig the
-// block's table of sincos2pi_tab.
+// frame stack, PHS_STATE * stack_depth doubles per thread of a BLOCK-thread block.
 // Checked build (phs_check.h): the event's channel, its whole x row, momentum row and event
 // entries, and its program's visit count, before anything is read or written.
 __device__ __forceinline__ bool event_in_bounds(const PhsLaunch &a, const PhsSegment &seg,
@@ -319,7 +310,7 @@ __device__ __forceinline__ double xrow_at(const double *xe, int k, int stride) {
 
 template <bool PER_EVENT, int BLOCK = PHS_FWD_BLOCK>
 __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegment &seg,
-                                              int64_t local, double *smem, const double2 *trig) {
+                                              int64_t local, double *smem) {
   if (!phs_in(seg.channel, a.n_programs, PHS_CHK_CHANNEL)) return;
   const PhsChannel &ch = a.channels[seg.channel];
   if (!event_in_bounds(a, seg, local, ch.n_out, ch.n_visits)) return;
@@ -354,7 +345,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
   double msq_b = s, m_b = sqrts, p_b = 0.0, mmax_b = sqrts, E_b = sqrts;
   double factor = 1.0;
   bool ok = true;
-  int sp = 0;
+  int sp = 0, halved = 0;
 
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
@@ -375,29 +366,36 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
         map_msq(C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
                 cmsq[j], f);
         factor *= f;
-        cm[j] = sqrt(cmsq[j]);
+        cm[j] = fx_sqrt(cmsq[j]);
       }
     }
     // Kallen function and kinematic test at the visited branch (phs_cpu.cpp:218-233)
-    double d = dsub(dsub(msq_b, cmsq[0]), cmsq[1]);
-    double lda = dsub(dmul(d, d), dmul(dmul(4.0, cmsq[0]), cmsq[1]));
-    ok = ok && (lda > 0.0) && (m_b > dadd(cm[0], cm[1])) && (m_b <= mmax_b);
+    const int massless = V.massless;
+    double sl;
+    ok = kallen_ok(massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
     // one reciprocal of m serves p_decay = sqrt(lda)/(2m), sqrt(lda)/m^2, bg, gamma and the
     // daughters' energies E = (m^2 + m_j^2 - m_k^2)/(2m) (the two-body energy, equal to the
-    // reference's sqrt(m_j^2 + p^2))
-    const double sl = sqrt(lda);
-    const double rm = m_b > 0.0 ? __drcp_rn(m_b) : 0.0;
-    const double hm = 0.5 * rm;
-    const double pc = sl * hm;
-    factor *= (sl * rm) * rm;
-    const double ce0 = (msq_b + cmsq[0] - cmsq[1]) * hm;
-    const double ce1 = (msq_b + cmsq[1] - cmsq[0]) * hm;
+    // reference's sqrt(m_j^2 + p^2)); a massless daughter's is p.  Two massless daughters
+    // share m equally, and their sqrt(lda)/m^2 is 1.  sqrt(lda)/m^2 is kept halved, the
+    // powers of two put back at the end.
+    double rm, hm, pc, ce0, ce1;
+    mass_reciprocals(m_b, rm, hm);
+    if (massless == 3) {
+      pc = ce0 = ce1 = 0.5 * m_b;
+    } else {
+      pc = sl * hm;
+      factor *= pc * rm;
+      halved++;
+      const double dc = cmsq[0] - cmsq[1];
+      ce0 = massless & 1 ? pc : (msq_b + dc) * hm;
+      ce1 = massless & 2 ? pc : (msq_b - dc) * hm;
+    }
 
     // rotation + boost of the visited branch (phs_cpu.cpp:299-330)
-    const double bg = p_b * rm;
+    const double bg = V.self_root ? 0.0 : p_b * rm;
     const double ga = V.self_root ? 1.0 : E_b * rm;
     double sphi, cphi;
-    sincos2pi_tab(xrow_at(xe, V.x_phi, seg.x_stride), trig, sphi, cphi);
+    sincos2pi(xrow_at(xe, V.x_phi, seg.x_stride), sphi, cphi);
     double b0 = V.b0, b1 = V.b1;
     if (PER_EVENT && V.ct_class == PHS_CT_COLLINEAR) {
       b0 = dmul(V.m, V.m) / s;
@@ -449,13 +447,11 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
           L[4 * r + c] = l0 * E1r[c] + l1 * E2r[c] + l2 * E3r[c] + l3 * E4r[c];
       }
     } else if (V.self_root && !lab) {
-      // parent frame is the identity: L0 * L1 = L1
-      double e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-      L[0] = ga;  L[1] = e01; L[2] = 0.0;  L[3] = e03;
-      L[4] = 0.0; L[5] = e11; L[6] = e12;  L[7] = e13;
-      L[8] = 0.0; L[9] = e21; L[10] = e22; L[11] = e23;
-      L[12] = bg; L[13] = e31; L[14] = 0.0; L[15] = e33;
+      // parent frame is the identity, and the root's boost too: L0 * L1 is the rotation
+      L[0] = 1.0;  L[1] = 0.0;       L[2] = 0.0;  L[3] = 0.0;
+      L[4] = 0.0;  L[5] = ct * cphi; L[6] = e12;  L[7] = e13;
+      L[8] = 0.0;  L[9] = ct * sphi; L[10] = e22; L[11] = e23;
+      L[12] = 0.0; L[13] = -st;      L[14] = 0.0; L[15] = ct;
     } else if (PER_EVENT && V.self_root) {
       // (per-event beams, where nearly every event has a lab boost; the uniform-beam kernels
       // keep the general product, which leaves their registers to the common case)
@@ -594,7 +590,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
   }
 
   a.volume[ev] = PER_EVENT ? channel_volume(ch, sqrts) : ch.volume;
-  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? factor : 0.0;
+  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? factor * (double)(1 << halved) : 0.0;
   a.ok[ev] = ok ? 1 : 0;
   if (!ok) {
     double2 *o = reinterpret_cast<double2 *>(out);
@@ -642,12 +638,11 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const PhsSegment 
         double f;
         map_msq(C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
                 cmsq[j], f);
-        cm[j] = sqrt(cmsq[j]);
+        cm[j] = fx_sqrt(cmsq[j]);
       }
     }
-    const double d = dsub(dsub(msq_b, cmsq[0]), cmsq[1]);
-    const double lda = dsub(dmul(d, d), dmul(dmul(4.0, cmsq[0]), cmsq[1]));
-    ok = ok && (lda > 0.0) && (m_b > dadd(cm[0], cm[1])) && (m_b <= mmax_b);
+    double sl;
+    ok = kallen_ok(V.massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
     if (V.push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
       const bool j0 = V.push == 0;
       stack_store<BLOCK>(smem, sp, 16, j0 ? cmsq[0] : cmsq[1]);

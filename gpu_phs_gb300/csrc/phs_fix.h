@@ -1,0 +1,277 @@
+// phs_fix.h -- FP64 functions evaluated beside the FP64 pipe (host and device).
+//
+// GB300 issues a warp's FP64 instruction over 16 cycles of an SM (two lanes a cycle); a
+// 32 x 32 -> 64 bit multiply-add takes 1.4, a 64 x 64 -> high 64 bit product 4.3 (measured).
+// The functions here therefore run on the integer and FP32 pipes:
+//
+//   * square root and reciprocal: the seed 1/sqrt(x) or 1/x to about 2^-45 from the FP32
+//     estimate and one Newton step in FP32 with the residual of the 48-bit operand, put
+//     together as a double with integer operations; then one Newton step in FP64 with the
+//     residual exact through the FMA (Markstein): 3 and 2 FP64 instructions;
+//   * sin and cos of 2 pi x, tan, exp: 64-bit fixed point.  The argument is reduced exactly
+//     (as integers), the Taylor series run in Horner form on 64-bit products, on 32-bit
+//     ones where a term's weight is below 2^-29, and the result has about 2^-60 of
+//     error before it is rounded to double.
+//
+// SM-cycles per call of a warp, measured with every warp in the same function (this header /
+// the CUDA library): square root 55 / 152, reciprocal 38 / 92 (__drcp_rn), tan 127 / 622,
+// exp 82 / 301, sin and cos of 2 pi x 122 with the conversion to double / 497 (sincospi).
+// Beside FP64 work of other warps most of it is free.
+//
+// The header also compiles as host C++ (tests/test_fix_host.py checks the bounds stated).
+#pragma once
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#if defined(__CUDACC__)
+#define FX_FN __host__ __device__ __forceinline__
+#else
+#define FX_FN inline
+#endif
+
+#if defined(__CUDA_ARCH__)
+FX_FN uint64_t fx_mulhi(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
+FX_FN uint32_t fx_mulhi32(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+FX_FN int fx_clz64(uint64_t a) { return __clzll((long long)a); }
+FX_FN uint32_t fx_hi(double d) { return (uint32_t)__double2hiint(d); }
+FX_FN uint32_t fx_lo(double d) { return (uint32_t)__double2loint(d); }
+FX_FN double fx_double(uint32_t hi, uint32_t lo) { return __hiloint2double((int)hi, (int)lo); }
+FX_FN uint64_t fx_bits(double d) { return (uint64_t)__double_as_longlong(d); }
+FX_FN double fx_from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
+FX_FN float fx_float(uint32_t b) { return __uint_as_float(b); }
+FX_FN uint32_t fx_fbits(float f) { return __float_as_uint(f); }
+FX_FN float fx_rsqrt_est(float a) { return rsqrtf(a); }
+FX_FN float fx_rcp_est(float a) { return __fdividef(1.0f, a); }
+FX_FN float fx_fmaf(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+FX_FN float fx_mulf(float a, float b) { return __fmul_rn(a, b); }
+FX_FN int fx_rint32(float a) { return __float2int_rn(a); }
+FX_FN uint32_t fx_trunc_u32(float a) { return __float2uint_rz(a); }
+FX_FN double fx_mul(double a, double b) { return __dmul_rn(a, b); }
+FX_FN double fx_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+#else
+FX_FN uint64_t fx_mulhi(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
+FX_FN uint32_t fx_mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+FX_FN int fx_clz64(uint64_t a) { return a ? __builtin_clzll(a) : 64; }
+FX_FN uint64_t fx_bits(double d) { uint64_t b; memcpy(&b, &d, 8); return b; }
+FX_FN double fx_from_bits(uint64_t b) { double d; memcpy(&d, &b, 8); return d; }
+FX_FN uint32_t fx_hi(double d) { return (uint32_t)(fx_bits(d) >> 32); }
+FX_FN uint32_t fx_lo(double d) { return (uint32_t)fx_bits(d); }
+FX_FN double fx_double(uint32_t hi, uint32_t lo) { return fx_from_bits((uint64_t)hi << 32 | lo); }
+FX_FN float fx_float(uint32_t b) { float f; memcpy(&f, &b, 4); return f; }
+FX_FN uint32_t fx_fbits(float f) { uint32_t b; memcpy(&b, &f, 4); return b; }
+FX_FN float fx_rsqrt_est(float a) { return 1.0f / sqrtf(a); }
+FX_FN float fx_rcp_est(float a) { return 1.0f / a; }
+FX_FN float fx_fmaf(float a, float b, float c) { return fmaf(a, b, c); }
+FX_FN float fx_mulf(float a, float b) { return a * b; }
+FX_FN int fx_rint32(float a) { return (int)lrintf(a); }
+FX_FN uint32_t fx_trunc_u32(float a) { return (uint32_t)a; }
+FX_FN double fx_mul(double a, double b) { return a * b; }
+FX_FN double fx_fma(double a, double b, double c) { return fma(a, b, c); }
+#endif
+
+// ------------------------------------------------------------ square root and reciprocal
+// y0 + c (y0 in [0.5, 1), |c| < 2^-22) as a double: y0's bits widened, c added in units of
+// y0's last place.
+FX_FN uint64_t fx_seed(float y0, float c) {
+  const uint32_t b = fx_fbits(y0);
+  const uint64_t d = (uint64_t)((b >> 3) + ((1023u - 127u) << 20)) << 32 | (uint64_t)(b << 29);
+  return d + (uint64_t)(int64_t)fx_rint32(fx_mulf(c, 0x1p53f));
+}
+
+// 1/sqrt(x) to about 2^-45 for a normal x > 0; the bits of a double.
+FX_FN uint64_t fx_rsqrt_seed(double x) {
+  const uint32_t hi = fx_hi(x), lo = fx_lo(x);
+  const uint32_t be = hi >> 20, even = (be & 1u) ^ 1u;   // x = m 4^j, m in [1, 4)
+  const float mh = fx_float(((127u + even) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const float ml = fx_mulf((float)(lo & 0x1fffffffu), even ? 0x1p-51f : 0x1p-52f);
+  float y0 = fx_rsqrt_est(mh);
+  y0 = y0 < 0x1.fffffep-1f ? y0 : 0x1.fffffep-1f;
+  const float p = fx_mulf(y0, y0), pl = fx_fmaf(y0, y0, -p);
+  float e = fx_fmaf(-mh, p, 1.0f);             // 1 - m y0^2
+  e = fx_fmaf(-mh, pl, e);
+  e = fx_fmaf(-ml, p, e);
+  const float c = fx_mulf(fx_mulf(y0, e), fx_fmaf(e, 0.375f, 0.5f));
+  const int j = ((int)be - 1023) >> 1;
+  return fx_seed(y0, c) - ((uint64_t)(int64_t)j << 52);
+}
+
+// sqrt(x): the correctly rounded value but for arguments whose root lies within 2^-30 ulp
+// of a rounding boundary.  Zeros, subnormals and the smallest normals (whose residual would
+// be subnormal), infinities and NaN go to the library's; negatives give NaN.
+FX_FN double fx_sqrt(double x) {
+  const uint32_t hi = fx_hi(x);
+  if (hi - 0x08000000u >= 0x77f00000u) {
+    if (hi > 0x80000000u) return fx_double(0x7fffffffu, 0xffffffffu);   // negative
+    return sqrt(x);
+  }
+  const uint64_t rb = fx_rsqrt_seed(x);
+  const double r = fx_from_bits(rb), h = fx_from_bits(rb - (1ull << 52));
+  const double s = fx_mul(x, r);
+  return fx_fma(fx_fma(-s, s, x), h, s);
+}
+
+// 1/x within an ulp (almost always correctly rounded) for x > 0.
+FX_FN double fx_rcp(double x) {
+  const uint32_t hi = fx_hi(x), lo = fx_lo(x);
+  if (hi - 0x04000000u >= 0x78000000u) return 1.0 / x;
+  const float mh = fx_float((127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const float ml = fx_mulf((float)(lo & 0x1fffffffu), 0x1p-52f);
+  float y0 = fx_rcp_est(mh);
+  y0 = y0 < 0x1.fffffep-1f ? y0 : 0x1.fffffep-1f;
+  float e = fx_fmaf(-mh, y0, 1.0f);
+  e = fx_fmaf(-ml, y0, e);
+  const float c = fx_mulf(y0, fx_fmaf(e, e, e));
+  const double r = fx_from_bits(fx_seed(y0, c) - ((uint64_t)(int64_t)((int)(hi >> 20) - 1023) << 52));
+  return fx_fma(fx_fma(-x, r, 1.0), r, r);
+}
+
+// a > b; as integers where neither is negative or NaN.
+FX_FN bool fx_gt(double a, double b) {
+  const uint32_t ah = fx_hi(a), bh = fx_hi(b);
+  if ((ah > bh ? ah : bh) <= 0x7fefffffu) return fx_bits(a) > fx_bits(b);
+  return a > b;
+}
+
+// ---------------------------------------------------------------------- packing
+// m 2^e (m > 0 an integer) as a double, rounded to nearest; e such that the result is normal.
+FX_FN double fx_pack(uint64_t m, int e) {
+  const int z = fx_clz64(m);
+  m <<= z;
+  // bit 63 of m lands on the exponent field's lowest bit: one less is put there
+  const uint64_t r = (m >> 11) + ((m >> 10) & 1u);
+  return fx_from_bits(r + ((uint64_t)(uint32_t)(e - z + 63 + 1022) << 52));
+}
+
+// A value of Q62 (v 2^-62) as a double.
+FX_FN double fx_from_q62(int64_t v) {
+  const uint64_t a = v < 0 ? (uint64_t)-v : (uint64_t)v;
+  if (a == 0) return 0.0;
+  const double d = fx_pack(a, -62);
+  return v < 0 ? -d : d;
+}
+
+// x 2^64 for 0 <= x < 1, truncated to an integer (exact for x >= 2^-11).
+FX_FN uint64_t fx_q64(double x) {
+  const uint64_t b = fx_bits(x);
+  const int be = (int)(b >> 52);
+  const uint64_t m = (b << 11) | (1ull << 63);
+  const int sh = 1022 - be;                     // >= 0
+  return sh < 64 ? m >> sh : 0;
+}
+
+// ---------------------------------------------------------------------- sin, cos, tan
+// For v = u^2 (Q64), 0 <= u <= pi/4: w = 1 - sin(u)/u and k = 1 - cos(u), both Q64, by
+// their Taylor series in Horner form (the next terms are below 2^-63 and 2^-68).  Terms of
+// weight below 2^-28 run on 32-bit products; together within 2^-59.
+FX_FN void fx_sincos_series(uint64_t v, uint64_t &w, uint64_t &k) {
+  const uint32_t vh = (uint32_t)(v >> 32);
+  // 1/11! - v (1/13! - v (1/15! - v / 17!)), Q57, and 1/12! - v (1/14! - v (1/16! - v / 18!)), Q60
+  uint32_t a = 0x1ae7fu - fx_mulhi32(vh, 0x195u);
+  uint32_t b = 0xd740u - fx_mulhi32(vh, 0xb4u);
+  a = 0x1612461u - fx_mulhi32(vh, a);
+  b = 0xc9cba5u - fx_mulhi32(vh, b);
+  a = 0xd7322b40u - fx_mulhi32(vh, a);
+  b = 0x8f76c780u - fx_mulhi32(vh, b);
+  uint64_t s = 0x2e3bc74aad8eull - (((uint64_t)vh * a) >> 25);   // 1/9! - v (...), Q64
+  uint64_t c = 0x49f93edde28ull - (((uint64_t)vh * b) >> 28);   // 1/10! - v (...)
+  s = 0xd00d00d00d00dull - fx_mulhi(v, s);                        // 1/7!
+  c = 0x1a01a01a01a02ull - fx_mulhi(v, c);                        // 1/8!
+  s = 0x222222222222222ull - fx_mulhi(v, s);                      // 1/5!
+  c = 0x5b05b05b05b05bull - fx_mulhi(v, c);                      // 1/6!
+  s = 0x2aaaaaaaaaaaaaabull - fx_mulhi(v, s);                      // 1/3!
+  c = 0xaaaaaaaaaaaaaabull - fx_mulhi(v, c);                      // 1/4!
+  c = 0x8000000000000000ull - fx_mulhi(v, c);                     // 1/2!
+  w = fx_mulhi(v, s);
+  k = fx_mulhi(v, c);
+}
+
+// sin and cos of 2 pi x for 0 <= x < 1 given as X = x 2^64, Q62, within 2^-58.
+FX_FN void fx_sincos2pi_q62(uint64_t X, int64_t &s, int64_t &c) {
+  const uint32_t q = (uint32_t)((X + (1ull << 61)) >> 62);        // nearest quarter turn, mod 4
+  const int64_t r = (int64_t)(X - ((uint64_t)q << 62));           // |r| <= 2^61
+  const uint64_t ar = r < 0 ? (uint64_t)-r : (uint64_t)r;
+  const uint64_t u = fx_mulhi(ar << 3, 0xc90fdaa22168c235ull);    // 2 pi r 2^-64, Q64
+  uint64_t w, k;
+  fx_sincos_series(fx_mulhi(u, u), w, k);
+  int64_t sn = (int64_t)((u - fx_mulhi(u, w)) >> 2);
+  const int64_t cs = (int64_t)((1ull << 62) - (k >> 2));
+  sn = r < 0 ? -sn : sn;
+  // quarter turns: (s, c) -> (c, -s) -> (-s, -c) -> (-c, s)
+  const int64_t a = q & 1u ? cs : sn, b = q & 1u ? sn : cs;
+  s = q & 2u ? -a : a;
+  c = ((q + 1u) & 2u) ? -b : b;
+}
+
+// n / d for n, d in [2^62, 2^64): the quotient in Q62, within 2^-60 of it.
+FX_FN uint64_t fx_div_q62(uint64_t n, uint64_t d) {
+  const float y0 = fx_rcp_est((float)(uint32_t)(d >> 32));        // in [2^-32, 2^-30]
+  const uint32_t Y0 = fx_trunc_u32(fx_mulf(y0, 0x1.fffffcp+61f)); // 2^94 / d to 2^-22, below it
+  // 1 - d Y0 2^-94, in units of 2^-62
+  const uint32_t dh = (uint32_t)(d >> 32), dl = (uint32_t)d;
+  const int64_t e = (int64_t)((1ull << 62) - ((uint64_t)dh * Y0 + (((uint64_t)dl * Y0) >> 32)));
+  // 2^126 / d to 2^-43
+  const uint64_t Y = ((uint64_t)Y0 << 32) + (uint64_t)(((int64_t)(int32_t)(e >> 12) * (int64_t)(Y0 >> 1)) >> 17);
+  const uint64_t q = fx_mulhi(n, Y);                              // n / d, Q62, to 2^-43
+  const int32_t r = (int32_t)(int64_t)((n >> 2) - fx_mulhi(q, d)); // its residual, 2^-62 d
+  return q + (uint64_t)(((int64_t)r * (int64_t)(uint32_t)(Y >> 33)) >> 29);
+}
+
+// tan(z) for |z| < pi/2 as doubles: within 0.51 ulp above pi/4 and for 2^-10 < |z|; below,
+// within 2^-62 absolute.  z and, above pi/4, pi/2 - |z| are reduced exactly.
+FX_FN double fx_tan(double z) {
+  const uint32_t zh = fx_hi(z);
+  const int be = (int)((zh >> 20) & 0x7ffu);                      // <= 1023
+  const uint64_t mn = (fx_bits(z) << 11) | (1ull << 63);          // |z| = mn 2^(be - 1086)
+  const uint64_t A = 1023 - be < 64 ? mn >> (1023 - be) : 0;      // |z|, Q63
+  uint64_t un = mn;                                               // u = un 2^(e - 63)
+  int e = be - 1023;
+  const bool big = A > 0x6487ed5110b4611aull;                     // above pi/4: u = pi/2 - |z|
+  if (big) {
+    const uint64_t d = 0xc90fdaa22168c234ull - A;                 // > 0: |z| below pi/2
+    const int sh = fx_clz64(d);
+    un = (d << sh) | ((0xc4c6628b80dc1cd1ull >> 1) >> (63 - sh));
+    e = -sh;
+  }
+  const uint64_t u = -1 - e < 64 ? un >> (-1 - e) : 0;            // Q64
+  uint64_t w, k;
+  fx_sincos_series(fx_mulhi(u, u), w, k);
+  const uint64_t sn = un - fx_mulhi(un, w);                       // sin u = sn 2^(e - 63)
+  const uint64_t cs = (1ull << 63) - (k >> 1);                    // cos u, Q63
+  const uint64_t q = fx_div_q62(big ? cs : sn, big ? sn : cs);
+  const double t = fx_pack(q, (big ? -e : e) - 62);
+  return (int32_t)zh < 0 ? -t : t;
+}
+
+// ---------------------------------------------------------------------- exp
+// exp(y): for 0 <= y < 708 in fixed point (2^n 2^(j/4) exp(u), u < ln(2)/4, Taylor terms
+// through u^12) within 0.51 ulp, else the library's.
+FX_FN double fx_exp(double y) {
+  const uint32_t yh = fx_hi(y);
+  if (yh >= 0x40862000u) return exp(y);
+  const int sh = 1085 - (int)(yh >> 20);                          // >= 53
+  const uint64_t mn = (fx_bits(y) << 11) | (1ull << 63);
+  const uint64_t L = 0xb8aa3b295c17f0bcull;                       // log2(e), Q63
+  const uint64_t ph = fx_mulhi(mn, L), pl = mn * L;               // y log2(e) = ph 2^-sh
+  const int n = sh < 64 ? (int)(ph >> sh) : 0;
+  const uint64_t f = sh < 64 ? (ph << (64 - sh)) | (pl >> sh) : (sh < 128 ? ph >> (sh - 64) : 0);
+  const uint32_t j = (uint32_t)(f >> 62);
+  const uint64_t u = fx_mulhi(f & 0x3fffffffffffffffull, 0xb17217f7d1cf79acull);   // Q64
+  const uint32_t uh = (uint32_t)(u >> 32);
+  // 1/7! + u (1/8! + u (... + u / 12!)), Q44
+  uint32_t a = 440721u + fx_mulhi32(uh, 36727u);
+  a = 4847935u + fx_mulhi32(uh, a);
+  a = 48479349u + fx_mulhi32(uh, a);
+  a = 436314138u + fx_mulhi32(uh, a);
+  a = 3490513104u + fx_mulhi32(uh, a);
+  uint64_t t = 0x5b05b05b05b05bull + (((uint64_t)uh * a) >> 12);   // 1/6! + u (...), Q64
+  t = 0x222222222222222ull + fx_mulhi(u, t);
+  t = 0xaaaaaaaaaaaaaabull + fx_mulhi(u, t);
+  t = 0x2aaaaaaaaaaaaaabull + fx_mulhi(u, t);
+  t = 0x8000000000000000ull + fx_mulhi(u, t);
+  t = 0x8000000000000000ull + (fx_mulhi(u, t) >> 1);    // 1 + u (1/2 + ...), Q63
+  t = 0x8000000000000000ull + fx_mulhi(u, t);           // exp(u), Q63
+  const uint64_t c = j & 2u ? (j & 1u ? 0xd744fccad69d6af4ull : 0xb504f333f9de6484ull)
+                            : (j & 1u ? 0x9837f0518db8a96full : 0x8000000000000000ull);
+  return fx_pack(fx_mulhi(t, c), n - 62);
+}

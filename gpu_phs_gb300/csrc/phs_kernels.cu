@@ -18,13 +18,6 @@
 
 namespace {
 
-// The sin/cos table sits after the frame stack and the queues (phs_forward_smem_bytes).
-template <int BLOCK = PHS_FWD_BLOCK>
-__device__ __forceinline__ double2 *phs_trig_table(double *smem, int stack_depth) {
-  return reinterpret_cast<double2 *>(smem + (size_t)stack_depth * PHS_STATE * BLOCK +
-                                     (size_t)(BLOCK / 32) * 64);
-}
-
 // COMPACT: events whose kinematic test fails need no angles or boosts.  Where many fail
 // (low ok fractions: multi-channel batches, hard cuts), pass A tests each event, writes
 // the failures, and queues the rest per warp; pass B runs them densely.  Where nearly all
@@ -37,9 +30,6 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  double2 *trig = phs_trig_table<BLOCK>(smem, a.stack_depth);
-  fill_trig_table(trig);
-  __syncthreads();
   if constexpr (COMPACT) {
     int64_t *q = reinterpret_cast<int64_t *>(smem + (size_t)a.stack_depth * PHS_STATE * BLOCK) +
                  (threadIdx.x >> 5) * 64;
@@ -47,7 +37,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
         a, q,
         [&](const PhsSegment &sg, int64_t loc) { return phs_ok_f64<PER_EVENT, BLOCK>(a, sg, loc, smem); },
         [&](int, const PhsSegment &sg, int64_t loc) {
-          phs_event_f64<PER_EVENT, BLOCK>(a, sg, loc, smem, trig);
+          phs_event_f64<PER_EVENT, BLOCK>(a, sg, loc, smem);
         });
   } else {
     for (int64_t tile = warp0; tile < a.n_tiles; tile += n_warps) {
@@ -61,7 +51,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
       const PhsSegment seg = segs[lo];
       const int64_t local = (tile - seg.tile_begin) * 32 + lane;
       if (local >= seg.ev_count) continue;
-      phs_event_f64<PER_EVENT, BLOCK>(a, seg, local, smem, trig);
+      phs_event_f64<PER_EVENT, BLOCK>(a, seg, local, smem);
     }
   }
 }
@@ -78,9 +68,6 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, 4)
     phs_forward_exact_kernel(const __grid_constant__ PhsLaunch a) {
   extern __shared__ double smem[];
   const int lane = threadIdx.x & 31;
-  double2 *trig = phs_trig_table(smem, a.stack_depth);
-  fill_trig_table(trig);
-  __syncthreads();
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
   const int64_t n_claims = a.exact_tile[a.n_segments];
   for (;;) {
@@ -100,7 +87,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, 4)
     if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
         !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
       continue;
-    phs_event_f64<PER_EVENT>(a, seg, a.exact_queue[seg.tile_begin * 32 + idx], smem, trig);
+    phs_event_f64<PER_EVENT>(a, seg, a.exact_queue[seg.tile_begin * 32 + idx], smem);
   }
 }
 
@@ -114,9 +101,6 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     phs_f64_walk_kernel(const __grid_constant__ PhsLaunch a) {
   extern __shared__ double smem[];
   const int lane = threadIdx.x & 31;
-  double2 *trig = phs_trig_table<BLOCK>(smem, a.stack_depth);
-  fill_trig_table(trig);
-  __syncthreads();
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
   const int64_t n_claims = a.pass_tile[a.n_segments];
   for (;;) {
@@ -136,7 +120,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
         !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
       continue;
-    phs_event_f64<false, BLOCK>(a, seg, a.pass_queue[seg.tile_begin * 32 + idx], smem, trig);
+    phs_event_f64<false, BLOCK>(a, seg, a.pass_queue[seg.tile_begin * 32 + idx], smem);
   }
 }
 
@@ -233,10 +217,9 @@ cudaError_t phs_launch_fma_rate(void *out, int fp64, int blocks, int threads, in
 }
 
 size_t phs_forward_smem_bytes(int stack_depth, int block) {
-  // frame stack, the compacting variant's per-warp queues (64 events per warp), the
-  // sin/cos table
+  // frame stack, the compacting variant's per-warp queues (64 events per warp)
   return (size_t)stack_depth * PHS_STATE * block * sizeof(double) +
-         (size_t)(block / 32) * 64 * sizeof(int64_t) + PHS_TRIG_N * sizeof(double2);
+         (size_t)(block / 32) * 64 * sizeof(int64_t);
 }
 
 // Variants (each at one block shape, BLOCK threads, and a register budget): 0: one pass,

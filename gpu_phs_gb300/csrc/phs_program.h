@@ -74,7 +74,7 @@ struct PhsVisit {
   int8_t parent_root;   // 1 when the visited branch is a daughter of the root: without a lab
                         // boost its parent frame is the root's rotation, rows
                         // (1,0,0,0), (0,*,*,*), (0,*,*,*), (0,*,0,*)
-  int8_t pad1;
+  int8_t massless;      // bit j: daughter j is a massless outgoing particle
 };
 
 struct PhsChannel {

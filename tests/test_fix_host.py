@@ -1,0 +1,106 @@
+"""Host-side checks of the functions of phs_fix.h (the header compiles as plain C++) against
+long double: square root, reciprocal, tan, exp, sin and cos of 2 pi x, the comparison and the
+conversions, over every range they serve and at the edges of their reductions."""
+import os
+import subprocess
+import tempfile
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "gpu_phs_gb300", "csrc")
+
+DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <random>
+#include "phs_fix.h"
+typedef long double Q;
+static const Q PI = 3.14159265358979323846264338327950288L;
+static double ulp(double a) { a = std::fabs(a); return std::nextafter(a, INFINITY) - a; }
+static double err(double got, Q want) { return std::fabs((double)((Q)got - want)) / ulp((double)want); }
+int main() {
+  std::mt19937_64 g(1);
+  std::uniform_real_distribution<double> U(0, 1);
+  const int n = 400000;
+  long root = 0;
+  double rcp = 0, tn = 0, tsmall = 0, ex = 0, exl = 0, sc = 0, cv = 0;
+  for (int i = 0; i < n; i++) {
+    const double a = std::ldexp(1 + U(g), (int)(U(g) * 2000) - 1000);
+    root += fx_sqrt(a) != std::sqrt(a);
+    const double b = std::ldexp(1 + U(g), (int)(U(g) * 1800) - 900);
+    rcp = std::fmax(rcp, err(fx_rcp(b), 1.0L / (Q)b));
+    double z;
+    switch (i % 4) {
+      case 0: z = (2 * U(g) - 1) * M_PI / 2; break;
+      case 1: z = M_PI / 2 - std::ldexp(U(g), -(int)(U(g) * 40)); break;
+      case 2: z = std::ldexp(U(g), -(int)(U(g) * 60)); break;
+      default: z = -M_PI / 4 + (U(g) - 0.5) * 1e-3;
+    }
+    if (std::fabs(z) < M_PI / 2) {
+      // near pi/2 as the cotangent of pi/2 - |z| (the double difference is exact)
+      const Q u = (Q)(M_PI / 2 - std::fabs(z)) + 6.123233995736766035868820147292e-17L;
+      const Q want = std::fabs(z) > 1.5 ? std::copysign(1.0L / tanl(u), (Q)z) : tanl((Q)z);
+      if (std::fabs(z) > 0x1p-9)
+        tn = std::fmax(tn, err(fx_tan(z), want));
+      else if (std::fabs(z) <= 0x1p-9)
+        tsmall = std::fmax(tsmall, std::fabs((double)((Q)fx_tan(z) - want)) - ulp((double)want));
+    }
+    const double y = i % 2 ? U(g) * 40 : std::ldexp(U(g), -(int)(U(g) * 60));
+    ex = std::fmax(ex, err(fx_exp(y), expl((Q)y)));
+    const double y2 = U(g) * 708;
+    exl = std::fmax(exl, err(fx_exp(y2), expl((Q)y2)));
+    const double x = i % 2 ? U(g) : std::ldexp(U(g), -(int)(U(g) * 70));
+    int64_t s, c;
+    fx_sincos2pi_q62(fx_q64(x), s, c);
+    sc = std::fmax(sc, std::fabs((double)((Q)s * 0x1p-62L - sinl(2 * PI * (Q)x))));
+    sc = std::fmax(sc, std::fabs((double)((Q)c * 0x1p-62L - cosl(2 * PI * (Q)x))));
+    if (s) cv = std::fmax(cv, err(fx_from_q62(s), (Q)s * 0x1p-62L));
+  }
+  // edges: exact values and the ends of the reductions
+  int bad = 0;
+  for (double a : {1.0, 4.0, 0.25, 2.0, 0.0, (double)INFINITY, 5e-324, 1e-310, 1.7e308, 0x1p-896, 0x1p-897})
+    bad += fx_sqrt(a) != std::sqrt(a);
+  for (double a = 0.5; a <= 8; a *= 2)
+    for (double b : {std::nextafter(a, 0.0), std::nextafter(a, 100.0)}) {
+      bad += fx_sqrt(b) != std::sqrt(b);
+      bad += err(fx_rcp(b), 1.0L / (Q)b) > 1.001;
+    }
+  bad += !std::isnan(fx_sqrt(-1.0)) + !std::isnan(fx_sqrt(NAN)) + (fx_rcp(INFINITY) != 0) + !std::isinf(fx_rcp(0.0));
+  bad += fx_exp(0.0) != 1 || !std::isinf(fx_exp(800.0)) || !std::isnan(fx_exp(NAN)) || std::fabs(fx_exp(-3.0) - std::exp(-3.0)) > 1e-16;
+  for (double x : {0.0, 0.25, 0.5, 0.75}) {   // quarter turns are exact
+    int64_t s, c;
+    fx_sincos2pi_q62(fx_q64(x), s, c);
+    bad += (double)s * 0x1p-62 != std::rint(std::sin(2 * M_PI * x)) || (double)c * 0x1p-62 != std::rint(std::cos(2 * M_PI * x));
+  }
+  const double v[] = {-(double)INFINITY, -1.0, -0.0, 0.0, 5e-324, 0.1, 0.5, 1.0, 100.0, 1e300, INFINITY, NAN};
+  for (double a : v)
+    for (double b : v) bad += fx_gt(a, b) != (a > b);
+  std::printf("%ld %.6f %.6f %.3e %.6f %.6f %.3e %.6f %d\n", root, rcp, tn, tsmall, ex, exl, sc, cv, bad);
+  return 0;
+}
+"""
+
+
+def test_fixed_point_functions():
+    try:
+        subprocess.run(["g++", "--version"], check=True, capture_output=True)
+    except (OSError, subprocess.CalledProcessError):
+        pytest.skip("g++ not available")
+    with tempfile.TemporaryDirectory() as d:
+        src, exe = os.path.join(d, "fx.cpp"), os.path.join(d, "fx")
+        with open(src, "w") as fh:
+            fh.write(DRIVER)
+        subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=gnu++17", "-I", CSRC, src, "-o", exe],
+                       check=True)
+        root, rcp, tn, tsmall, ex, exl, sc, cv, bad = subprocess.run(
+            [exe], check=True, capture_output=True, text=True).stdout.split()
+    # half an ulp plus the fixed point's 2^-59 .. 2^-58 (and the long double's own 2^-64)
+    assert int(root) == 0                    # correctly rounded
+    assert float(rcp) <= 1.001
+    assert float(tn) <= 0.55
+    assert float(tsmall) <= 2.0 ** -61       # below 2^-9: an ulp or 2^-61
+    assert float(ex) <= 0.55 and float(exl) <= 0.75
+    assert float(sc) <= 2.0 ** -59
+    assert float(cv) <= 0.501
+    assert int(bad) == 0
