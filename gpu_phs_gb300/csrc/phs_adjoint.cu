@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
                        double *__restrict__ xbar, double *__restrict__ thbar, int th_stride,
                        AdjLayout lay, double *__restrict__ store, int64_t store_events) {
   extern __shared__ double sm[];
+  const FxRegs kr = fx_regs();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
     L[15] = L[0];
     L[3] = lab ? ch.lab_bg : 0.0;
     L[12] = L[3];
-    double msq_b = s, m_b = sqrts, p_b = 0.0, mmax_b = sqrts, E_b = sqrts;
+    double msq_b = s, m_b = sqrts, p_b = 0.0, E_b = sqrts;
     bool ok = true;
     int sp = 0, np = 0;
     for (int v = 0; v < n_visits; v++) {
@@ -253,21 +254,20 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 1) = m_b;
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 2) = p_b;
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 3) = E_b;
-      double cmsq[2], cm[2], cmax[2];
+      double cmsq[2], cm[2];
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const PhsChild &C = V.child[j];
         if (!C.internal) {
           cmsq[j] = C.msq_leaf;
           cm[j] = C.m_leaf;
-          cmax[j] = 0.0;
         } else {
           double f, aux;
           const double xm = xrow_at(xe, C.x_msq, seg.x_stride);
-          map_msq(C.map_id, xm, s, C.m, C.w, C.msq_min, C.msq_max, C.a0, C.a1, C.a2, cmsq[j], f,
+          map_msq(kr, C.map_id, xm, s, C.m, C.w, C.msq_min, C.msq_max, C.a0, C.a1, C.a2, cmsq[j], f,
                   aux);
-          cm[j] = fx_sqrt(cmsq[j]);
-          cmax[j] = C.m_max;
+          cm[j] = fx_sqrt(cmsq[j], kr);
+          ok = ok && !fx_gt(cm[j], C.m_max);
           double dd[6];
           map_derivs(C, ad.visit[v].child[j], xm, aux, dd[0], dd[1], dd[2], dd[3], dd[4], dd[5]);
           const int cv = ad.visit[v].child_visit[j];
@@ -278,8 +278,8 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
         }
       }
       double sl, rm, hm;
-      ok = kallen_ok(V.massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
-      mass_reciprocals(m_b, rm, hm);
+      ok = kallen_ok(kr, V.massless, msq_b, m_b, cmsq, cm, sl) && ok;
+      mass_reciprocals(kr, m_b, rm, hm);
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 4) = sl;
       slot(sm, lay.state0 + PHS_ADJ_STATE * v + 5) = rm;
       const double pc = sl * hm;
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
       const double x_phi = xrow_at(xe, V.x_phi, seg.x_stride);
       const double x_ct = xrow_at(xe, V.x_ct, seg.x_stride);
       sincos2pi(x_phi, sphi, cphi);
-      map_ct(V.ct_class, x_ct, V.b0, V.b1, ct, st, fct);
+      map_ct(kr, V.ct_class, x_ct, V.b0, V.b1, ct, st, fct);
       {
         double dct, dst, dlf;
         ct_derivs(V.ct_class, x_ct, V.b0, V.b1, ct, st, dct, dst, dlf);
@@ -369,8 +369,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
         slot(sm, base + 16) = j0 ? cmsq[0] : cmsq[1];
         slot(sm, base + 17) = j0 ? cm[0] : cm[1];
         slot(sm, base + 18) = j0 ? pc : -pc;
-        slot(sm, base + 19) = j0 ? cmax[0] : cmax[1];
-        slot(sm, base + 20) = j0 ? ce0 : ce1;
+        slot(sm, base + 19) = j0 ? ce0 : ce1;
         sp++;
       }
       if (V.carry >= 0) {
@@ -378,7 +377,6 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
         msq_b = j0 ? cmsq[0] : cmsq[1];
         m_b = j0 ? cm[0] : cm[1];
         p_b = j0 ? pc : -pc;
-        mmax_b = j0 ? cmax[0] : cmax[1];
         E_b = j0 ? ce0 : ce1;
       } else if (sp > 0) {
         // the frame the reverse walk resumes with after this pop
@@ -394,8 +392,7 @@ __global__ void __launch_bounds__(PHS_ADJ_BLOCK)
         msq_b = slot(sm, base + 16);
         m_b = slot(sm, base + 17);
         p_b = slot(sm, base + 18);
-        mmax_b = slot(sm, base + 19);
-        E_b = slot(sm, base + 20);
+        E_b = slot(sm, base + 19);
       }
     }
     if (!ok) continue;  // zero derivatives

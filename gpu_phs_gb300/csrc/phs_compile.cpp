@@ -181,6 +181,8 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
   out.n_out = p.n_out;
   out.n_x_used = 3 * p.n_out - 4;
   out.m_tot = m_tot;
+  out.f0 = 1.0;
+  out.inv_sqrts = 1.0 / sqrts;
 
   auto fill_child = [&](int code, PhsChild &ch) {
     memset(&ch, 0, sizeof(ch));
@@ -253,6 +255,15 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
     V.massless = 0;
     for (int j = 0; j < 2; j++)
       if (!V.child[j].internal && V.child[j].msq_leaf == 0.0) V.massless |= 1 << j;
+    V.kind = V.friend_sign    ? PHS_KIND_FRIEND
+             : V.self_root    ? PHS_KIND_ROOT
+             : V.both_leaves  ? (V.parent_root ? PHS_KIND_LEAVES_FIRST : PHS_KIND_LEAVES)
+             : V.parent_root  ? PHS_KIND_FIRST
+                              : PHS_KIND_INNER;
+    for (const PhsChild &C : V.child) {
+      if (!C.internal || C.map_id == PHS_MAP_STEP_E || C.map_id == PHS_MAP_STEP_H) continue;
+      out.f0 *= C.map_id == PHS_MAP_NO ? (C.msq_max - C.msq_min) / s : C.a2;
+    }
     V.push = V.carry = -1;
     if (i0 && i1) {
       int n0 = __builtin_popcount(kid(cur, 0)), n1 = __builtin_popcount(kid(cur, 1));

@@ -2,15 +2,28 @@
 // FP64 kernel and, as the exact fallback near kinematic limits, by the FP32-pair kernel).
 //
 // Arithmetic follows the reference CPU path (phs_cpu.cpp), whose expression order it keeps
-// with explicit round-to-nearest intrinsics wherever a value feeds the kinematic ok test
+// with separately rounded products and sums wherever a value feeds the kinematic ok test
 // (msq mappings, the Kallen function and the mass sums), so ok flags match the reference
 // bit for bit whenever the transcendental functions agree; factors and boosts use FMA.
 //
-// The FP64 pipe bounds this code (two lanes a cycle and SM).  What can run beside it does:
-// the elementary functions, square roots and reciprocals (phs_fix.h), the comparisons of the
-// kinematic test (as integers), and with a massless daughter the Kallen function needs
-// neither its product nor its square root.  1e7 tt events: 13.82 -> 8.28 ms; 3e6 events of
-// the 13 TeV caterpillar (split form) 0.346 -> 0.278 ms.
+// The FP64 pipe bounds this code (two lanes a cycle and SM), so the walk is written for few
+// FP64 instructions:
+//   * what can run beside the pipe does: the elementary functions, square roots and
+//     reciprocals (phs_fix.h), halvings and doublings, the comparisons of the kinematic test;
+//   * sums and products alone are FMAs with register constants (FxRegs: 16 cycles, not 19);
+//   * a visit's frame step has a form per position in the tree (PHS_KIND_*), so that known
+//     zeros cost nothing, and a visit of two outgoing daughters computes their momenta in its
+//     own rest frame and takes them through its parent's frame, with no frame of its own;
+//   * with massless daughters the Kallen function needs no product or square root, and two
+//     of them need no 1/m, beta or gamma either: gamma E = E_b/2, beta gamma E = p_b/2;
+//   * blocks that a visit skips are real branches: the compiler turns short ones into
+//     predicated instructions, which take their turn on the FP64 pipe all the same.
+// A tt event takes 297 FP64 instructions (445 before, 81 of them predicated off), the pipe is
+// 88 % busy.  Against the library's functions and the plain product of matrices: 1e7 tt events
+// 13.84 -> 8.29 (functions) -> 5.36 ms; 3e6 events of the 13 TeV caterpillar 0.346 -> 0.241,
+// 2^22 events over 64 channels 1.10 -> 0.62, 5e5 tt events with their own beams 0.936 -> 0.420,
+// 3e5 12-particle events 0.502 -> 0.265 ms.  Momenta are nearer the exact map (median error
+// of tt 3.1e-16 -> 2.2e-16 of the energy, against an 80-bit evaluation).
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -24,7 +37,7 @@
 #define PHS_PI 3.14159265358979323846
 #define PHS_TWOPI2 39.47841760435743447534
 #define PHS_TWOPI5 9792.62991312900650440772
-#define PHS_STATE 21  // doubles per saved frame: L[16], msq, m, p, m_max, E
+#define PHS_STATE 20  // doubles per saved frame: L[16], msq, m, p, E
 
 namespace {
 
@@ -33,26 +46,27 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
-// msq from x (phs_cpu.cpp:12-61), same expression order, no contraction.  aux receives the
-// mapping's transcendental term for the adjoint's derivatives: tan z (Breit-Wigner), the
-// exponential term a0 exp(.) (collinear, infrared, radiation, t/u channel), exp(.)(1 + a1)
-// (STEP_E); 0 otherwise.
-__device__ __forceinline__ void map_msq(int t, double x, double s, double m, double w,
-                                        double msq_min, double msq_max, double a0, double a1,
-                                        double a2, double &msq, double &f, double &aux) {
+// msq from x (phs_cpu.cpp:12-61), same expression order, no contraction.  f receives the
+// mapping's factor without its constant part (a2; the range over s of the uniform map: the
+// caller's, PhsChannel::f0 for uniform beams).  aux receives the mapping's transcendental
+// term for the adjoint's derivatives: tan z (Breit-Wigner), the exponential term a0 exp(.)
+// (collinear, infrared, radiation, t/u channel), exp(.)(1 + a1) (STEP_E); 0 otherwise.
+__device__ __forceinline__ void map_msq(const FxRegs &k, int t, double x, double s, double m,
+                                        double w, double msq_min, double msq_max, double a0,
+                                        double a1, double a2, double &msq, double &f, double &aux) {
   aux = 0.0;
   switch (t) {
     case PHS_MAP_NO:
-      msq = dadd(dmul(dsub(1.0, x), msq_min), dmul(x, msq_max));
-      f = (msq_max - msq_min) / s;
+      msq = fx_add(k, fx_mul(k, fx_sub(k, k.one, x), msq_min), fx_mul(k, x, msq_max));
+      f = 1.0;
       break;
     case PHS_MAP_SCHANNEL: {
-      double z = dadd(dmul(dsub(1.0, x), a0), dmul(x, a1));
+      const double z = fx_add(k, fx_mul(k, fx_sub(k, k.one, x), a0), fx_mul(k, x, a1));
       // |z| < pi / 2, as integers (NaN is not)
       if ((fx_bits(z) & 0x7fffffffffffffffull) < 0x3ff921fb54442d18ull) {
-        double tz = fx_tan(z);
-        msq = dmul(m, dadd(m, dmul(w, tz)));
-        f = a2 * (1.0 + tz * tz);
+        const double tz = fx_tan(z);
+        msq = fx_mul(k, m, fx_add(k, fx_mul(k, w, tz), m));
+        f = fma(tz, tz, k.one);
         aux = tz;
       } else {
         msq = 0.0;
@@ -63,19 +77,20 @@ __device__ __forceinline__ void map_msq(int t, double x, double s, double m, dou
     case PHS_MAP_COLLINEAR:
     case PHS_MAP_INFRARED:
     case PHS_MAP_RADIATION: {
-      double msq1 = dmul(a0, fx_exp(dmul(x, a1)));
-      msq = dadd(dsub(msq1, a0), msq_min);
-      f = a2 * msq1;
+      const double msq1 = fx_mul(k, a0, fx_exp(fx_mul(k, x, a1)));
+      msq = fx_add(k, fx_sub(k, msq1, a0), msq_min);
+      f = msq1;
       aux = msq1;
       break;
     }
     case PHS_MAP_TCHANNEL:
     case PHS_MAP_UCHANNEL: {
       // one exponential per lane: the side of x = 0.5 selects its argument and the sum
-      const bool lower = x < 0.5;
-      const double msq1 = dmul(a0, fx_exp(dmul(lower ? x : dsub(1.0, x), a1)));
-      msq = lower ? dadd(dsub(msq1, a0), msq_min) : dadd(-dsub(msq1, a0), msq_max);
-      f = a2 * msq1;
+      const bool lower = fx_gt(0.5, x);
+      const double msq1 = fx_mul(k, a0, fx_exp(fx_mul(k, lower ? x : fx_sub(k, k.one, x), a1)));
+      const double d = fx_sub(k, msq1, a0);
+      msq = fx_add(k, lower ? d : fx_neg(d), lower ? msq_min : msq_max);
+      f = msq1;
       aux = msq1;
       break;
     }
@@ -100,33 +115,30 @@ __device__ __forceinline__ void map_msq(int t, double x, double s, double m, dou
   }
 }
 
-__device__ __forceinline__ void map_msq(int t, double x, double s, double m, double w,
-                                        double msq_min, double msq_max, double a0, double a1,
-                                        double a2, double &msq, double &f) {
-  double aux;
-  map_msq(t, x, s, m, w, msq_min, msq_max, a0, a1, a2, msq, f, aux);
-}
-
 // cos(theta) from x (phs_cpu.cpp:112-146).  The collinear branch keeps the reference's
-// rounding: sin(theta) = sqrt(1 - ct^2) is ill-conditioned as |ct| -> 1.
-__device__ __forceinline__ void map_ct(int ct_class, double x, double b0, double b1, double &ct,
-                                       double &st, double &f) {
+// rounding: sin(theta) = sqrt(1 - ct^2) is ill-conditioned as |ct| -> 1.  The uniform map's
+// ct = 2x - 1 and st = sqrt(4 x (1 - x)) have one rounding each before the root (the
+// reference forms 1 - x first).
+__device__ __forceinline__ void map_ct(const FxRegs &k, int ct_class, double x, double b0,
+                                       double b1, double &ct, double &st, double &f) {
   if (ct_class == PHS_CT_COLLINEAR) {
-    const bool lower = x < 0.5;
-    const double tmp = dmul(b0, fx_exp(dmul(dmul(2.0, lower ? x : dsub(1.0, x)), b1)));
-    ct = lower ? dsub(dsub(tmp, b0), 1.0) : dadd(-dsub(tmp, b0), 1.0);
+    const bool lower = fx_gt(0.5, x);
+    const double y = lower ? x : fx_sub(k, k.one, x);
+    const double tmp = fx_mul(k, b0, fx_exp(fx_mul(k, fx_scale(y, 1), b1)));
+    const double d = fx_sub(k, tmp, b0);
+    ct = fx_sub(k, lower ? d : fx_neg(d), lower ? k.one : fx_neg(k.one));
     if (ct >= -1.0 && ct <= 1.0) {
-      st = fx_sqrt(dsub(1.0, dmul(ct, ct)));
-      f = tmp * b1;
+      st = fx_sqrt(fx_sub(k, k.one, fx_mul(k, ct, ct)), k);
+      f = fx_mul(k, tmp, b1);
     } else {
       ct = 1.0;
       st = 0.0;
       f = 0.0;
     }
   } else {
-    double tmp = 2.0 * (1.0 - x);
-    ct = 1.0 - tmp;
-    st = fx_sqrt(tmp * (2.0 - tmp));
+    ct = fx_sub(k, fx_scale(x, 1), k.one);
+    const double x4 = fx_scale(x, 2);
+    st = fx_sqrt(fma(-x4, x, x4), k);
     f = 1.0;
   }
 }
@@ -179,27 +191,33 @@ __device__ __forceinline__ double channel_volume(const PhsChannel &ch, double sq
 // m w; here they are products with 1/s (once per event) and the compiled 1/(m w), within an
 // ulp of the quotients (a2 weights the factor; a1 = atan(u) at u >= 10^3 moves by ulp/u).
 // msq_min = m_min^2 and m^2 do not depend on sqrt(s): the compiled values (the same bits).
-__device__ void child_constants(const PhsChild &C, double sqrts, double m_tot, double inv_s,
-                                double &a0, double &a1, double &a2, double &msq_min,
-                                double &msq_max, double &m_max) {
+__device__ void child_constants(const FxRegs &k, const PhsChild &C, double sqrts, double m_tot,
+                                double inv_s, double &a0, double &a1, double &a2,
+                                double &msq_min, double &msq_max, double &m_max) {
   double m = C.m, w = C.w, m_min = C.m_min;
-  m_max = dadd(dsub(sqrts, m_tot), m_min);
+  m_max = fx_add(k, fx_sub(k, sqrts, m_tot), m_min);
   msq_min = C.msq_min;
-  msq_max = dmul(m_max, m_max);
+  msq_max = fx_mul(k, m_max, m_max);
   a0 = a1 = a2 = 0.0;
   switch (C.map_id) {
     case PHS_MAP_NO:
-      a1 = msq_max - msq_min;
-      a2 = a1 * inv_s;
+      a1 = fx_sub(k, msq_max, msq_min);
+      a2 = fx_mul(k, a1, inv_s);
       break;
     case PHS_MAP_SCHANNEL: {
       // a0 = atan((msq_min - m^2) / (m w)) does not depend on sqrt(s): the compiled
       // program's value (the host's atan of the same argument bits, as the reference's CPU
       // path computes it) serves every event
-      const double mw = dmul(m, w);
       a0 = C.a0;
-      a1 = phs_atan_bw(dsub(msq_max, C.msq0) * C.inv_mw);   // argument >= 10^3 here in practice
-      a2 = dmul(dsub(a1, a0), mw) * inv_s;
+      const double u = fx_mul(k, fx_sub(k, msq_max, C.msq0), C.inv_mw);
+      if (!fx_gt(1024.0, u)) {   // phs_atan_large in the walk's forms (u >= 10^3 in practice)
+        const double r = fx_rcp(u, k), r2 = fx_mul(k, r, r);
+        const double at = fma(fx_mul(k, r, r2), fma(r2, 0.2, -1.0 / 3.0), r);
+        a1 = (PHS_PIO2_HI - at) + PHS_PIO2_LO;
+      } else {
+        a1 = atan(u);
+      }
+      a2 = fx_mul(k, fx_mul(k, fx_sub(k, a1, a0), fx_mul(k, m, w)), inv_s);
       break;
     }
     case PHS_MAP_RADIATION:
@@ -252,29 +270,36 @@ __device__ __forceinline__ void sincos2pi(double x, double &s, double &c) {
 
 // 1 / m and 1 / (2 m) of the visited branch's mass; 0 where m is not positive (its event
 // fails the kinematic test).
-__device__ __forceinline__ void mass_reciprocals(double m, double &rm, double &hm) {
-  rm = fx_hi(m) - 1u < 0x7fefffffu ? fx_rcp(m) : 0.0;
-  hm = fx_hi(m) - 0x04000000u < 0x78000000u ? fx_from_bits(fx_bits(rm) - (1ull << 52)) : 0.5 * rm;
+__device__ __forceinline__ void mass_reciprocals(const FxRegs &k, double m, double &rm, double &hm) {
+  rm = fx_hi(m) - 1u < 0x7fefffffu ? fx_rcp(m, k) : 0.0;
+  hm = fx_scale(rm, -1);
 }
 
 // The Kallen function of the visited branch with the kinematic test, in the reference's
-// rounding: sl = sqrt(lambda); V.massless has bit j set for a massless outgoing daughter j.
+// rounding: sl = sqrt(lambda); `massless` has bit j set for a massless outgoing daughter j.
 // With one of them lambda is d^2 and its rounded square root |d| itself (no over- or
-// underflow for 2^-500 < |d| < 2^500; other d take the general form).
-__device__ __forceinline__ bool kallen_ok(int massless, double msq_b, double m_b, double mmax_b,
+// underflow for 2^-500 < |d| < 2^500; other d take the general form).  The test's upper
+// bound, m <= m_max, is the caller's (per internal daughter, as its mass is formed).
+__device__ __forceinline__ bool kallen_ok(const FxRegs &k, int massless, double msq_b, double m_b,
                                           const double cmsq[2], const double cm[2], double &sl) {
-  const double d = massless == 3 ? msq_b : dsub(dsub(msq_b, cmsq[0]), cmsq[1]);
+  double d = msq_b, msum = cm[0];
+  if (massless == 0) {
+    d = fx_sub(k, fx_sub(k, d, cmsq[0]), cmsq[1]);
+    msum = fx_add(k, cm[0], cm[1]);
+  } else if (massless != 3) {
+    d = fx_sub(k, d, massless & 1 ? cmsq[1] : cmsq[0]);
+    msum = massless & 1 ? cm[1] : cm[0];
+  }
   bool positive;
   if (massless != 0 && (fx_hi(d) & 0x7fffffffu) - 0x20b00000u < 0x3e800000u) {
     sl = fx_from_bits(fx_bits(d) & 0x7fffffffffffffffull);
     positive = true;
   } else {
-    const double lda = dsub(dmul(d, d), dmul(dmul(4.0, cmsq[0]), cmsq[1]));
-    sl = fx_sqrt(lda);
+    const double lda = fx_sub(k, fx_mul(k, d, d), fx_mul(k, fx_scale(cmsq[0], 2), cmsq[1]));
+    sl = fx_sqrt(lda, k);
     positive = fx_gt(lda, 0.0);
   }
-  const double msum = massless & 1 ? cm[1] : (massless & 2 ? cm[0] : dadd(cm[0], cm[1]));
-  return positive && fx_gt(m_b, msum) && !fx_gt(m_b, mmax_b);
+  return positive && fx_gt(m_b, msum);
 }
 
 // Frame stack slot k of depth `depth`: one column per thread of a BLOCK-thread block.
@@ -308,9 +333,67 @@ __device__ __forceinline__ double xrow_at(const double *xe, int k, int stride) {
   return phs_in(k, stride, PHS_CHK_X) ? xe[k] : 0.0;
 }
 
+// A leaf's momentum row.
+__device__ __forceinline__ void put_momentum(double *out, int index, int n_out, double q0, double q1,
+                                             double q2, double q3) {
+  if (!phs_in(index, n_out, PHS_CHK_P)) return;
+  double2 *o = reinterpret_cast<double2 *>(out + 4 * index);
+  o[0] = make_double2(q0, q1);
+  o[1] = make_double2(q2, q3);
+}
+
+// The frame steps.  L is the parent's frame on entry and the visited branch's on return:
+// L B_z(bg, ga) R_z(phi) R_y(theta), the boost along z first and the two rotations after it
+// (phs_cpu.cpp:299-330 multiplies the same matrices), row by row in place: 12 FP64
+// instructions for a full row where the product with the multiplied-out matrix takes 12 and
+// 8 more to form its entries.
+struct Step {
+  double bg, ga, cp, sp, ct, st;
+};
+// Row (l0 l1 l2 l3); Z0: l0 = 0, Z2: l2 = 0.
+template <bool Z0, bool Z2>
+__device__ __forceinline__ void frame_row(const FxRegs &k, const Step &t, double *l) {
+  const double n0 = Z0 ? fx_mul(k, l[3], t.bg) : fma(l[0], t.ga, fx_mul(k, l[3], t.bg));
+  const double z = Z0 ? fx_mul(k, l[3], t.ga) : fma(l[0], t.bg, fx_mul(k, l[3], t.ga));
+  const double u = Z2 ? fx_mul(k, t.cp, l[1]) : fma(t.sp, l[2], fx_mul(k, t.cp, l[1]));
+  const double w = Z2 ? fx_mul(k, -t.sp, l[1]) : fma(t.cp, l[2], fx_mul(k, -t.sp, l[1]));
+  l[0] = n0;
+  l[1] = fma(t.ct, u, fx_mul(k, -t.st, z));
+  l[2] = w;
+  l[3] = fma(t.st, u, fx_mul(k, t.ct, z));
+}
+
+// The friend boost (phs.cu:853-910): the decay angles are measured from the friend beam's
+// direction in the branch's rest frame, B_z(-bg) L^-1 (1, 0, 0, ff) (only its direction
+// matters, so the lab boost inside L needs no special case); the step's matrix is
+// B_z(bg) diag(1, R_f R(theta, phi)).  Uniform per channel: no divergence.
+__device__ __forceinline__ void friend_step(double ff, const Step &t, double L[16]) {
+  const double u0 = L[0] - ff * L[12];
+  double Rf[9];
+  rot_z_onto(-(L[1] - ff * L[13]), -(L[2] - ff * L[14]), -t.bg * u0 - t.ga * (L[3] - ff * L[15]), Rf);
+  const double A[9] = {t.ct * t.cp, -t.sp, t.st * t.cp, t.ct * t.sp, t.cp, t.st * t.sp, -t.st, 0.0, t.ct};
+  double Q[9];
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      Q[3 * r + c] = Rf[3 * r] * A[c] + Rf[3 * r + 1] * A[3 + c] + Rf[3 * r + 2] * A[6 + c];
+  const double E1r[4] = {t.ga, t.bg * Q[6], t.bg * Q[7], t.bg * Q[8]};
+  const double E2r[4] = {0.0, Q[0], Q[1], Q[2]};
+  const double E3r[4] = {0.0, Q[3], Q[4], Q[5]};
+  const double E4r[4] = {t.bg, t.ga * Q[6], t.ga * Q[7], t.ga * Q[8]};
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      L[4 * r + c] = l0 * E1r[c] + l1 * E2r[c] + l2 * E3r[c] + l3 * E4r[c];
+  }
+}
+
 template <bool PER_EVENT, int BLOCK = PHS_FWD_BLOCK>
-__device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegment &seg,
-                                              int64_t local, double *smem) {
+__device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &k,
+                                              const PhsSegment &seg, int64_t local, double *smem) {
   if (!phs_in(seg.channel, a.n_programs, PHS_CHK_CHANNEL)) return;
   const PhsChannel &ch = a.channels[seg.channel];
   if (!event_in_bounds(a, seg, local, ch.n_out, ch.n_visits)) return;
@@ -320,240 +403,202 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
 
   double sqrts = ch.sqrts;
   double lab_bg = ch.lab_bg, lab_ga = ch.lab_gamma;
-  bool lab = ch.lab != 0;
+  const bool lab = PER_EVENT || ch.lab != 0;
   if (PER_EVENT) {
-    double E1 = a.E1[ev], E2 = a.E2[ev];
-    double r = sqrt(dmul(E1, E2));
-    sqrts = dmul(2.0, r);
-    lab = E1 != E2;
-    lab_bg = dsub(E1, E2) / dmul(2.0, r);
-    lab_ga = sqrt(1.0 + lab_bg * lab_bg);
+    const double E1 = a.E1[ev], E2 = a.E2[ev];
+    const double r = fx_sqrt(fx_mul(k, E1, E2), k);
+    sqrts = fx_add(k, r, r);
+    lab_bg = fx_hi(sqrts) - 0x04000000u < 0x78000000u ? fx_div(fx_sub(k, E1, E2), sqrts, k)
+                                                      : dsub(E1, E2) / sqrts;
+    lab_ga = fx_sqrt(fma(lab_bg, lab_bg, k.one), k);
   }
-  const double s = dmul(sqrts, sqrts);
-  const double inv_s = PER_EVENT ? 1.0 / s : 0.0;   // per-event mapping constants
+  const double s = fx_mul(k, sqrts, sqrts);
+  const double inv_s = PER_EVENT ? fx_rcp(s, k) : 0.0;   // per-event mapping constants
 
-  // frame of the visited branch; the root's parent frame is the lab boost (or 1)
+  // frame of the visited branch (the root's parent frame, the lab boost or 1, is in its step)
   double L[16];
 #pragma unroll
   for (int i = 0; i < 16; i++) L[i] = 0.0;
-  L[0] = lab ? lab_ga : 1.0;
-  L[5] = 1.0;
-  L[10] = 1.0;
-  L[15] = L[0];
-  L[3] = lab ? lab_bg : 0.0;
-  L[12] = L[3];
-  double msq_b = s, m_b = sqrts, p_b = 0.0, mmax_b = sqrts, E_b = sqrts;
-  double factor = 1.0;
+  double msq_b = s, m_b = sqrts, p_b = 0.0, E_b = sqrts;
+  double factor = PER_EVENT ? 1.0 : ch.f0;
   bool ok = true;
   int sp = 0, halved = 0;
 
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
-    double cmsq[2], cm[2], cmax[2];
+    double cmsq[2], cm[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
       if (!C.internal) {
         cmsq[j] = C.msq_leaf;
         cm[j] = C.m_leaf;
-        cmax[j] = 0.0;
       } else {
-        double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max;
-        cmax[j] = C.m_max;
-        if (PER_EVENT) child_constants(C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, cmax[j]);
-        double f;
-        map_msq(C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
-                cmsq[j], f);
-        factor *= f;
-        cm[j] = fx_sqrt(cmsq[j]);
+        double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
+        if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
+        double f, aux;
+        map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
+                cmsq[j], f, aux);
+        if (PER_EVENT && C.map_id != PHS_MAP_STEP_E && C.map_id != PHS_MAP_STEP_H) factor = fx_mul(k, factor, a2);
+        if (C.map_id != PHS_MAP_NO) factor = fx_mul(k, factor, f);
+        cm[j] = fx_sqrt(cmsq[j], k);
+        ok = ok && !fx_gt(cm[j], mmax);   // NaN fails at the daughter's own visit
       }
     }
     // Kallen function and kinematic test at the visited branch (phs_cpu.cpp:218-233)
     const int massless = V.massless;
     double sl;
-    ok = kallen_ok(massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
+    ok = kallen_ok(k, massless, msq_b, m_b, cmsq, cm, sl) && ok;
     // one reciprocal of m serves p_decay = sqrt(lda)/(2m), sqrt(lda)/m^2, bg, gamma and the
     // daughters' energies E = (m^2 + m_j^2 - m_k^2)/(2m) (the two-body energy, equal to the
-    // reference's sqrt(m_j^2 + p^2)); a massless daughter's is p.  Two massless daughters
-    // share m equally, and their sqrt(lda)/m^2 is 1.  sqrt(lda)/m^2 is kept halved, the
-    // powers of two put back at the end.
-    double rm, hm, pc, ce0, ce1;
-    mass_reciprocals(m_b, rm, hm);
+    // reference's sqrt(m_j^2 + p^2)); a massless daughter's is p, the other's then m - p.
+    // Two massless daughters share m equally, their sqrt(lda)/m^2 is 1, and as the last
+    // visit of their line nothing else needs 1/m.  sqrt(lda)/m^2 is kept halved, the powers
+    // of two put back at the end.
+    int kind = V.kind;
+    if (lab)
+      kind = kind == PHS_KIND_ROOT ? PHS_KIND_ROOT_LAB
+             : kind == PHS_KIND_FIRST ? PHS_KIND_FIRST_LAB
+             : kind == PHS_KIND_LEAVES_FIRST ? PHS_KIND_LEAVES : kind;
+    const bool pair = kind == PHS_KIND_LEAVES || kind == PHS_KIND_LEAVES_FIRST;
+    double rm = 0.0, pc, ce0, ce1;
     if (massless == 3) {
-      pc = ce0 = ce1 = 0.5 * m_b;
+      pc = ce0 = ce1 = fx_scale(m_b, -1);
+      if (!pair) rm = fx_hi(m_b) - 1u < 0x7fefffffu ? fx_rcp(m_b, k) : 0.0;   // a friend's, or n_out = 2
     } else {
-      pc = sl * hm;
-      factor *= pc * rm;
+      double hm;
+      if (!PER_EVENT && V.self_root) {
+        rm = ch.inv_sqrts;
+        hm = fx_scale(rm, -1);
+      } else {
+        mass_reciprocals(k, m_b, rm, hm);
+      }
+      pc = fx_mul(k, sl, hm);
+      factor = fx_mul(k, factor, fx_mul(k, pc, rm));
       halved++;
-      const double dc = cmsq[0] - cmsq[1];
-      ce0 = massless & 1 ? pc : (msq_b + dc) * hm;
-      ce1 = massless & 2 ? pc : (msq_b - dc) * hm;
+      if (massless == 0) {
+        const double dc = fx_sub(k, cmsq[0], cmsq[1]);
+        ce0 = fx_mul(k, fx_add(k, msq_b, dc), hm);
+        ce1 = fx_mul(k, fx_sub(k, msq_b, dc), hm);
+      } else {
+        const double eo = fx_sub(k, m_b, pc);
+        ce0 = massless & 1 ? pc : eo;
+        ce1 = massless & 1 ? eo : pc;
+      }
     }
 
-    // rotation + boost of the visited branch (phs_cpu.cpp:299-330)
-    const double bg = V.self_root ? 0.0 : p_b * rm;
-    const double ga = V.self_root ? 1.0 : E_b * rm;
-    double sphi, cphi;
-    sincos2pi(xrow_at(xe, V.x_phi, seg.x_stride), sphi, cphi);
+    // the decay angles
+    Step t;
+    sincos2pi(xrow_at(xe, V.x_phi, seg.x_stride), t.sp, t.cp);
     double b0 = V.b0, b1 = V.b1;
     if (PER_EVENT && V.ct_class == PHS_CT_COLLINEAR) {
       b0 = dmul(V.m, V.m) / s;
       b1 = log(dadd(b0, 1.0) / b0);
     }
-    double ct, st, fct;
-    map_ct(V.ct_class, xrow_at(xe, V.x_ct, seg.x_stride), b0, b1, ct, st, fct);
-    if (V.ct_class == PHS_CT_COLLINEAR) factor *= fct;   // the uniform map's factor is 1
-    const double e03 = bg * ct, e12 = -sphi, e13 = st * cphi;
-    const double e22 = cphi, e23 = st * sphi, e33 = ga * ct;
-    // the entries of L1 that only the frame's columns 1 and 2 read: formed in the branches
-    // that write those (a leaf-only visit writes columns 0 and 3 only)
-    const auto col12 = [&](double &e01, double &e11, double &e21, double &e31) {
-      e01 = -bg * st;
-      e11 = ct * cphi;
-      e21 = ct * sphi;
-      e31 = -ga * st;
-    };
+    double fct;
+    map_ct(k, V.ct_class, xrow_at(xe, V.x_ct, seg.x_stride), b0, b1, t.ct, t.st, fct);
+    if (V.ct_class == PHS_CT_COLLINEAR) factor = fx_mul(k, factor, fct);   // the uniform map's factor is 1
 
-    // the frame is updated in place: row r of L L1 depends on row r of L only
-    if (V.friend_sign != 0) {
-      // friend boost (phs.cu:853-910): the decay angles are measured from the friend
-      // beam's direction in the branch's rest frame, B_z(-bg) L^-1 (1, 0, 0, ff) (only
-      // its direction matters, so the lab boost inside L needs no special case);
-      // L1 = B_z(bg) diag(1, R_f R(theta, phi)).  Uniform per channel: no divergence.
-      const double ff = V.friend_sign;
-      const double u0 = L[0] - ff * L[12];
-      double Rf[9];
-      rot_z_onto(-(L[1] - ff * L[13]), -(L[2] - ff * L[14]),
-                 -bg * u0 - ga * (L[3] - ff * L[15]), Rf);
-      double e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-      const double A[9] = {e11, e12, e13, e21, e22, e23, -st, 0.0, ct};
-      double Q[9];
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          Q[3 * r + c] = Rf[3 * r] * A[c] + Rf[3 * r + 1] * A[3 + c] + Rf[3 * r + 2] * A[6 + c];
-      const double E1r[4] = {ga, bg * Q[6], bg * Q[7], bg * Q[8]};
-      const double E2r[4] = {0.0, Q[0], Q[1], Q[2]};
-      const double E3r[4] = {0.0, Q[3], Q[4], Q[5]};
-      const double E4r[4] = {bg, ga * Q[6], ga * Q[7], ga * Q[8]};
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-          L[4 * r + c] = l0 * E1r[c] + l1 * E2r[c] + l2 * E3r[c] + l3 * E4r[c];
+    if (pair) {
+      // two outgoing daughters: (E, 0, 0, +-p) rotated by (theta, phi), boosted along z by
+      // (bg, gamma) and taken through the parent's frame; the transverse part is shared up
+      // to its sign
+      const double pst = fx_mul(k, pc, t.st), qx = fx_mul(k, pst, t.cp), qy = fx_mul(k, pst, t.sp);
+      double qa0, qa3, qb0, qb3;   // daughters 0 and 1 along t and z
+      if (massless == 3) {
+        const double eh = fx_scale(E_b, -1), ph = fx_scale(p_b, -1);
+        qa0 = fma(ph, t.ct, eh);
+        qb0 = fma(-ph, t.ct, eh);
+        qa3 = fma(eh, t.ct, ph);
+        qb3 = fma(-eh, t.ct, ph);
+      } else {
+        const double bg = fx_mul(k, p_b, rm), ga = fx_mul(k, E_b, rm), qz = fx_mul(k, pc, t.ct);
+        const double z0 = fx_mul(k, bg, qz), z3 = fx_mul(k, ga, qz);
+        qa0 = fma(ga, ce0, z0);
+        qb0 = fma(ga, ce1, -z0);
+        qa3 = fma(bg, ce0, z3);
+        qb3 = fma(bg, ce1, -z3);
       }
-    } else if (V.self_root && !lab) {
-      // parent frame is the identity, and the root's boost too: L0 * L1 is the rotation
-      L[0] = 1.0;  L[1] = 0.0;       L[2] = 0.0;  L[3] = 0.0;
-      L[4] = 0.0;  L[5] = ct * cphi; L[6] = e12;  L[7] = e13;
-      L[8] = 0.0;  L[9] = ct * sphi; L[10] = e22; L[11] = e23;
-      L[12] = 0.0; L[13] = -st;      L[14] = 0.0; L[15] = ct;
-    } else if (PER_EVENT && V.self_root) {
-      // (per-event beams, where nearly every event has a lab boost; the uniform-beam kernels
-      // keep the general product, which leaves their registers to the common case)
-      // the parent frame is the lab boost B_z(lab_bg): rows 1 and 2 are unit rows, and the
-      // root's bg is 0 and its gamma 1
-      double e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-      const double g0 = L[0], b0 = L[3], b3 = L[12], g3 = L[15];
-      L[0] = g0;     L[1] = b0 * e31;    L[2] = 0.0;  L[3] = b0 * e33;
-      L[4] = 0.0;    L[5] = e11;         L[6] = e12;  L[7] = e13;
-      L[8] = 0.0;    L[9] = e21;         L[10] = e22; L[11] = e23;
-      L[12] = b3;    L[13] = g3 * e31;   L[14] = 0.0; L[15] = g3 * e33;
-    } else if (V.parent_root && !lab) {
-      // the parent frame is the root's rotation (its bg is 0 and its gamma 1): row 0 is
-      // (1, 0, 0, 0) and L[4], L[8], L[12], L[14] are 0, so half the products drop out
-      double e01 = 0.0, e11 = 0.0, e21 = 0.0, e31 = 0.0;
-      if (!V.both_leaves) col12(e01, e11, e21, e31);
-      L[0] = ga;  L[1] = e01; L[2] = 0.0;  L[3] = e03;
+      double qa[4], qb[4];
+      if (kind == PHS_KIND_LEAVES_FIRST) {
+        // the parent's frame is the root's rotation: (1,0,0,0) (0,*,*,*) (0,*,*,*) (0,*,0,*)
+        qa[0] = qa0;
+        qb[0] = qb0;
 #pragma unroll
-      for (int r = 1; r < 4; r++) {
-        const double l1 = L[4 * r + 1], l2 = r < 3 ? L[4 * r + 2] : 0.0, l3 = L[4 * r + 3];
-        L[4 * r + 0] = l3 * bg;
-        L[4 * r + 3] = r < 3 ? l1 * e13 + l2 * e23 + l3 * e33 : l1 * e13 + l3 * e33;
-        if (!V.both_leaves) {
-          L[4 * r + 1] = r < 3 ? l1 * e11 + l2 * e21 + l3 * e31 : l1 * e11 + l3 * e31;
-          L[4 * r + 2] = r < 3 ? l1 * e12 + l2 * e22 : l1 * e12;
-        } else {
-          L[4 * r + 1] = 0.0;
-          L[4 * r + 2] = 0.0;
+        for (int r = 1; r < 4; r++) {
+          const double l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
+          const double w = r < 3 ? fma(l2, qy, fx_mul(k, l1, qx)) : fx_mul(k, l1, qx);
+          qa[r] = fma(l3, qa3, w);
+          qb[r] = fma(l3, qb3, -w);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
+          const double w = fma(l2, qy, fx_mul(k, l1, qx));
+          qa[r] = fma(l0, qa0, fma(l3, qa3, w));
+          qb[r] = fma(l0, qb0, fma(l3, qb3, -w));
         }
       }
-    } else if (PER_EVENT && V.parent_root) {
-      // the root's frame with the lab boost: entries (0,2), (1,0), (2,0), (3,2) are 0
-      double e01 = 0.0, e11 = 0.0, e21 = 0.0, e31 = 0.0;
-      if (!V.both_leaves) col12(e01, e11, e21, e31);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        const bool edge = r == 0 || r == 3;   // l2 = 0; otherwise l0 = 0
-        L[4 * r + 0] = edge ? l0 * ga + l3 * bg : l3 * bg;
-        L[4 * r + 3] = edge ? l0 * e03 + l1 * e13 + l3 * e33 : l1 * e13 + l2 * e23 + l3 * e33;
-        if (!V.both_leaves) {
-          L[4 * r + 1] = edge ? l0 * e01 + l1 * e11 + l3 * e31 : l1 * e11 + l2 * e21 + l3 * e31;
-          L[4 * r + 2] = edge ? l1 * e12 : l1 * e12 + l2 * e22;
-        } else {
-          L[4 * r + 1] = 0.0;
-          L[4 * r + 2] = 0.0;
-        }
-      }
-    } else if (V.both_leaves) {
-      // both daughters are leaves: their momenta read the frame's columns 0 and 3 only
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        L[4 * r + 0] = l0 * ga + l3 * bg;
-        L[4 * r + 3] = l0 * e03 + l1 * e13 + l2 * e23 + l3 * e33;
-        L[4 * r + 1] = 0.0;
-        L[4 * r + 2] = 0.0;
-      }
+      put_momentum(out, V.child[0].out_index, ch.n_out, qa[0], qa[1], qa[2], qa[3]);
+      put_momentum(out, V.child[1].out_index, ch.n_out, qb[0], qb[1], qb[2], qb[3]);
     } else {
-      double e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const double l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        L[4 * r + 0] = l0 * ga + l3 * bg;
-        L[4 * r + 3] = l0 * e03 + l1 * e13 + l2 * e23 + l3 * e33;
-        L[4 * r + 1] = l0 * e01 + l1 * e11 + l2 * e21 + l3 * e31;
-        L[4 * r + 2] = l1 * e12 + l2 * e22;
+      // rotation + boost of the visited branch (phs_cpu.cpp:299-330)
+      if (!V.self_root) {
+        t.bg = fx_mul(k, p_b, rm);
+        t.ga = fx_mul(k, E_b, rm);
       }
-    }
-
-    // leaf momenta: L_new * (E, 0, 0, +-p) (phs_cpu.cpp:286-291); the two leaves of a
-    // leaf-only visit share the products L_new[r][3] p
-    if (V.both_leaves) {
-      double t3[4];
+      switch (kind) {
+        case PHS_KIND_ROOT:
+          // parent frame and boost are the identity: the rotation alone
+          L[0] = 1.0;  L[1] = 0.0;                       L[2] = 0.0;          L[3] = 0.0;
+          L[4] = 0.0;  L[5] = fx_mul(k, t.ct, t.cp);     L[6] = fx_neg(t.sp); L[7] = fx_mul(k, t.st, t.cp);
+          L[8] = 0.0;  L[9] = fx_mul(k, t.ct, t.sp);     L[10] = t.cp;        L[11] = fx_mul(k, t.st, t.sp);
+          L[12] = 0.0; L[13] = fx_neg(t.st);             L[14] = 0.0;         L[15] = t.ct;
+          break;
+        case PHS_KIND_ROOT_LAB:
+          // behind the lab boost B_z(lab_bg): rows 1 and 2 as above
+          L[0] = lab_ga;  L[1] = fx_mul(k, -lab_bg, t.st);  L[2] = 0.0;          L[3] = fx_mul(k, lab_bg, t.ct);
+          L[4] = 0.0;     L[5] = fx_mul(k, t.ct, t.cp);     L[6] = fx_neg(t.sp); L[7] = fx_mul(k, t.st, t.cp);
+          L[8] = 0.0;     L[9] = fx_mul(k, t.ct, t.sp);     L[10] = t.cp;        L[11] = fx_mul(k, t.st, t.sp);
+          L[12] = lab_bg; L[13] = fx_mul(k, -lab_ga, t.st); L[14] = 0.0;         L[15] = fx_mul(k, lab_ga, t.ct);
+          break;
+        case PHS_KIND_FIRST:
+          // row 0 of the root's rotation is (1, 0, 0, 0)
+          L[0] = t.ga;
+          L[1] = fx_mul(k, -t.st, t.bg);
+          L[2] = 0.0;
+          L[3] = fx_mul(k, t.ct, t.bg);
+          frame_row<true, false>(k, t, L + 4);
+          frame_row<true, false>(k, t, L + 8);
+          frame_row<true, true>(k, t, L + 12);
+          break;
+        case PHS_KIND_FIRST_LAB:
+          // the root's frame with the lab boost: entries (0,2), (1,0), (2,0), (3,2) are 0
+          frame_row<false, true>(k, t, L);
+          frame_row<true, false>(k, t, L + 4);
+          frame_row<true, false>(k, t, L + 8);
+          frame_row<false, true>(k, t, L + 12);
+          break;
+        case PHS_KIND_FRIEND:
+          friend_step((double)V.friend_sign, t, L);
+          break;
+        default:
 #pragma unroll
-      for (int r = 0; r < 4; r++) t3[r] = L[4 * r + 3] * pc;
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const PhsChild &C = V.child[j];
-        if (phs_in(C.out_index, ch.n_out, PHS_CHK_P)) {
-          const double E = j == 0 ? ce0 : ce1;
-          double q[4];
-#pragma unroll
-          for (int r = 0; r < 4; r++) q[r] = fma(L[4 * r], E, j == 0 ? t3[r] : -t3[r]);
-          double2 *o = reinterpret_cast<double2 *>(out + 4 * C.out_index);
-          o[0] = make_double2(q[0], q[1]);
-          o[1] = make_double2(q[2], q[3]);
-        }
+          for (int r = 0; r < 4; r++) frame_row<false, false>(k, t, L + 4 * r);
       }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
+      // leaf momenta: L_new * (E, 0, 0, +-p) (phs_cpu.cpp:286-291).  (A loop that is not
+      // unrolled: the compiler would issue the FP64 instructions of an absent leaf too.)
+#pragma unroll 1
+      for (int j = V.child[0].internal ? (V.child[1].internal ? 2 : 1) : 0; j < 2; j++) {
         const PhsChild &C = V.child[j];
-        if (!C.internal && phs_in(C.out_index, ch.n_out, PHS_CHK_P)) {
-          double pj = j == 0 ? pc : -pc;
-          const double E = j == 0 ? ce0 : ce1;
-          double2 *o = reinterpret_cast<double2 *>(out + 4 * C.out_index);
-          o[0] = make_double2(L[0] * E + L[3] * pj, L[4] * E + L[7] * pj);
-          o[1] = make_double2(L[8] * E + L[11] * pj, L[12] * E + L[15] * pj);
-        }
+        if (C.internal) break;
+        const double E = j == 0 ? ce0 : ce1, pj = j == 0 ? pc : fx_neg(pc);
+        double q[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) q[r] = fma(L[4 * r], E, fx_mul(k, L[4 * r + 3], pj));
+        put_momentum(out, C.out_index, ch.n_out, q[0], q[1], q[2], q[3]);
       }
     }
 
@@ -565,17 +610,15 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
       for (int i = 0; i < 16; i++) stack_store<BLOCK>(smem, sp, i, L[i]);
       stack_store<BLOCK>(smem, sp, 16, j0 ? cmsq[0] : cmsq[1]);
       stack_store<BLOCK>(smem, sp, 17, j0 ? cm[0] : cm[1]);
-      stack_store<BLOCK>(smem, sp, 18, j0 ? pc : -pc);
-      stack_store<BLOCK>(smem, sp, 19, j0 ? cmax[0] : cmax[1]);
-      stack_store<BLOCK>(smem, sp, 20, j0 ? ce0 : ce1);
+      stack_store<BLOCK>(smem, sp, 18, j0 ? pc : fx_neg(pc));
+      stack_store<BLOCK>(smem, sp, 19, j0 ? ce0 : ce1);
       sp++;
     }
     if (V.carry >= 0) {
       const bool j0 = V.carry == 0;
       msq_b = j0 ? cmsq[0] : cmsq[1];
       m_b = j0 ? cm[0] : cm[1];
-      p_b = j0 ? pc : -pc;
-      mmax_b = j0 ? cmax[0] : cmax[1];
+      p_b = j0 ? pc : fx_neg(pc);
       E_b = j0 ? ce0 : ce1;
     } else if (sp > 0) {
       sp--;
@@ -584,13 +627,13 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
       msq_b = stack_load<BLOCK>(smem, sp, 16);
       m_b = stack_load<BLOCK>(smem, sp, 17);
       p_b = stack_load<BLOCK>(smem, sp, 18);
-      mmax_b = stack_load<BLOCK>(smem, sp, 19);
-      E_b = stack_load<BLOCK>(smem, sp, 20);
+      E_b = stack_load<BLOCK>(smem, sp, 19);
     }
   }
 
   a.volume[ev] = PER_EVENT ? channel_volume(ch, sqrts) : ch.volume;
-  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? factor * (double)(1 << halved) : 0.0;
+  a.factor[ev * a.factor_stride + seg.factor_col] =
+      ok ? fx_mul(k, factor, fx_double((1023u + halved) << 20, 0u)) : 0.0;
   a.ok[ev] = ok ? 1 : 0;
   if (!ok) {
     double2 *o = reinterpret_cast<double2 *>(out);
@@ -604,78 +647,65 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const PhsSegme
 // same arithmetic, so the flag is the same bit -- without angles or boosts.  An event that
 // fails gets its outputs here (momenta 0, factor 0, ok 0, the channel volume); one that
 // passes gets them from phs_event_f64 in pass B.  Returns ok.  smem: the event's frame
-// stack (only the msq, m and m_max slots are used).
+// stack (only the msq and m slots are used).
 template <bool PER_EVENT, int BLOCK = PHS_FWD_BLOCK>
-__device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const PhsSegment &seg,
-                                           int64_t local, double *smem) {
+__device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
+                                           const PhsSegment &seg, int64_t local, double *smem) {
   if (!phs_in(seg.channel, a.n_programs, PHS_CHK_CHANNEL)) return false;
   const PhsChannel &ch = a.channels[seg.channel];
   if (!event_in_bounds(a, seg, local, ch.n_out, ch.n_visits)) return false;
   const int64_t ev = seg.ev_begin + local;
   const double *xe = a.x + seg.x_base + local * seg.x_stride;
   double sqrts = ch.sqrts;
-  if (PER_EVENT) sqrts = dmul(2.0, sqrt(dmul(a.E1[ev], a.E2[ev])));
-  const double s = dmul(sqrts, sqrts);
-  const double inv_s = PER_EVENT ? 1.0 / s : 0.0;   // per-event mapping constants
-  double msq_b = s, m_b = sqrts, mmax_b = sqrts;
+  if (PER_EVENT) {
+    const double r = fx_sqrt(fx_mul(k, a.E1[ev], a.E2[ev]), k);
+    sqrts = fx_add(k, r, r);
+  }
+  const double s = fx_mul(k, sqrts, sqrts);
+  const double inv_s = PER_EVENT ? fx_rcp(s, k) : 0.0;   // per-event mapping constants
+  double msq_b = s, m_b = sqrts;
   bool ok = true;
   int sp = 0;
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
-    double cmsq[2], cm[2], cmax[2];
+    double cmsq[2], cm[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
       if (!C.internal) {
         cmsq[j] = C.msq_leaf;
         cm[j] = C.m_leaf;
-        cmax[j] = 0.0;
       } else {
-        double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max;
-        cmax[j] = C.m_max;
-        if (PER_EVENT) child_constants(C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, cmax[j]);
-        double f;
-        map_msq(C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
-                cmsq[j], f);
-        cm[j] = fx_sqrt(cmsq[j]);
+        double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
+        if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
+        double f, aux;
+        map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
+                cmsq[j], f, aux);
+        cm[j] = fx_sqrt(cmsq[j], k);
+        ok = ok && !fx_gt(cm[j], mmax);
       }
     }
     double sl;
-    ok = kallen_ok(V.massless, msq_b, m_b, mmax_b, cmsq, cm, sl) && ok;
+    ok = kallen_ok(k, V.massless, msq_b, m_b, cmsq, cm, sl) && ok;
     if (V.push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
       const bool j0 = V.push == 0;
       stack_store<BLOCK>(smem, sp, 16, j0 ? cmsq[0] : cmsq[1]);
       stack_store<BLOCK>(smem, sp, 17, j0 ? cm[0] : cm[1]);
-      stack_store<BLOCK>(smem, sp, 19, j0 ? cmax[0] : cmax[1]);
       sp++;
     }
     if (V.carry >= 0) {
       const bool j0 = V.carry == 0;
       msq_b = j0 ? cmsq[0] : cmsq[1];
       m_b = j0 ? cm[0] : cm[1];
-      mmax_b = j0 ? cmax[0] : cmax[1];
     } else if (sp > 0) {
       sp--;
       msq_b = stack_load<BLOCK>(smem, sp, 16);
       m_b = stack_load<BLOCK>(smem, sp, 17);
-      mmax_b = stack_load<BLOCK>(smem, sp, 19);
     }
   }
   if (!ok) {
-    double volume = ch.volume;
-    if (PER_EVENT) {
-      double vol[PHS_MAX_VISITS];
-      const double c_int = 4 * PHS_TWOPI2, c_root = 4 * PHS_TWOPI5;
-      for (int i = 0; i < ch.n_vol; i++) {
-        int k1 = ch.vol_child[i][0], k2 = ch.vol_child[i][1];
-        double v1 = k1 >= 0 ? vol[k1] : 1.0, v2 = k2 >= 0 ? vol[k2] : 1.0;
-        vol[i] = ch.vol_is_root[i] ? dmul(v1, v2) / c_root
-                                   : dmul(dmul(dmul(v1, v2), sqrts), sqrts) / c_int;
-      }
-      volume = vol[ch.n_vol - 1];
-    }
-    a.volume[ev] = volume;
+    a.volume[ev] = PER_EVENT ? channel_volume(ch, sqrts) : ch.volume;
     a.factor[ev * a.factor_stride + seg.factor_col] = 0.0;
     a.ok[ev] = 0;
     double2 *o = reinterpret_cast<double2 *>(a.p + seg.p_base + local * 4 * (int64_t)ch.n_out);

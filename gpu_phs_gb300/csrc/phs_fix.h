@@ -30,6 +30,25 @@
 #define FX_FN inline
 #endif
 
+// FP64 sums and products alone, with the same bits: a b = fma(a, b, -0), a + b = fma(a, 1, b).
+// A fused multiply-add whose operands all sit in registers takes an SM's FP64 pipe 16 cycles a
+// warp; a plain product or sum, and an FMA with a constant operand, 19 (measured, at any
+// occupancy).  The two constants therefore live in registers: the caller reads them once per
+// thread from memory (fx_regs), where the compiler cannot see their values.
+struct FxRegs {
+  double nz, one;   // -0.0 and 1.0
+};
+#if defined(__CUDACC__)
+namespace {
+__constant__ double fx_reg_values[4] = {-0.0, 1.0, -0.0, 1.0};
+}
+// Per thread (not warp-uniform to the compiler, which would keep them as constant operands).
+__device__ __forceinline__ FxRegs fx_regs() {
+  const int i = (threadIdx.x & 1) * 2;
+  return {fx_reg_values[i], fx_reg_values[i + 1]};
+}
+#endif
+
 #if defined(__CUDA_ARCH__)
 FX_FN uint64_t fx_mulhi(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
 FX_FN uint32_t fx_mulhi32(uint32_t a, uint32_t b) { return __umulhi(a, b); }
@@ -47,7 +66,6 @@ FX_FN float fx_fmaf(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 FX_FN float fx_mulf(float a, float b) { return __fmul_rn(a, b); }
 FX_FN int fx_rint32(float a) { return __float2int_rn(a); }
 FX_FN uint32_t fx_trunc_u32(float a) { return __float2uint_rz(a); }
-FX_FN double fx_mul(double a, double b) { return __dmul_rn(a, b); }
 FX_FN double fx_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 #else
 FX_FN uint64_t fx_mulhi(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
@@ -66,9 +84,18 @@ FX_FN float fx_fmaf(float a, float b, float c) { return fmaf(a, b, c); }
 FX_FN float fx_mulf(float a, float b) { return a * b; }
 FX_FN int fx_rint32(float a) { return (int)lrintf(a); }
 FX_FN uint32_t fx_trunc_u32(float a) { return (uint32_t)a; }
-FX_FN double fx_mul(double a, double b) { return a * b; }
 FX_FN double fx_fma(double a, double b, double c) { return fma(a, b, c); }
 #endif
+
+FX_FN double fx_mul(const FxRegs &k, double a, double b) { return fx_fma(a, b, k.nz); }
+FX_FN double fx_add(const FxRegs &k, double a, double b) { return fx_fma(a, k.one, b); }
+FX_FN double fx_sub(const FxRegs &k, double a, double b) { return fx_fma(-b, k.one, a); }
+FX_FN double fx_neg(double a) { return fx_double(fx_hi(a) ^ 0x80000000u, fx_lo(a)); }
+// a 2^e for a normal result (zeros, subnormals, infinities and NaN come back unchanged).
+FX_FN double fx_scale(double a, int e) {
+  const uint32_t h = fx_hi(a);
+  return (h & 0x7ff00000u) - 0x00300000u < 0x7f900000u ? fx_double(h + (uint32_t)(e << 20), fx_lo(a)) : a;
+}
 
 // ------------------------------------------------------------ square root and reciprocal
 // y0 + c (y0 in [0.5, 1), |c| < 2^-22) as a double: y0's bits widened, c added in units of
@@ -99,7 +126,7 @@ FX_FN uint64_t fx_rsqrt_seed(double x) {
 // sqrt(x): the correctly rounded value but for arguments whose root lies within 2^-30 ulp
 // of a rounding boundary.  Zeros, subnormals and the smallest normals (whose residual would
 // be subnormal), infinities and NaN go to the library's; negatives give NaN.
-FX_FN double fx_sqrt(double x) {
+FX_FN double fx_sqrt(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   const uint32_t hi = fx_hi(x);
   if (hi - 0x08000000u >= 0x77f00000u) {
     if (hi > 0x80000000u) return fx_double(0x7fffffffu, 0xffffffffu);   // negative
@@ -107,12 +134,12 @@ FX_FN double fx_sqrt(double x) {
   }
   const uint64_t rb = fx_rsqrt_seed(x);
   const double r = fx_from_bits(rb), h = fx_from_bits(rb - (1ull << 52));
-  const double s = fx_mul(x, r);
+  const double s = fx_mul(k, x, r);
   return fx_fma(fx_fma(-s, s, x), h, s);
 }
 
 // 1/x within an ulp (almost always correctly rounded) for x > 0.
-FX_FN double fx_rcp(double x) {
+FX_FN double fx_rcp(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   const uint32_t hi = fx_hi(x), lo = fx_lo(x);
   if (hi - 0x04000000u >= 0x78000000u) return 1.0 / x;
   const float mh = fx_float((127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
@@ -123,7 +150,15 @@ FX_FN double fx_rcp(double x) {
   e = fx_fmaf(-ml, y0, e);
   const float c = fx_mulf(y0, fx_fmaf(e, e, e));
   const double r = fx_from_bits(fx_seed(y0, c) - ((uint64_t)(int64_t)((int)(hi >> 20) - 1023) << 52));
-  return fx_fma(fx_fma(-x, r, 1.0), r, r);
+  return fx_fma(fx_fma(-x, r, k.one), r, r);
+}
+
+// a / b for b > 0: the quotient from the reciprocal, corrected once with its residual
+// (correctly rounded but for quotients within 2^-50 ulp of a rounding boundary, and where the
+// residual would be subnormal).
+FX_FN double fx_div(double a, double b, const FxRegs &k) {
+  const double r = fx_rcp(b, k), q = fx_mul(k, a, r);
+  return fx_fma(fx_fma(-q, b, a), r, q);
 }
 
 // a > b; as integers where neither is negative or NaN.
@@ -148,7 +183,7 @@ FX_FN double fx_from_q62(int64_t v) {
   const uint64_t a = v < 0 ? (uint64_t)-v : (uint64_t)v;
   if (a == 0) return 0.0;
   const double d = fx_pack(a, -62);
-  return v < 0 ? -d : d;
+  return v < 0 ? fx_neg(d) : d;
 }
 
 // x 2^64 for 0 <= x < 1, truncated to an integer (exact for x >= 2^-11).
@@ -240,7 +275,7 @@ FX_FN double fx_tan(double z) {
   const uint64_t cs = (1ull << 63) - (k >> 1);                    // cos u, Q63
   const uint64_t q = fx_div_q62(big ? cs : sn, big ? sn : cs);
   const double t = fx_pack(q, (big ? -e : e) - 62);
-  return (int32_t)zh < 0 ? -t : t;
+  return (int32_t)zh < 0 ? fx_neg(t) : t;
 }
 
 // ---------------------------------------------------------------------- exp

@@ -27,6 +27,7 @@ template <bool PER_EVENT, bool COMPACT, int MIN_BLOCKS, int BLOCK = PHS_FWD_BLOC
 __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     phs_forward_f64_kernel(const __grid_constant__ PhsLaunch a) {
   extern __shared__ double smem[];
+  const FxRegs k = fx_regs();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -35,9 +36,9 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
                  (threadIdx.x >> 5) * 64;
     compacting_loop<PHS_CHUNK_TILES>(
         a, q,
-        [&](const PhsSegment &sg, int64_t loc) { return phs_ok_f64<PER_EVENT, BLOCK>(a, sg, loc, smem); },
+        [&](const PhsSegment &sg, int64_t loc) { return phs_ok_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem); },
         [&](int, const PhsSegment &sg, int64_t loc) {
-          phs_event_f64<PER_EVENT, BLOCK>(a, sg, loc, smem);
+          phs_event_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem);
         });
   } else {
     for (int64_t tile = warp0; tile < a.n_tiles; tile += n_warps) {
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
       const PhsSegment seg = segs[lo];
       const int64_t local = (tile - seg.tile_begin) * 32 + lane;
       if (local >= seg.ev_count) continue;
-      phs_event_f64<PER_EVENT, BLOCK>(a, seg, local, smem);
+      phs_event_f64<PER_EVENT, BLOCK>(a, k, seg, local, smem);
     }
   }
 }
@@ -67,6 +68,7 @@ template <bool PER_EVENT>
 __global__ void __launch_bounds__(PHS_FWD_BLOCK, 4)
     phs_forward_exact_kernel(const __grid_constant__ PhsLaunch a) {
   extern __shared__ double smem[];
+  const FxRegs k = fx_regs();
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
   const int64_t n_claims = a.exact_tile[a.n_segments];
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, 4)
     if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
         !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
       continue;
-    phs_event_f64<PER_EVENT>(a, seg, a.exact_queue[seg.tile_begin * 32 + idx], smem);
+    phs_event_f64<PER_EVENT>(a, k, seg, a.exact_queue[seg.tile_begin * 32 + idx], smem);
   }
 }
 
@@ -100,6 +102,7 @@ template <int MIN_BLOCKS, int BLOCK = PHS_FWD_BLOCK>
 __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     phs_f64_walk_kernel(const __grid_constant__ PhsLaunch a) {
   extern __shared__ double smem[];
+  const FxRegs k = fx_regs();
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
   const int64_t n_claims = a.pass_tile[a.n_segments];
@@ -120,7 +123,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
         !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
       continue;
-    phs_event_f64<false, BLOCK>(a, seg, a.pass_queue[seg.tile_begin * 32 + idx], smem);
+    phs_event_f64<false, BLOCK>(a, k, seg, a.pass_queue[seg.tile_begin * 32 + idx], smem);
   }
 }
 

@@ -63,7 +63,7 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C) {
 __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChild &C64,
                                               double sqrts, double m_tot, double inv_s) {
   double a0, a1, a2, mn, mx, mmax;
-  child_constants(C64, sqrts, m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
+  child_constants(fx_regs(), C64, sqrts, m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
   // to pairs with integer operations: the FP64 pipe is the per-event path's scarce one
   ChildVar r;
   r.a2 = ff_from_double_int(a2);

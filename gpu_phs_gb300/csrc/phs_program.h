@@ -36,6 +36,18 @@ enum {
 // cos(theta) mapping classes (phs_cpu.cpp:112-146).
 enum { PHS_CT_UNIFORM = 0, PHS_CT_COLLINEAR = 1 };
 
+// The forms of a visit's frame step without a lab boost (the FP64 walk picks the lab forms).
+enum {
+  PHS_KIND_ROOT = 0,          // the root: its frame is the decay rotation
+  PHS_KIND_FIRST = 1,         // a daughter of the root with an internal daughter of its own
+  PHS_KIND_INNER = 2,         // any other branch with an internal daughter
+  PHS_KIND_LEAVES = 3,        // two outgoing daughters: their momenta, no frame
+  PHS_KIND_LEAVES_FIRST = 4,  // the same for a daughter of the root
+  PHS_KIND_FRIEND = 5,        // decay angles measured from a beam
+  PHS_KIND_ROOT_LAB = 6,      // ROOT and FIRST behind a lab boost
+  PHS_KIND_FIRST_LAB = 7
+};
+
 // One daughter of a visited branch.
 struct PhsChild {
   int32_t internal;   // 0: outgoing particle (leaf); 1: internal branch
@@ -75,6 +87,8 @@ struct PhsVisit {
                         // boost its parent frame is the root's rotation, rows
                         // (1,0,0,0), (0,*,*,*), (0,*,*,*), (0,*,0,*)
   int8_t massless;      // bit j: daughter j is a massless outgoing particle
+  int32_t kind;         // PHS_KIND_*: the form of the visit's frame step (FP64 walk)
+  int32_t pad0;
 };
 
 struct PhsChannel {
@@ -84,6 +98,9 @@ struct PhsChannel {
   int32_t n_vol;      // entries of the volume program
   double m_tot;       // sum of all outgoing masses
   double volume;      // channel volume at the handle's sqrt(s) (phs_cpu.cpp:194-213)
+  double f0;          // product of the msq mappings' constant factors at the handle's sqrt(s)
+                      // (all mappings but the STEP ones)
+  double inv_sqrts;   // 1 / sqrts
   double sqrts;       // uniform beams: sqrt(s) = 2 sqrt(E1 E2) the constants were made for
   double lab_bg;      // uniform beams: longitudinal lab boost (E1-E2)/(2 sqrt(E1 E2))
   double lab_gamma;   //   and its gamma (phs.cu:1286-1301)

@@ -104,3 +104,55 @@ def test_fixed_point_functions():
     assert float(sc) <= 2.0 ** -59
     assert float(cv) <= 0.501
     assert int(bad) == 0
+
+
+REG_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <cstring>
+#include <random>
+#include "phs_fix.h"
+static bool same(double a, double b) { return (a != a && b != b) || std::memcmp(&a, &b, 8) == 0; }
+int main() {
+  const FxRegs k{-0.0, 1.0};
+  std::mt19937_64 g(2);
+  std::uniform_real_distribution<double> U(0, 1);
+  const double edge[] = {0.0, -0.0, 1.0, -1.0, 5e-324, -5e-324, 2.2250738585072014e-308, 1.7976931348623157e308,
+                         -1.7976931348623157e308, INFINITY, -INFINITY, NAN, 0.1, -3.0};
+  long form = 0, div = 0, scale = 0;
+  auto forms = [&](double a, double b) {
+    form += !same(fx_mul(k, a, b), a * b);
+    form += !same(fx_add(k, a, b), a + b);
+    form += !same(fx_sub(k, a, b), a - b);
+  };
+  for (double a : edge) {
+    form += a == a && !same(fx_neg(a), -a);
+    for (double b : edge) forms(a, b);
+  }
+  const int n = 400000;
+  for (int i = 0; i < n; i++) {
+    const double a = std::ldexp(2 * U(g) - 1, (int)(U(g) * 400) - 200);
+    const double b = std::ldexp(1 + U(g), (int)(U(g) * 400) - 200);
+    forms(a, b);
+    forms(b, a);
+    div += fx_div(a, b, k) != a / b;
+    for (int e : {-2, -1, 1, 2}) scale += fx_scale(a, e) != std::ldexp(a, e);
+  }
+  for (double a : {0.0, -0.0, (double)INFINITY, 5e-324}) scale += !same(fx_scale(a, 1), a);
+  printf("%ld %ld %ld %d\n", form, div, scale, n);
+}
+"""
+
+
+def test_register_constant_forms_and_division(tmp_path):
+    """Products, sums and differences through an FMA with -0 or 1 are the plain operations' bits
+    (signed zeros, subnormals, overflow and non-finite values included), scaling by a power of
+    two is exact, and the corrected quotient is the division's."""
+    src, exe = tmp_path / "r.cpp", tmp_path / "r"
+    src.write_text(REG_DRIVER)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True)
+    form, div, scale, n = (int(v) for v in subprocess.run([str(exe)], capture_output=True, text=True,
+                                                          check=True).stdout.split())
+    assert form == 0 and scale == 0
+    assert div <= n // 1000
