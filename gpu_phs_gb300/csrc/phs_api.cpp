@@ -921,7 +921,7 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
                           const double *E1, const double *E2, const double *p, const uint8_t *ok,
                           const double *x_own, const double *factor_own, double *all_factors,
                           double *x_out, cudaStream_t st, int order_lo = 0, int order_hi = -1,
-                          bool write_fixed = true, int64_t x_ch_stride = 0);
+                          int64_t x_ch_stride = 0);
 
 extern "C" int phs_inverse_device(phs_process_t h, int64_t n_events, const int64_t *counts,
                                   const double *E1, const double *E2, const double *p,
@@ -970,7 +970,7 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
                           const double *E1, const double *E2, const double *p, const uint8_t *ok,
                           const double *x_own, const double *factor_own, double *all_factors,
                           double *x_out, cudaStream_t st, int order_lo, int order_hi,
-                          bool write_fixed, int64_t x_ch_stride) {
+                          int64_t x_ch_stride) {
   const int nch = h->p.n_channels;
   PhsInvLaunch a;
   memset(&a, 0, sizeof a);
@@ -993,20 +993,28 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
   a.max_visits = h->max_visits;
   a.group_order = h->d_inv_groups.as<int32_t>();
   a.group_begin = a.group_order + nch;
-  const bool cache = phs_inverse_fits_cache(a.n_out, a.stack_depth, a.max_visits);
+  // mapping results are kept only where some shape has a second channel to reuse them
+  const bool cache = h->n_inv_groups < nch && phs_inverse_fits_cache(a.n_out, a.stack_depth, a.max_visits);
   a.group_reuse = cache ? reinterpret_cast<const uint64_t *>(
                               static_cast<const char *>(h->d_inv_groups.ptr) + h->inv_reuse_offset)
                         : nullptr;
   a.n_groups = h->n_inv_groups;
   a.order_lo = order_lo;
   a.order_hi = order_hi < 0 ? nch : order_hi;
-  a.write_fixed = write_fixed ? 1 : 0;
   a.lab = h->prog.empty() ? 0 : h->prog[0].lab;
-  const int64_t tiles = (n_events + PHS_INV_BLOCK - 1) / PHS_INV_BLOCK;
-  const int64_t cap = (int64_t)sm_count(h->device) *
-                      phs_inverse_blocks_per_sm(a.n_out, a.stack_depth, a.max_visits,
-                                                E1 != nullptr, cache, !a.lab);
-  CUDA_TRY(phs_launch_inverse(a, (int)std::max<int64_t>(1, std::min(tiles, cap)), st));
+  const std::vector<int32_t> &gb = h->inv_group_begin;
+  a.group_lo = (int32_t)(std::upper_bound(gb.begin(), gb.end(), a.order_lo) - gb.begin()) - 1;
+  a.group_hi = (int32_t)(std::lower_bound(gb.begin(), gb.end(), a.order_hi) - gb.begin());
+  if (a.order_lo >= a.order_hi) return PHS_OK;
+  // events per block: long tiles fill the warps with ok events, short ones give blocks to
+  // every SM; halved until the grid is four times what is resident (measured for 2e5 events x
+  // 16 channels: 2.79 ms, 2.85 at eight times)
+  const int64_t resident = (int64_t)sm_count(h->device) *
+                           phs_inverse_blocks_per_sm(a.n_out, a.stack_depth, a.max_visits,
+                                                     E1 != nullptr, cache, !a.lab);
+  a.tile = PHS_INV_TILE;
+  while (a.tile > 64 && (n_events + a.tile - 1) / a.tile * (a.group_hi - a.group_lo) < 4 * resident) a.tile /= 2;
+  CUDA_TRY(phs_launch_inverse(a, st));
   return PHS_OK;
 }
 
@@ -1945,8 +1953,7 @@ extern "C" void c_whizard_gen_phs_from_x_gpu(double *E1_in, double *E2_in,
         if (e == cudaSuccess) e = cudaStreamWaitEvent(cs[1], W.done[0], 0);
         if (e != cudaSuccess) rc = fail(PHS_ERR_CUDA, "%s", cudaGetErrorString(e));
         // do_inverse_mapping is forced on (whizard_gpu_phs.cpp:118): every channel's factor
-        // and x; the generating channel keeps its own x and factor (phs.cu:1580-1585), written
-        // with the other no-arithmetic outputs by the first launch (over every event)
+        // and x; the generating channel keeps its own x and factor (phs.cu:1580-1585)
         for (size_t u = 0; u < units.size() && rc == PHS_OK; u++) {
           const Unit &U = units[u];
           const int64_t e0 = U.e0;
@@ -1954,7 +1961,7 @@ extern "C" void c_whizard_gen_phs_from_x_gpu(double *E1_in, double *E2_in,
                               uniform ? nullptr : dE1 + e0, uniform ? nullptr : dE2 + e0,
                               dp + e0 * 4 * n_out, dok + e0, dx + e0 * n_x, df + e0,
                               W.dfa.as<double>() + e0 * nch, dxo + e0 * n_x, cs[u & 1], U.lo, U.hi,
-                              u == 0, n);
+                              n);
           if (rc == PHS_OK && (e = cudaEventRecord(W.done[u + 1], cs[u & 1])) != cudaSuccess)
             rc = fail(PHS_ERR_CUDA, "%s", cudaGetErrorString(e));
         }
@@ -1963,7 +1970,7 @@ extern "C" void c_whizard_gen_phs_from_x_gpu(double *E1_in, double *E2_in,
         rc = fail(PHS_ERR_CUDA, "copy back: %s", cudaGetErrorString(e));
       const int32_t *order = W.proc->inv_order.data();
       // the copy stream waits for the launches in order: launch u's rows are copied after
-      // every launch up to u (the first one's fixed outputs included) is done
+      // every launch up to u is done
       for (size_t u = 0; u < units.size() && rc == PHS_OK && e == cudaSuccess; u++) {
         const Unit &U = units[u];
         e = cudaStreamWaitEvent(ms, W.done[u + 1], 0);

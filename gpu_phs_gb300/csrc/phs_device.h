@@ -146,10 +146,10 @@ void phs_adjoint_sizes(int max_visits, int max_pops, int stack_depth, bool frien
 #define PHS_ADJ_BLOCK_HOST 64
 
 // Inverse map (phs_inverse.cu): for every event and every channel, the x row and factor
-// that channel assigns to the event's momenta.  Threads per block (and events per tile and
-// per walk): with ~84 doubles of shared memory per thread, 64-thread blocks keep 5 blocks
-// (10 warps) resident per SM where 128-thread blocks keep 2 (8 warps).
-#define PHS_INV_BLOCK 64
+// that channel assigns to the event's momenta.  Threads per block: with ~84 doubles of shared
+// memory per thread, 64-thread blocks keep 5 blocks (10 warps) resident per SM where
+// 128-thread blocks keep 2 (8 warps).
+#define PHS_INV_BLOCK 128
 struct PhsInvLaunch {
   const PhsChannel *channels;  // device, per channel (uniform-beam constants)
   const int64_t *ch_begin;     // device, [n_channels]: first event of each generating channel
@@ -169,16 +169,17 @@ struct PhsInvLaunch {
                                 // null: no reuse (and no shared memory for it)
   int32_t n_groups;
   // this launch inverts the channels at group_order positions [order_lo, order_hi) (all:
-  // 0, n_channels); write_fixed: it also writes every channel's outputs that need no
-  // arithmetic (own rows, x padding, ok = false events), which one launch of a split set does
-  int32_t order_lo, order_hi, write_fixed;
+  // 0, n_channels), which lie in the groups [group_lo, group_hi)
+  int32_t order_lo, order_hi, group_lo, group_hi;
+  int32_t tile;                // events per block (a multiple of 32, at most PHS_INV_TILE)
   int64_t n_events;
   int64_t x_ch_stride;         // rows per channel in x_out (n_events, or more for a launch
                                // over a range of the events of a longer array)
   int32_t n_channels, n_out, n_x, stack_depth, max_visits;
   int32_t lab;                 // uniform beams: 1 when E1 != E2 (the programs' lab boost)
 };
-cudaError_t phs_launch_inverse(const PhsInvLaunch &a, int n_blocks, cudaStream_t stream);
+cudaError_t phs_launch_inverse(const PhsInvLaunch &a, cudaStream_t stream);
+#define PHS_INV_TILE 1024
 // cache: the per-visit mapping results that channels of a shape reuse (a.group_reuse set);
 // phs_inverse_fits_cache tells whether the block's shared memory holds them.  lab_rows:
 // uniform beams without a lab boost, where the kernel reads the outgoing momenta from p

@@ -46,6 +46,30 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
+// The STEP maps: calls, as they are rare and their library functions and divisions would be
+// much of the kernels' code.
+struct StepMap {
+  double msq, f, aux;
+};
+__device__ __noinline__ StepMap map_msq_step(int t, double x, double s, double msq_min,
+                                             double msq_max, double a0, double a1, double a2) {
+  StepMap r;
+  double z;
+  if (t == PHS_MAP_STEP_H) {
+    const double am = dsub(a0, x);
+    z = dadd(dsub(a1 / am, a1 / a0), dmul(a2, x));
+    r.f = (a1 / (am * am) + a2) * (msq_max - msq_min) / s;
+    r.aux = 0.0;
+  } else {
+    const double tmp = dmul(exp(dmul(-x, a0) / a2), dadd(1.0, a1));
+    z = dmul(-a2, log(dsub(tmp, a1)));
+    r.f = a0 / (1.0 - a1 / tmp) * (msq_max - msq_min) / s;
+    r.aux = tmp;
+  }
+  r.msq = dadd(dmul(z, msq_max), dmul(dsub(1.0, z), msq_min));
+  return r;
+}
+
 // msq from x (phs_cpu.cpp:12-61), same expression order, no contraction.  f receives the
 // mapping's factor without its constant part (a2; the range over s of the uniform map: the
 // caller's, PhsChannel::f0 for uniform beams).  aux receives the mapping's transcendental
@@ -94,19 +118,12 @@ __device__ __forceinline__ void map_msq(const FxRegs &k, int t, double x, double
       aux = msq1;
       break;
     }
-    case PHS_MAP_STEP_H: {
-      double am = dsub(a0, x);
-      double z = dadd(dsub(a1 / am, a1 / a0), dmul(a2, x));
-      msq = dadd(dmul(z, msq_max), dmul(dsub(1.0, z), msq_min));
-      f = (a1 / (am * am) + a2) * (msq_max - msq_min) / s;
-      break;
-    }
+    case PHS_MAP_STEP_H:
     case PHS_MAP_STEP_E: {
-      double tmp = dmul(exp(dmul(-x, a0) / a2), dadd(1.0, a1));
-      double z = dmul(-a2, log(dsub(tmp, a1)));
-      msq = dadd(dmul(z, msq_max), dmul(dsub(1.0, z), msq_min));
-      f = a0 / (1.0 - a1 / tmp) * (msq_max - msq_min) / s;
-      aux = tmp;
+      const StepMap r = map_msq_step(t, x, s, msq_min, msq_max, a0, a1, a2);
+      msq = r.msq;
+      f = r.f;
+      aux = r.aux;
       break;
     }
     default:
@@ -215,7 +232,7 @@ __device__ void child_constants(const FxRegs &k, const PhsChild &C, double sqrts
         const double at = fma(fx_mul(k, r, r2), fma(r2, 0.2, -1.0 / 3.0), r);
         a1 = (PHS_PIO2_HI - at) + PHS_PIO2_LO;
       } else {
-        a1 = atan(u);
+        a1 = fx_lib_atan2(u, 1.0);
       }
       a2 = fx_mul(k, fx_mul(k, fx_sub(k, a1, a0), fx_mul(k, m, w)), inv_s);
       break;
@@ -255,6 +272,9 @@ __device__ void child_constants(const FxRegs &k, const PhsChild &C, double sqrts
   }
 }
 
+__device__ __noinline__ double lib_sinpi(double x) { return sinpi(x); }
+__device__ __noinline__ double lib_cospi(double x) { return cospi(x); }
+
 // sin and cos of 2 pi x for a phi mapping's x: in fixed point for 0 <= x < 1 (absolute
 // error 2^-60), else the library's.
 __device__ __forceinline__ void sincos2pi(double x, double &s, double &c) {
@@ -264,7 +284,8 @@ __device__ __forceinline__ void sincos2pi(double x, double &s, double &c) {
     s = fx_from_q62(si);
     c = fx_from_q62(ci);
   } else {
-    sincospi(2.0 * x, &s, &c);
+    s = lib_sinpi(2.0 * x);
+    c = lib_cospi(2.0 * x);
   }
 }
 
@@ -408,8 +429,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
     const double E1 = a.E1[ev], E2 = a.E2[ev];
     const double r = fx_sqrt(fx_mul(k, E1, E2), k);
     sqrts = fx_add(k, r, r);
-    lab_bg = fx_hi(sqrts) - 0x04000000u < 0x78000000u ? fx_div(fx_sub(k, E1, E2), sqrts, k)
-                                                      : dsub(E1, E2) / sqrts;
+    lab_bg = fx_div(fx_sub(k, E1, E2), sqrts, k);
     lab_ga = fx_sqrt(fma(lab_bg, lab_bg, k.one), k);
   }
   const double s = fx_mul(k, sqrts, sqrts);
@@ -427,23 +447,29 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
-    double cmsq[2], cm[2];
-#pragma unroll
+    double cmsq[2] = {V.child[0].msq_leaf, V.child[1].msq_leaf}, cm[2] = {V.child[0].m_leaf, V.child[1].m_leaf};
+    // (not unrolled: the mapping code of one daughter serves both)
+#pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
-      if (!C.internal) {
-        cmsq[j] = C.msq_leaf;
-        cm[j] = C.m_leaf;
-      } else {
+      if (C.internal) {
+        double mq, mj;
         double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
         if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
         double f, aux;
         map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
-                cmsq[j], f, aux);
+                mq, f, aux);
         if (PER_EVENT && C.map_id != PHS_MAP_STEP_E && C.map_id != PHS_MAP_STEP_H) factor = fx_mul(k, factor, a2);
         if (C.map_id != PHS_MAP_NO) factor = fx_mul(k, factor, f);
-        cm[j] = fx_sqrt(cmsq[j], k);
-        ok = ok && !fx_gt(cm[j], mmax);   // NaN fails at the daughter's own visit
+        mj = fx_sqrt(mq, k);
+        ok = ok && !fx_gt(mj, mmax);   // NaN fails at the daughter's own visit
+        if (j == 0) {
+          cmsq[0] = mq;
+          cm[0] = mj;
+        } else {
+          cmsq[1] = mq;
+          cm[1] = mj;
+        }
       }
     }
     // Kallen function and kinematic test at the visited branch (phs_cpu.cpp:218-233)
@@ -669,21 +695,27 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
-    double cmsq[2], cm[2];
-#pragma unroll
+    double cmsq[2] = {V.child[0].msq_leaf, V.child[1].msq_leaf}, cm[2] = {V.child[0].m_leaf, V.child[1].m_leaf};
+    // (not unrolled: the mapping code of one daughter serves both)
+#pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
-      if (!C.internal) {
-        cmsq[j] = C.msq_leaf;
-        cm[j] = C.m_leaf;
-      } else {
+      if (C.internal) {
+        double mq, mj;
         double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
         if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
         double f, aux;
         map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
-                cmsq[j], f, aux);
-        cm[j] = fx_sqrt(cmsq[j], k);
-        ok = ok && !fx_gt(cm[j], mmax);
+                mq, f, aux);
+        mj = fx_sqrt(mq, k);
+        ok = ok && !fx_gt(mj, mmax);
+        if (j == 0) {
+          cmsq[0] = mq;
+          cm[0] = mj;
+        } else {
+          cmsq[1] = mq;
+          cm[1] = mj;
+        }
       }
     }
     double sl;

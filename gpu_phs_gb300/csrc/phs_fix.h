@@ -97,6 +97,22 @@ FX_FN double fx_scale(double a, int e) {
   return (h & 0x7ff00000u) - 0x00300000u < 0x7f900000u ? fx_double(h + (uint32_t)(e << 20), fx_lo(a)) : a;
 }
 
+// The library's functions for the arguments that the forms here leave out.  On the device they
+// are calls: inlined at every use they would be most of the kernels' code, and the walks'
+// instruction fetches already limit them.
+#if defined(__CUDACC__)
+#define FX_RARE static __host__ __device__ __noinline__
+#else
+#define FX_RARE inline
+#endif
+FX_RARE double fx_lib_sqrt(double x) { return sqrt(x); }
+FX_RARE double fx_lib_div(double a, double b) { return a / b; }
+FX_RARE double fx_lib_exp(double x) { return exp(x); }
+FX_RARE double fx_lib_log(double x) { return log(x); }
+FX_RARE double fx_lib_atan2(double y, double x) { return atan2(y, x); }
+FX_RARE double fx_lib_sin(double x) { return sin(x); }
+FX_RARE double fx_lib_cos(double x) { return cos(x); }
+
 // ------------------------------------------------------------ square root and reciprocal
 // y0 + c (y0 in [0.5, 1), |c| < 2^-22) as a double: y0's bits widened, c added in units of
 // y0's last place.
@@ -130,7 +146,7 @@ FX_FN double fx_sqrt(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   const uint32_t hi = fx_hi(x);
   if (hi - 0x08000000u >= 0x77f00000u) {
     if (hi > 0x80000000u) return fx_double(0x7fffffffu, 0xffffffffu);   // negative
-    return sqrt(x);
+    return fx_lib_sqrt(x);
   }
   const uint64_t rb = fx_rsqrt_seed(x);
   const double r = fx_from_bits(rb), h = fx_from_bits(rb - (1ull << 52));
@@ -141,7 +157,7 @@ FX_FN double fx_sqrt(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
 // 1/x within an ulp (almost always correctly rounded) for x > 0.
 FX_FN double fx_rcp(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   const uint32_t hi = fx_hi(x), lo = fx_lo(x);
-  if (hi - 0x04000000u >= 0x78000000u) return 1.0 / x;
+  if (hi - 0x04000000u >= 0x78000000u) return fx_lib_div(1.0, x);
   const float mh = fx_float((127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
   const float ml = fx_mulf((float)(lo & 0x1fffffffu), 0x1p-52f);
   float y0 = fx_rcp_est(mh);
@@ -153,12 +169,18 @@ FX_FN double fx_rcp(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   return fx_fma(fx_fma(-x, r, k.one), r, r);
 }
 
-// a / b for b > 0: the quotient from the reciprocal, corrected once with its residual
-// (correctly rounded but for quotients within 2^-50 ulp of a rounding boundary, and where the
-// residual would be subnormal).
-FX_FN double fx_div(double a, double b, const FxRegs &k) {
-  const double r = fx_rcp(b, k), q = fx_mul(k, a, r);
+// a / b given r = fx_rcp(b): the product corrected once with its residual, the correctly rounded
+// quotient (Markstein) where r is 1/b correctly rounded, as it is but for about one b in 2^36,
+// and the residual is not subnormal.
+FX_FN double fx_quot(double a, double b, double r, const FxRegs &k) {
+  const double q = fx_mul(k, a, r);
   return fx_fma(fx_fma(-q, b, a), r, q);
+}
+// b such that fx_quot serves a / b: normal, positive, and neither huge nor tiny.
+FX_FN bool fx_quot_serves(double b) { return fx_hi(b) - 0x04000000u < 0x78000000u; }
+FX_FN double fx_div(double a, double b, const FxRegs &k) {
+  if (!fx_quot_serves(b)) return fx_lib_div(a, b);
+  return fx_quot(a, b, fx_rcp(b, k), k);
 }
 
 // a > b; as integers where neither is negative or NaN.
@@ -238,15 +260,19 @@ FX_FN void fx_sincos2pi_q62(uint64_t X, int64_t &s, int64_t &c) {
   c = ((q + 1u) & 2u) ? -b : b;
 }
 
-// n / d for n, d in [2^62, 2^64): the quotient in Q62, within 2^-60 of it.
-FX_FN uint64_t fx_div_q62(uint64_t n, uint64_t d) {
+// 2^126 / d for d in [2^62, 2^64), to 2^-43.
+FX_FN uint64_t fx_recip_q62(uint64_t d) {
   const float y0 = fx_rcp_est((float)(uint32_t)(d >> 32));        // in [2^-32, 2^-30]
   const uint32_t Y0 = fx_trunc_u32(fx_mulf(y0, 0x1.fffffcp+61f)); // 2^94 / d to 2^-22, below it
   // 1 - d Y0 2^-94, in units of 2^-62
   const uint32_t dh = (uint32_t)(d >> 32), dl = (uint32_t)d;
   const int64_t e = (int64_t)((1ull << 62) - ((uint64_t)dh * Y0 + (((uint64_t)dl * Y0) >> 32)));
-  // 2^126 / d to 2^-43
-  const uint64_t Y = ((uint64_t)Y0 << 32) + (uint64_t)(((int64_t)(int32_t)(e >> 12) * (int64_t)(Y0 >> 1)) >> 17);
+  return ((uint64_t)Y0 << 32) + (uint64_t)(((int64_t)(int32_t)(e >> 12) * (int64_t)(Y0 >> 1)) >> 17);
+}
+
+// n / d for n, d in [2^62, 2^64): the quotient in Q62, within 2^-60 of it.
+FX_FN uint64_t fx_div_q62(uint64_t n, uint64_t d) {
+  const uint64_t Y = fx_recip_q62(d);
   const uint64_t q = fx_mulhi(n, Y);                              // n / d, Q62, to 2^-43
   const int32_t r = (int32_t)(int64_t)((n >> 2) - fx_mulhi(q, d)); // its residual, 2^-62 d
   return q + (uint64_t)(((int64_t)r * (int64_t)(uint32_t)(Y >> 33)) >> 29);
@@ -283,7 +309,7 @@ FX_FN double fx_tan(double z) {
 // through u^12) within 0.51 ulp, else the library's.
 FX_FN double fx_exp(double y) {
   const uint32_t yh = fx_hi(y);
-  if (yh >= 0x40862000u) return exp(y);
+  if (yh >= 0x40862000u) return fx_lib_exp(y);
   const int sh = 1085 - (int)(yh >> 20);                          // >= 53
   const uint64_t mn = (fx_bits(y) << 11) | (1ull << 63);
   const uint64_t L = 0xb8aa3b295c17f0bcull;                       // log2(e), Q63
@@ -309,4 +335,110 @@ FX_FN double fx_exp(double y) {
   const uint64_t c = j & 2u ? (j & 1u ? 0xd744fccad69d6af4ull : 0xb504f333f9de6484ull)
                             : (j & 1u ? 0x9837f0518db8a96full : 0x8000000000000000ull);
   return fx_pack(fx_mulhi(t, c), n - 62);
+}
+
+// ---------------------------------------------------------------------- inverse functions
+// sin and cos of phi (radians, 0 <= phi < 8): the phase in turns, then fx_sincos2pi_q62; within
+// 2^-58, and correctly rounded like the library's but for about one value in a hundred.
+FX_FN void fx_sincos(double phi, double &s, double &c) {
+  const uint32_t hi = fx_hi(phi);
+  if (hi >= 0x40200000u) {   // 8 and above, negative, NaN
+    s = fx_lib_sin(phi);
+    c = fx_lib_cos(phi);
+    return;
+  }
+  const uint64_t mn = (fx_bits(phi) << 11) | (1ull << 63);        // phi = mn 2^(be - 1086)
+  const int sh = 1024 - (int)(hi >> 20);                          // >= -1
+  const uint64_t C = 0xa2f9836e4e44152aull;                       // 2^66 / (2 pi)
+  const uint64_t ph = fx_mulhi(mn, C), pl = mn * C;               // phi 2^64 / (2 pi) = ph 2^-sh
+  const uint64_t X = sh < 0 ? (ph << 1) | (pl >> 63) : (sh < 64 ? ph >> sh : 0);
+  int64_t si, ci;
+  fx_sincos2pi_q62(X, si, ci);
+  s = fx_from_q62(si);
+  c = fx_from_q62(ci);
+}
+
+// atan2(y, x) for finite arguments whose exponents lie within 2^+-400 (others: the library's).
+// With t the smaller over the larger magnitude: below 2^-9 the series of atan(t) in FP64;
+// else an FP32 estimate u of atan(t) and the remaining angle, tan(d) = (lo cos u - hi sin u) /
+// (hi cos u + lo sin u), in fixed point (|d| < 2^-20, so d^3/3 is below 2^-61 of it).  Within
+// 0.51 ulp above 2^-4 and an ulp everywhere.
+FX_FN double fx_atan2(double y, double x) {
+  const uint32_t yh = fx_hi(y) & 0x7fffffffu, xh = fx_hi(x) & 0x7fffffffu;
+  if (yh - 0x26f00000u >= 0x32000000u || xh - 0x26f00000u >= 0x32000000u) return fx_lib_atan2(y, x);
+  const uint64_t yb = fx_bits(y) & 0x7fffffffffffffffull, xb = fx_bits(x) & 0x7fffffffffffffffull;
+  const bool swap = yb > xb, back = (int32_t)fx_hi(x) < 0;
+  const uint64_t hb = swap ? yb : xb, lb = swap ? xb : yb;
+  const int d = (int)(hb >> 52) - (int)(lb >> 52);                // >= 0
+  uint64_t th;                                                    // atan(t), Q64
+  double r;
+  if (d > 9) {
+    const double t = fx_from_bits(lb) / fx_from_bits(hb), t2 = t * t;
+    r = t + t * t2 * (-1.0 / 3.0 + t2 * (0.2 + t2 * (-1.0 / 7.0 + t2 * (1.0 / 9.0))));
+    const int sh = 1022 - (int)(fx_hi(r) >> 20);                  // r < 2^-8
+    th = sh < 64 ? ((fx_bits(r) << 11) | (1ull << 63)) >> sh : 0;
+  } else {
+    const uint64_t H = (hb << 11) | (1ull << 63), L = ((lb << 11) | (1ull << 63)) >> d;   // Q63
+    const float t = fx_mulf((float)(uint32_t)(L >> 32), fx_rcp_est((float)(uint32_t)(H >> 32)));
+    const uint32_t u = fx_trunc_u32(fx_mulf(atanf(t), 0x1p32f));
+    uint64_t w, k;
+    fx_sincos_series((uint64_t)u * u, w, k);
+    const uint64_t U = (uint64_t)u << 32;
+    const uint64_t sn = U - fx_mulhi(U, w), cs = 0 - k;           // Q64 (t >= 2^-10: cos u < 1)
+    // lo cos u - hi sin u, 2^-127 units, kept in 2^-82
+    const uint64_t a1 = fx_mulhi(L, cs), a0 = L * cs;
+    const uint64_t b1 = fx_mulhi(H, sn), b0 = H * sn;
+    const uint64_t n0 = a0 - b0, n1 = a1 - b1 - (a0 < b0 ? 1 : 0);
+    const int64_t N = (int64_t)((n1 << 19) | (n0 >> 45));
+    const uint64_t Y = fx_recip_q62((fx_mulhi(H, cs) >> 1) + (fx_mulhi(L, sn) >> 1));   // 2^126 / (.)
+    // N Y 2^-64, signed: tan(d) in 2^-82
+    const uint64_t an = N < 0 ? (uint64_t)-N : (uint64_t)N;
+    const uint64_t q = fx_mulhi(an, Y) >> 18;
+    th = N < 0 ? U - q : U + q;
+    r = fx_pack(th, -64);
+  }
+  if (swap || back) {
+    uint64_t T = th >> 3;                                         // Q61
+    if (swap) T = 0x3243f6a8885a308dull - T;                      // pi/2 - .
+    if (back) T = 0x6487ed5110b4611aull - T;                      // pi - .
+    r = fx_pack(T, -61);
+  }
+  return (int32_t)fx_hi(y) < 0 ? fx_neg(r) : r;
+}
+
+// log(v) for a normal v > 0 (others: the library's): m in [sqrt(1/2), sqrt(2)), s = (m - 1) /
+// (m + 1), log m = 2 s (1 + s^2/3 + s^4/5 + ...) in fixed point with a relative error of 2^-59,
+// and e log 2 added in FP64.  Within 0.51 ulp where e is 0, an ulp elsewhere.
+FX_FN double fx_log(double v) {
+  const uint32_t hi = fx_hi(v);
+  if (hi - 0x00100000u >= 0x7fe00000u) return fx_lib_log(v);
+  const uint64_t f = (fx_bits(v) << 11) | (1ull << 63);           // 1.f, Q63
+  const bool up = f >= 0xb504f333f9de6484ull;                     // above sqrt(2): m = f / 2
+  const int e = (int)(hi >> 20) - 1023 + (up ? 1 : 0);
+  // |m - 1| and m + 1
+  uint64_t n = up ? 0 - f : (f << 1) >> 1;                        // Q64 : Q63
+  const uint64_t dn = (1ull << 62) + (f >> (up ? 2 : 1));         // Q62
+  if (n == 0) return (double)e * 0x1.62e42fefa39efp-1;
+  const int z = fx_clz64(n);
+  n <<= z;
+  const uint64_t q = fx_div_q62(n, dn);
+  const int ex = (up ? 2 : 1) + z;                                // s = q 2^-62 2^-ex
+  const uint64_t S = ex < 2 ? q << (2 - ex) : (ex < 66 ? q >> (ex - 2) : 0);    // Q64, below 0.172
+  const uint64_t w = fx_mulhi(S, S);
+  const uint32_t wh = (uint32_t)(w >> 32);
+  uint32_t p = 0xb21642du + fx_mulhi32(wh, 0xa3d70a4u);           // 1/23 + w/25, Q32
+  p = 0xc30c30cu + fx_mulhi32(wh, p);
+  p = 0xd79435eu + fx_mulhi32(wh, p);
+  p = 0xf0f0f0fu + fx_mulhi32(wh, p);
+  p = 0x11111111u + fx_mulhi32(wh, p);
+  p = 0x13b13b14u + fx_mulhi32(wh, p);
+  uint64_t P = 0x1745d1745d1745d1ull + (uint64_t)wh * p;          // 1/11 + w (...), Q64
+  P = 0x1c71c71c71c71c72ull + fx_mulhi(w, P);
+  P = 0x2492492492492492ull + fx_mulhi(w, P);
+  P = 0x3333333333333333ull + fx_mulhi(w, P);
+  P = 0x5555555555555555ull + fx_mulhi(w, P);
+  const uint64_t t = (1ull << 63) + (fx_mulhi(w, P) >> 1);        // 1 + w P, Q63
+  const double lm = fx_pack(fx_mulhi(q, t), -60 - ex);       // 2 s t
+  const double l = up ? fx_neg(lm) : lm;
+  return e == 0 ? l : fx_fma((double)e, 0x1.62e42fefa39efp-1, fx_fma((double)e, 0x1.abc9e3b39803fp-56, l));
 }

@@ -6,12 +6,19 @@
 // The reference runs this as a host loop over channels, each iteration a chain of
 // event-parallel kernels (combine, msq, one launch per boost level, with and without
 // friends) that round-trip msq, p_decay, phi/ct/st and a 4x4 matrix per boost through HBM.
-// Here one persistent kernel does all of it: a block takes PHS_INV_BLOCK consecutive events
-// at a time, queues the ok ones, stages their CM-frame momenta in shared memory once, and
-// every thread then walks the visit
-// program (phs_program.h) of each channel in turn for its event, with the running frame in
-// registers and the channel's branch momenta in its shared-memory column.  Per (event,
-// channel) the only HBM traffic is the x row and the factor written.
+// Here one kernel does all of it: a block takes a tile of events and the channels of one tree
+// shape, lists the ok events, and each thread walks the shape's visit program (phs_program.h)
+// for one of them, with the running frame in registers and the branch momenta in its
+// shared-memory column; then the mappings of each channel of the shape.  Per (event, channel)
+// the only HBM traffic is the x row and the factor written.
+//
+// The FP64 pipe bounds it, so square roots, reciprocals, angles, arctangents and logarithms
+// come from phs_fix.h, the separately rounded products and sums are FMAs with register
+// constants (the same bits), and what is rare is called rather than inlined: four warps of a
+// block walk the same program, but different blocks do not, and with twice the code the
+// instruction fetches took a sixth of the time.  2e5 events of 16 channels (6 particles):
+// 6.09 -> 2.60 ms (FP64 pipe 79 % busy; 3.45 ms with 64-thread blocks and the rare code
+// inlined, 4.0 ms with 32-thread blocks).
 //
 // At a visit of branch b, with Gp and (theta, phi) the frame and angles of b's parent:
 //   G   = [R_f^-1] B_z(-bg_b) R_y(-theta) R_z(-phi) Gp   b's rest frame, z along its flight
@@ -41,51 +48,52 @@
 
 namespace {
 
+// (x, f) of the STEP maps: a call, for the code's size (as map_msq_step).
+__device__ __noinline__ double2 map_msq_step_inverse(int t, double msq, double s, double msq_min,
+                                                     double msq_max, double a0, double a1, double a2) {
+  const double z1 = (msq - msq_min) / (msq_max - msq_min);
+  if (t == PHS_MAP_STEP_E) {
+    const double z2 = 1.0 + a1 * exp(z1 / a2);
+    return make_double2((z1 - a2 * log(z2 / (1.0 + a1))) / a0, a0 * z2 * (msq_max - msq_min) / s);
+  }
+  const double z3 = a0 - z1 / a2;
+  const double x = ((a0 + z1 / a2 + z1) - sqrt(z3 * z3 + 2.0 * z1 * (a0 + z1 / a2) + z1 * z1)) / 2.0;
+  return make_double2(x, (a1 / (a0 - x) / (a0 - x) + a2) * (msq_max - msq_min) / s);
+}
+
 // mappings_gpu.hpp:15-172 (mapping_x_from_msq_*), constants as in phs_cpu.cpp:452-531.
-__device__ __forceinline__ void map_msq_inverse(int t, double msq, double s, double m, double w,
-                                                double msq_min, double msq_max, double a0,
-                                                double a1, double a2, double &x, double &f) {
+__device__ __forceinline__ void map_msq_inverse(const FxRegs &k, int t, double msq, double s,
+                                                double m, double w, double msq_min,
+                                                double msq_max, double a0, double a1, double a2,
+                                                double &x, double &f) {
   switch (t) {
     case PHS_MAP_NO:
-      x = (msq - msq_min) / (msq_max - msq_min);
-      f = (msq_max - msq_min) / s;
+      x = fx_div(fx_sub(k, msq, msq_min), fx_sub(k, msq_max, msq_min), k);
+      f = a2;
       break;
-    case PHS_MAP_SCHANNEL: {
-      const double z = (msq - m * m) / (m * w);
-      x = (atan(z) - a0) / (a1 - a0);
-      f = a2 * (1.0 + z * z);
-      break;
-    }
     case PHS_MAP_COLLINEAR:
     case PHS_MAP_INFRARED:
     case PHS_MAP_RADIATION: {
-      const double z = msq - msq_min + a0;
-      x = log(z / a0) / a1;
-      f = a2 * z;
+      const double z = fx_add(k, fx_sub(k, msq, msq_min), a0);
+      x = fx_div(fx_log(fx_div(z, a0, k)), a1, k);
+      f = fx_mul(k, a2, z);
       break;
     }
     case PHS_MAP_TCHANNEL:
     case PHS_MAP_UCHANNEL: {
       // one logarithm per lane: the side of the midpoint selects its argument
-      const bool lower = msq < (msq_max + msq_min) / 2;
-      const double z = lower ? msq - msq_min + a0 : msq_max - msq + a0;
-      const double lx = log(z / a0) / a1;
-      x = lower ? lx : 1.0 - lx;
-      f = a2 * z;
+      const bool lower = fx_gt(fx_scale(fx_add(k, msq_max, msq_min), -1), msq);
+      const double z = fx_add(k, lower ? fx_sub(k, msq, msq_min) : fx_sub(k, msq_max, msq), a0);
+      const double lx = fx_div(fx_log(fx_div(z, a0, k)), a1, k);
+      x = lower ? lx : fx_sub(k, k.one, lx);
+      f = fx_mul(k, a2, z);
       break;
     }
-    case PHS_MAP_STEP_E: {
-      const double z1 = (msq - msq_min) / (msq_max - msq_min);
-      const double z2 = 1.0 + a1 * exp(z1 / a2);
-      x = (z1 - a2 * log(z2 / (1.0 + a1))) / a0;
-      f = a0 * z2 * (msq_max - msq_min) / s;
-      break;
-    }
+    case PHS_MAP_STEP_E:
     case PHS_MAP_STEP_H: {
-      const double z1 = (msq - msq_min) / (msq_max - msq_min);
-      const double z3 = a0 - z1 / a2;
-      x = ((a0 + z1 / a2 + z1) - sqrt(z3 * z3 + 2.0 * z1 * (a0 + z1 / a2) + z1 * z1)) / 2.0;
-      f = (a1 / (a0 - x) / (a0 - x) + a2) * (msq_max - msq_min) / s;
+      const double2 r = map_msq_step_inverse(t, msq, s, msq_min, msq_max, a0, a1, a2);
+      x = r.x;
+      f = r.y;
       break;
     }
     default:
@@ -95,17 +103,17 @@ __device__ __forceinline__ void map_msq_inverse(int t, double msq, double s, dou
 }
 
 // mappings_gpu.hpp:184-219 (mapping_x_from_ct_*).
-__device__ __forceinline__ void map_ct_inverse(int ct_class, double ct, double b0, double b1,
-                                               double &x, double &f) {
+__device__ __forceinline__ void map_ct_inverse(const FxRegs &k, int ct_class, double ct, double b0,
+                                               double b1, double &x, double &f) {
   if (ct_class == PHS_CT_COLLINEAR) {
     // one logarithm per lane, as for the msq maps
     const bool lower = ct < 0.0;
-    const double ct1 = lower ? ct + b0 + 1.0 : -ct + b0 + 1.0;
-    const double lx = log(ct1 / b0) / (2.0 * b1);
-    x = lower ? lx : 1.0 - lx;
-    f = ct1 * b1;
+    const double ct1 = fx_add(k, fx_add(k, lower ? ct : fx_neg(ct), b0), k.one);
+    const double lx = fx_div(fx_log(fx_div(ct1, b0, k)), fx_scale(b1, 1), k);
+    x = lower ? lx : fx_sub(k, k.one, lx);
+    f = fx_mul(k, ct1, b1);
   } else {
-    x = (ct + 1.0) / 2.0;
+    x = fx_scale(fx_add(k, ct, k.one), -1);
     f = 1.0;
   }
 }
@@ -150,15 +158,18 @@ struct InvMomenta {
 // exceptions are divisions by constants of an output that is not ill-conditioned in them,
 // done as products with the constant's reciprocal (one rounding more): x_phi = phi / 2 pi
 // and the Breit-Wigner inverse's divisions by m w and a1 - a0.
-__device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, double sqrts,
+__device__ void inverse_geometry(const FxRegs &k, const PhsChannel &ch, const InvMomenta &pm, double sqrts,
                                  double *stk, double *geo, int stack_depth) {
-  const double s = sqrts * sqrts;
+  const double s = fx_mul(k, sqrts, sqrts);
+  const auto mul = [&](double u, double v) { return fx_mul(k, u, v); };
+  const auto add = [&](double u, double v) { return fx_add(k, u, v); };
+  const auto sub = [&](double u, double v) { return fx_sub(k, u, v); };
   // internal momenta as sums of their daughters in post-order (_combine_particles,
   // phs.cu:1262-1283); the root's (the last) is never a daughter
   for (int i = 0; i + 1 < ch.n_vol; i++) {
     const int a = ch.comb[i][0], b = ch.comb[i][1], o = ch.n_out + i;
 #pragma unroll
-    for (int mu = 0; mu < 4; mu++) pm.set_internal(o, mu, pm.get(a, mu) + pm.get(b, mu));
+    for (int mu = 0; mu < 4; mu++) pm.set_internal(o, mu, add(pm.get(a, mu), pm.get(b, mu)));
   }
   // carried state of the visited branch: its parent's frame Gp and angles, its msq, decay
   // momentum and mass
@@ -169,6 +180,9 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
+    // one reciprocal of the mass serves both divisions by it
+    const bool serves = fx_quot_serves(m_b);
+    const double rm = serves ? fx_rcp(m_b, k) : 0.0;
     // the branch's frame G: CM momenta -> its rest frame, z along its flight (or friend)
     // axis.  The root's is the identity; else L_r3_r2_b3(-bg, gamma, ct0, -st0, cp0, -sp0)
     // times the parent's (phs.cu:1114-1125)
@@ -177,29 +191,37 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
 #pragma unroll
       for (int i = 0; i < 16; i++) G[i] = (i % 5 == 0) ? 1.0 : 0.0;
     } else {
-      const double bg = m_b > 0.0 ? pd_b / m_b : 0.0;
-      const double ga = sqrt(1.0 + bg * bg);
-      const double t01 = -bg * st0 * cp0, t02 = -bg * st0 * sp0, t03 = -bg * ct0;
-      const double t11 = ct0 * cp0, t12 = ct0 * sp0;
-      const double t31 = ga * st0 * cp0, t32 = ga * st0 * sp0, t33 = ga * ct0;
+      const double bg = fx_gt(m_b, 0.0) ? (serves ? fx_quot(pd_b, m_b, rm, k) : fx_lib_div(pd_b, m_b)) : 0.0;
+      const double ga = fx_sqrt(add(mul(bg, bg), k.one), k);
+      const double bs = mul(-bg, st0), gs = mul(ga, st0);
+      const double t01 = mul(bs, cp0), t02 = mul(bs, sp0), t03 = mul(-bg, ct0);
+      const double t11 = mul(ct0, cp0), t12 = mul(ct0, sp0);
+      const double t31 = mul(gs, cp0), t32 = mul(gs, sp0), t33 = mul(ga, ct0);
       if (V.parent_root) {
         // the parent's frame is the root's, the identity: G is the step's own matrix (the
         // product below with Gp = 1 gives the same bits)
         G[0] = ga;    G[1] = t01;   G[2] = t02;  G[3] = t03;
-        G[4] = 0.0;   G[5] = t11;   G[6] = t12;  G[7] = -st0;
-        G[8] = 0.0;   G[9] = -sp0;  G[10] = cp0; G[11] = 0.0;
-        G[12] = -bg;  G[13] = t31;  G[14] = t32; G[15] = t33;
+        G[4] = 0.0;   G[5] = t11;   G[6] = t12;  G[7] = fx_neg(st0);
+        G[8] = 0.0;   G[9] = fx_neg(sp0); G[10] = cp0; G[11] = 0.0;
+        G[12] = fx_neg(bg); G[13] = t31;  G[14] = t32; G[15] = t33;
       } else {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
           const double g0 = Gp[c], g1 = Gp[4 + c], g2 = Gp[8 + c], g3 = Gp[12 + c];
           // row 0 only feeds the frames of internal daughters
-          if (!V.both_leaves) G[c] = ga * g0 + t01 * g1 + t02 * g2 + t03 * g3;
-          G[4 + c] = t11 * g1 + t12 * g2 + (-st0) * g3;
-          G[8 + c] = (-sp0) * g1 + cp0 * g2;
-          G[12 + c] = (-bg) * g0 + t31 * g1 + t32 * g2 + t33 * g3;
+          G[c] = g0;   // row 0 below
+          G[4 + c] = add(add(mul(t11, g1), mul(t12, g2)), mul(-st0, g3));
+          G[8 + c] = add(mul(-sp0, g1), mul(cp0, g2));
+          G[12 + c] = add(add(add(mul(-bg, g0), mul(t31, g1)), mul(t32, g2)), mul(t33, g3));
         }
-        if (V.both_leaves) G[0] = G[1] = G[2] = G[3] = 0.0;
+        // row 0 only feeds the frames of internal daughters (a loop: the compiler would issue
+        // a short block's FP64 instructions also where it is skipped)
+#pragma unroll 1
+        for (int c = V.both_leaves ? 4 : 0; c < 4; c += 4) {
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            G[i] = add(add(add(mul(ga, Gp[i]), mul(t01, Gp[4 + i])), mul(t02, Gp[8 + i])), mul(t03, Gp[12 + i]));
+        }
       }
       if (V.friend_sign != 0) {
         // rotate the friend beam's direction G (1, 0, 0, ff) onto z (phs.cu:1183-1206);
@@ -226,28 +248,33 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
       q1[mu] = pm.get(V.slot[1], mu);
     }
     double cmsq[2];
-    cmsq[0] = q0[0] * q0[0] - q0[1] * q0[1] - q0[2] * q0[2] - q0[3] * q0[3];
-    cmsq[1] = q1[0] * q1[0] - q1[1] * q1[1] - q1[2] * q1[2] - q1[3] * q1[3];
+    cmsq[0] = sub(sub(sub(mul(q0[0], q0[0]), mul(q0[1], q0[1])), mul(q0[2], q0[2])), mul(q0[3], q0[3]));
+    cmsq[1] = sub(sub(sub(mul(q1[0], q1[0]), mul(q1[1], q1[1])), mul(q1[2], q1[2])), mul(q1[3], q1[3]));
 
     geo[(PHS_INV_GEO * v + 0) * PHS_INV_BLOCK] = cmsq[0];
     geo[(PHS_INV_GEO * v + 1) * PHS_INV_BLOCK] = cmsq[1];
 
     // Kallen function at the visited branch
-    const double d = msq_b - cmsq[0] - cmsq[1];
-    const double sl = sqrt(d * d - 4.0 * cmsq[0] * cmsq[1]);
-    const double pd = sl / (2.0 * m_b);
-    geo[(PHS_INV_GEO * v + 4) * PHS_INV_BLOCK] = sl / msq_b;
+    const double d = sub(sub(msq_b, cmsq[0]), cmsq[1]);
+    const double sl = fx_sqrt(sub(mul(d, d), mul(fx_scale(cmsq[0], 2), cmsq[1])), k);
+    // (halving sl / m and dividing by 2 m round alike)
+    const double pd = serves ? fx_scale(fx_quot(sl, m_b, rm, k), -1) : fx_lib_div(sl, 2.0 * m_b);
+    geo[(PHS_INV_GEO * v + 4) * PHS_INV_BLOCK] = fx_div(sl, msq_b, k);
 
     // angles of daughter 1 in the branch's frame (azimuthal_angle, polar_angle_ct,
     // phs.cu:913-922)
     // (the root's frame is the identity: the same bits without the products)
-    const double qx = V.self_root ? q0[1] : G[4] * q0[0] + G[5] * q0[1] + G[6] * q0[2] + G[7] * q0[3];
-    const double qy = V.self_root ? q0[2] : G[8] * q0[0] + G[9] * q0[1] + G[10] * q0[2] + G[11] * q0[3];
-    const double qz = V.self_root ? q0[3] : G[12] * q0[0] + G[13] * q0[1] + G[14] * q0[2] + G[15] * q0[3];
-    double phi = atan2(qy, qx);
-    if (phi < 0.0) phi += 2.0 * PHS_PI;
-    geo[(PHS_INV_GEO * v + 3) * PHS_INV_BLOCK] = phi * (1.0 / (2.0 * PHS_PI));   // x_phi
-    const double ct = qz / sqrt(qx * qx + qy * qy + qz * qz);
+    double qx = q0[1], qy = q0[2], qz = q0[3];
+#pragma unroll 1
+    for (int r = V.self_root ? 1 : 0; r < 1; r++) {
+      qx = add(add(add(mul(G[4], q0[0]), mul(G[5], q0[1])), mul(G[6], q0[2])), mul(G[7], q0[3]));
+      qy = add(add(add(mul(G[8], q0[0]), mul(G[9], q0[1])), mul(G[10], q0[2])), mul(G[11], q0[3]));
+      qz = add(add(add(mul(G[12], q0[0]), mul(G[13], q0[1])), mul(G[14], q0[2])), mul(G[15], q0[3]));
+    }
+    double phi = fx_atan2(qy, qx);
+    if ((int32_t)fx_hi(phi) < 0) phi = add(phi, 2.0 * PHS_PI);
+    geo[(PHS_INV_GEO * v + 3) * PHS_INV_BLOCK] = mul(phi, 1.0 / (2.0 * PHS_PI));   // x_phi
+    const double ct = fx_div(qz, fx_sqrt(add(add(mul(qx, qx), mul(qy, qy)), mul(qz, qz)), k), k);
     geo[(PHS_INV_GEO * v + 2) * PHS_INV_BLOCK] = ct;
     if (V.both_leaves) {
       if (sp > 0) {
@@ -264,9 +291,9 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
       }
       continue;
     }
-    const double st = sqrt(1.0 - ct * ct);
+    const double st = fx_sqrt(sub(k.one, mul(ct, ct)), k);
     double sph, cph;
-    sincos(phi, &sph, &cph);
+    fx_sincos(phi, sph, cph);
     if (V.push >= 0 && phs_in(sp, stack_depth, PHS_CHK_STACK)) {
       const bool j0 = V.push == 0;
 #pragma unroll
@@ -277,8 +304,8 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
       inv_store(stk, sp, 19, sph);
       const double mq = j0 ? cmsq[0] : cmsq[1];
       inv_store(stk, sp, 20, mq);
-      inv_store(stk, sp, 21, j0 ? pd : -pd);
-      inv_store(stk, sp, 22, sqrt(mq));
+      inv_store(stk, sp, 21, j0 ? pd : fx_neg(pd));
+      inv_store(stk, sp, 22, fx_sqrt(mq, k));
       sp++;
     }
     if (V.carry >= 0) {
@@ -290,8 +317,8 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
       cp0 = cph;
       sp0 = sph;
       msq_b = j0 ? cmsq[0] : cmsq[1];
-      pd_b = j0 ? pd : -pd;
-      m_b = sqrt(msq_b);
+      pd_b = j0 ? pd : fx_neg(pd);
+      m_b = fx_sqrt(msq_b, k);
     }
   }
 }
@@ -303,15 +330,15 @@ __device__ void inverse_geometry(const PhsChannel &ch, const InvMomenta &pm, dou
 // cache (null: no cache, reuse 0).  xr null: the mappings run (the next channel may reuse
 // them) but write nothing.
 template <bool PER_EVENT>
-__device__ double inverse_maps(const PhsChannel &ch, double sqrts, const double *geo,
+__device__ double inverse_maps(const FxRegs &k, const PhsChannel &ch, double sqrts, const double *geo,
                                double *cache, double *xr, uint64_t reuse, int n_x) {
-  const double s = sqrts * sqrts;
+  const double s = fx_mul(k, sqrts, sqrts);
   double factor = 1.0;
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
-    // inverse msq maps of the internal daughters
-#pragma unroll
+    // inverse msq maps of the internal daughters (not unrolled: the code of one serves both)
+#pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
       if (C.internal) {
@@ -322,16 +349,17 @@ __device__ double inverse_maps(const PhsChannel &ch, double sqrts, const double 
           f = slot[PHS_INV_BLOCK];
         } else {
           double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax;
-          if (PER_EVENT) child_constants(fx_regs(), C, sqrts, ch.m_tot, 1.0 / s, a0, a1, a2, mn, mx, mmax);
+          if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, fx_rcp(s, k), a0, a1, a2, mn, mx, mmax);
           const double msq = geo[(PHS_INV_GEO * v + j) * PHS_INV_BLOCK];
           if (C.map_id == PHS_MAP_SCHANNEL) {
             // mapping_x_from_msq_schannel with its divisors m w and a1 - a0 (constants of the
             // channel) as compiled reciprocals
-            const double z = (msq - C.msq0) * C.inv_mw;
-            x = PER_EVENT ? (atan(z) - a0) / (a1 - a0) : (atan(z) - a0) * C.inv_da;
-            f = a2 * (1.0 + z * z);
+            const double z = fx_mul(k, fx_sub(k, msq, C.msq0), C.inv_mw);
+            const double da = fx_sub(k, fx_atan2(z, 1.0), a0);
+            x = PER_EVENT ? fx_div(da, fx_sub(k, a1, a0), k) : fx_mul(k, da, C.inv_da);
+            f = fx_mul(k, a2, fx_add(k, fx_mul(k, z, z), k.one));
           } else {
-            map_msq_inverse(C.map_id, msq, s, C.m, C.w, mn, mx, a0, a1, a2, x, f);
+            map_msq_inverse(k, C.map_id, msq, s, C.m, C.w, mn, mx, a0, a1, a2, x, f);
           }
           if (slot) {
             slot[0] = x;
@@ -339,10 +367,10 @@ __device__ double inverse_maps(const PhsChannel &ch, double sqrts, const double 
           }
         }
         if (xr && phs_in(C.x_msq, n_x, PHS_CHK_INV)) xr[C.x_msq] = x;
-        factor *= f;
+        factor = fx_mul(k, factor, f);
       }
     }
-    factor *= geo[(PHS_INV_GEO * v + 4) * PHS_INV_BLOCK];  // sqrt(lambda) / msq
+    factor = fx_mul(k, factor, geo[(PHS_INV_GEO * v + 4) * PHS_INV_BLOCK]);  // sqrt(lambda) / msq
     if (xr && phs_in(V.x_phi, n_x, PHS_CHK_INV)) xr[V.x_phi] = geo[(PHS_INV_GEO * v + 3) * PHS_INV_BLOCK];
     double *slot = cache ? cache + (PHS_INV_CACHE * v + 4) * PHS_INV_BLOCK : nullptr;
     double x, f;
@@ -355,144 +383,150 @@ __device__ double inverse_maps(const PhsChannel &ch, double sqrts, const double 
         b0 = V.m * V.m / s;
         b1 = log((b0 + 1.0) / b0);
       }
-      map_ct_inverse(V.ct_class, geo[(PHS_INV_GEO * v + 2) * PHS_INV_BLOCK], b0, b1, x, f);
+      map_ct_inverse(k, V.ct_class, geo[(PHS_INV_GEO * v + 2) * PHS_INV_BLOCK], b0, b1, x, f);
       if (slot) {
         slot[0] = x;
         slot[PHS_INV_BLOCK] = f;
       }
     }
     if (xr && phs_in(V.x_ct, n_x, PHS_CHK_INV)) xr[V.x_ct] = x;
-    factor *= f;
+    if (V.ct_class == PHS_CT_COLLINEAR) factor = fx_mul(k, factor, f);   // uniform: 1
   }
   return factor;
 }
 
+// One block: `tile` events and the channels of one tree shape (in the launch's slice of the
+// group order).  It writes their outputs that need no arithmetic, gathers the tile's ok events
+// and walks them, a warp 32 at a time.  What bounds the kernel is the FP64 pipe; events are ok
+// in very different shares from channel to channel, so blocks are many and short and the
+// hardware's block scheduler spreads them.  (Persistent blocks that each took 64 events through
+// every channel left most SMs idle: 40 000 ok events of 2e5 are 600 such walks.)
 // LAB_ROWS: no lab boost (uniform beams with E1 = E2): the outgoing momenta are read from p
 // instead of staged in shared memory (InvMomenta).
 template <bool PER_EVENT, bool LAB_ROWS>
-__global__ void __launch_bounds__(PHS_INV_BLOCK)
+__global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
     phs_inverse_kernel(const __grid_constant__ PhsInvLaunch a) {
   static_assert(!(PER_EVENT && LAB_ROWS), "per-event beams stage their CM momenta");
+  constexpr int kWarps = PHS_INV_BLOCK / 32;
   extern __shared__ double sm[];
+  const FxRegs k = fx_regs();
   double *pm = sm;  // [4 (n_out - 1), or 4 (2 n_out - 1) with staging][block]
   double *stk = sm + (size_t)4 * (LAB_ROWS ? a.n_out - 1 : 2 * a.n_out - 1) * PHS_INV_BLOCK;  // frame stack
   double *geo = stk + (size_t)PHS_INV_STATE * a.stack_depth * PHS_INV_BLOCK;  // per-visit geometry
   double *cache = a.group_reuse ? geo + (size_t)PHS_INV_GEO * a.max_visits * PHS_INV_BLOCK
                                 : nullptr;  // per-visit mapping results
-  const int tid = threadIdx.x;
-  const int64_t n_tiles = (a.n_events + PHS_INV_BLOCK - 1) / PHS_INV_BLOCK;
-  const PhsChannel &ch0 = a.channels[0];
+  __shared__ uint16_t listed[PHS_INV_TILE];  // the tile's ok events
+  __shared__ int warp_ok[kWarps];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int n_groups = a.group_hi - a.group_lo;
+  const int64_t n_items = (a.n_events + a.tile - 1) / a.tile * n_groups;
+  const bool has_own = a.x_own != nullptr;
 
-  // the ok events of this block's tiles, queued: a walk takes PHS_INV_BLOCK of them at a
-  // time, so every thread has an event (the rest, fewer, wait for the next tile)
-  __shared__ int64_t q_ev[2 * PHS_INV_BLOCK];
-  __shared__ int q_own[2 * PHS_INV_BLOCK];
-  __shared__ int warp_ok[PHS_INV_BLOCK / 32];
-  const int lane = tid & 31, wid = tid >> 5;
-  int queued = 0;  // block-uniform
-
-  for (int64_t tile = blockIdx.x;; tile += gridDim.x) {
-    const bool more = tile < n_tiles;
-    // 1. per event: the outputs that need no arithmetic (the generating channel's own x and
-    // factor, x padding beyond a channel's n_x_used, zeros for ok = false events)
-    const int64_t ev = tile * PHS_INV_BLOCK + tid;
-    const bool valid = more && ev < a.n_events;
-    int own = 0;
-    bool ok = false;
-    if (valid) {
-      // the generating channel: the last c with ch_begin[c] <= ev
-      int lo = 0, hi = a.n_channels - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a.ch_begin[mid] <= ev) lo = mid; else hi = mid - 1;
-      }
-      own = lo;
-      ok = a.ok ? a.ok[ev] != 0 : true;
-      const double *xo = a.x_own ? a.x_own + ev * a.n_x : nullptr;
-      // (checked build: a row beyond x_out's events writes nothing; no early exit, the
-      // block's barriers below must be reached by every thread)
-      const bool rows_in = phs_in(ev, a.x_ch_stride, PHS_CHK_INV);
-      for (int c = 0; c < (a.write_fixed && rows_in ? a.n_channels : 0); c++) {
-        double *xr = a.x_out + ((int64_t)c * a.x_ch_stride + ev) * a.n_x;
-        double *fo = a.all_factors + ev * a.n_channels + c;
-        if (c == own && xo) {
-          // the generating channel keeps its own x and factor (_move_x/_move_factors)
-          for (int k = 0; k < a.n_x; k++) xr[k] = xo[k];
-          *fo = a.factor_own ? a.factor_own[ev] : 0.0;
-          continue;
-        }
-        const int n_used = a.channels[c].n_x_used;
-        for (int k = n_used; k < a.n_x; k++) xr[k] = xo ? xo[k] : 0.0;
-        if (!ok) {
-          for (int k = 0; k < n_used; k++) xr[k] = 0.0;
-          *fo = 0.0;
-        }
-      }
-    }
-    // 2. queue the ok events: the inversions run in full warps (an FP64 instruction costs
-    // the pipe the same whatever the number of active lanes)
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (lane == 0) warp_ok[wid] = __popc(m);
-    __syncthreads();
-    int before = 0, n_ok = 0;
-    for (int w = 0; w < PHS_INV_BLOCK / 32; w++) {
-      if (w < wid) before += warp_ok[w];
-      n_ok += warp_ok[w];
-    }
-    if (ok) {
-      const int d = queued + before + __popc(m & ((1u << lane) - 1u));
-      if (phs_in(d, 2 * PHS_INV_BLOCK, PHS_CHK_SLOT)) {
-        q_ev[d] = ev;
-        q_own[d] = own;
-      }
-    }
-    queued += n_ok;
-    __syncthreads();  // the queue is complete; warp_ok is read
-    if (queued < PHS_INV_BLOCK && (more || queued == 0)) {
-      if (!more) break;
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int g = a.group_lo + (int)(item % n_groups);
+    const int64_t e0 = item / n_groups * a.tile;
+    const int n_ev = (int)min((int64_t)a.tile, a.n_events - e0);
+    const int gb = a.group_begin[g], ge = a.group_begin[g + 1];
+    const int lo = max(gb, a.order_lo), hi = min(ge, a.order_hi);
+    // checked build: the group's entries, its shape's program, the regions sized for it and
+    // the tile (block-uniform: every thread leaves together)
+    if (!phs_in(gb, a.n_channels, PHS_CHK_SLOT) || !phs_in(hi - 1, a.n_channels, PHS_CHK_SLOT) ||
+        !phs_in(a.group_order[gb], a.n_channels, PHS_CHK_CHANNEL) ||
+        !phs_in(a.channels[a.group_order[gb]].n_visits - 1, a.max_visits, PHS_CHK_VISITS) ||
+        !phs_in(a.channels[a.group_order[gb]].n_out - 1, a.n_out, PHS_CHK_SLOT) ||
+        !phs_in(n_ev - 1, PHS_INV_TILE, PHS_CHK_SLOT) || !phs_in(e0 + n_ev - 1, a.x_ch_stride, PHS_CHK_INV))
       continue;
-    }
-    const int n_walk = min(queued, PHS_INV_BLOCK);
-    // 3. every other channel of the tid-th queued event
-    if (tid < n_walk && phs_in(q_ev[tid], a.n_events, PHS_CHK_SLOT) &&
-        phs_in(q_ev[tid], a.x_ch_stride, PHS_CHK_INV)) {
-      const int64_t e = q_ev[tid];
-      const int own_e = q_own[tid];
-      double sqrts = ch0.sqrts, lab_bg = ch0.lab ? ch0.lab_bg : 0.0;
-      double lab_ga = ch0.lab ? ch0.lab_gamma : 1.0;
-      if (PER_EVENT) {
-        const double E1 = a.E1[e], E2 = a.E2[e], r = sqrt(E1 * E2);
-        sqrts = 2.0 * r;
-        lab_bg = (E1 - E2) / (2.0 * r);
-        lab_ga = sqrt(1.0 + lab_bg * lab_bg);
-      }
-      // this event's momenta, lab -> CM (the inverse of phs.cu:1286-1301)
-      const double *prow = a.p + e * 4 * (int64_t)a.n_out;
-      if (!LAB_ROWS) {
-        const double2 *pe = reinterpret_cast<const double2 *>(prow);
-        for (int k = 0; k < a.n_out; k++) {
-          const double2 e_x = pe[2 * k], y_z = pe[2 * k + 1];
-          pm[(4 * k + 0) * PHS_INV_BLOCK + tid] = dsub(dmul(lab_ga, e_x.x), dmul(lab_bg, y_z.y));
-          pm[(4 * k + 1) * PHS_INV_BLOCK + tid] = e_x.y;
-          pm[(4 * k + 2) * PHS_INV_BLOCK + tid] = y_z.x;
-          pm[(4 * k + 3) * PHS_INV_BLOCK + tid] = dadd(dmul(-lab_bg, e_x.x), dmul(lab_ga, y_z.y));
+
+    // 1. per channel: the outputs that need no arithmetic (the generating channel's own x and
+    // factor, x padding beyond a channel's n_x_used, zeros for ok = false events); rows of
+    // consecutive events are contiguous
+    for (int i = lo; i < hi; i++) {
+      const int c = a.group_order[i];
+      if (!phs_in(c, a.n_channels, PHS_CHK_CHANNEL)) continue;
+      // the generating channel of an event: the last c with ch_begin[c] <= event
+      const int64_t own0 = a.ch_begin[c] - e0;
+      const int64_t own1 = (c + 1 < a.n_channels ? a.ch_begin[c + 1] : a.n_events) - e0;
+      const int n_used = a.channels[c].n_x_used;
+      double *xr = a.x_out + ((int64_t)c * a.x_ch_stride + e0) * a.n_x;
+      const double *xo = has_own ? a.x_own + e0 * a.n_x : nullptr;
+      int ev = tid / a.n_x, kx = tid - ev * a.n_x;
+      const int dev = PHS_INV_BLOCK / a.n_x, dkx = PHS_INV_BLOCK - dev * a.n_x;
+      for (int j = tid; j < n_ev * a.n_x; j += PHS_INV_BLOCK) {
+        const bool own = has_own && ev >= own0 && ev < own1;
+        if (own || kx >= n_used)
+          xr[j] = xo ? xo[j] : 0.0;
+        else if (a.ok && !a.ok[e0 + ev])
+          xr[j] = 0.0;
+        ev += dev;
+        kx += dkx;
+        if (kx >= a.n_x) {
+          kx -= a.n_x;
+          ev++;
         }
       }
-      const InvMomenta mom{pm + tid, LAB_ROWS ? prow : nullptr, a.n_out};
-      // the geometry once per tree shape, then the mappings of each channel of that shape
-      // (of this launch's slice of the group order)
-      const bool has_own = a.x_own != nullptr;
-      for (int g = 0; g < a.n_groups; g++) {
-        const int gb = a.group_begin[g], ge = a.group_begin[g + 1];
-        const int lo = max(gb, a.order_lo), hi = min(ge, a.order_hi);
-        if (lo >= hi || (has_own && hi - lo == 1 && a.group_order[lo] == own_e)) continue;
-        // checked build: the group's entries, its shape's program and the regions sized for it
-        if (!phs_in(gb, a.n_channels, PHS_CHK_SLOT) || !phs_in(hi - 1, a.n_channels, PHS_CHK_SLOT) ||
-            !phs_in(a.group_order[gb], a.n_channels, PHS_CHK_CHANNEL) ||
-            !phs_in(a.channels[a.group_order[gb]].n_visits - 1, a.max_visits, PHS_CHK_VISITS) ||
-            !phs_in(a.channels[a.group_order[gb]].n_out - 1, a.n_out, PHS_CHK_SLOT))
-          continue;
-        inverse_geometry(a.channels[a.group_order[gb]], mom, sqrts, stk, geo + tid, a.stack_depth);
+      for (int j = tid; j < n_ev; j += PHS_INV_BLOCK) {
+        double *fo = a.all_factors + (e0 + j) * a.n_channels + c;
+        if (has_own && j >= own0 && j < own1)
+          *fo = a.factor_own ? a.factor_own[e0 + j] : 0.0;
+        else if (a.ok && !a.ok[e0 + j])
+          *fo = 0.0;
+      }
+    }
+
+    // 2. the ok events, listed in order: the inversions run in full warps (an FP64 instruction
+    // costs the pipe the same whatever the number of active lanes).  A shape's only channel
+    // does not invert the events that it generated.
+    const bool skip_own = has_own && hi - lo == 1;
+    const int c0 = a.group_order[lo];
+    const int64_t skip0 = skip_own ? a.ch_begin[c0] - e0 : 0;
+    const int64_t skip1 = skip_own ? (c0 + 1 < a.n_channels ? a.ch_begin[c0 + 1] : a.n_events) - e0 : 0;
+    int n_list = 0;  // block-uniform
+    for (int base = 0; base < n_ev; base += PHS_INV_BLOCK) {
+      const int j = base + tid;
+      const bool take = j < n_ev && (!a.ok || a.ok[e0 + j]) && !(j >= skip0 && j < skip1);
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (lane == 0) warp_ok[wid] = __popc(m);
+      __syncthreads();
+      int before = n_list, total = 0;
+      for (int w = 0; w < kWarps; w++) {
+        if (w < wid) before += warp_ok[w];
+        total += warp_ok[w];
+      }
+      const int d = before + __popc(m & ((1u << lane) - 1u));
+      if (take && phs_in(d, PHS_INV_TILE, PHS_CHK_SLOT)) listed[d] = (uint16_t)j;
+      n_list += total;
+      __syncthreads();  // warp_ok is read, the entries are written
+    }
+
+    // 3. the geometry once per event, then the mappings of each channel of the shape
+    for (int at = wid * 32; at < n_list; at += PHS_INV_BLOCK) {
+      const int slot = at + lane;
+      if (slot < n_list && phs_in(listed[slot], n_ev, PHS_CHK_SLOT)) {
+        const int j = listed[slot];
+        const int64_t e = e0 + j;
+        const PhsChannel &ch0 = a.channels[0];
+        double sqrts = ch0.sqrts, lab_bg = ch0.lab ? ch0.lab_bg : 0.0;
+        double lab_ga = ch0.lab ? ch0.lab_gamma : 1.0;
+        if (PER_EVENT) {
+          const double E1 = a.E1[e], E2 = a.E2[e], r = fx_sqrt(fx_mul(k, E1, E2), k);
+          sqrts = fx_add(k, r, r);
+          lab_bg = fx_div(fx_sub(k, E1, E2), sqrts, k);
+          lab_ga = fx_sqrt(fx_add(k, fx_mul(k, lab_bg, lab_bg), k.one), k);
+        }
+        // this event's momenta, lab -> CM (the inverse of phs.cu:1286-1301)
+        const double *prow = a.p + e * 4 * (int64_t)a.n_out;
+        if (!LAB_ROWS) {
+          const double2 *pe = reinterpret_cast<const double2 *>(prow);
+          for (int q = 0; q < a.n_out; q++) {
+            const double2 e_x = pe[2 * q], y_z = pe[2 * q + 1];
+            pm[(4 * q + 0) * PHS_INV_BLOCK + tid] = fx_sub(k, fx_mul(k, lab_ga, e_x.x), fx_mul(k, lab_bg, y_z.y));
+            pm[(4 * q + 1) * PHS_INV_BLOCK + tid] = e_x.y;
+            pm[(4 * q + 2) * PHS_INV_BLOCK + tid] = y_z.x;
+            pm[(4 * q + 3) * PHS_INV_BLOCK + tid] = fx_add(k, fx_mul(k, -lab_bg, e_x.x), fx_mul(k, lab_ga, y_z.y));
+          }
+        }
+        const InvMomenta mom{pm + tid, LAB_ROWS ? prow : nullptr, a.n_out};
+        inverse_geometry(k, a.channels[a.group_order[gb]], mom, sqrts, stk, geo + tid, a.stack_depth);
         for (int i = lo; i < hi; i++) {
           const int c = a.group_order[i];
           if (!phs_in(c, a.n_channels, PHS_CHK_CHANNEL) ||
@@ -500,34 +534,19 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK)
             continue;
           // the generating channel keeps its own row, but its mappings still run when a
           // later channel of the shape reuses them
-          const bool own_row = c == own_e && has_own;
+          const bool own_row = has_own && e >= a.ch_begin[c] &&
+                               (c + 1 == a.n_channels || e < a.ch_begin[c + 1]);
           if (own_row && (!cache || i + 1 == hi || a.group_reuse[i + 1] == 0)) continue;
           double *xr = own_row ? nullptr : a.x_out + ((int64_t)c * a.x_ch_stride + e) * a.n_x;
           // the first channel of a shape (or of the slice) computes every mapping
           const uint64_t reuse = i == lo || !cache ? 0ull : a.group_reuse[i];
-          const double fac = inverse_maps<PER_EVENT>(a.channels[c], sqrts, geo + tid,
+          const double fac = inverse_maps<PER_EVENT>(k, a.channels[c], sqrts, geo + tid,
                                                      cache ? cache + tid : nullptr, xr, reuse, a.n_x);
           if (!own_row) a.all_factors[e * a.n_channels + c] = fac;
         }
       }
     }
-    __syncthreads();  // every walked entry is read
-    // the events beyond the walked ones move to the front (fewer than PHS_INV_BLOCK)
-    const int rest = queued - n_walk;
-    int64_t e_rest = 0;
-    int o_rest = 0;
-    if (tid < rest && phs_in(PHS_INV_BLOCK + tid, 2 * PHS_INV_BLOCK, PHS_CHK_SLOT)) {
-      e_rest = q_ev[PHS_INV_BLOCK + tid];
-      o_rest = q_own[PHS_INV_BLOCK + tid];
-    }
-    __syncthreads();
-    if (tid < rest) {
-      q_ev[tid] = e_rest;
-      q_own[tid] = o_rest;
-    }
-    queued = rest;
-    __syncthreads();
-    if (!more && queued == 0) break;
+    __syncthreads();  // the list is read
   }
 }
 
@@ -563,8 +582,8 @@ int phs_inverse_blocks_per_sm(int n_out, int stack_depth, int max_visits, bool p
   return n > 0 ? n : 1;
 }
 
-cudaError_t phs_launch_inverse(const PhsInvLaunch &a, int n_blocks, cudaStream_t stream) {
-  if (a.n_events <= 0) return cudaSuccess;
+cudaError_t phs_launch_inverse(const PhsInvLaunch &a, cudaStream_t stream) {
+  if (a.n_events <= 0 || a.group_lo >= a.group_hi) return cudaSuccess;
   const bool per_event = a.E1 && a.E2;
   const bool lab_rows = !per_event && !a.lab;
   const size_t smem = phs_inverse_smem_bytes(a.n_out, a.stack_depth, a.max_visits,
@@ -574,12 +593,14 @@ cudaError_t phs_launch_inverse(const PhsInvLaunch &a, int n_blocks, cudaStream_t
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
+  const int64_t n_blocks = (a.n_events + a.tile - 1) / a.tile * (a.group_hi - a.group_lo);
+  const unsigned grid = (unsigned)(n_blocks < 0x7fffffff ? n_blocks : 0x7fffffff);
   if (per_event)
-    phs_inverse_kernel<true, false><<<n_blocks, PHS_INV_BLOCK, smem, stream>>>(a);
+    phs_inverse_kernel<true, false><<<grid, PHS_INV_BLOCK, smem, stream>>>(a);
   else if (lab_rows)
-    phs_inverse_kernel<false, true><<<n_blocks, PHS_INV_BLOCK, smem, stream>>>(a);
+    phs_inverse_kernel<false, true><<<grid, PHS_INV_BLOCK, smem, stream>>>(a);
   else
-    phs_inverse_kernel<false, false><<<n_blocks, PHS_INV_BLOCK, smem, stream>>>(a);
+    phs_inverse_kernel<false, false><<<grid, PHS_INV_BLOCK, smem, stream>>>(a);
   return cudaGetLastError();
 }
 

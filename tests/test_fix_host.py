@@ -156,3 +156,70 @@ def test_register_constant_forms_and_division(tmp_path):
                                                           check=True).stdout.split())
     assert form == 0 and scale == 0
     assert div <= n // 1000
+
+
+INVERSE_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <random>
+#include "phs_fix.h"
+typedef long double Q;
+static double ulp(double a) { a = std::fabs(a); return std::nextafter(a, INFINITY) - a; }
+static double err(double got, Q want) { return std::fabs((double)((Q)got - want)) / ulp((double)want); }
+static bool close(double a, double b) { return a == b || (a != a && b != b) || std::fabs(a - b) <= ulp(b); }
+int main() {
+  std::mt19937_64 g(3);
+  std::uniform_real_distribution<double> U(0, 1);
+  double at = 0, small = 0, lg = 0, near1 = 0, sc = 0;
+  for (int i = 0; i < 400000; i++) {
+    const double a = 2 * M_PI * U(g), r = std::ldexp(1 + U(g), (int)(U(g) * 40) - 20);
+    double y = r * std::sin(a), x = r * std::cos(a);
+    if (i % 3 == 1) y = std::ldexp(y, -(int)(U(g) * 40));
+    if (i % 3 == 2) x = std::ldexp(x, -(int)(U(g) * 40));
+    const Q w = atan2l((Q)y, (Q)x);
+    double &e = fabsl(w) > 0.0625L ? at : small;
+    e = std::fmax(e, err(fx_atan2(y, x), w));
+    const double v = i % 2 ? std::ldexp(1 + U(g), (int)(U(g) * 200) - 100)
+                           : 1 + std::ldexp(2 * U(g) - 1, -(int)(U(g) * 50) - 1);
+    const Q l = logl((Q)v);
+    if (l != 0) {
+      double &f = v > 0.71 && v < 1.41 ? near1 : lg;
+      f = std::fmax(f, err(fx_log(v), l));
+    }
+    const double phi = i % 2 ? 2 * M_PI * U(g) : std::ldexp(U(g), -(int)(U(g) * 50));
+    double s, c;
+    fx_sincos(phi, s, c);
+    sc = std::fmax(sc, std::fabs((double)((Q)s - sinl((Q)phi))) - ulp(s) / 2);
+    sc = std::fmax(sc, std::fabs((double)((Q)c - cosl((Q)phi))) - ulp(c) / 2);
+  }
+  int bad = 0;
+  const double e[] = {0.0, -0.0, 1.0, -1.0, 0x1p-9, 0x1.fffffffffffffp-10, 1e-300, -1e300, 5e-324, INFINITY, -INFINITY, NAN};
+  for (double a : e)
+    for (double b : e) bad += !close(fx_atan2(a, b), std::atan2(a, b));
+  for (double a : {1.0, 2.0, 0.5, 0.0, -1.0, (double)INFINITY, (double)NAN, 5e-324, 1.4142135623730951, 1.414213562373095,
+                   0.7071067811865475, 0.7071067811865476, 1.0000000000000002, 0.9999999999999999})
+    bad += !close(fx_log(a), std::log(a));
+  double s, c;
+  for (double a : {0.0, 7.999, 8.0, -1.0, 1e6}) {
+    fx_sincos(a, s, c);
+    bad += !close(s, std::sin(a)) || !close(c, std::cos(a));
+  }
+  printf("%.6f %.6f %.6f %.6f %.3e %d\n", at, small, lg, near1, sc, bad);
+}
+"""
+
+
+def test_inverse_functions(tmp_path):
+    """atan2, log and sin / cos of an angle in radians against long double, at their edges against
+    the C library: half an ulp and the fixed point's 2^-59 where the result is large, an ulp at
+    small angles (2^-62 absolute) and where e log 2 is added with a second rounding."""
+    src, exe = tmp_path / "i.cpp", tmp_path / "i"
+    src.write_text(INVERSE_DRIVER)
+    subprocess.run(["g++", "-O2", "-std=gnu++17", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True)
+    at, small, lg, near1, sc, bad = subprocess.run([str(exe)], capture_output=True, text=True,
+                                                   check=True).stdout.split()
+    assert float(at) <= 0.55 and float(small) <= 1.05
+    assert float(near1) <= 0.55 and float(lg) <= 1.05
+    assert float(sc) <= 2.0 ** -58
+    assert int(bad) == 0
