@@ -143,7 +143,6 @@ struct Segments {
   DevBuf dev;
   std::vector<PhsSegment> uploaded;  // content of dev
   DevBuf work;                       // chunk counter of the compacting kernels
-  DevBuf exact_n, exact_q, exact_t;  // FP32-pair launches: the exact-path queues
   DevBuf pass_n, pass_t, pass_q;     // FP32-pair split form: pre-test survivors per segment
   int64_t n_tiles = 0;
   int64_t n_chunks = 0;
@@ -151,9 +150,6 @@ struct Segments {
   void release() {
     dev.release();
     work.release();
-    exact_n.release();
-    exact_q.release();
-    exact_t.release();
     pass_n.release();
     pass_t.release();
     pass_q.release();
@@ -214,7 +210,7 @@ int attach_segments(Segments &S, PhsLaunch &a, cudaStream_t stream) {
     a.ev_len = std::max(a.ev_len, g.ev_begin + g.ev_count);
   }
   a.segments = nullptr;
-  if (int rc = S.work.reserve(2 * sizeof(unsigned long long))) return rc;
+  if (int rc = S.work.reserve(sizeof(unsigned long long))) return rc;
   a.work = S.work.as<unsigned long long>();
   if (S.host.size() <= PHS_INLINE_SEGS) {
     std::copy(S.host.begin(), S.host.end(), a.seg_inline);
@@ -305,9 +301,6 @@ int launch_tuned(int &variant, int n_variants, int64_t n_events, cudaStream_t st
   return PHS_OK;
 }
 
-// FP32-pair launch: the float-float kernel, then the exact FP64 path over the events it
-// queued (a handful of blocks: they are about 0.1 % of the events, or all events of a
-// channel without a float-float form).
 // Scratch of the split forms: pre-test survivors per segment, their claim numbering and
 // their indices (n_tiles * 32 entries).
 int attach_pass_buffers(Segments &S, PhsLaunch &a) {
@@ -324,17 +317,7 @@ int attach_pass_buffers(Segments &S, PhsLaunch &a) {
 
 int launch_ff_tuned(int &variant, Segments &S, PhsLaunch a, int device, int depth,
                     int64_t n_events, cudaStream_t st) {
-  const size_t n_seg = (size_t)std::max(a.n_segments, 1);
-  if (int rc = S.exact_n.reserve(n_seg * sizeof(unsigned int))) return rc;
-  if (int rc = S.exact_t.reserve((n_seg + 1) * sizeof(int64_t))) return rc;
-  if (int rc = S.exact_q.reserve((size_t)std::max<int64_t>(a.n_tiles, 1) * 32 * sizeof(int32_t)))
-    return rc;
   if (int rc = attach_pass_buffers(S, a)) return rc;
-  a.exact_work = a.work + 1;  // attach_segments reserved two counters
-  a.exact_count = S.exact_n.as<unsigned int>();
-  a.exact_queue = S.exact_q.as<int32_t>();
-  a.exact_tile = S.exact_t.as<int64_t>();
-  const int exact_grid = sm_count(device) * 4;
   // per-event beams: the float-float one pass at either register budget (variants 0, 1;
   // the pre-test needs uniform constants), or the FP64 compacting kernel (2, 3: FP64
   // variants 1, 2), whose FP64 results meet this precision's bar too and which wins where
@@ -343,18 +326,17 @@ int launch_ff_tuned(int &variant, Segments &S, PhsLaunch a, int device, int dept
   return launch_tuned(variant, per_event ? 4 : PHS_FF_VARIANTS, n_events, st, [&](int v) {
     if (per_event && v >= 2) {
       const int f64v = v >= 4 ? 1 + (v & 1) : v - 1;
-      cudaError_t e = cudaMemsetAsync(a.work, 0, 2 * sizeof(unsigned long long), st);
+      cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
       if (e == cudaSuccess)
         e = phs_launch_forward_f64(a, grid_for(a.n_tiles, device, depth, true, f64v), f64v, st);
       return e;
     }
     if (per_event) v &= 1;
-    cudaError_t e = cudaMemsetAsync(a.exact_count, 0, (size_t)a.n_segments * sizeof(unsigned int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.work, 0, 2 * sizeof(unsigned long long), st);
+    cudaError_t e = cudaSuccess;
+    if (v >= 2) e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
     if (e == cudaSuccess && v >= 4)
       e = cudaMemsetAsync(a.pass_count, 0, (size_t)a.n_segments * sizeof(unsigned int), st);
     if (e == cudaSuccess) e = phs_launch_forward_ff(a, grid_for_ff(a.n_tiles, device, depth, v), v, st);
-    if (e == cudaSuccess) e = phs_launch_forward_exact(a, exact_grid, st);
     return e;
   });
 }
@@ -370,7 +352,7 @@ int launch_f64_tuned(int &variant, Segments &S, PhsLaunch a, int device, int dep
     // one-pass form of the same block shape
     if (per_event && v >= PHS_F64_VARIANTS_PER_EVENT) v -= 4;
     cudaError_t e = cudaSuccess;
-    if (a.work) e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
+    if (v != 0 && v != 3 && v != 4) e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
     if (e == cudaSuccess && v >= PHS_F64_VARIANTS_PER_EVENT)
       e = cudaMemsetAsync(a.pass_count, 0, (size_t)a.n_segments * sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;

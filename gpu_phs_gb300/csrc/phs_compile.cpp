@@ -363,6 +363,8 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
   out.s = split(in.sqrts * in.sqrts);
   out.lab_bg = split(in.lab_bg);
   out.lab_gamma = split(in.lab_gamma);
+  out.f0 = split(in.f0);
+  out.inv_sqrts = split(in.inv_sqrts);
   out.m_tot = split(in.m_tot);
   out.volume = in.volume;
   for (int v = 0; v < in.n_visits; v++) {
@@ -401,11 +403,10 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
     F.carry = V.carry;
     F.push = V.push;
     F.self_root = V.self_root;
-    F.both_leaves = V.both_leaves;
-    F.parent_root = V.parent_root;
+    F.massless = V.massless;
+    F.kind = V.kind;
     F.b0 = split(V.b0);
     F.b1 = split(V.b1);
-    F.self_m_max = split(V.self_m_max);
     PhsTestVisit &P = out.test[v];
     for (int j = 0; j < 2; j++) {
       const PhsChildFF &G = F.child[j];

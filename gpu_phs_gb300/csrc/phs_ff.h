@@ -173,6 +173,30 @@ FF_FN ff ff_dot2(ff a0, ff b0, ff a1, ff b1) {
   return fast_two_sum(s.hi, f_add(e, s.lo));
 }
 
+// The same without the final normalization (|lo| may reach a few ulps of hi): for a value that
+// is widened to a double next.
+FF_FN ff ff_dot2_raw(ff a0, ff b0, ff a1, ff b1) {
+  const ff p0 = two_prod(a0.hi, b0.hi), p1 = two_prod(a1.hi, b1.hi);
+  float e = f_fma(a0.hi, b0.lo, f_fma(a0.lo, b0.hi, p0.lo));
+  e = f_add(e, f_fma(a1.hi, b1.lo, f_fma(a1.lo, b1.hi, p1.lo)));
+  const ff s = two_sum(p0.hi, p1.hi);
+  return ff_make(s.hi, f_add(e, s.lo));
+}
+
+// a0 b0 + a1 b1 + c, not normalized.
+FF_FN ff ff_dot2_add_raw(ff a0, ff b0, ff a1, ff b1, ff c) {
+  const ff p0 = two_prod(a0.hi, b0.hi), p1 = two_prod(a1.hi, b1.hi);
+  float e = f_fma(a0.hi, b0.lo, f_fma(a0.lo, b0.hi, p0.lo));
+  e = f_add(e, f_fma(a1.hi, b1.lo, f_fma(a1.lo, b1.hi, p1.lo)));
+  e = f_add(e, c.lo);
+  ff s = two_sum(p0.hi, p1.hi);
+  e = f_add(e, s.lo);
+  s = two_sum(s.hi, c.hi);
+  return ff_make(s.hi, f_add(e, s.lo));
+}
+
+FF_FN ff ff_normalize(ff a) { return fast_two_sum(a.hi, a.lo); }
+
 FF_FN ff ff_dot3(ff a0, ff b0, ff a1, ff b1, ff a2, ff b2) {
   const ff p0 = two_prod(a0.hi, b0.hi), p1 = two_prod(a1.hi, b1.hi);
   const ff p2 = two_prod(a2.hi, b2.hi);
@@ -366,8 +390,8 @@ FF_FN void ff_sincos2pi(ff x, const FFTables &T, ff &s, ff &c) {
   int k = ((int)kf) & 63;
   float4 t = T.trig[k];
   ff sk = ff_make(t.x, t.y), ck = ff_make(t.z, t.w);
-  s = ff_add(ff_mul(sk, cf), ff_mul(ck, sf));
-  c = ff_sub(ff_mul(ck, cf), ff_mul(sk, sf));
+  s = ff_dot2(sk, cf, ck, sf);
+  c = ff_dot2(ck, cf, ff_neg(sk), sf);
 }
 
 // sin and cos of z (radians), |z| <= pi/2 + pi/64: Cody-Waite reduction by k pi/32.
@@ -381,8 +405,8 @@ FF_FN void ff_sincos(ff z, const FFTables &T, ff &s, ff &c) {
   int k = ((int)kf) & 63;
   float4 t = T.trig[k];
   ff sk = ff_make(t.x, t.y), ck = ff_make(t.z, t.w);
-  s = ff_add(ff_mul(sk, cf), ff_mul(ck, sf));
-  c = ff_sub(ff_mul(ck, cf), ff_mul(sk, sf));
+  s = ff_dot2(sk, cf, ck, sf);
+  c = ff_dot2(ck, cf, ff_neg(sk), sf);
 }
 
 // tan(z) for |z| < pi/2 (radians).

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
         a, q,
         [&](const PhsSegment &sg, int64_t loc) { return phs_ok_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem); },
         [&](int, const PhsSegment &sg, int64_t loc) {
-          phs_event_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem);
+          if (loc >= 0) phs_event_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem);
         });
   } else {
     for (int64_t tile = warp0; tile < a.n_tiles; tile += n_warps) {
@@ -54,42 +54,6 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
       if (local >= seg.ev_count) continue;
       phs_event_f64<PER_EVENT, BLOCK>(a, k, seg, local, smem);
     }
-  }
-}
-
-// The exact FP64 path for the events the FP32-pair kernel queued, per segment
-// (a.exact_queue from tile_begin * 32 on, a.exact_count entries, claims numbered by
-// a.exact_tile).  Those are events within 1e-5 of a kinematic limit, and all events of
-// channels whose mappings or boosts have no float-float form; keeping their FP64 code out
-// of the FP32-pair kernel keeps that kernel's body small.  Warps claim 32 events of one
-// segment (a.exact_work counts the claims), so each runs one channel's program; the counts
-// are read on the device, so the launch can sit in a CUDA graph behind the FP32-pair one.
-template <bool PER_EVENT>
-__global__ void __launch_bounds__(PHS_FWD_BLOCK, 4)
-    phs_forward_exact_kernel(const __grid_constant__ PhsLaunch a) {
-  extern __shared__ double smem[];
-  const FxRegs k = fx_regs();
-  const int lane = threadIdx.x & 31;
-  const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
-  const int64_t n_claims = a.exact_tile[a.n_segments];
-  for (;;) {
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(a.exact_work, 1ull);
-    const int64_t t = (int64_t)__shfl_sync(0xffffffffu, c, 0);
-    if (t >= n_claims) break;
-    int lo = 0, hi = a.n_segments - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.exact_tile[mid] <= t) lo = mid; else hi = mid - 1;
-    }
-    const PhsSegment seg = segs[lo];
-    const int64_t idx = (t - a.exact_tile[lo]) * 32 + lane;
-    if (idx >= (int64_t)a.exact_count[lo]) continue;
-    // the queue slot lies in the segment's run of a.n_tiles * 32 entries, the event in the segment
-    if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
-        !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
-      continue;
-    phs_event_f64<PER_EVENT>(a, k, seg, a.exact_queue[seg.tile_begin * 32 + idx], smem);
   }
 }
 
@@ -318,21 +282,6 @@ cudaError_t phs_launch_forward_f64(const PhsLaunch &a, int n_blocks, int variant
   }
   return a.E1 && a.E2 ? launch_f64<true>(a, n_blocks, variant, stream)
                       : launch_f64<false>(a, n_blocks, variant, stream);
-}
-
-cudaError_t phs_launch_forward_exact(const PhsLaunch &a, int n_blocks, cudaStream_t stream) {
-  if (a.n_tiles <= 0) return cudaSuccess;
-  cudaError_t e = phs_launch_count_scan(a.exact_count, a.exact_tile, a.n_segments, stream);
-  if (e != cudaSuccess) return e;
-  const size_t smem = phs_forward_smem_bytes(a.stack_depth, PHS_FWD_BLOCK);
-  e = allow_smem(a.E1 && a.E2 ? (const void *)phs_forward_exact_kernel<true>
-                              : (const void *)phs_forward_exact_kernel<false>, smem);
-  if (e != cudaSuccess) return e;
-  if (a.E1 && a.E2)
-    phs_forward_exact_kernel<true><<<n_blocks, PHS_FWD_BLOCK, smem, stream>>>(a);
-  else
-    phs_forward_exact_kernel<false><<<n_blocks, PHS_FWD_BLOCK, smem, stream>>>(a);
-  return cudaGetLastError();
 }
 
 // SMs of the current device (grid caps of the grid-stride kernels below).

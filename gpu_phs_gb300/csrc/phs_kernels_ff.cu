@@ -9,10 +9,17 @@
 // decided in float-float only when the margins |m - m1 - m2| and |m_max - m| exceed
 // 1e-5 of the mass (and msq is not within 1e-10 s of zero).  Otherwise -- and for channels
 // with STEP mappings or friend boosts, which have no float-float form -- the event is
-// queued for the exact FP64 path (phs_event_f64.cuh, launched behind this kernel by
-// phs_launch_forward_exact), which also keeps p_decay near threshold in FP64.
+// queued for the exact FP64 path (phs_event_f64.cuh; ExactQueue below), which also keeps
+// p_decay near threshold in FP64.
 // The Kallen function is evaluated in factored form, (m-m1-m2)(m+m1+m2)(m-m1+m2)(m+m1-m2),
 // which keeps its relative accuracy close to threshold.
+//
+// The walk waits on FP32 latencies (16 warps a SM at 128 registers, issue slots half used), so
+// fewer dependent operations are what counts: frame steps and daughter pairs in the FP64 walk's
+// forms and the energies from the masses took 1e6 tt events from 372 to 357 us (7.9 to 7.0
+// thousand instructions a warp), and the error of the momenta from 2.1e-14 to 1.2e-14.  Five or
+// six blocks a SM (96, 80 registers, spills) and the mappings of both daughters unrolled were
+// slower.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -22,7 +29,7 @@
 #include "phs_ff.h"
 #include "phs_program.h"
 
-#define PHS_FF_STATE 40   // floats per saved frame: L[16], msq, m, p, m_max as pairs
+#define PHS_FF_STATE 40   // floats per saved frame: L[16], msq, m, p, E as pairs
 #define PHS_FF_MARGIN 1e-5f     // kinematic margins decided in float-float
 #define PHS_FF_MSQ_ZERO 1e-10f  // |msq| below this fraction of s takes the exact path
 #define PHS_FF_TEST_MIN_BLOCKS 8  // resident blocks per SM of the stand-alone pre-test kernel
@@ -111,7 +118,8 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChil
   return child_var(C, C64, sqrts64, m_tot64, 1.0 / s64);
 }
 
-// msq from x in float-float; returns false when the event must take the exact path.
+// msq from x in float-float; returns false when the event must take the exact path.  f: the
+// mapping's factor without its constant part a2 (as map_msq).
 // x arrives as a float-float pair truncated from the double, so x < 0.5 is decided on its
 // high part exactly as the reference decides it on the double.
 __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &cv, double xd,
@@ -120,7 +128,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
   switch (C.map_id) {
     case PHS_MAP_NO:
       msq = ff_add(ld(C.msq_min), ff_mul(x, ff_sub(cv.msq_max, ld(C.msq_min))));
-      f = cv.a2;
+      f = ff_from_float(1.0f);
       return true;
     case PHS_MAP_SCHANNEL: {
       // z = (1-x) a0 + x a1; next to +-pi/2, tan z = -+cot(pi/2 -+ z) with pi/2 -+ z formed
@@ -137,7 +145,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
       ff t = ff_div_fast(cot ? cw : sw, cot ? sw : cw);
       if (ls) t = ff_neg(t);
       msq = ff_add(ld(C.m2), ff_mul(ld(C.mw), t));
-      f = ff_mul(cv.a2, ff_add_f(ff_sqr(t), 1.0f));
+      f = ff_add_f(ff_sqr(t), 1.0f);
       return true;
     }
     case PHS_MAP_COLLINEAR:
@@ -151,7 +159,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
       const ff msq1 = ff_mul(ld(C.a0), ff_exp(ff_mul(upper ? ff_one_minus_double_int(xd) : x, cv.a1), T));
       msq = upper ? ff_add(ff_sub(ld(C.a0), msq1), cv.msq_max)
                   : ff_add(ff_sub(msq1, ld(C.a0)), ld(C.msq_min));
-      f = ff_mul(cv.a2, msq1);
+      f = msq1;
       return true;
     }
   }
@@ -169,10 +177,40 @@ __device__ __forceinline__ double widen(ff a) {
 __device__ __forceinline__ ff ff_twice(ff a) { return ff_make(f_add(a.hi, a.hi), f_add(a.lo, a.lo)); }
 __device__ __forceinline__ ff ff_half(ff a) { return ff_make(f_mul(a.hi, 0.5f), f_mul(a.lo, 0.5f)); }
 
+// A leaf's momentum row, from pairs that need not be normalized.
+template <bool INT>
+__device__ __forceinline__ void put_momentum_ff(double *out, int index, int n_out, const ff q[4]) {
+  if (!phs_in(index, n_out, PHS_CHK_P)) return;
+  double2 *o = reinterpret_cast<double2 *>(out + 4 * index);
+  double d[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) d[r] = widen<INT>(INT ? ff_normalize(q[r]) : q[r]);
+  o[0] = make_double2(d[0], d[1]);
+  o[1] = make_double2(d[2], d[3]);
+}
+
+// The frame step of phs_event_f64.cuh (boost along z, then the two rotations) in float-float.
+struct StepFF {
+  ff bg, ga, cp, sp, ct, st;
+};
+template <bool Z0, bool Z2>
+__device__ __forceinline__ void frame_row_ff(const StepFF &t, ff *l) {
+  const ff n0 = Z0 ? ff_mul(l[3], t.bg) : ff_dot2(l[0], t.ga, l[3], t.bg);
+  const ff z = Z0 ? ff_mul(l[3], t.ga) : ff_dot2(l[0], t.bg, l[3], t.ga);
+  const ff u = Z2 ? ff_mul(t.cp, l[1]) : ff_dot2(l[1], t.cp, l[2], t.sp);
+  const ff w = Z2 ? ff_mul(ff_neg(t.sp), l[1]) : ff_dot2(l[2], t.cp, l[1], ff_neg(t.sp));
+  l[0] = n0;
+  l[1] = ff_dot2(t.ct, u, ff_neg(t.st), z);
+  l[2] = w;
+  l[3] = ff_dot2(t.st, u, t.ct, z);
+}
+
 // One event in float-float.  Returns false if it must be recomputed on the exact path
 // (outputs written so far are then overwritten).  PER_EVENT: beam energies a.E1/a.E2 per
 // event; the constants that depend on sqrt(s) come from FP64 per event (as the FP64 path
-// computes them) and the walk stays in float-float.
+// computes them) and the walk stays in float-float.  The walk has the FP64 walk's forms
+// (phs_event_f64.cuh): frame steps by kind, two outgoing daughters as vectors through the
+// parent's frame, massless daughters without square roots or reciprocals.
 template <bool PER_EVENT = false>
 __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegment &seg,
                                              int64_t local, const FFTables &T, float *fst) {
@@ -191,7 +229,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 
   // beams: the channel's, or this event's (phs_event_f64's expressions)
   ff sqrts_f = ld(ch.sqrts), s_f = ld(ch.s), lab_bg = ld(ch.lab_bg), lab_ga = ld(ch.lab_gamma);
-  bool lab = ch.lab != 0;
+  const bool lab = PER_EVENT || ch.lab != 0;
   double sqrts64 = 0.0, s64 = 0.0;
   ff inv_s_f = zero;
   if (PER_EVENT) {
@@ -205,7 +243,6 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
     sqrts_f = ff_twice(r);
     s_f = ff_sqr(sqrts_f);
     inv_s_f = ff_recip_fast(s_f);
-    lab = E1 != E2;
     lab_bg = ff_div_fast(ff_sub(e1, e2), sqrts_f);
     lab_ga = ff_sqrt_fast(ff_add_f(ff_sqr(lab_bg), 1.0f));
   }
@@ -215,76 +252,101 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
   ff L[16];
 #pragma unroll
   for (int i = 0; i < 16; i++) L[i] = zero;
-  L[0] = lab ? lab_ga : one;
-  L[5] = one;
-  L[10] = one;
-  L[15] = L[0];
-  L[3] = lab ? lab_bg : zero;
-  L[12] = L[3];
-  ff msq_b = s_f, m_b = sqrts_f, p_b = zero, mmax_b = sqrts_f;
-  ff factor = one;
+  ff msq_b = s_f, m_b = sqrts_f, p_b = zero, E_b = sqrts_f;
+  ff factor = PER_EVENT ? one : ld(ch.f0);
   bool ok = true;
   int sp = 0;
 
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisitFF &V = ch.visit[v];
-    ff cmsq[2], cm[2], cmax[2];
-#pragma unroll
+    ff cmsq[2] = {ld(V.child[0].msq_leaf), ld(V.child[1].msq_leaf)};
+    ff cm[2] = {ld(V.child[0].m_leaf), ld(V.child[1].m_leaf)};
+    bool exact = false;
+    // (not unrolled: the mapping code of one daughter serves both)
+#pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChildFF &C = V.child[j];
-      if (!C.internal) {
-        cmsq[j] = ld(C.msq_leaf);
-        cm[j] = ld(C.m_leaf);
-        cmax[j] = zero;
+      if (!C.internal) continue;
+      ff f = one, mq = zero;
+      const ChildVar cv = PER_EVENT
+          ? child_var(C, a.channels[seg.channel].visit[v].child[j], sqrts_f, inv_s_f, ld(ch.m_tot),
+                      sqrts64, a.channels[seg.channel].m_tot)
+          : child_var(C);
+      if (!map_msq_ff(C, cv, xrow_at(xe, C.x_msq, seg.x_stride), T, mq, f)) exact = true;
+      if (PER_EVENT) factor = ff_mul(factor, cv.a2);
+      if (C.map_id != PHS_MAP_NO) factor = ff_mul(factor, f);
+      if (msq_near_zero(mq, s_scale)) exact = true;
+      if (mq.hi < 0.0f) {  // the reference takes sqrt of a negative: not ok
+        ok = false;
+        mq = zero;
+      }
+      const ff mj = ff_sqrt_fast(mq);
+      // the kinematic test's upper bound m <= m_max, decided here only away from it
+      const ff dhi = ff_sub(cv.m_max, mj);
+      if (near_zero(dhi, cv.m_max.hi)) exact = true;
+      ok = ok && dhi.hi > 0.0f;
+      if (j == 0) {
+        cmsq[0] = mq;
+        cm[0] = mj;
       } else {
-        ff f;
-        const ChildVar cv = PER_EVENT
-            ? child_var(C, a.channels[seg.channel].visit[v].child[j], sqrts_f, inv_s_f, ld(ch.m_tot),
-                        sqrts64, a.channels[seg.channel].m_tot)
-            : child_var(C);
-        if (!map_msq_ff(C, cv, xrow_at(xe, C.x_msq, seg.x_stride), T, cmsq[j], f)) return false;
-        factor = ff_mul(factor, f);
-        if (msq_near_zero(cmsq[j], s_scale)) return false;
-        if (cmsq[j].hi < 0.0f) {  // the reference takes sqrt of a negative: not ok
-          ok = false;
-          cmsq[j] = zero;
-        }
-        cm[j] = ff_sqrt_fast(cmsq[j]);
-        cmax[j] = cv.m_max;
+        cmsq[1] = mq;
+        cm[1] = mj;
       }
     }
-    // kinematic test at the visited branch, decided here only away from its limits
-    const ff msum = ff_add(cm[0], cm[1]);
-    const ff dlo = ff_sub(m_b, msum);
+    if (exact) return false;
+    // the test's lower bound m > m1 + m2, likewise
+    const int massless = V.massless;
+    const ff msum = massless == 0 ? ff_add(cm[0], cm[1]) : massless == 3 ? zero : ffsel(massless & 1, cm[1], cm[0]);
+    const ff dlo = massless == 3 ? m_b : ff_sub(m_b, msum);
     if (near_zero(dlo, m_b.hi)) return false;
     ok = ok && dlo.hi > 0.0f;
-    if (!V.self_root) {
-      const ff dhi = ff_sub(mmax_b, m_b);
-      if (near_zero(dhi, mmax_b.hi)) return false;
-      ok = ok && dhi.hi > 0.0f;
+    int kind = V.kind;
+    if (lab)
+      kind = kind == PHS_KIND_ROOT ? PHS_KIND_ROOT_LAB
+             : kind == PHS_KIND_FIRST ? PHS_KIND_FIRST_LAB
+             : kind == PHS_KIND_LEAVES_FIRST ? PHS_KIND_LEAVES : kind;
+    const bool pair = kind == PHS_KIND_LEAVES || kind == PHS_KIND_LEAVES_FIRST;
+    // Kallen function, factored; one reciprocal of m serves p_decay, the factor, the energies
+    // and the boost
+    ff rm = zero, pc, ce0, ce1;
+    if (massless == 3) {
+      pc = ce0 = ce1 = ff_half(m_b);
+      if (!pair && m_b.hi > 0.0f) rm = ff_recip_fast(m_b);   // n_out = 2
+    } else {
+      rm = !PER_EVENT && V.self_root ? ld(ch.inv_sqrts) : (m_b.hi > 0.0f ? ff_recip_fast(m_b) : zero);
+      ff sl;
+      if (massless != 0) {
+        sl = ff_mul(dlo, ff_add(m_b, msum));               // m^2 - m_j^2
+        if (!(sl.hi > 0.0f)) sl = zero;
+      } else {
+        const ff mdiff = ff_sub(cm[0], cm[1]);
+        ff lda = ff_mul(ff_mul(dlo, ff_add(m_b, msum)),
+                        ff_mul(ff_sub(m_b, mdiff), ff_add(m_b, mdiff)));
+        if (!(lda.hi > 0.0f)) lda = zero;
+        sl = ff_sqrt_fast(lda);
+      }
+      const ff slrm = ff_mul(sl, rm);
+      pc = ff_half(slrm);                                  // sqrt(lambda) / (2 m)
+      factor = ff_mul(factor, ff_mul(slrm, rm));           // sqrt(lambda) / m^2
+      if (massless == 0) {
+        const ff dc = ff_sub(cmsq[0], cmsq[1]), hm = ff_half(rm);
+        ce0 = ff_mul(ff_add(msq_b, dc), hm);
+        ce1 = ff_mul(ff_sub(msq_b, dc), hm);
+      } else {
+        const ff eo = ff_sub(m_b, pc);
+        ce0 = ffsel(massless & 1, pc, eo);
+        ce1 = ffsel(massless & 1, eo, pc);
+      }
     }
-    // Kallen function, factored; one reciprocal of m serves p_decay, the factor and bg
-    const ff mdiff = ff_sub(cm[0], cm[1]);
-    ff lda = ff_mul(ff_mul(dlo, ff_add(m_b, msum)),
-                    ff_mul(ff_sub(m_b, mdiff), ff_add(m_b, mdiff)));
-    if (!(lda.hi > 0.0f)) lda = zero;
-    const ff sl = ff_sqrt_fast(lda);
-    const ff rm = m_b.hi > 0.0f ? ff_recip_fast(m_b) : zero;
-    const ff slrm = ff_mul(sl, rm);
-    const ff pc = ff_half(slrm);                       // sqrt(lambda) / (2 m)
-    factor = ff_mul(factor, ff_mul(slrm, rm));         // sqrt(lambda) / m^2
 
-    // rotation + boost of the visited branch
-    const ff bg = ff_mul(p_b, rm);
-    const ff ga = ff_sqrt_fast(ff_add_f(ff_sqr(bg), 1.0f));
-    ff sphi, cphi;
-    ff_sincos2pi(ff_from_double_int(xrow_at(xe, V.x_phi, seg.x_stride)), T, sphi, cphi);
+    // the decay angles
+    StepFF t;
+    ff_sincos2pi(ff_from_double_int(xrow_at(xe, V.x_phi, seg.x_stride)), T, t.sp, t.cp);
     const double xctd = xrow_at(xe, V.x_ct, seg.x_stride);
     const ff xct = ff_from_double_int(xctd);
-    ff ct, st, fct;
     if (V.ct_class == PHS_CT_COLLINEAR) {
-      ff b0 = ld(V.b0), b1 = ld(V.b1);
+      ff b0 = ld(V.b0), b1 = ld(V.b1), fct;
       if (PER_EVENT) {
         const double m = a.channels[seg.channel].visit[v].m;
         const double b0d = dmul(m, m) / s64;
@@ -293,121 +355,111 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       }
       const bool lower = xct.hi < 0.5f;
       const ff tmp = ff_mul(b0, ff_exp(ff_mul(ff_twice(lower ? xct : ff_one_minus_double_int(xctd)), b1), T));
-      ct = lower ? ff_add_f(ff_sub(tmp, b0), -1.0f) : ff_add_f(ff_sub(b0, tmp), 1.0f);
-      if (ct.hi >= -1.0f && ct.hi <= 1.0f) {
+      t.ct = lower ? ff_add_f(ff_sub(tmp, b0), -1.0f) : ff_add_f(ff_sub(b0, tmp), 1.0f);
+      if (t.ct.hi >= -1.0f && t.ct.hi <= 1.0f) {
         // 1 - ct^2 = (1 - ct)(1 + ct), each factor without cancellation
-        st = ff_sqrt_fast(ff_mul(ff_sub(one, ct), ff_add_f(ct, 1.0f)));
+        t.st = ff_sqrt_fast(ff_mul(ff_sub(one, t.ct), ff_add_f(t.ct, 1.0f)));
         fct = ff_mul(tmp, b1);
       } else {
-        ct = one;
-        st = zero;
+        t.ct = one;
+        t.st = zero;
         fct = zero;
       }
+      factor = ff_mul(factor, fct);   // the uniform map's is 1
     } else {
-      // tmp = 2(1 - x), ct = 1 - tmp, st = sqrt(tmp (2 - tmp)) = 2 sqrt((1-x) x)
-      const ff u = ff_one_minus_double_int(xctd);
-      ct = ff_sub(xct, u);
-      st = ff_twice(ff_sqrt_fast(ff_mul(u, xct)));
-      fct = one;
-    }
-    if (V.ct_class == PHS_CT_COLLINEAR) factor = ff_mul(factor, fct);   // uniform: 1
-    const ff e03 = ff_mul(bg, ct), e12 = ff_neg(sphi), e13 = ff_mul(st, cphi), e22 = cphi;
-    const ff e23 = ff_mul(st, sphi), e33 = ff_mul(ga, ct);
-    // the entries of L1 that only the frame's columns 1 and 2 read: formed in the branches
-    // that write those (a leaf-only visit writes columns 0 and 3 only)
-    const auto col12 = [&](ff &e01, ff &e11, ff &e21, ff &e31) {
-      e01 = ff_neg(ff_mul(bg, st));
-      e11 = ff_mul(ct, cphi);
-      e21 = ff_mul(ct, sphi);
-      e31 = ff_neg(ff_mul(ga, st));
-    };
-
-    if (V.self_root && !lab) {
-      ff e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-      L[0] = ga;   L[1] = e01;  L[2] = zero;  L[3] = e03;
-      L[4] = zero; L[5] = e11;  L[6] = e12;   L[7] = e13;
-      L[8] = zero; L[9] = e21;  L[10] = e22;  L[11] = e23;
-      L[12] = bg;  L[13] = e31; L[14] = zero; L[15] = e33;
-    } else if (PER_EVENT && V.self_root) {
-      // (per-event beams, where nearly every event has a lab boost; the uniform-beam kernels
-      // keep the general product, which leaves their registers to the common case)
-      // the parent frame is the lab boost B_z(lab_bg): rows 1 and 2 are unit rows
-      ff e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-      const ff g0 = L[0], b0 = L[3];
-      L[0] = ff_dot2(g0, ga, b0, bg);   L[1] = ff_dot2(g0, e01, b0, e31);
-      L[2] = zero;                      L[3] = ff_dot2(g0, e03, b0, e33);
-      L[4] = zero; L[5] = e11;  L[6] = e12;   L[7] = e13;
-      L[8] = zero; L[9] = e21;  L[10] = e22;  L[11] = e23;
-      L[12] = ff_dot2(b0, ga, g0, bg);  L[13] = ff_dot2(b0, e01, g0, e31);
-      L[14] = zero;                     L[15] = ff_dot2(b0, e03, g0, e33);
-    } else if (V.parent_root && !lab) {
-      // the parent frame is the root's rotation (its bg is 0 and its gamma 1): row 0 is
-      // (1, 0, 0, 0) and L[4], L[8], L[12], L[14] are 0, so half the products drop out
-      ff e01 = zero, e11 = zero, e21 = zero, e31 = zero;
-      if (!V.both_leaves) col12(e01, e11, e21, e31);
-      L[0] = ga;   L[1] = e01;  L[2] = zero;  L[3] = e03;
-#pragma unroll
-      for (int r = 1; r < 4; r++) {
-        const ff l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        L[4 * r + 0] = ff_mul(l3, bg);
-        L[4 * r + 3] = r < 3 ? ff_dot3(l1, e13, l2, e23, l3, e33) : ff_dot2(l1, e13, l3, e33);
-        if (!V.both_leaves) {
-          L[4 * r + 1] = r < 3 ? ff_dot3(l1, e11, l2, e21, l3, e31) : ff_dot2(l1, e11, l3, e31);
-          L[4 * r + 2] = r < 3 ? ff_dot2(l1, e12, l2, e22) : ff_mul(l1, e12);
-        }
-      }
-    } else if (PER_EVENT && V.parent_root) {
-      // the root's frame with the lab boost: entries (0,2), (1,0), (2,0), (3,2) are 0
-      ff e01 = zero, e11 = zero, e21 = zero, e31 = zero;
-      if (!V.both_leaves) col12(e01, e11, e21, e31);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const ff l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        const bool edge = r == 0 || r == 3;   // l2 = 0; otherwise l0 = 0
-        L[4 * r + 0] = edge ? ff_dot2(l0, ga, l3, bg) : ff_mul(l3, bg);
-        L[4 * r + 3] = edge ? ff_dot3(l0, e03, l1, e13, l3, e33) : ff_dot3(l1, e13, l2, e23, l3, e33);
-        if (!V.both_leaves) {
-          L[4 * r + 1] = edge ? ff_dot3(l0, e01, l1, e11, l3, e31) : ff_dot3(l1, e11, l2, e21, l3, e31);
-          L[4 * r + 2] = edge ? ff_mul(l1, e12) : ff_dot2(l1, e12, l2, e22);
-        }
-      }
-    } else if (V.both_leaves) {
-      // both daughters are leaves: their momenta read the frame's columns 0 and 3 only
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const ff l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        L[4 * r + 0] = ff_dot2(l0, ga, l3, bg);
-        L[4 * r + 3] = ff_dot4(l0, e03, l1, e13, l2, e23, l3, e33);
-      }
-    } else {
-      // row r of L L1 depends on row r of L only: update in place
-      ff e01, e11, e21, e31;
-      col12(e01, e11, e21, e31);
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const ff l0 = L[4 * r], l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
-        L[4 * r + 0] = ff_dot2(l0, ga, l3, bg);
-        L[4 * r + 3] = ff_dot4(l0, e03, l1, e13, l2, e23, l3, e33);
-        L[4 * r + 1] = ff_dot4(l0, e01, l1, e11, l2, e21, l3, e31);
-        L[4 * r + 2] = ff_dot2(l1, e12, l2, e22);
-      }
+      // ct = 2x - 1, st = sqrt(2(1 - x) 2x) = 2 sqrt((1-x) x)
+      t.ct = ff_add_f(ff_twice(xct), -1.0f);
+      t.st = ff_twice(ff_sqrt_fast(ff_mul(ff_one_minus_double_int(xctd), xct)));
     }
 
-    // leaf momenta L_new (E, 0, 0, +-p)
+    if (pair) {
+      // two outgoing daughters (see phs_event_f64)
+      const ff pst = ff_mul(pc, t.st), qx = ff_mul(pst, t.cp), qy = ff_mul(pst, t.sp);
+      ff qa0, qa3, qb0, qb3;
+      if (massless == 3) {
+        const ff eh = ff_half(E_b), ph = ff_half(p_b), c0 = ff_mul(ph, t.ct), c3 = ff_mul(eh, t.ct);
+        qa0 = ff_add(eh, c0);
+        qb0 = ff_sub(eh, c0);
+        qa3 = ff_add(ph, c3);
+        qb3 = ff_sub(ph, c3);
+      } else {
+        const ff bg = ff_mul(p_b, rm), ga = ff_mul(E_b, rm), qz = ff_mul(pc, t.ct), nz = ff_neg(qz);
+        qa0 = ff_dot2(ga, ce0, bg, qz);
+        qb0 = ff_dot2(ga, ce1, bg, nz);
+        qa3 = ff_dot2(bg, ce0, ga, qz);
+        qb3 = ff_dot2(bg, ce1, ga, nz);
+      }
+      ff qa[4], qb[4];
+      if (kind == PHS_KIND_LEAVES_FIRST) {
+        // the parent's frame is the root's rotation: (1,0,0,0) (0,*,*,*) (0,*,*,*) (0,*,0,*)
+        qa[0] = qa0;
+        qb[0] = qb0;
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const PhsChildFF &C = V.child[j];
-      if (!C.internal && phs_in(C.out_index, ch.n_out, PHS_CHK_P)) {
-        const ff pj = j == 0 ? pc : ff_neg(pc);
-        const ff E = ff_sqrt_fast(ff_add(cmsq[j], ff_sqr(pj)));
-        double2 *o = reinterpret_cast<double2 *>(out + 4 * C.out_index);
-        // to double on the (otherwise idle) FP64 pipe: two exact widenings and one add
-        o[0] = make_double2(widen<PER_EVENT>(ff_dot2(L[0], E, L[3], pj)),
-                            widen<PER_EVENT>(ff_dot2(L[4], E, L[7], pj)));
-        o[1] = make_double2(widen<PER_EVENT>(ff_dot2(L[8], E, L[11], pj)),
-                            widen<PER_EVENT>(ff_dot2(L[12], E, L[15], pj)));
+        for (int r = 1; r < 4; r++) {
+          const ff l1 = L[4 * r + 1], l2 = L[4 * r + 2], l3 = L[4 * r + 3];
+          const ff w = r < 3 ? ff_dot2(l1, qx, l2, qy) : ff_mul(l1, qx);
+          qa[r] = ff_add(ff_mul(l3, qa3), w);
+          qb[r] = ff_sub(ff_mul(l3, qb3), w);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const ff l0 = L[4 * r], l3 = L[4 * r + 3];
+          const ff w = ff_dot2(L[4 * r + 1], qx, L[4 * r + 2], qy);
+          qa[r] = ff_dot2_add_raw(l0, qa0, l3, qa3, w);
+          qb[r] = ff_dot2_add_raw(l0, qb0, l3, qb3, ff_neg(w));
+        }
+      }
+      put_momentum_ff<PER_EVENT>(out, V.child[0].out_index, ch.n_out, qa);
+      put_momentum_ff<PER_EVENT>(out, V.child[1].out_index, ch.n_out, qb);
+    } else {
+      // rotation + boost of the visited branch (friend steps take the exact path)
+      if (!V.self_root) {
+        t.bg = ff_mul(p_b, rm);
+        t.ga = ff_mul(E_b, rm);
+      }
+      switch (kind) {
+        case PHS_KIND_ROOT:
+          L[0] = one;   L[1] = zero;               L[2] = zero;        L[3] = zero;
+          L[4] = zero;  L[5] = ff_mul(t.ct, t.cp); L[6] = ff_neg(t.sp); L[7] = ff_mul(t.st, t.cp);
+          L[8] = zero;  L[9] = ff_mul(t.ct, t.sp); L[10] = t.cp;       L[11] = ff_mul(t.st, t.sp);
+          L[12] = zero; L[13] = ff_neg(t.st);      L[14] = zero;       L[15] = t.ct;
+          break;
+        case PHS_KIND_ROOT_LAB:
+          L[0] = lab_ga;  L[1] = ff_neg(ff_mul(lab_bg, t.st));  L[2] = zero;         L[3] = ff_mul(lab_bg, t.ct);
+          L[4] = zero;    L[5] = ff_mul(t.ct, t.cp);            L[6] = ff_neg(t.sp); L[7] = ff_mul(t.st, t.cp);
+          L[8] = zero;    L[9] = ff_mul(t.ct, t.sp);            L[10] = t.cp;        L[11] = ff_mul(t.st, t.sp);
+          L[12] = lab_bg; L[13] = ff_neg(ff_mul(lab_ga, t.st)); L[14] = zero;        L[15] = ff_mul(lab_ga, t.ct);
+          break;
+        case PHS_KIND_FIRST:
+          L[0] = t.ga;
+          L[1] = ff_neg(ff_mul(t.st, t.bg));
+          L[2] = zero;
+          L[3] = ff_mul(t.ct, t.bg);
+          frame_row_ff<true, false>(t, L + 4);
+          frame_row_ff<true, false>(t, L + 8);
+          frame_row_ff<true, true>(t, L + 12);
+          break;
+        case PHS_KIND_FIRST_LAB:
+          frame_row_ff<false, true>(t, L);
+          frame_row_ff<true, false>(t, L + 4);
+          frame_row_ff<true, false>(t, L + 8);
+          frame_row_ff<false, true>(t, L + 12);
+          break;
+        default:
+#pragma unroll
+          for (int r = 0; r < 4; r++) frame_row_ff<false, false>(t, L + 4 * r);
+      }
+      // leaf momenta L_new (E, 0, 0, +-p) (a loop that is not unrolled, as in phs_event_f64)
+#pragma unroll 1
+      for (int j = V.child[0].internal ? (V.child[1].internal ? 2 : 1) : 0; j < 2; j++) {
+        const PhsChildFF &C = V.child[j];
+        if (C.internal) break;
+        const ff E = ffsel(j == 0, ce0, ce1), pj = j == 0 ? pc : ff_neg(pc);
+        ff q[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) q[r] = ff_dot2_raw(L[4 * r], E, L[4 * r + 3], pj);
+        put_momentum_ff<PER_EVENT>(out, C.out_index, ch.n_out, q);
       }
     }
 
@@ -418,7 +470,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       fstack_store(fst, sp, 16, ffsel(j0, cmsq[0], cmsq[1]));
       fstack_store(fst, sp, 17, ffsel(j0, cm[0], cm[1]));
       fstack_store(fst, sp, 18, j0 ? pc : ff_neg(pc));
-      fstack_store(fst, sp, 19, ffsel(j0, cmax[0], cmax[1]));
+      fstack_store(fst, sp, 19, ffsel(j0, ce0, ce1));
       sp++;
     }
     if (V.carry >= 0) {
@@ -426,7 +478,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       msq_b = ffsel(j0, cmsq[0], cmsq[1]);
       m_b = ffsel(j0, cm[0], cm[1]);
       p_b = j0 ? pc : ff_neg(pc);
-      mmax_b = ffsel(j0, cmax[0], cmax[1]);
+      E_b = ffsel(j0, ce0, ce1);
     } else if (sp > 0) {
       sp--;
 #pragma unroll
@@ -434,7 +486,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       msq_b = fstack_load(fst, sp, 16);
       m_b = fstack_load(fst, sp, 17);
       p_b = fstack_load(fst, sp, 18);
-      mmax_b = fstack_load(fst, sp, 19);
+      E_b = fstack_load(fst, sp, 19);
     }
   }
 
@@ -494,16 +546,45 @@ __device__ __forceinline__ float msq_f32(int map_id, float4 c, float c4, float c
   return 0.0f;
 }
 
-// Queues event `local` of segment si for the exact FP64 launch (each event at most once,
-// so the slot stays below the segment's event count).
-__device__ __forceinline__ void queue_exact(const PhsLaunch &a, int si, int64_t local) {
-  if (!phs_in(si, a.n_segments, PHS_CHK_SEGMENT)) return;
-  const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
-  const unsigned slot = atomicAdd(a.exact_count + si, 1u);
-  if (phs_in(slot, segs[si].ev_count, PHS_CHK_QUEUE) &&
-      phs_in(segs[si].tile_begin * 32 + slot, a.n_tiles * 32, PHS_CHK_QUEUE))
-    a.exact_queue[segs[si].tile_begin * 32 + slot] = (int32_t)local;
+// The exact FP64 walk of one event.  It shares the float-float frame stack's memory (slots of 8 bytes, 20 a
+// frame: a thread uses one walk at a time, and no slot of one thread overlaps another's).
+static_assert(PHS_FF_STATE * sizeof(float) == PHS_STATE * sizeof(double), "one frame stack serves both walks");
+template <bool PER_EVENT>
+__device__ __forceinline__ void exact_event(const PhsLaunch &a, const PhsSegment &seg, int64_t local, double *stack) {
+  phs_event_f64<PER_EVENT>(a, fx_regs(), seg, local, stack);
 }
+
+// Events that the float-float walk cannot decide (about 0.1 %, and all of a channel without a
+// float-float form) wait in a queue per warp and take the exact FP64 walk 32 at a time, or as
+// many as there are when the warp goes on to another segment or ends.  (A kernel behind the
+// walk for all of them took 35 to 50 us more a call, the latency of one FP64 walk and of two
+// launches.)
+template <bool PER_EVENT>
+struct ExactQueue {
+  int32_t *slots;   // 64, in shared memory
+  double *stack;
+  int n = 0, seg = 0;   // warp-uniform
+  __device__ __forceinline__ void flush(const PhsLaunch &a, const PhsSegment *segs, int least) {
+    const int lane = threadIdx.x & 31;
+    while (n >= least && n > 0) {
+      const int take = n < 32 ? n : 32;
+      __syncwarp();
+      const int32_t l = lane < take && phs_in(n - take + lane, 64, PHS_CHK_QUEUE) ? slots[n - take + lane] : -1;
+      __syncwarp();
+      n -= take;
+      if (l >= 0) exact_event<PER_EVENT>(a, segs[seg], l, stack);
+      __syncwarp();
+    }
+  }
+  // Collective: the lanes with `want` queue event `local` of segment si (at most 31 wait, of si).
+  __device__ __forceinline__ void push(bool want, int si, int64_t local) {
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    const int slot = n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+    if (want && phs_in(slot, 64, PHS_CHK_QUEUE)) slots[slot] = (int32_t)local;
+    n += __popc(m);
+    seg = si;
+  }
+};
 
 // The reduction tables of the float-float functions, built per block in shared memory,
 // exact at multiples of pi/2 (threads 0..95; the caller synchronises).
@@ -687,19 +768,19 @@ __device__ __forceinline__ void write_failed_tile(const PhsLaunch &a, const PhsS
 }
 
 // MIN_BLOCKS: resident blocks per SM the register allocation targets; COMPACT: the
-// two-pass form of phs_kernels.cu (pass A, here in FP32, settles the events that clearly
-// fail; pass B computes the rest densely).  The autotuner in phs_api.cpp picks the faster instantiation per process.
+// two-pass form of phs_kernels.cu (pass A, the FP32 pre-test, settles the events that clearly
+// fail; pass B computes the rest densely).  The autotuner in phs_api.cpp picks the faster
+// instantiation per process.
 template <int MIN_BLOCKS, bool COMPACT, bool PER_EVENT = false>
 __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
     phs_forward_ff_kernel(const __grid_constant__ PhsLaunch a) {
   static_assert(!(COMPACT && PER_EVENT), "the FP32 pre-test needs uniform beams");
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int32_t exact_slots[PHS_FWD_BLOCK / 32][64];
   FFTables &T = *reinterpret_cast<FFTables *>(smem_raw);
-  // the float-float frame stack and the FP64 one share memory (fstack_store): a thread
-  // uses one at a time, and no slot of one thread overlaps another thread's
   float *fst = reinterpret_cast<float *>(smem_raw + sizeof(FFTables));
-  // events the float-float walk cannot decide go to the exact FP64 launch behind this one
-  auto to_exact = [&](int si, int64_t loc) { queue_exact(a, si, loc); };
+  ExactQueue<PER_EVENT> exact{exact_slots[threadIdx.x >> 5], reinterpret_cast<double *>(fst)};
+  const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
 
   fill_ff_tables(T);
   __syncthreads();
@@ -720,22 +801,26 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
           return false;
         },
         [&](int si, const PhsSegment &sg, int64_t loc) {
-          if (!phs_event_ff(a, sg, loc, T, fst)) to_exact(si, loc);
+          exact.flush(a, segs, si == exact.seg ? 32 : 1);
+          exact.push(loc >= 0 && !phs_event_ff(a, sg, loc, T, fst), si, loc);
         });
   } else {
-    for (int64_t tile = warp0; tile < a.n_tiles; tile += n_warps) {
-      const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
+    // (one call site of the exact walk, ahead of each tile: its code is large)
+    for (int64_t tile = warp0;; tile += n_warps) {
+      const bool more = tile < a.n_tiles;
       int lo = 0, hi = a.n_segments - 1;
       while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
         if (segs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
       }
+      exact.flush(a, segs, more && lo == exact.seg ? 32 : 1);
+      if (!more) break;
       const PhsSegment seg = segs[lo];
       const int64_t local = (tile - seg.tile_begin) * 32 + lane;
-      if (local >= seg.ev_count) continue;
-      if (!phs_event_ff<PER_EVENT>(a, seg, local, T, fst)) to_exact(lo, local);
+      exact.push(local < seg.ev_count && !phs_event_ff<PER_EVENT>(a, seg, local, T, fst), lo, local);
     }
   }
+  if constexpr (COMPACT) exact.flush(a, segs, 1);
 }
 
 // Split form, kernel 1 of 3: the FP32 pre-test alone, at the occupancy its few registers
@@ -806,7 +891,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, PHS_FF_TEST_MIN_BLOCKS)
 
 // Kernel 2 of 3 (one block): tile[s] = sum over the segments before s of
 // ceil(count / 32), the dense numbering of the next kernel's warp claims; tile[n] is their
-// total.  Also serves the exact path's queues.
+// total.
 __global__ void __launch_bounds__(1024)
     phs_count_scan_kernel(const unsigned int *count, int64_t *tile, int n) {
   __shared__ int64_t warp_sum[32];
@@ -846,6 +931,8 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
   float *fst = reinterpret_cast<float *>(smem_raw + sizeof(FFTables));
   fill_ff_tables(T);
   __syncthreads();
+  __shared__ int32_t exact_slots[PHS_FWD_BLOCK / 32][64];
+  ExactQueue<false> exact{exact_slots[threadIdx.x >> 5], reinterpret_cast<double *>(fst)};
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
   const int64_t n_claims = a.pass_tile[a.n_segments];
@@ -853,23 +940,21 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
     unsigned long long c = 0;
     if (lane == 0) c = atomicAdd(a.work, 1ull);
     const int64_t t = (int64_t)__shfl_sync(0xffffffffu, c, 0);
-    if (t >= n_claims) break;
     // the last segment whose first claim is <= t (empty segments share the next one's)
     int lo = 0, hi = a.n_segments - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (a.pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
     }
+    // (one call site of the exact walk, ahead of each claim: its code is large)
+    exact.flush(a, segs, t < n_claims && lo == exact.seg ? 32 : 1);
+    if (t >= n_claims) break;
     const PhsSegment &seg = segs[lo];
     const int64_t idx = (t - a.pass_tile[lo]) * 32 + lane;
-    if (idx >= (int64_t)a.pass_count[lo]) continue;
-    if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
-        !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))
-      continue;
-    const int64_t local = a.pass_queue[seg.tile_begin * 32 + idx];
-    if (!phs_event_ff(a, seg, local, T, fst)) {
-      queue_exact(a, lo, local);
-    }
+    const bool valid = idx < (int64_t)a.pass_count[lo] && phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) &&
+                       phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE);
+    const int64_t local = valid ? a.pass_queue[seg.tile_begin * 32 + idx] : 0;
+    exact.push(valid && !phs_event_ff(a, seg, local, T, fst), lo, local);
   }
 }
 
@@ -890,12 +975,6 @@ cudaError_t phs_launch_pretest(const PhsLaunch &a, cudaStream_t stream) {
   const int64_t cap = (int64_t)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   phs_ff_test_kernel<<<(int)(want < cap ? want : cap), PHS_FWD_BLOCK, 0, stream>>>(a);
   phs_count_scan_kernel<<<1, 1024, 0, stream>>>(a.pass_count, a.pass_tile, a.n_segments);
-  return cudaGetLastError();
-}
-
-cudaError_t phs_launch_count_scan(const unsigned int *count, int64_t *tile, int n,
-                                  cudaStream_t stream) {
-  phs_count_scan_kernel<<<1, 1024, 0, stream>>>(count, tile, n);
   return cudaGetLastError();
 }
 

@@ -155,9 +155,9 @@ struct PhsChildFF {
 
 struct PhsVisitFF {
   PhsChildFF child[2];
-  int32_t x_phi, x_ct, ct_class, carry, push, self_root, both_leaves;
-  int32_t parent_root;  // as PhsVisit::parent_root
-  PhsFF b0, b1, self_m_max;
+  int32_t x_phi, x_ct, ct_class, carry, push, self_root;
+  int32_t massless, kind;  // as in PhsVisit
+  PhsFF b0, b1;
 };
 
 // The FP32 pre-test's view of a visit (high parts only), four 16-byte loads.  Per child
@@ -178,6 +178,7 @@ struct PhsChannelFF {
   int32_t exact_only;  // 1: STEP_E/STEP_H mappings or a friend boost: FP64 path
   int32_t lab;
   PhsFF sqrts, s, lab_bg, lab_gamma;
+  PhsFF f0, inv_sqrts;  // as in PhsChannel
   PhsFF m_tot;        // the sum of all outgoing masses (per-event m_max)
   double volume;
   PhsVisitFF visit[PHS_MAX_VISITS];
