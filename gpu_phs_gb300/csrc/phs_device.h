@@ -124,8 +124,7 @@ cudaError_t phs_launch_adjoint(const PhsLaunch &a, const PhsAdjChannel *adj, con
 int phs_adjoint_blocks_per_sm(int max_visits, int max_pops, int stack_depth, bool friends,
                               bool stored = false);
 void phs_adjoint_sizes(int max_visits, int max_pops, int stack_depth, bool friends, int *state0,
-                       int *ang0, int *der0, int *pop0, int *stack0, int *fr0,
-                       size_t *smem);
+                       int *ang0, int *pop0, int *stack0, int *fr0, size_t *smem);
 #define PHS_ADJ_BLOCK_HOST 64
 
 // Inverse map (phs_inverse.cu): for every event and every channel, the x row and factor

@@ -191,6 +191,7 @@ struct PhsAdjChild {
   double da0_dm, da0_dw, da1_dm, da1_dw;  // Breit-Wigner: derivatives of the atan bounds
   double dlf_dm0, dlf_dw0;  // the x-independent parts of dlog f/dm and dlog f/dw:
                             // (da1 - da0)/(a1 - a0) + 1/m (and 1/w)
+  double da, mw, two_m;     // a1 - a0, m w, 2 m
 };
 
 struct PhsAdjVisit {

@@ -283,3 +283,52 @@ def test_adjoint_lab_boost_and_leaf_pairs_against_finite_differences(torch, buil
     jbar = torch.randn(n, generator=g, device="cuda", dtype=torch.float64)
     check_x_derivatives(torch, ps, proc, x, pbar, jbar, h, 0.7,
                         f"{proc.name} E1 {E1:g} E2 {E2:g} dx")
+
+
+@pytest.mark.parametrize("n_out,lab", [(2, False), (2, True), (3, False), (4, True), (5, False), (6, True)])
+def test_adjoint_random_trees_every_mapping_against_finite_differences(torch, n_out, lab):
+    """Channels of random trees with every mapping kind and random leaf masses: each form of
+    the reverse frame step (root, its daughters, inner branches, leaf pairs massive and
+    massless, with and without the lab boost), against finite differences as above."""
+    from conftest import all_maps_process
+    from gpu_phs_gb300.api import PhaseSpace
+    every = all_maps_process(70 + n_out, n_out, 3)
+    h, n, tested = 1e-6, 3000, 0
+    for c in range(every.n_channels):
+        proc = every.subset([c])
+        E1, E2 = (600.0, 500.0) if lab else (500.0, 500.0)
+        proc.sqrts = 2.0 * np.sqrt(E1 * E2)
+        x = torch.from_numpy(uniform_x(1200 + 10 * n_out + c, n, proc.n_x)).cuda()
+        x[:, :max(0, n_out - 2)] *= 0.5        # lighter branches: more events pass the test
+        ps = PhaseSpace(proc, E1, E2)
+        g = torch.Generator(device="cuda").manual_seed(60 + 10 * n_out + c)
+        pbar = torch.randn((n, proc.n_out, 4), generator=g, device="cuda", dtype=torch.float64)
+        jbar = torch.randn(n, generator=g, device="cuda", dtype=torch.float64)
+        if x_keep(torch, ps.generate(x), x, proc, h).sum() < 60:
+            continue                           # a channel whose events (nearly) all fail
+        check_x_derivatives(torch, ps, proc, x, pbar, jbar, h, 0.0, f"n_out {n_out} channel {c} lab {lab} dx")
+        tested += 1
+    assert tested >= 1
+
+
+def test_adjoint_at_the_end_of_cos_theta(torch):
+    """x = 0 for every cos(theta): sin(theta) = 0 counts as constant there, and every derivative
+    stays finite; those of the other x are the ones at x = 2^-200, where sin(theta) = 2^-99 is
+    below any rounding of theirs."""
+    from gpu_phs_gb300.api import PhaseSpace
+    proc = P.tt()
+    n = 2000
+    x = torch.from_numpy(uniform_x(77, n, proc.n_x)).cuda()
+    cts = torch.arange(proc.n_out - 1, 3 * proc.n_out - 4, 2)
+    ps = PhaseSpace(proc, 500.0, 500.0)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    pbar = torch.randn((n, proc.n_out, 4), generator=g, device="cuda", dtype=torch.float64)
+    at, inside = x.clone(), x.clone()
+    at[:, cts] = 0.0
+    inside[:, cts] = 2.0 ** -200
+    a, ta = ps.vjp(at, pbar)
+    b, _ = ps.vjp(inside, pbar)
+    assert torch.isfinite(a).all() and torch.isfinite(ta).all()
+    rest = [k for k in range(3 * proc.n_out - 4) if k not in cts.tolist()]
+    scale = 1.0 + b[:, rest].abs().amax(dim=1, keepdim=True)
+    assert ((a - b)[:, rest].abs() / scale).max() < 1e-12
