@@ -146,6 +146,7 @@ struct Segments {
   DevBuf pass_n, pass_t, pass_q;     // FP32-pair split form: pre-test survivors per segment
   int64_t n_tiles = 0;
   int64_t n_chunks = 0;
+  int32_t chunk_tiles = PHS_CHUNK_TILES;
   int64_t n_events = 0;
   void release() {
     dev.release();
@@ -166,6 +167,14 @@ int build_segments(Segments &S, const int64_t *counts, int n_channels,
                    const std::vector<ChanLayout> &lay, int64_t ev0, int64_t x0, int64_t p0,
                    bool whizard_cols) {
   S.host.clear();
+  // tiles per work chunk: long chunks append to the pre-test's queues with fewer atomics, short
+  // ones share the work evenly over its resident warps (152 SMs x 32): at least 8 chunks a warp,
+  // or single tiles.  With 8 tiles always, 3e5 events left three warps of four idle: 12-particle
+  // trees 264 us (226 so), 3e5 events over 64 channels 107 (82), 2^22 610 (582).
+  int64_t total = 0;
+  for (int c = 0; c < n_channels; c++) total += counts[c] > 0 ? counts[c] : 0;
+  S.chunk_tiles = PHS_CHUNK_TILES;
+  while (S.chunk_tiles > 1 && total / 32 < (int64_t)S.chunk_tiles * 8 * 4864) S.chunk_tiles /= 2;
   int64_t ev = ev0, x = x0, p = p0, tile = 0, chunk = 0;
   for (int c = 0; c < n_channels; c++) {
     const int64_t n = counts[c];
@@ -186,7 +195,7 @@ int build_segments(Segments &S, const int64_t *counts, int n_channels,
     S.host.push_back(g);
     const int64_t tiles = (n + 31) / 32;
     tile += tiles;
-    chunk += (tiles + PHS_CHUNK_TILES - 1) / PHS_CHUNK_TILES;
+    chunk += (tiles + S.chunk_tiles - 1) / S.chunk_tiles;
     ev += n;
     x += n * lay[c].x_stride;
     p += n * 4 * lay[c].n_out;
@@ -202,6 +211,7 @@ int attach_segments(Segments &S, PhsLaunch &a, cudaStream_t stream) {
   a.n_segments = (int32_t)S.host.size();
   a.n_tiles = S.n_tiles;
   a.n_chunks = S.n_chunks;
+  a.chunk_tiles = S.chunk_tiles;
   // the arrays' extents as the segments address them (the checked build's bounds)
   a.x_len = a.p_len = a.ev_len = 0;
   for (const PhsSegment &g : S.host) {

@@ -18,6 +18,7 @@ struct PhsLaunch {
   int32_t stack_depth;         // max push depth over the launched channels
   int64_t n_tiles;             // total 32-event warp tiles
   int64_t n_chunks;            // total work chunks (PhsSegment::chunk_begin)
+  int32_t chunk_tiles;         // tiles of a work chunk (at most PHS_CHUNK_TILES)
   const double *x;
   double *p;
   double *factor;

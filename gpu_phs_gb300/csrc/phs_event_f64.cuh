@@ -755,7 +755,7 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
 // call site each, which keeps the (large) event code once in the kernel.
 //
 // Work is claimed in chunks of CHUNK consecutive tiles of one segment: CHUNK = 1 (single
-// tiles), or PHS_CHUNK_TILES (PhsSegment::chunk_begin; a segment's last chunk may be
+// tiles), or a.chunk_tiles (CHUNK = 0; PhsSegment::chunk_begin; a segment's last chunk may be
 // shorter), whichever was measured faster for the kernel.  With a.work set, a warp claims
 // its next chunk from that counter when it finishes one (events of different channels and
 // kinematics cost very different amounts, and static shares leave SMs idle at the end);
@@ -780,7 +780,7 @@ __device__ __forceinline__ void compacting_loop(const PhsLaunch &a, int64_t *q, 
   int cseg = 0;          // segment of the current chunk
   int64_t tile = 0, tile_end = 0;
   bool done = false;
-  static_assert(CHUNK == 1 || CHUNK == PHS_CHUNK_TILES, "chunks of 1 or PHS_CHUNK_TILES tiles");
+  static_assert(CHUNK == 1 || CHUNK == 0, "chunks of 1 or a.chunk_tiles tiles");
   auto claim = [&]() {
     const int64_t c = next_chunk();
     done = c >= (CHUNK == 1 ? a.n_tiles : a.n_chunks);
@@ -797,8 +797,8 @@ __device__ __forceinline__ void compacting_loop(const PhsLaunch &a, int64_t *q, 
       return;
     }
     const int64_t seg_tiles = (segs[lo].ev_count + 31) / 32;
-    tile = segs[lo].tile_begin + (c - segs[lo].chunk_begin) * CHUNK;
-    const int64_t end = tile + CHUNK, seg_end = segs[lo].tile_begin + seg_tiles;
+    tile = segs[lo].tile_begin + (c - segs[lo].chunk_begin) * a.chunk_tiles;
+    const int64_t end = tile + a.chunk_tiles, seg_end = segs[lo].tile_begin + seg_tiles;
     tile_end = end < seg_end ? end : seg_end;
   };
   claim();

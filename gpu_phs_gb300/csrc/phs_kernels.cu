@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
   if constexpr (COMPACT) {
     int64_t *q = reinterpret_cast<int64_t *>(smem + (size_t)a.stack_depth * PHS_STATE * BLOCK) +
                  (threadIdx.x >> 5) * 64;
-    compacting_loop<PHS_CHUNK_TILES>(
+    compacting_loop<0>(
         a, q,
         [&](const PhsSegment &sg, int64_t loc) { return phs_ok_f64<PER_EVENT, BLOCK>(a, k, sg, loc, smem); },
         [&](int, const PhsSegment &sg, int64_t loc) {

@@ -825,7 +825,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
 
 // Split form, kernel 1 of 3: the FP32 pre-test alone, at the occupancy its few registers
 // allow (the fused kernel runs it at the float-float walk's).  A warp takes a chunk of
-// PHS_CHUNK_TILES tiles of one segment; events that fail for certain get their outputs
+// a.chunk_tiles tiles of one segment; events that fail for certain get their outputs
 // here, the others are gathered in shared memory and appended to their segment's queue
 // (local event indices from tile_begin * 32 on, in any order) with one atomic per chunk.
 __global__ void __launch_bounds__(PHS_FWD_BLOCK, PHS_FF_TEST_MIN_BLOCKS)
@@ -847,9 +847,9 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, PHS_FF_TEST_MIN_BLOCKS)
       if (segs[mid].chunk_begin <= chunk) lo = mid; else hi = mid - 1;
     }
     const PhsSegment &seg = segs[lo];
-    const int64_t t0 = (chunk - seg.chunk_begin) * PHS_CHUNK_TILES;
+    const int64_t t0 = (chunk - seg.chunk_begin) * a.chunk_tiles;
     const int64_t seg_tiles = (seg.ev_count + 31) / 32;
-    const int n_t = (int)(seg_tiles - t0 < PHS_CHUNK_TILES ? seg_tiles - t0 : PHS_CHUNK_TILES);
+    const int n_t = (int)(seg_tiles - t0 < a.chunk_tiles ? seg_tiles - t0 : a.chunk_tiles);
     if (seg.channel != staged_channel && phs_in(seg.channel, a.n_programs, PHS_CHK_CHANNEL)) {
       const PhsChannelFF &ch = a.channels_ff[seg.channel];
       const int nv = ch.n_visits < PHS_MAX_VISITS ? ch.n_visits : PHS_MAX_VISITS;
