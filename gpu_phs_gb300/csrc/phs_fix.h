@@ -247,7 +247,8 @@ FX_FN void fx_sincos_series(uint64_t v, uint64_t &w, uint64_t &k) {
 FX_FN void fx_sincos2pi_q62(uint64_t X, int64_t &s, int64_t &c) {
   const uint32_t q = (uint32_t)((X + (1ull << 61)) >> 62);        // nearest quarter turn, mod 4
   const int64_t r = (int64_t)(X - ((uint64_t)q << 62));           // |r| <= 2^61
-  const uint64_t ar = r < 0 ? (uint64_t)-r : (uint64_t)r;
+  uint64_t ar = r < 0 ? (uint64_t)-r : (uint64_t)r;
+  ar -= ar >> 61;                                                 // an odd eighth: below 2^61
   const uint64_t u = fx_mulhi(ar << 3, 0xc90fdaa22168c235ull);    // 2 pi r 2^-64, Q64
   uint64_t w, k;
   fx_sincos_series(fx_mulhi(u, u), w, k);

@@ -223,3 +223,35 @@ def test_inverse_functions(tmp_path):
     assert float(near1) <= 0.55 and float(lg) <= 1.05
     assert float(sc) <= 2.0 ** -58
     assert int(bad) == 0
+
+
+EIGHTHS_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include "phs_fix.h"
+int main() {
+  const long double PI = 3.14159265358979323846264338327950288L;
+  double worst = 0;
+  for (int k = 0; k < 4096; k++)
+    for (int64_t d : {-1, 0, 1}) {
+      const uint64_t X = ((uint64_t)k << 52) + (uint64_t)d;
+      int64_t s, c;
+      fx_sincos2pi_q62(X, s, c);
+      const long double a = 2 * PI * ((long double)X * 0x1p-64L);
+      worst = std::fmax(worst, (double)std::fmax(fabsl((long double)s * 0x1p-62L - sinl(a)),
+                                                 fabsl((long double)c * 0x1p-62L - cosl(a))));
+    }
+  printf("%.3e\n", worst);
+}
+"""
+
+
+def test_sincos_at_simple_fractions(tmp_path):
+    """sin and cos of 2 pi x at every multiple of 1/4096 of a turn and one unit beside it: the
+    odd eighths lie on the edge of the quarter-turn reduction."""
+    src, exe = tmp_path / "e.cpp", tmp_path / "e"
+    src.write_text(EIGHTHS_DRIVER)
+    subprocess.run(["g++", "-O2", "-std=gnu++17", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True)
+    worst = float(subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout)
+    assert worst <= 2.0 ** -58
