@@ -233,7 +233,7 @@ int main() {
   const long double PI = 3.14159265358979323846264338327950288L;
   double worst = 0;
   for (int k = 0; k < 4096; k++)
-    for (int64_t d : {-1, 0, 1}) {
+    for (int64_t d = -1; d <= 1; d++) {
       const uint64_t X = ((uint64_t)k << 52) + (uint64_t)d;
       int64_t s, c;
       fx_sincos2pi_q62(X, s, c);
