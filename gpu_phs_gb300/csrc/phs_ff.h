@@ -8,9 +8,10 @@
 // break an error-free step.  The elementary functions reduce their argument with a table
 // of exact multiples (kept in shared memory by the kernel) and evaluate short Taylor
 // series; leading terms in float-float, the small tail in plain float.  Accuracy against
-// long double on the host: 3e-14 relative for the arithmetic, 5e-14 absolute for sin and
-// cos, 1.5e-13 relative for tan and exp, far inside what the forward map needs for momenta
-// within 1e-6.
+// long double on the host: 3e-14 relative for the arithmetic, 6e-15 absolute for sin and
+// cos, 1.5e-13 relative for exp, 3e-14 relative for tan up to pi/4 (3.7e-13 within 0.04 of
+// pi/2, where the callers take the cotangent of the complement), far inside what the forward
+// map needs for momenta within 1e-6.
 //
 // The header also compiles as host C++ (for CPU validation of the functions).
 #pragma once
@@ -146,21 +147,25 @@ FF_FN ff ff_recip_fast(ff b) {
   return fast_two_sum(y, f_mul(y, e));
 }
 
-// a/b with the reciprocal estimate: q1 = a.hi y, then one correction from a - b q1.
+// a/b with the reciprocal estimate: q1 = a.hi y, then one correction from a - b q1 (its leading
+// difference is exact: b q1 lies within a few ulps of a).
 FF_FN ff ff_div_fast(ff a, ff b) {
   const float y = f_rcp_approx(b.hi);
   const float q1 = f_mul(a.hi, y);
-  const ff r = ff_sub(a, ff_mul_f(b, q1));
-  return fast_two_sum(q1, f_mul(r.hi, y));
+  const ff p = two_prod(b.hi, q1);
+  const float r = f_add(f_sub(a.hi, p.hi), f_sub(a.lo, f_fma(b.lo, q1, p.lo)));
+  return fast_two_sum(q1, f_mul(r, y));
 }
 
-// sqrt(a), a >= 0, from the hardware rsqrt estimate and one Newton step in float-float.
+// sqrt(a), a >= 0, from the hardware rsqrt estimate and one Newton step in float-float (the
+// residual as in ff_div_fast).
 FF_FN ff ff_sqrt_fast(ff a) {
   if (!(a.hi > 0.0f)) return ff_make(0.0f, 0.0f);
   const float y = f_rsqrt_approx(a.hi);
   const float s = f_mul(a.hi, y);
-  const ff r = ff_sub(a, two_prod(s, s));
-  return fast_two_sum(s, f_mul(f_mul(r.hi, y), 0.5f));
+  const ff p = two_prod(s, s);
+  const float r = f_add(f_sub(a.hi, p.hi), f_sub(a.lo, p.lo));
+  return fast_two_sum(s, f_mul(f_mul(r, y), 0.5f));
 }
 
 // a0 b0 + a1 b1 (+ a2 b2 + a3 b3): exact products of the high parts summed with TwoSum,
@@ -249,28 +254,21 @@ FF_FN float ff_bitsf(uint32_t b) { float f; memcpy(&f, &b, 4); return f; }
 FF_FN int ff_clz(uint32_t v) { return v ? __builtin_clz(v) : 32; }
 #endif
 
-// The same conversions with integer operations only (no FP64 instructions): the mantissa
-// bits of the double are cut into a 24-bit and a 29-bit field.  Truncates toward zero, so
-// for 0 <= d < 1 the order against 0.5 is kept exactly (d < 0.5 iff hi < 0.5f).  Values
-// below 2^-74 in magnitude (or non-finite) are not handled: their low part reads as 0.
+// The same conversions without FP64 instructions: the significand's upper 24 bits are the high
+// part's, the 29 bits below it are converted as an integer and scaled (rounded to 24 bits).  The
+// high part is truncated, so for 0 <= d < 1 the order against 0.5 is kept exactly (d < 0.5 iff
+// hi < 0.5f).  Values below 2^-103 in magnitude (or non-finite) are not handled: their low part
+// reads as 0.
 FF_FN ff ff_from_double_int(double d) {
   const uint64_t b = ff_dbits(d);
-  const uint32_t hw = (uint32_t)(b >> 32), lw = (uint32_t)b;
-  const int e = (int)((hw >> 20) & 0x7ff) - 1023;   // unbiased exponent
-  if (e < -126) return ff_make(0.0f, 0.0f);
-  const uint32_t sign = hw & 0x80000000u;
-  const uint32_t hi = sign | ((uint32_t)(e + 127) << 23) | ((hw & 0xfffffu) << 3) | (lw >> 29);
-  const uint32_t r = lw & 0x1fffffffu;              // remaining 29 bits, weight 2^(e-52)
-  float lo = 0.0f;
-  if (r != 0) {
-    const int p = 31 - ff_clz(r);                   // leading one of r
-    const int fe = e - 52 + p + 127;                // biased exponent of the low part
-    if (fe >= 1) {
-      const uint32_t m = p >= 23 ? (r >> (p - 23)) : (r << (23 - p));
-      lo = ff_bitsf(sign | ((uint32_t)fe << 23) | (m & 0x7fffffu));
-    }
-  }
-  return ff_make(ff_bitsf(hi), lo);
+  const uint32_t hw = (uint32_t)(b >> 32), lw = (uint32_t)b, sign = hw & 0x80000000u;
+  const uint32_t mag = hw & 0x7fffffffu;
+  if (mag < (897u << 20)) return ff_make(0.0f, 0.0f);           // below 2^-126
+  const uint32_t hi = sign | ((mag - (896u << 20)) << 3) | (lw >> 29);
+  // the low field has weight 2^(e - 52), e the unbiased exponent: r 2^-29 2^(e - 23)
+  const int fe = (int)(mag >> 20) - 919;
+  const float scale = ff_bitsf(fe > 0 ? sign | ((uint32_t)fe << 23) : 0u);
+  return ff_make(ff_bitsf(hi), f_mul(f_mul((float)(lw & 0x1fffffffu), 0x1p-29f), scale));
 }
 
 // D * 2^e2 for an integer 0 < D < 2^63, truncated to 48 bits, with integer operations only.
@@ -340,73 +338,68 @@ FF_FN double ff_to_double_int(ff a) {
 
 // ------------------------------------------------------------------ elementary functions
 // Cody-Waite splits (three floats summing to the constant to ~2^-72 relative).
-#define FF_PI32_1 0.098174773156642914f
-#define FF_PI32_2 -2.7319617679211206e-09f
-#define FF_PI32_3 -1.0719528187536762e-16f
+#define FF_PI128_1 0.024543693289160729f
+#define FF_PI128_2 -6.8299044198028015e-10f
+#define FF_PI128_3 -2.6798820468841905e-17f
+#define FF_SIXTH_LO -4.9670538793122887e-09f  // 1/6 - (float)(1/6)
 #define FF_LN2_32_1 0.021660849452018738f
 #define FF_LN2_32_2 -5.9520444128935424e-11f
 #define FF_LN2_32_3 -2.7447449183091686e-18f
-#define FF_INV_PI32 10.185915946960449f     // 32/pi, for choosing the table index only
+#define FF_INV_PI128 40.743663787841797f    // 128/pi, for choosing the table index only
 #define FF_INV_LN2_32 46.166240692138672f   // 32/ln 2, likewise
 #define FF_PI_HI 3.1415927410125732f
 #define FF_PI_LO -8.7422776573475858e-08f
-#define FF_SIXTH_LO -4.9670538793122887e-09f  // 1/6 - (float)(1/6)
-
-// sin and cos of f, |f| <= pi/64 (radians), float-float.
-FF_FN void ff_sincos_small(ff f, ff &s, ff &c) {
-  ff f2 = ff_sqr(f);
-  float y = f2.hi;
-  // sin f = f - f^3/6 + f^5 (1/120 - f^2/5040 + f^4/362880)
-  ff f3 = ff_mul(f2, f);
-  float ts = f_mul(f_mul(y, y), f_fma(y, f_fma(y, 1.0f / 362880.0f, -1.0f / 5040.0f), 1.0f / 120.0f));
-  ff s1 = ff_sub(f, ff_mul_f(f3, 1.0f / 6.0f));
-  // 1/6 is not exact in float: correct with the float-float constant's low part
-  s1 = ff_add_f(s1, f_mul(-f3.hi, FF_SIXTH_LO));
-  s = ff_add_f(s1, f_mul(f.hi, ts));
-  // cos f = 1 - f^2/2 + f^4 (1/24 - f^2/720 + f^4/40320)
-  float tc = f_mul(f_mul(y, y), f_fma(y, f_fma(y, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f));
-  ff c1 = ff_add(ff_from_float(1.0f), ff_mul_f(f2, -0.5f));
-  c = ff_add_f(c1, tc);
-}
 
 // Tables (built on the host, phs_ff_tables in phs_kernels_ff.cu):
-//   trig[k] = {sin(k pi/32).hi, .lo, cos(k pi/32).hi, .lo}, k = 0..63
+//   trig[k] = {sin(k pi/128).hi, .lo, cos(k pi/128).hi, .lo}, k = 0..255
 //   exp2[j] = {2^(j/32).hi, .lo}, j = 0..31
 struct FFTables {
-  float4 trig[64];
+  float4 trig[256];
   float2 exp2[32];
 };
 
 FF_FN ff ff_pi() { return ff_make(FF_PI_HI, FF_PI_LO); }
 
-// sin(2 pi x), cos(2 pi x) for x in [0, 1]: the reduction 64x - k is exact.
-FF_FN void ff_sincos2pi(ff x, const FFTables &T, ff &s, ff &c) {
-  ff y = ff_make(f_mul(x.hi, 64.0f), f_mul(x.lo, 64.0f));
-  float kf = rintf(y.hi);
-  ff g = ff_add_f(y, -kf);                       // exact: |g| <= 1/2
-  ff f = ff_mul(g, ff_make(FF_PI32_1, FF_PI32_2)); // radians, |f| <= pi/64
-  ff sf, cf;
-  ff_sincos_small(f, sf, cf);
-  int k = ((int)kf) & 63;
-  float4 t = T.trig[k];
-  ff sk = ff_make(t.x, t.y), ck = ff_make(t.z, t.w);
-  s = ff_dot2(sk, cf, ck, sf);
-  c = ff_dot2(ck, cf, ff_neg(sk), sf);
+// sin and cos of k pi/128 + f for |f| <= pi/256 (radians): sin f = f - f^3/6 + f^5/120 (the
+// cubic term as a pair: tan next to 0 and cot next to pi/2 keep their relative accuracy) and
+// q = 1 - cos f = f^2/2 - f^4/24 + f^6/720; terms below 2^-27 of the result run in float.  Then
+// s_k + (c_k sin f - s_k q) and c_k - (s_k sin f + c_k q), where the parenthesis is below 2^-6.
+// (80 instructions; a table of 64 entries, with a longer series in pairs, took 120.)
+FF_FN void ff_sincos_table(int k, ff f, const FFTables &T, ff &s, ff &c) {
+  const ff f2 = two_prod(f.hi, f.hi);
+  const float f2lo = f_fma(f_add(f.hi, f.hi), f.lo, f2.lo);
+  // g = f^2/6 - f^4/120, sin f = f - f g
+  const float gh = f_mul(f2.hi, 1.0f / 6.0f);
+  float gl = f_fma(f2.hi, 1.0f / 6.0f, -gh);
+  gl = f_fma(f2.hi, FF_SIXTH_LO, f_fma(f2lo, 1.0f / 6.0f, gl));
+  gl = f_fma(f_mul(f2.hi, f2.hi), -1.0f / 120.0f, gl);
+  const float th = f_mul(f.hi, gh);
+  const float tl = f_fma(f.lo, gh, f_fma(f.hi, gl, f_fma(f.hi, gh, -th)));
+  const ff s1 = fast_two_sum(f.hi, -th);
+  const ff sf = fast_two_sum(s1.hi, f_add(s1.lo, f_sub(f.lo, tl)));
+  const float quart = f_mul(f_mul(f2.hi, f2.hi), f_fma(f2.hi, 1.0f / 720.0f, -1.0f / 24.0f));
+  const ff q = ff_make(f_mul(f2.hi, 0.5f), f_fma(f2lo, 0.5f, quart));
+  const float4 t = T.trig[k & 255];
+  const ff sk = ff_make(t.x, t.y), ck = ff_make(t.z, t.w);
+  s = ff_add(sk, ff_dot2_raw(ck, sf, ff_neg(sk), q));
+  c = ff_sub(ck, ff_dot2_raw(sk, sf, ck, q));
 }
 
-// sin and cos of z (radians), |z| <= pi/2 + pi/64: Cody-Waite reduction by k pi/32.
+// sin(2 pi x), cos(2 pi x) for x in [0, 1]: the reduction 256x - k is exact.
+FF_FN void ff_sincos2pi(ff x, const FFTables &T, ff &s, ff &c) {
+  const ff y = ff_make(f_mul(x.hi, 256.0f), f_mul(x.lo, 256.0f));
+  const float kf = rintf(y.hi);
+  const ff g = fast_two_sum(f_sub(y.hi, kf), y.lo);   // |g| <= 1/2; y.lo is below an ulp of y.hi
+  ff_sincos_table((int)kf, ff_mul(g, ff_make(FF_PI128_1, FF_PI128_2)), T, s, c);
+}
+
+// sin and cos of z (radians), |z| <= pi/2 + pi/64: Cody-Waite reduction by k pi/128.
 FF_FN void ff_sincos(ff z, const FFTables &T, ff &s, ff &c) {
-  float kf = rintf(f_mul(z.hi, FF_INV_PI32));
-  ff f = ff_sub(z, two_prod(kf, FF_PI32_1));
-  f = ff_add_f(f, f_mul(-kf, FF_PI32_2));
-  f = ff_add_f(f, f_mul(-kf, FF_PI32_3));
-  ff sf, cf;
-  ff_sincos_small(f, sf, cf);
-  int k = ((int)kf) & 63;
-  float4 t = T.trig[k];
-  ff sk = ff_make(t.x, t.y), ck = ff_make(t.z, t.w);
-  s = ff_dot2(sk, cf, ck, sf);
-  c = ff_dot2(ck, cf, ff_neg(sk), sf);
+  const float kf = rintf(f_mul(z.hi, FF_INV_PI128));
+  ff f = ff_sub(z, two_prod(kf, FF_PI128_1));
+  f = ff_add_f(f, f_mul(-kf, FF_PI128_2));
+  f = ff_make(f.hi, f_fma(-kf, FF_PI128_3, f.lo));
+  ff_sincos_table((int)kf, f, T, s, c);
 }
 
 // tan(z) for |z| < pi/2 (radians).
@@ -446,12 +439,12 @@ FF_FN ff ff_exp(ff y, const FFTables &T) {
 // Fills the tables (host side).  Entries whose angle is a multiple of pi/2 are set to the
 // exact 0 / +-1, so that tan near +-pi/2 keeps its relative accuracy.
 inline void ff_fill_tables(FFTables &T) {
-  for (int k = 0; k < 64; k++) {
-    long double a = (long double)k * 3.14159265358979323846264338327950288L / 32.0L;
+  for (int k = 0; k < 256; k++) {
+    long double a = (long double)k * 3.14159265358979323846264338327950288L / 128.0L;
     long double sv = sinl(a), cv = cosl(a);
-    if (k % 16 == 0) {
-      sv = (k == 16) ? 1.0L : (k == 48 ? -1.0L : 0.0L);
-      cv = (k == 0) ? 1.0L : (k == 32 ? -1.0L : 0.0L);
+    if (k % 64 == 0) {
+      sv = (k == 64) ? 1.0L : (k == 192 ? -1.0L : 0.0L);
+      cv = (k == 0) ? 1.0L : (k == 128 ? -1.0L : 0.0L);
     }
     float sh = (float)sv, ch = (float)cv;
     T.trig[k].x = sh;

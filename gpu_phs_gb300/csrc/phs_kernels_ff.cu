@@ -17,9 +17,11 @@
 // The walk waits on FP32 latencies (16 warps a SM at 128 registers, issue slots half used), so
 // fewer dependent operations are what counts: frame steps and daughter pairs in the FP64 walk's
 // forms and the energies from the masses took 1e6 tt events from 372 to 357 us (7.9 to 7.0
-// thousand instructions a warp), and the error of the momenta from 2.1e-14 to 1.2e-14.  Five or
-// six blocks a SM (96, 80 registers, spills) and the mappings of both daughters unrolled were
-// slower.
+// thousand instructions a warp); a sin/cos table of 256 entries with a shorter series, exact
+// leading differences in roots and quotients, conversions through the integer-to-float unit,
+// and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 315 us.  The error of the momenta
+// went from 2.1e-14 to 1.0e-14.  Five or six blocks a SM (96, 80 registers, spills) and the
+// mappings of both daughters unrolled were slower.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -118,10 +120,17 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChil
   return child_var(C, C64, sqrts64, m_tot64, 1.0 / s64);
 }
 
+// 1 - x: on the FP64 pipe (uniform beams, where it is mostly idle), or with integer operations.
+template <bool INT>
+__device__ __forceinline__ ff one_minus(double x) {
+  return INT ? ff_one_minus_double_int(x) : ff_from_double_int(1.0 - x);
+}
+
 // msq from x in float-float; returns false when the event must take the exact path.  f: the
 // mapping's factor without its constant part a2 (as map_msq).
 // x arrives as a float-float pair truncated from the double, so x < 0.5 is decided on its
 // high part exactly as the reference decides it on the double.
+template <bool INT>
 __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &cv, double xd,
                                            const FFTables &T, ff &msq, ff &f) {
   const ff x = ff_from_double_int(xd);
@@ -139,7 +148,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
       if (!(fabsf(z.hi) < 1.5707962f)) return false;   // the reference's |z| < pi/2 test
       const bool hs = z.hi > 0.78539816f, ls = z.hi < -0.78539816f, cot = hs || ls;
       ff w = z;
-      if (cot) w = ff_add(hs ? cv.u1 : ld(C.u0), ff_mul(hs ? ff_one_minus_double_int(xd) : x, cv.a1));
+      if (cot) w = ff_add(hs ? cv.u1 : ld(C.u0), ff_mul(hs ? one_minus<INT>(xd) : x, cv.a1));
       ff sw, cw;
       ff_sincos(w, T, sw, cw);
       ff t = ff_div_fast(cot ? cw : sw, cot ? sw : cw);
@@ -156,7 +165,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
       // one exponential for all five: the t/u-channel maps take x >= 0.5 from the other
       // end, with the argument and the sum selected per lane
       const bool upper = (C.map_id == PHS_MAP_TCHANNEL || C.map_id == PHS_MAP_UCHANNEL) && !(x.hi < 0.5f);
-      const ff msq1 = ff_mul(ld(C.a0), ff_exp(ff_mul(upper ? ff_one_minus_double_int(xd) : x, cv.a1), T));
+      const ff msq1 = ff_mul(ld(C.a0), ff_exp(ff_mul(upper ? one_minus<INT>(xd) : x, cv.a1), T));
       msq = upper ? ff_add(ff_sub(ld(C.a0), msq1), cv.msq_max)
                   : ff_add(ff_sub(msq1, ld(C.a0)), ld(C.msq_min));
       f = msq1;
@@ -273,7 +282,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
           ? child_var(C, a.channels[seg.channel].visit[v].child[j], sqrts_f, inv_s_f, ld(ch.m_tot),
                       sqrts64, a.channels[seg.channel].m_tot)
           : child_var(C);
-      if (!map_msq_ff(C, cv, xrow_at(xe, C.x_msq, seg.x_stride), T, mq, f)) exact = true;
+      if (!map_msq_ff<PER_EVENT>(C, cv, xrow_at(xe, C.x_msq, seg.x_stride), T, mq, f)) exact = true;
       if (PER_EVENT) factor = ff_mul(factor, cv.a2);
       if (C.map_id != PHS_MAP_NO) factor = ff_mul(factor, f);
       if (msq_near_zero(mq, s_scale)) exact = true;
@@ -283,9 +292,10 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       }
       const ff mj = ff_sqrt_fast(mq);
       // the kinematic test's upper bound m <= m_max, decided here only away from it
-      const ff dhi = ff_sub(cv.m_max, mj);
-      if (near_zero(dhi, cv.m_max.hi)) exact = true;
-      ok = ok && dhi.hi > 0.0f;
+      // (in float: its rounding is 1e-7 of m_max, the margin 1e-5)
+      const float dhi = f_sub(cv.m_max.hi, mj.hi);
+      if (fabsf(dhi) <= PHS_FF_MARGIN * cv.m_max.hi) exact = true;
+      ok = ok && dhi > 0.0f;
       if (j == 0) {
         cmsq[0] = mq;
         cm[0] = mj;
@@ -344,8 +354,8 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
     StepFF t;
     ff_sincos2pi(ff_from_double_int(xrow_at(xe, V.x_phi, seg.x_stride)), T, t.sp, t.cp);
     const double xctd = xrow_at(xe, V.x_ct, seg.x_stride);
-    const ff xct = ff_from_double_int(xctd);
     if (V.ct_class == PHS_CT_COLLINEAR) {
+      const ff xct = ff_from_double_int(xctd);
       ff b0 = ld(V.b0), b1 = ld(V.b1), fct;
       if (PER_EVENT) {
         const double m = a.channels[seg.channel].visit[v].m;
@@ -354,7 +364,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
         b1 = ff_from_double_int(log(dadd(b0d, 1.0) / b0d));
       }
       const bool lower = xct.hi < 0.5f;
-      const ff tmp = ff_mul(b0, ff_exp(ff_mul(ff_twice(lower ? xct : ff_one_minus_double_int(xctd)), b1), T));
+      const ff tmp = ff_mul(b0, ff_exp(ff_mul(ff_twice(lower ? xct : one_minus<PER_EVENT>(xctd)), b1), T));
       t.ct = lower ? ff_add_f(ff_sub(tmp, b0), -1.0f) : ff_add_f(ff_sub(b0, tmp), 1.0f);
       if (t.ct.hi >= -1.0f && t.ct.hi <= 1.0f) {
         // 1 - ct^2 = (1 - ct)(1 + ct), each factor without cancellation
@@ -368,8 +378,14 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       factor = ff_mul(factor, fct);   // the uniform map's is 1
     } else {
       // ct = 2x - 1, st = sqrt(2(1 - x) 2x) = 2 sqrt((1-x) x)
-      t.ct = ff_add_f(ff_twice(xct), -1.0f);
-      t.st = ff_twice(ff_sqrt_fast(ff_mul(ff_one_minus_double_int(xctd), xct)));
+      if (PER_EVENT) {
+        const ff xct = ff_from_double_int(xctd);
+        t.ct = ff_add_f(ff_twice(xct), -1.0f);
+        t.st = ff_twice(ff_sqrt_fast(ff_mul(ff_one_minus_double_int(xctd), xct)));
+      } else {
+        t.ct = ff_from_double_int(fma(2.0, xctd, -1.0));
+        t.st = ff_twice(ff_sqrt_fast(ff_from_double_int(fma(-xctd, xctd, xctd))));
+      }
     }
 
     if (pair) {
@@ -586,24 +602,30 @@ struct ExactQueue {
   }
 };
 
-// The reduction tables of the float-float functions, built per block in shared memory,
-// exact at multiples of pi/2 (threads 0..95; the caller synchronises).
+// 2^(j/32) to 24 + 24 bits is built from these doubles.
+__constant__ double exp2_32nds[32] = {
+    0x1.0000000000000p+0, 0x1.059b0d3158574p+0, 0x1.0b5586cf9890fp+0, 0x1.11301d0125b51p+0,
+    0x1.172b83c7d517bp+0, 0x1.1d4873168b9aap+0, 0x1.2387a6e756238p+0, 0x1.29e9df51fdee1p+0,
+    0x1.306fe0a31b715p+0, 0x1.371a7373aa9cbp+0, 0x1.3dea64c123422p+0, 0x1.44e086061892dp+0,
+    0x1.4bfdad5362a27p+0, 0x1.5342b569d4f82p+0, 0x1.5ab07dd485429p+0, 0x1.6247eb03a5585p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.71f75e8ec5f74p+0, 0x1.7a11473eb0187p+0, 0x1.82589994cce13p+0,
+    0x1.8ace5422aa0dbp+0, 0x1.93737b0cdc5e5p+0, 0x1.9c49182a3f090p+0, 0x1.a5503b23e255dp+0,
+    0x1.ae89f995ad3adp+0, 0x1.b7f76f2fb5e47p+0, 0x1.c199bdd85529cp+0, 0x1.cb720dcef9069p+0,
+    0x1.d5818dcfba487p+0, 0x1.dfc97337b9b5fp+0, 0x1.ea4afa2a490dap+0, 0x1.f50765b6e4540p+0};
+
+// The reduction tables of the float-float functions, built per block in shared memory in fixed
+// point (exact at multiples of pi/2; the library's sincospi took 4 us of a call).  The caller
+// synchronises.
 __device__ __forceinline__ void fill_ff_tables(FFTables &T) {
-  if (threadIdx.x < 64) {
-    const int k = threadIdx.x;
-    double sv, cv;
-    sincospi(k / 32.0, &sv, &cv);
-    if (k % 16 == 0) {
-      sv = k == 16 ? 1.0 : (k == 48 ? -1.0 : 0.0);
-      cv = k == 0 ? 1.0 : (k == 32 ? -1.0 : 0.0);
-    }
-    const float sh = (float)sv, chh = (float)cv;
-    T.trig[k] = make_float4(sh, (float)(sv - (double)sh), chh, (float)(cv - (double)chh));
-  } else if (threadIdx.x < 96) {
-    const int j = threadIdx.x - 64;
-    const double v = exp2(j / 32.0);
-    const float h = (float)v;
-    T.exp2[j] = make_float2(h, (float)(v - (double)h));
+  for (int k = threadIdx.x; k < 256; k += blockDim.x) {
+    int64_t si, ci;
+    fx_sincos2pi_q62((uint64_t)k << 56, si, ci);
+    const ff sv = ff_from_double_int(fx_from_q62(si)), cv = ff_from_double_int(fx_from_q62(ci));
+    T.trig[k] = make_float4(sv.hi, sv.lo, cv.hi, cv.lo);
+  }
+  if (threadIdx.x < 32) {
+    const ff v = ff_from_double_int(exp2_32nds[threadIdx.x]);
+    T.exp2[threadIdx.x] = make_float2(v.hi, v.lo);
   }
 }
 
