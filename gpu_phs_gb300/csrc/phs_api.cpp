@@ -325,8 +325,18 @@ int attach_pass_buffers(Segments &S, PhsLaunch &a) {
   return PHS_OK;
 }
 
-int launch_ff_tuned(int &variant, Segments &S, PhsLaunch a, int device, int depth,
+// Few tiles: the time is one walk's latency, which the wide form shortens (the FP64 kernels'
+// bits, which meet the FP32-pair precision's bar too).
+bool wide_serves(const PhsLaunch &a, int tiles_per_visit) {
+  return !a.friends && a.n_tiles <= (int64_t)tiles_per_visit * a.max_visits;
+}
+
+int launch_ff_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int device, int depth,
                     int64_t n_events, cudaStream_t st) {
+  if (!pinned && wide_serves(a, PHS_WIDE_TILES / 2)) {   // (2e4 tt events: 25 us in pairs, 29 wide)
+    CUDA_TRY(phs_launch_forward_f64(a, 0, PHS_F64_WIDE, st));
+    return PHS_OK;
+  }
   if (int rc = attach_pass_buffers(S, a)) return rc;
   // per-event beams: the float-float one pass at either register budget (variants 0, 1;
   // the pre-test needs uniform constants), or the FP64 compacting kernel (2, 3: FP64
@@ -351,9 +361,13 @@ int launch_ff_tuned(int &variant, Segments &S, PhsLaunch a, int device, int dept
   });
 }
 
-int launch_f64_tuned(int &variant, Segments &S, PhsLaunch a, int device, int depth,
+int launch_f64_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int device, int depth,
                      int64_t n_events, cudaStream_t st) {
   const bool per_event = a.E1 != nullptr;
+  if (!pinned && wide_serves(a, PHS_WIDE_TILES)) {
+    CUDA_TRY(phs_launch_forward_f64(a, 0, PHS_F64_WIDE, st));
+    return PHS_OK;
+  }
   if (!per_event)
     if (int rc = attach_pass_buffers(S, a)) return rc;
   const int n_variants = per_event ? PHS_F64_VARIANTS_PER_EVENT : PHS_F64_VARIANTS;
@@ -440,6 +454,7 @@ struct phs_process {
   int precision = PHS_PRECISION_F64;
   int ff_variant_ev[2] = {-1, -1};  // autotuned FP32-pair variant: uniform, per-event beams
   int f64_variant[2] = {-1, -1};  // autotuned FP64 variant: uniform, per-event beams
+  bool pinned = false, ff_pinned = false;  // the variants were set, not tuned
   std::vector<PhsChannel> prog;
   std::vector<PhsChannelFF> prog_ff;
   std::vector<PhsAdjChannel> prog_adj;
@@ -729,6 +744,8 @@ extern "C" int phs_process_set_variants(phs_process_t h, int ff_variant, int f64
     if (int rc = check_variants(ff_variant, f64_variant)) return rc;
     h->ff_variant_ev[0] = h->ff_variant_ev[1] = ff_variant;
     h->f64_variant[0] = h->f64_variant[1] = f64_variant;
+    h->pinned = f64_variant >= 0;
+    h->ff_pinned = ff_variant >= 0;
     return PHS_OK;
   });
 }
@@ -786,6 +803,8 @@ static int launch_process(phs_process_t h, Segments &S, int64_t n_events, const 
   a.channels = h->d_prog.as<PhsChannel>();
   a.channels_ff = h->d_prog_ff.as<PhsChannelFF>();
   a.stack_depth = h->stack_depth;
+  a.max_visits = h->max_visits;
+  a.friends = h->has_friends ? 1 : 0;
   a.x = x;
   a.p = p;
   a.factor = f;
@@ -800,9 +819,9 @@ static int launch_process(phs_process_t h, Segments &S, int64_t n_events, const 
   if ((rc = attach_segments(S, a, stream))) return rc;
   if (a.n_tiles == 0) return PHS_OK;
   if (h->precision == PHS_PRECISION_F32X2)
-    return launch_ff_tuned(h->ff_variant_ev[E1 != nullptr], S, a, h->device, h->stack_depth,
+    return launch_ff_tuned(h->ff_variant_ev[E1 != nullptr], h->ff_pinned, S, a, h->device, h->stack_depth,
                            n_events, stream);
-  return launch_f64_tuned(h->f64_variant[E1 != nullptr], S, a, h->device, h->stack_depth, n_events,
+  return launch_f64_tuned(h->f64_variant[E1 != nullptr], h->pinned, S, a, h->device, h->stack_depth, n_events,
                           stream);
 }
 
@@ -1095,7 +1114,9 @@ struct phs_batch {
   std::vector<PhsChannel> prog;
   std::vector<PhsChannelFF> prog_ff;
   std::vector<ChanLayout> lay;
-  int stack_depth = 0;
+  int stack_depth = 0, max_visits = 0;
+  bool friends = false;
+  bool pinned = false, ff_pinned = false;  // the variants were set, not tuned
   DevBuf d_prog, d_prog_ff;
   Segments segs;
 };
@@ -1117,6 +1138,8 @@ extern "C" int phs_batch_create(phs_batch_t *out, int n_procs, const phs_process
       b->prog_ff.insert(b->prog_ff.end(), h->prog_ff.begin(), h->prog_ff.end());
       b->lay.insert(b->lay.end(), h->lay.begin(), h->lay.end());
       b->stack_depth = std::max(b->stack_depth, h->stack_depth);
+      b->max_visits = std::max(b->max_visits, h->max_visits);
+      b->friends = b->friends || h->has_friends;
     }
     DeviceGuard g(b->device);
     int rc = b->d_prog.reserve(b->prog.size() * sizeof(PhsChannel));
@@ -1197,6 +1220,8 @@ extern "C" int phs_batch_generate_device(phs_batch_t b, const int64_t *counts, c
     a.channels = b->d_prog.as<PhsChannel>();
     a.channels_ff = b->d_prog_ff.as<PhsChannelFF>();
     a.stack_depth = b->stack_depth;
+    a.max_visits = b->max_visits;
+    a.friends = b->friends ? 1 : 0;
     a.x = x;
     a.p = p;
     a.factor = f;
@@ -1207,9 +1232,9 @@ extern "C" int phs_batch_generate_device(phs_batch_t b, const int64_t *counts, c
     if ((rc = attach_segments(b->segs, a, (cudaStream_t)stream))) return rc;
     if (a.n_tiles == 0) return PHS_OK;
     if (b->precision == PHS_PRECISION_F32X2)
-      return launch_ff_tuned(b->ff_variant, b->segs, a, b->device, b->stack_depth, n_events,
+      return launch_ff_tuned(b->ff_variant, b->ff_pinned, b->segs, a, b->device, b->stack_depth, n_events,
                              (cudaStream_t)stream);
-    return launch_f64_tuned(b->f64_variant, b->segs, a, b->device, b->stack_depth, n_events,
+    return launch_f64_tuned(b->f64_variant, b->pinned, b->segs, a, b->device, b->stack_depth, n_events,
                             (cudaStream_t)stream);
   });
 }
@@ -1220,6 +1245,8 @@ extern "C" int phs_batch_set_variants(phs_batch_t b, int ff_variant, int f64_var
     if (int rc = check_variants(ff_variant, f64_variant)) return rc;
     b->ff_variant = ff_variant;
     b->f64_variant = f64_variant;
+    b->pinned = f64_variant >= 0;
+    b->ff_pinned = ff_variant >= 0;
     return PHS_OK;
   });
 }

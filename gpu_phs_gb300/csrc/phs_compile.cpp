@@ -282,6 +282,27 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
     }
   }
   out.n_visits = v;
+  {
+    // the visit of each internal daughter: the next one (carry), or the one after the pop
+    std::vector<std::pair<int, int>> pushed;
+    for (int u = 0; u < v; u++) out.visit[u].child_visit[0] = out.visit[u].child_visit[1] = -1;
+    out.visit[0].parent_visit = -1;
+    auto link = [&](int parent, int j, int child) {
+      out.visit[parent].child_visit[j] = (int8_t)child;
+      out.visit[child].parent_visit = (int8_t)parent;
+      out.visit[child].parent_child = (int8_t)j;
+    };
+    for (int u = 0; u < v; u++) {
+      const PhsVisit &V = out.visit[u];
+      if (V.push >= 0) pushed.push_back({u, V.push});
+      if (V.carry >= 0) {
+        link(u, V.carry, u + 1);
+      } else if (u + 1 < v) {
+        link(pushed.back().first, pushed.back().second, u + 1);
+        pushed.pop_back();
+      }
+    }
+  }
   if (depth > PHS_STACK_DEPTH) { err = where + "tree too deep for the visit stack"; return PHS_ERR_UNSUPPORTED; }
   info.stack_depth = depth;
   info.n_internal = v;

@@ -16,6 +16,8 @@ struct PhsLaunch {
   PhsSegment seg_inline[PHS_INLINE_SEGS];  // sorted by tile_begin
   int32_t n_segments;
   int32_t stack_depth;         // max push depth over the launched channels
+  int32_t max_visits;          // max visits over the launched channels
+  int32_t friends;             // 1: some launched channel has a friend visit
   int64_t n_tiles;             // total 32-event warp tiles
   int64_t n_chunks;            // total work chunks (PhsSegment::chunk_begin)
   int32_t chunk_tiles;         // tiles of a work chunk (at most PHS_CHUNK_TILES)
@@ -50,9 +52,16 @@ struct PhsLaunch {
 // pass, 256 x 2 and 64 x 8; 5-8: split (the FP32 pre-test of phs_launch_pretest, then the
 // FP64 walk over its survivors; uniform beams only, needs the a.pass_* buffers and a.work
 // zeroed), 128 x 4, 128 x 3, 256 x 2, 64 x 8.  PHS_F64_VARIANTS of them; the first
-// PHS_F64_VARIANTS_PER_EVENT serve per-event beams.
+// PHS_F64_VARIANTS_PER_EVENT serve per-event beams.  PHS_F64_WIDE (not tried by the autotuner,
+// no friend visits): the form for launches that leave the GPU idle, a block of five warps per
+// 32 events.
 #define PHS_F64_VARIANTS 9
 #define PHS_F64_VARIANTS_PER_EVENT 5
+#define PHS_F64_WIDE 9
+// Tiles a visit of the largest tree up to which the wide form is the faster one (us a call, wide
+// against one pass / split: 3 visits 1e4 events 12.4 / 14.5, 2e4 18.6 / 18.5, 4e4 27 / 21; 5 visits
+// 2e4 29 / 33, 4e4 45 / 38; 11 visits 4e4 92 / 95, 1.6e5 287 / 268).
+#define PHS_WIDE_TILES 160
 cudaError_t phs_launch_forward_f64(const PhsLaunch &a, int n_blocks, int variant,
                                    cudaStream_t stream);
 int phs_forward_blocks_per_sm(int stack_depth, bool per_event, int variant);

@@ -91,6 +91,298 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
   }
 }
 
+// The wide form, for launches that leave the GPU idle: there the time is the latency of one
+// event's walk, some 5000 instructions in a row, so a block of five warps takes the 32 events of
+// a tile.  What does not depend on the frames is computed for all visits at once, a visit per
+// warp (mappings and angles; then, with every msq known, masses, momenta and energies); the
+// frames follow with a warp per row (a frame step works row by row, and component r of a
+// momentum reads row r alone), while the fifth warp multiplies the factor.  Every value comes
+// from the same operations in the same order as in phs_event_f64: the same bits.  No friend
+// visits (their axis mixes rows).  Slots of a visit (one column per event):
+enum {
+  kWMsq, kWM,                  // the visited branch
+  kWSp, kWCp, kWCt, kWSt,      // its decay angles
+  kWFct, kWF, kWA2,            // factors: cos(theta) map; the branch's msq map and (per-event
+                               // beams) its constant
+  kWPc, kWE0, kWE1, kWRm, kWFk,  // p_decay, daughters' energies, 1/m, sqrt(lambda) / (2 m^2)
+  PHS_WIDE_SLOTS
+};
+#define PHS_WIDE_WARPS 5
+
+template <bool PER_EVENT>
+__global__ void __launch_bounds__(PHS_WIDE_WARPS * 32)
+    phs_forward_f64_wide_kernel(const __grid_constant__ PhsLaunch a) {
+  extern __shared__ double smem[];
+  __shared__ unsigned ok_mask;
+  const FxRegs k = fx_regs();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
+  const auto at = [&](int v, int i) -> double & { return smem[(v * PHS_WIDE_SLOTS + i) * 32 + lane]; };
+  for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
+    int lo = 0, hi = a.n_segments - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (segs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    }
+    const PhsSegment &seg = segs[lo];
+    const int64_t first = (tile - seg.tile_begin) * 32;
+    const bool valid = first + lane < seg.ev_count;
+    const int64_t local = valid ? first + lane : first;   // (a copy of the tile's first event)
+    // checked build: the channel, its slots and the event's rows (block-uniform on the first
+    // event; an event out of range writes nothing)
+    if (!phs_in(seg.channel, a.n_programs, PHS_CHK_CHANNEL)) continue;
+    const PhsChannel &ch = a.channels[seg.channel];
+    if (!phs_in(ch.n_visits - 1, a.max_visits, PHS_CHK_VISITS)) continue;
+    const bool inside = event_in_bounds(a, seg, local, ch.n_out, ch.n_visits);
+    const int64_t ev = seg.ev_begin + local;
+    const double *xe = a.x + seg.x_base + local * seg.x_stride;
+    double *out = a.p + seg.p_base + local * 4 * (int64_t)ch.n_out;
+    const bool lab = PER_EVENT || ch.lab != 0;
+    double sqrts = ch.sqrts, lab_bg = ch.lab_bg, lab_ga = ch.lab_gamma;
+    if (PER_EVENT) {
+      const double E1 = inside ? a.E1[ev] : 1.0, E2 = inside ? a.E2[ev] : 1.0;
+      const double r = fx_sqrt(fx_mul(k, E1, E2), k);
+      sqrts = fx_add(k, r, r);
+      lab_bg = fx_div(fx_sub(k, E1, E2), sqrts, k);
+      lab_ga = fx_sqrt(fma(lab_bg, lab_bg, k.one), k);
+    }
+    const double s = fx_mul(k, sqrts, sqrts);
+    const double inv_s = PER_EVENT ? fx_rcp(s, k) : 0.0;
+    const int n_visits = ch.n_visits;
+    bool ok = true;
+    if (threadIdx.x == 0) ok_mask = 0xffffffffu;
+
+    // 1. mappings of each visit's internal daughters, and its angles
+    for (int v = wid; v < n_visits; v += PHS_WIDE_WARPS) {
+      const PhsVisit &V = ch.visit[v];
+      if (v == 0) {
+        at(0, kWMsq) = s;
+        at(0, kWM) = sqrts;
+      }
+#pragma unroll 1
+      for (int j = 0; j < 2; j++) {
+        const PhsChild &C = V.child[j];
+        if (!C.internal || !phs_in(V.child_visit[j], n_visits, PHS_CHK_VISITS)) continue;
+        double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
+        if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
+        double mq, f, aux;
+        map_msq(k, C.map_id, inside ? xrow_at(xe, C.x_msq, seg.x_stride) : 0.5, s, C.m, C.w, mn, mx, a0, a1,
+                a2, mq, f, aux);
+        const double mj = fx_sqrt(mq, k);
+        ok = ok && !fx_gt(mj, mmax);
+        const int cv = V.child_visit[j];
+        at(cv, kWMsq) = mq;
+        at(cv, kWM) = mj;
+        at(cv, kWF) = f;
+        if (PER_EVENT) at(cv, kWA2) = a2;
+      }
+      double sp, cp, ct, st, fct, b0 = V.b0, b1 = V.b1;
+      sincos2pi(inside ? xrow_at(xe, V.x_phi, seg.x_stride) : 0.5, sp, cp);
+      if (PER_EVENT && V.ct_class == PHS_CT_COLLINEAR) {
+        b0 = dmul(V.m, V.m) / s;
+        b1 = log(dadd(b0, 1.0) / b0);
+      }
+      map_ct(k, V.ct_class, inside ? xrow_at(xe, V.x_ct, seg.x_stride) : 0.5, b0, b1, ct, st, fct);
+      at(v, kWSp) = sp;
+      at(v, kWCp) = cp;
+      at(v, kWCt) = ct;
+      at(v, kWSt) = st;
+      at(v, kWFct) = fct;
+    }
+    __syncthreads();
+
+    // 2. kinematics of each visit
+    for (int v = wid; v < n_visits; v += PHS_WIDE_WARPS) {
+      const PhsVisit &V = ch.visit[v];
+      double cmsq[2], cm[2];
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const bool in = V.child[j].internal && phs_in(V.child_visit[j], n_visits, PHS_CHK_VISITS);
+        cmsq[j] = in ? at(V.child_visit[j], kWMsq) : V.child[j].msq_leaf;
+        cm[j] = in ? at(V.child_visit[j], kWM) : V.child[j].m_leaf;
+      }
+      const double msq_b = at(v, kWMsq), m_b = at(v, kWM);
+      const int massless = V.massless;
+      double sl;
+      ok = kallen_ok(k, massless, msq_b, m_b, cmsq, cm, sl) && ok;
+      double rm = 0.0, pc, ce0, ce1;
+      if (massless == 3) {
+        pc = ce0 = ce1 = fx_scale(m_b, -1);
+        if (V.kind == PHS_KIND_ROOT) rm = fx_hi(m_b) - 1u < 0x7fefffffu ? fx_rcp(m_b, k) : 0.0;   // n_out = 2
+      } else {
+        double hm;
+        if (!PER_EVENT && V.self_root) {
+          rm = ch.inv_sqrts;
+          hm = fx_scale(rm, -1);
+        } else {
+          mass_reciprocals(k, m_b, rm, hm);
+        }
+        pc = fx_mul(k, sl, hm);
+        at(v, kWFk) = fx_mul(k, pc, rm);
+        if (massless == 0) {
+          const double dc = fx_sub(k, cmsq[0], cmsq[1]);
+          ce0 = fx_mul(k, fx_add(k, msq_b, dc), hm);
+          ce1 = fx_mul(k, fx_sub(k, msq_b, dc), hm);
+        } else {
+          const double eo = fx_sub(k, m_b, pc);
+          ce0 = massless & 1 ? pc : eo;
+          ce1 = massless & 1 ? eo : pc;
+        }
+      }
+      at(v, kWPc) = pc;
+      at(v, kWE0) = ce0;
+      at(v, kWE1) = ce1;
+      at(v, kWRm) = rm;
+    }
+    const unsigned mine = __ballot_sync(0xffffffffu, ok && valid);
+    if (lane == 0) atomicAnd(&ok_mask, mine);
+    __syncthreads();
+    const unsigned passed = ok_mask;
+    ok = passed >> lane & 1;
+
+    // 3. the factor (warp 4), and the frames and momenta, row `wid` (warps 0 .. 3)
+    if (wid == 4) {
+      double factor = PER_EVENT ? 1.0 : ch.f0;
+      int halved = 0;
+      for (int v = 0; v < n_visits && passed; v++) {
+        const PhsVisit &V = ch.visit[v];
+        for (int j = 0; j < 2; j++) {
+          const PhsChild &C = V.child[j];
+          if (!C.internal || !phs_in(V.child_visit[j], n_visits, PHS_CHK_VISITS)) continue;
+          if (PER_EVENT && C.map_id != PHS_MAP_STEP_E && C.map_id != PHS_MAP_STEP_H)
+            factor = fx_mul(k, factor, at(V.child_visit[j], kWA2));
+          if (C.map_id != PHS_MAP_NO) factor = fx_mul(k, factor, at(V.child_visit[j], kWF));
+        }
+        if (V.massless != 3) {
+          factor = fx_mul(k, factor, at(v, kWFk));
+          halved++;
+        }
+        if (V.ct_class == PHS_CT_COLLINEAR) factor = fx_mul(k, factor, at(v, kWFct));
+      }
+      if (valid && inside) {
+        a.volume[ev] = PER_EVENT ? channel_volume(ch, sqrts) : ch.volume;
+        a.factor[ev * a.factor_stride + seg.factor_col] =
+            ok ? fx_mul(k, factor, fx_double((1023u + halved) << 20, 0u)) : 0.0;
+        a.ok[ev] = ok ? 1 : 0;
+      }
+    } else if (passed == 0) {
+      if (valid && inside)
+        for (int i = 0; i < ch.n_out; i++) out[4 * i + wid] = 0.0;
+    } else {
+      const bool first_row = wid == 0, edge = wid == 0 || wid == 3;
+      double l[4] = {0.0, 0.0, 0.0, 0.0}, s0[4] = {}, s1[4] = {};   // the row, and saved ones
+      int sp = 0;
+      const auto put = [&](int index, double q) {
+        if (valid && inside && phs_in(index, ch.n_out, PHS_CHK_P)) out[4 * index + wid] = ok ? q : 0.0;
+      };
+      for (int v = 0; v < n_visits; v++) {
+        const PhsVisit &V = ch.visit[v];
+        int kind = V.kind;
+        if (lab)
+          kind = kind == PHS_KIND_ROOT ? PHS_KIND_ROOT_LAB
+                 : kind == PHS_KIND_FIRST ? PHS_KIND_FIRST_LAB
+                 : kind == PHS_KIND_LEAVES_FIRST ? PHS_KIND_LEAVES : kind;
+        const bool pair = kind == PHS_KIND_LEAVES || kind == PHS_KIND_LEAVES_FIRST;
+        // the branch's momentum and energy in its parent's frame
+        double p_b = 0.0, E_b = 0.0;
+        if (phs_in(V.parent_visit + 1, n_visits + 1, PHS_CHK_VISITS) && V.parent_visit >= 0) {
+          const double pp = at(V.parent_visit, kWPc);
+          p_b = V.parent_child == 0 ? pp : fx_neg(pp);
+          E_b = at(V.parent_visit, V.parent_child == 0 ? kWE0 : kWE1);
+        }
+        const double pc = at(v, kWPc), ce0 = at(v, kWE0), ce1 = at(v, kWE1), rm = at(v, kWRm);
+        Step t;
+        t.sp = at(v, kWSp);
+        t.cp = at(v, kWCp);
+        t.ct = at(v, kWCt);
+        t.st = at(v, kWSt);
+        if (pair) {
+          const double pst = fx_mul(k, pc, t.st), qx = fx_mul(k, pst, t.cp), qy = fx_mul(k, pst, t.sp);
+          double qa0, qa3, qb0, qb3;
+          if (V.massless == 3) {
+            const double eh = fx_scale(E_b, -1), ph = fx_scale(p_b, -1);
+            qa0 = fma(ph, t.ct, eh);
+            qb0 = fma(-ph, t.ct, eh);
+            qa3 = fma(eh, t.ct, ph);
+            qb3 = fma(-eh, t.ct, ph);
+          } else {
+            const double bg = fx_mul(k, p_b, rm), ga = fx_mul(k, E_b, rm), qz = fx_mul(k, pc, t.ct);
+            const double z0 = fx_mul(k, bg, qz), z3 = fx_mul(k, ga, qz);
+            qa0 = fma(ga, ce0, z0);
+            qb0 = fma(ga, ce1, -z0);
+            qa3 = fma(bg, ce0, z3);
+            qb3 = fma(bg, ce1, -z3);
+          }
+          double qa, qb;
+          if (kind == PHS_KIND_LEAVES_FIRST) {
+            const double w = wid == 3 ? fx_mul(k, l[1], qx) : fma(l[2], qy, fx_mul(k, l[1], qx));
+            qa = first_row ? qa0 : fma(l[3], qa3, w);
+            qb = first_row ? qb0 : fma(l[3], qb3, -w);
+          } else {
+            const double w = fma(l[2], qy, fx_mul(k, l[1], qx));
+            qa = fma(l[0], qa0, fma(l[3], qa3, w));
+            qb = fma(l[0], qb0, fma(l[3], qb3, -w));
+          }
+          put(V.child[0].out_index, qa);
+          put(V.child[1].out_index, qb);
+        } else {
+          if (!V.self_root) {
+            t.bg = fx_mul(k, p_b, rm);
+            t.ga = fx_mul(k, E_b, rm);
+          }
+          if (kind == PHS_KIND_ROOT || kind == PHS_KIND_ROOT_LAB) {
+            if (edge) {
+              const double g = kind == PHS_KIND_ROOT ? (first_row ? 1.0 : 0.0) : (first_row ? lab_ga : lab_bg);
+              const double h = kind == PHS_KIND_ROOT ? (first_row ? 0.0 : 1.0) : (first_row ? lab_bg : lab_ga);
+              l[0] = g;
+              l[1] = fx_mul(k, -h, t.st);
+              l[2] = 0.0;
+              l[3] = fx_mul(k, h, t.ct);
+            } else {
+              const double c = wid == 1 ? t.cp : t.sp;
+              l[0] = 0.0;
+              l[1] = fx_mul(k, t.ct, c);
+              l[2] = wid == 1 ? fx_neg(t.sp) : t.cp;
+              l[3] = fx_mul(k, t.st, c);
+            }
+          } else if (kind == PHS_KIND_FIRST) {
+            if (first_row) {
+              l[0] = t.ga;
+              l[1] = fx_mul(k, -t.st, t.bg);
+              l[2] = 0.0;
+              l[3] = fx_mul(k, t.ct, t.bg);
+            } else if (wid == 3) {
+              frame_row<true, true>(k, t, l);
+            } else {
+              frame_row<true, false>(k, t, l);
+            }
+          } else if (kind == PHS_KIND_FIRST_LAB) {
+            if (edge) frame_row<false, true>(k, t, l); else frame_row<true, false>(k, t, l);
+          } else {
+            frame_row<false, false>(k, t, l);
+          }
+          for (int j = 0; j < 2; j++)
+            if (!V.child[j].internal)
+              put(V.child[j].out_index, fma(l[0], j == 0 ? ce0 : ce1, fx_mul(k, l[3], j == 0 ? pc : fx_neg(pc))));
+        }
+        if (V.push >= 0) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            if (sp == 0) s0[i] = l[i]; else s1[i] = l[i];
+          }
+          sp++;
+        }
+        if (V.carry < 0 && sp > 0) {
+          sp--;
+#pragma unroll
+          for (int i = 0; i < 4; i++) l[i] = sp == 0 ? s0[i] : s1[i];
+        }
+      }
+    }
+    __syncthreads();   // the slots are read
+  }
+}
+
 // Whizard's sparse momentum buffer from the dense one (layout in phs_device.h): one thread
 // per 32-byte slot, consecutive threads on consecutive slots.
 __global__ void phs_whizard_sparse_kernel(const __grid_constant__ PhsSparseLaunch a) {
@@ -237,6 +529,17 @@ int phs_forward_blocks_per_sm(int stack_depth, bool per_event, int variant) {
 }
 
 template <bool PER_EVENT>
+static cudaError_t launch_wide(const PhsLaunch &a, cudaStream_t stream) {
+  const size_t smem = (size_t)a.max_visits * PHS_WIDE_SLOTS * 32 * sizeof(double);
+  const cudaError_t e = allow_smem((const void *)phs_forward_f64_wide_kernel<PER_EVENT>, smem);
+  if (e != cudaSuccess) return e;
+  const int64_t cap = 1 << 20;
+  phs_forward_f64_wide_kernel<PER_EVENT>
+      <<<(int)(a.n_tiles < cap ? a.n_tiles : cap), PHS_WIDE_WARPS * 32, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
+template <bool PER_EVENT>
 static cudaError_t launch_f64(const PhsLaunch &a, int n_blocks, int variant, cudaStream_t stream) {
   const int block = f64_block(variant);
   const size_t smem = phs_forward_smem_bytes(a.stack_depth, block);
@@ -264,6 +567,10 @@ static cudaError_t launch_f64(const PhsLaunch &a, int n_blocks, int variant, cud
 cudaError_t phs_launch_forward_f64(const PhsLaunch &a, int n_blocks, int variant,
                                    cudaStream_t stream) {
   if (a.n_tiles <= 0) return cudaSuccess;
+  if (variant == PHS_F64_WIDE) {
+    if (a.friends) return cudaErrorInvalidValue;
+    return a.E1 && a.E2 ? launch_wide<true>(a, stream) : launch_wide<false>(a, stream);
+  }
   if (variant >= 5) {
     if (a.E1 || a.E2) return cudaErrorInvalidValue;  // the pre-test needs uniform beams
     cudaError_t e = phs_launch_pretest(a, stream);

@@ -88,7 +88,9 @@ struct PhsVisit {
                         // (1,0,0,0), (0,*,*,*), (0,*,*,*), (0,*,0,*)
   int8_t massless;      // bit j: daughter j is a massless outgoing particle
   int32_t kind;         // PHS_KIND_*: the form of the visit's frame step (FP64 walk)
-  int32_t pad0;
+  int8_t child_visit[2];  // visit where internal daughter j is the visited branch, -1: leaf
+  int8_t parent_visit;    // visit whose daughter the visited branch is, -1: the root
+  int8_t parent_child;    // which daughter
 };
 
 struct PhsChannel {
