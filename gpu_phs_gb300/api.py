@@ -26,8 +26,10 @@ def _ptr(t) -> Optional[int]:
 
 def _stream(stream) -> Optional[int]:
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the current stream's handle without a Stream object (0.3 us instead of 3)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 @dataclass
