@@ -315,11 +315,13 @@ int launch_tuned(int &variant, int n_variants, int64_t n_events, cudaStream_t st
 // their indices (n_tiles * 32 entries).
 int attach_pass_buffers(Segments &S, PhsLaunch &a) {
   const size_t n_seg = (size_t)std::max(a.n_segments, 1);
-  if (int rc = S.pass_n.reserve(n_seg * sizeof(unsigned int))) return rc;
+  // the walk's claim counter and the segments' counts, one memset
+  if (int rc = S.pass_n.reserve(sizeof(unsigned long long) + n_seg * sizeof(unsigned int))) return rc;
   if (int rc = S.pass_t.reserve((n_seg + 1) * sizeof(int64_t))) return rc;
   if (int rc = S.pass_q.reserve((size_t)std::max<int64_t>(a.n_tiles, 1) * 32 * sizeof(int32_t)))
     return rc;
-  a.pass_count = S.pass_n.as<unsigned int>();
+  a.work = S.pass_n.as<unsigned long long>();
+  a.pass_count = reinterpret_cast<unsigned int *>(a.work + 1);
   a.pass_tile = S.pass_t.as<int64_t>();
   a.pass_queue = S.pass_q.as<int32_t>();
   return PHS_OK;
@@ -353,9 +355,8 @@ int launch_ff_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int dev
     }
     if (per_event) v &= 1;
     cudaError_t e = cudaSuccess;
-    if (v >= 2) e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
-    if (e == cudaSuccess && v >= 4)
-      e = cudaMemsetAsync(a.pass_count, 0, (size_t)a.n_segments * sizeof(unsigned int), st);
+    if (v >= 2)
+      e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long) + (v >= 4 ? (size_t)a.n_segments * sizeof(unsigned int) : 0), st);
     if (e == cudaSuccess) e = phs_launch_forward_ff(a, grid_for_ff(a.n_tiles, device, depth, v), v, st);
     return e;
   });
@@ -376,9 +377,9 @@ int launch_f64_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int de
     // one-pass form of the same block shape
     if (per_event && v >= PHS_F64_VARIANTS_PER_EVENT) v -= 4;
     cudaError_t e = cudaSuccess;
-    if (v != 0 && v != 3 && v != 4) e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), st);
-    if (e == cudaSuccess && v >= PHS_F64_VARIANTS_PER_EVENT)
-      e = cudaMemsetAsync(a.pass_count, 0, (size_t)a.n_segments * sizeof(unsigned int), st);
+    const bool split = v >= PHS_F64_VARIANTS_PER_EVENT;
+    if (v != 0 && v != 3 && v != 4)
+      e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long) + (split ? (size_t)a.n_segments * sizeof(unsigned int) : 0), st);
     if (e != cudaSuccess) return e;
     return phs_launch_forward_f64(a, grid_for(a.n_tiles, device, depth, per_event, v), v, st);
   });

@@ -746,6 +746,33 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
   return ok;
 }
 
+// The split forms' claim numbering: tile[s] = sum over the segments before s of ceil(count / 32),
+// tile[n] the total.  Up to PHS_INLINE_SEGS segments every block of the walk forms it from the
+// pre-test's counts in shared memory (a launch for it, and one for its counters, took 5 us of a
+// call); more come from phs_count_scan_kernel.  Collective over the block.
+__device__ __forceinline__ const int64_t *claim_numbering(const PhsLaunch &a, int64_t *shared) {
+  if (a.n_segments > PHS_INLINE_SEGS) return a.pass_tile;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int64_t carry = 0;
+    for (int base = 0; base < a.n_segments; base += 32) {
+      const int s = base + lane;
+      const int64_t v = s < a.n_segments ? ((int64_t)a.pass_count[s] + 31) / 32 : 0;
+      int64_t inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (s < a.n_segments) shared[s] = carry + inc - v;
+      carry += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) shared[a.n_segments] = carry;
+  }
+  __syncthreads();
+  return shared;
+}
+
 // The persistent loop of the compacting kernels.  Each warp runs pass A on its 32-event
 // tiles (`pass_a(seg, local)` tests an event, writes it if it fails, and returns whether it
 // passed) and appends the passing events to its queue in shared memory (q: 64 slots);

@@ -69,7 +69,9 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
   const FxRegs k = fx_regs();
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
-  const int64_t n_claims = a.pass_tile[a.n_segments];
+  __shared__ int64_t tiles[PHS_INLINE_SEGS + 1];
+  const int64_t *pass_tile = claim_numbering(a, tiles);
+  const int64_t n_claims = pass_tile[a.n_segments];
   for (;;) {
     unsigned long long c = 0;
     if (lane == 0) c = atomicAdd(a.work, 1ull);
@@ -79,10 +81,10 @@ __global__ void __launch_bounds__(BLOCK, MIN_BLOCKS)
     int lo = 0, hi = a.n_segments - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (a.pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
+      if (pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
     }
     const PhsSegment seg = segs[lo];
-    const int64_t idx = (t - a.pass_tile[lo]) * 32 + lane;
+    const int64_t idx = (t - pass_tile[lo]) * 32 + lane;
     if (idx >= (int64_t)a.pass_count[lo]) continue;
     if (!phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) ||
         !phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE))

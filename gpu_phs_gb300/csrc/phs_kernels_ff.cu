@@ -520,30 +520,45 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 // that an event FAILS.  Each internal msq is evaluated in FP32 together with a bound on its
 // absolute error, 64 FP32 epsilons times the magnitudes of the terms it is made of (the
 // Breit-Wigner tails through the same cot reformulation as the float-float path, whose
-// tan error grows with 1 + tan^2; the exponential mappings through expm1f, whose error
-// grows with the exponent): the reference's FP64 msq, and the exact one, lie inside
+// tan error grows with 1 + tan^2; the exponential mappings, whose error grows with the
+// exponent): the reference's FP64 msq, and the exact one, lie inside
 // [msq - e, msq + e].  Masses are then intervals, and a test fails here only if it fails
 // for every value in them (with a further 1e-6 relative slack for the FP64 roundings of
 // the reference's own sums and bounds), so such an event fails the reference's test too.
 // Its outputs are written here.  Every other event goes to pass B, whose float-float /
 // FP64 walk decides its flag exactly.  Returns false for a failed event.
+//
+// Against those 64 epsilons (3.8e-6), per unit of the magnitudes: the angle of the tangent is
+// within 5e-7 (x, the constants, product and sum, rounded to nearest, of magnitudes up to pi),
+// the hardware sine and cosine within 2^-21.4 and 2^-21.2 (|w| <= pi/4), so tan or cot within
+// 1.3e-6 (1 + tan^2); the hardware exponential within 2 + 1.2 |y| epsilons, its argument within
+// 3 epsilons of |y|.  Square roots and quotients approximate to 2 epsilons, inside the 1e-6.
 #define PHS_F32_EPS_BOUND (64.0f * 5.9604645e-8f)
+// A double to the nearest float (ties away) with integer operations: the conversion unit for
+// doubles takes 16 cycles of an SM a warp.  Below 2^-126: 0; for |d| < 2^128.
+__device__ __forceinline__ float f32_of(double d) {
+  const uint64_t b = fx_bits(d) + 0x10000000ull;
+  const uint32_t hw = (uint32_t)(b >> 32), mag = hw & 0x7fffffffu;
+  return mag < (897u << 20) ? 0.0f
+                            : fx_float((hw & 0x80000000u) | ((mag - (896u << 20)) << 3) | ((uint32_t)b >> 29));
+}
+
 // c0..c5: the packed constants of PhsTestChild.
 __device__ __forceinline__ float msq_f32(int map_id, float4 c, float c4, float c5, double xd,
                                          float &e) {
-  const float x = (float)xd, k = PHS_F32_EPS_BOUND;
+  const float x = f32_of(xd), k = PHS_F32_EPS_BOUND;
   switch (map_id) {
     case PHS_MAP_NO:
       e = k * (fabsf(c.x) + fabsf(c.y));
       return c.x + x * (c.y - c.x);
     case PHS_MAP_SCHANNEL: {
-      // one tanf per lane, on z or on pi/2 -+ z (selected, not branched: lanes of a warp
+      // one tangent per lane, of z or of pi/2 -+ z (selected, not branched: lanes of a warp
       // take different sides)
       const float z = c.x + x * c.y;  // c.y holds a1 - a0
-      const bool hi_side = z > 0.78539816f, lo_side = z < -0.78539816f;
-      const float w = hi_side ? c.w + (float)(1.0 - xd) * c.y : (lo_side ? c.z + x * c.y : z);
-      const float tw = tanf(w);
-      const float t = hi_side ? 1.0f / tw : (lo_side ? -1.0f / tw : tw);
+      const bool hi_side = z > 0.78539816f, lo_side = z < -0.78539816f, cot = hi_side || lo_side;
+      const float w = hi_side ? c.w + (1.0f - x) * c.y : (lo_side ? c.z + x * c.y : z);
+      const float sw = __sinf(w), cw = __cosf(w);
+      const float q = __fdividef(cot ? cw : sw, cot ? sw : cw), t = lo_side ? -q : q;
       e = k * (fabsf(c4) + fabsf(c5) * (1.0f + t * t));
       return c4 + c5 * t;
     }
@@ -553,7 +568,7 @@ __device__ __forceinline__ float msq_f32(int map_id, float4 c, float c4, float c
     case PHS_MAP_TCHANNEL:
     case PHS_MAP_UCHANNEL: {
       const bool upper = (map_id == PHS_MAP_TCHANNEL || map_id == PHS_MAP_UCHANNEL) && !(xd < 0.5);
-      const float y = (upper ? (float)(1.0 - xd) : x) * c.y, em = expm1f(y);
+      const float y = (upper ? 1.0f - x : x) * c.y, em = __expf(y) - 1.0f;
       e = k * (fabsf(upper ? c.w : c.z) + fabsf(c.x) * (em + 1.0f) * (1.0f + fabsf(y)));
       return upper ? c.w - c.x * em : c.x * em + c.z;
     }
@@ -676,6 +691,12 @@ struct RegBounds {
   }
 };
 
+__device__ __forceinline__ float sqrt_approx(float a) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
 // staged: the channel's packed visits (PhsChannelFF::test as 4 float4 per visit) staged in
 // shared memory by the caller, or null: read from the channel program in global memory.
 template <class Bounds>
@@ -717,8 +738,8 @@ __device__ __forceinline__ bool phs_ok_f32(const PhsLaunch &a, const PhsSegment 
         const float msq = msq_f32((code >> 1) & 127, A[j], B[j].x, B[j].y,
                                   phs_in(xi, seg.x_stride, PHS_CHK_X) ? ld_x_narrow(xe + xi) : 0.0, e);
         fails = fails || msq + e < 0.0f;                // negative for certain: not ok
-        lo[j] = sqrtf(fmaxf(msq - e, 0.0f)) * dn;       // NaN bounds decide nothing
-        hi[j] = sqrtf(fmaxf(msq + e, 0.0f)) * up;
+        lo[j] = sqrt_approx(fmaxf(msq - e, 0.0f)) * dn;       // NaN bounds decide nothing
+        hi[j] = sqrt_approx(fmaxf(msq + e, 0.0f)) * up;
         cmax[j] = B[j].z;
       }
     }
@@ -957,7 +978,9 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
   ExactQueue<false> exact{exact_slots[threadIdx.x >> 5], reinterpret_cast<double *>(fst)};
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
-  const int64_t n_claims = a.pass_tile[a.n_segments];
+  __shared__ int64_t tiles[PHS_INLINE_SEGS + 1];
+  const int64_t *pass_tile = claim_numbering(a, tiles);
+  const int64_t n_claims = pass_tile[a.n_segments];
   for (;;) {
     unsigned long long c = 0;
     if (lane == 0) c = atomicAdd(a.work, 1ull);
@@ -966,13 +989,13 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
     int lo = 0, hi = a.n_segments - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (a.pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
+      if (pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
     }
     // (one call site of the exact walk, ahead of each claim: its code is large)
     exact.flush(a, segs, t < n_claims && lo == exact.seg ? 32 : 1);
     if (t >= n_claims) break;
     const PhsSegment &seg = segs[lo];
-    const int64_t idx = (t - a.pass_tile[lo]) * 32 + lane;
+    const int64_t idx = (t - pass_tile[lo]) * 32 + lane;
     const bool valid = idx < (int64_t)a.pass_count[lo] && phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) &&
                        phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE);
     const int64_t local = valid ? a.pass_queue[seg.tile_begin * 32 + idx] : 0;
@@ -996,7 +1019,8 @@ cudaError_t phs_launch_pretest(const PhsLaunch &a, cudaStream_t stream) {
   const int64_t want = (a.n_chunks + PHS_FWD_BLOCK / 32 - 1) / (PHS_FWD_BLOCK / 32);
   const int64_t cap = (int64_t)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   phs_ff_test_kernel<<<(int)(want < cap ? want : cap), PHS_FWD_BLOCK, 0, stream>>>(a);
-  phs_count_scan_kernel<<<1, 1024, 0, stream>>>(a.pass_count, a.pass_tile, a.n_segments);
+  if (a.n_segments > PHS_INLINE_SEGS)   // (up to that many: claim_numbering)
+    phs_count_scan_kernel<<<1, 1024, 0, stream>>>(a.pass_count, a.pass_tile, a.n_segments);
   return cudaGetLastError();
 }
 

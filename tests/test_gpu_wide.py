@@ -67,3 +67,29 @@ def test_wide_form_in_a_batch(torch):
     x = torch.rand(size, dtype=torch.float64, device="cuda", generator=g)
     for u, v in zip(wide.generate(x, counts), plain.generate(x, counts)):
         assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("n_channels", [1, 31, 64, 65, 90])
+def test_split_forms_over_many_segments(torch, n_channels):
+    """The split forms number their claims in shared memory up to 64 segments and with a scan
+    kernel beyond: the one-pass form's bits either way (FP64), its flags (FP32 pairs)."""
+    from gpu_phs_gb300.api import PRECISION_F32X2, Batch, PhaseSpace
+    procs, counts = P.batched(21, n_channels, 60 * n_channels)
+    spaces = [PhaseSpace(p, 0.5 * p.sqrts, 0.5 * p.sqrts) for p in procs]
+    g = torch.Generator(device="cuda").manual_seed(n_channels)
+    size = int(sum(p.n_x * int(c) for p, c in zip(procs, counts)))
+    x = torch.rand(size, dtype=torch.float64, device="cuda", generator=g)
+    plain = Batch(spaces)
+    plain.set_variants(-1, 0)
+    want = plain.generate(x, counts)
+    for v in (5, 6, 7, 8):
+        split = Batch(spaces)
+        split.set_variants(-1, v)
+        for _ in range(2):
+            for u, w in zip(split.generate(x, counts), want):
+                assert torch.equal(u, w)
+    for v in (4, 5):
+        pairs = Batch(spaces)
+        pairs.set_precision(PRECISION_F32X2)
+        pairs.set_variants(v, -1)
+        assert torch.equal(pairs.generate(x, counts)[3], want[3])
