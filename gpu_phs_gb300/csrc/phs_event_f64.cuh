@@ -133,9 +133,11 @@ __device__ __forceinline__ void map_msq(const FxRegs &k, int t, double x, double
 }
 
 // cos(theta) from x (phs_cpu.cpp:112-146).  The collinear branch keeps the reference's
-// rounding: sin(theta) = sqrt(1 - ct^2) is ill-conditioned as |ct| -> 1.  The uniform map's
-// ct = 2x - 1 and st = sqrt(4 x (1 - x)) have one rounding each before the root (the
-// reference forms 1 - x first).
+// rounding: sin(theta) = sqrt(1 - ct^2) is ill-conditioned as |ct| -> 1.  The uniform map keeps
+// the bits of ct = 1 - tmp and st = sqrt(tmp (2 - tmp)), tmp = 2 (1 - x): with 1 - x rounded, tmp
+// and ct are exact, and so tmp (2 - tmp) = 1 - ct^2 is one FMA.  (sqrt(4 x (1 - x)) is an addition
+// less and nearer to sin(theta) of x itself, but below x ~ 1e-3 it is another number than the
+// reference's, and the derivatives divide by it: 3e-12 between the gradients of 1e6 WW events.)
 __device__ __forceinline__ void map_ct(const FxRegs &k, int ct_class, double x, double b0,
                                        double b1, double &ct, double &st, double &f) {
   if (ct_class == PHS_CT_COLLINEAR) {
@@ -153,9 +155,8 @@ __device__ __forceinline__ void map_ct(const FxRegs &k, int ct_class, double x, 
       f = 0.0;
     }
   } else {
-    ct = fx_sub(k, fx_scale(x, 1), k.one);
-    const double x4 = fx_scale(x, 2);
-    st = fx_sqrt(fma(-x4, x, x4), k);
+    ct = fx_sub(k, k.one, fx_scale(fx_sub(k, k.one, x), 1));
+    st = fx_sqrt(fma(-ct, ct, k.one), k);
     f = 1.0;
   }
 }
