@@ -19,8 +19,10 @@
 // forms and the energies from the masses took 1e6 tt events from 372 to 357 us (7.9 to 7.0
 // thousand instructions a warp); a sin/cos table of 256 entries with a shorter series, exact
 // leading differences in roots and quotients, conversions through the integer-to-float unit,
-// and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 315 us.  The error of the momenta
-// went from 2.1e-14 to 1.0e-14.  Five or six blocks a SM (96, 80 registers, spills) and the
+// and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 322 us, a constant's pair in one
+// load (PhsFF) to 304 us.  The error of the momenta went from 2.1e-14 to 1.0e-14.  What waits on
+// global loads (18 % of the stalls) is the program's constants: prefetches of the x rows changed
+// nothing, and the program staged in shared memory gave tt 1 % and cost the 64-channel batch 2 %.  Five or six blocks a SM (96, 80 registers, spills) and the
 // mappings of both daughters unrolled were slower.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -866,7 +868,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
   if constexpr (COMPACT) exact.flush(a, segs, 1);
 }
 
-// Split form, kernel 1 of 3: the FP32 pre-test alone, at the occupancy its few registers
+// Split form, first kernel: the FP32 pre-test alone, at the occupancy its few registers
 // allow (the fused kernel runs it at the float-float walk's).  A warp takes a chunk of
 // a.chunk_tiles tiles of one segment; events that fail for certain get their outputs
 // here, the others are gathered in shared memory and appended to their segment's queue
@@ -932,9 +934,9 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, PHS_FF_TEST_MIN_BLOCKS)
   }
 }
 
-// Kernel 2 of 3 (one block): tile[s] = sum over the segments before s of
-// ceil(count / 32), the dense numbering of the next kernel's warp claims; tile[n] is their
-// total.
+// Between the two with more than PHS_INLINE_SEGS segments (one block): tile[s] = sum over the
+// segments before s of ceil(count / 32), the dense numbering of the next kernel's warp claims;
+// tile[n] is their total.
 __global__ void __launch_bounds__(1024)
     phs_count_scan_kernel(const unsigned int *count, int64_t *tile, int n) {
   __shared__ int64_t warp_sum[32];
@@ -963,7 +965,7 @@ __global__ void __launch_bounds__(1024)
   if (threadIdx.x == 0) tile[n] = carry;
 }
 
-// Kernel 3 of 3: the float-float walk over the queued events, 32 of one segment per warp
+// Second kernel: the float-float walk over the queued events, 32 of one segment per warp
 // claim (a.work counts the claims, zeroed before the launch), so every warp runs one
 // channel's program with all lanes busy except at a segment's last claim.
 template <int MIN_BLOCKS>
@@ -1025,7 +1027,7 @@ cudaError_t phs_launch_pretest(const PhsLaunch &a, cudaStream_t stream) {
 }
 
 // variant bit 0: register budget for 4 (1) or 3 (0) resident blocks; bit 1: compacting
-// (fused pre-test); variants 4 and 5: the split form (pre-test kernel, scan, walk kernel).
+// (fused pre-test); variants 4 and 5: the split form (pre-test kernel, walk kernel).
 static size_t ff_walk_smem_bytes(int stack_depth) {
   return sizeof(FFTables) + (size_t)stack_depth * (PHS_FF_STATE / 2) * PHS_FWD_BLOCK * sizeof(float2);
 }
