@@ -331,8 +331,8 @@ def measure_variants(torch, steps: int, warmup: int, x_tt, out_tt, ms_tt64, pin=
         "n_channels": 64, "n_events": n, "n_out_range": [3, 8],
         "counts": "power law, exponent 1.5, seed 2024",
         "launch": "one CUDA-graph replay per step: one pass and compacting are one "
-                  "persistent kernel; the split forms replay the FP32 pre-test, a scan, the "
-                  "walk and (FP32 pairs) the exact FP64 path's scan and kernel",
+                  "persistent kernel; the split forms replay the FP32 pre-test and the walk "
+                  "(FP32 pairs: undecided events in the walk's own FP64 queue)",
         **{f"{k}_events_per_s": n / bres[k] * 1e3 for k, _, _ in forms},
         "kernel_variants": tuned,
         "speedup_vs_plain_fp64": bres["fp64_one_pass"] / bres["fp32_mixed"],
