@@ -20,10 +20,11 @@
 // thousand instructions a warp); a sin/cos table of 256 entries with a shorter series, exact
 // leading differences in roots and quotients, conversions through the integer-to-float unit,
 // and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 322 us, a constant's pair in one
-// load (PhsFF) to 304 us.  The error of the momenta went from 2.1e-14 to 1.0e-14.  What waits on
-// global loads (18 % of the stalls) is the program's constants: prefetches of the x rows changed
-// nothing, and the program staged in shared memory gave tt 1 % and cost the 64-channel batch 2 %.  Five or six blocks a SM (96, 80 registers, spills) and the
-// mappings of both daughters unrolled were slower.
+// load (PhsFF) to 304 us, outputs widened with integers (ff_to_double_int) to 267 us.  The error
+// of the momenta went from 2.1e-14 to 1.0e-14.  What waits on global loads (18 % of the stalls) is
+// the program's constants: prefetches of the x rows changed nothing, and the program staged in
+// shared memory gave tt 1 % and cost the 64-channel batch 2 %.  Five or six blocks a SM (96, 80
+// registers, spills) and the mappings of both daughters unrolled were slower.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -177,25 +178,16 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
   return false;
 }
 
-// A pair as a double: two exact widenings and one add on the FP64 pipe (uniform beams,
-// where the walk is bound by FP32 issue), or with integer operations (per-event beams, where
-// the per-event constants keep the FP64 pipe busy).
-template <bool INT>
-__device__ __forceinline__ double widen(ff a) {
-  return INT ? ff_to_double_int(a) : ff_to_double(a);
-}
-
 __device__ __forceinline__ ff ff_twice(ff a) { return ff_make(f_add(a.hi, a.hi), f_add(a.lo, a.lo)); }
 __device__ __forceinline__ ff ff_half(ff a) { return ff_make(f_mul(a.hi, 0.5f), f_mul(a.lo, 0.5f)); }
 
 // A leaf's momentum row, from pairs that need not be normalized.
-template <bool INT>
 __device__ __forceinline__ void put_momentum_ff(double *out, int index, int n_out, const ff q[4]) {
   if (!phs_in(index, n_out, PHS_CHK_P)) return;
   double2 *o = reinterpret_cast<double2 *>(out + 4 * index);
   double d[4];
 #pragma unroll
-  for (int r = 0; r < 4; r++) d[r] = widen<INT>(INT ? ff_normalize(q[r]) : q[r]);
+  for (int r = 0; r < 4; r++) d[r] = ff_to_double_int(q[r]);
   o[0] = make_double2(d[0], d[1]);
   o[1] = make_double2(d[2], d[3]);
 }
@@ -428,8 +420,8 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
           qb[r] = ff_dot2_add_raw(l0, qb0, l3, qb3, ff_neg(w));
         }
       }
-      put_momentum_ff<PER_EVENT>(out, V.child[0].out_index, ch.n_out, qa);
-      put_momentum_ff<PER_EVENT>(out, V.child[1].out_index, ch.n_out, qb);
+      put_momentum_ff(out, V.child[0].out_index, ch.n_out, qa);
+      put_momentum_ff(out, V.child[1].out_index, ch.n_out, qb);
     } else {
       // rotation + boost of the visited branch (friend steps take the exact path)
       if (!V.self_root) {
@@ -477,7 +469,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
         ff q[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) q[r] = ff_dot2_raw(L[4 * r], E, L[4 * r + 3], pj);
-        put_momentum_ff<PER_EVENT>(out, C.out_index, ch.n_out, q);
+        put_momentum_ff(out, C.out_index, ch.n_out, q);
       }
     }
 
@@ -509,7 +501,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
   }
 
   a.volume[ev] = PER_EVENT ? channel_volume(a.channels[seg.channel], sqrts64) : ch.volume;
-  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? widen<PER_EVENT>(factor) : 0.0;
+  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? ff_to_double_int(factor) : 0.0;
   a.ok[ev] = ok ? 1 : 0;
   if (!ok) {
     double2 *o = reinterpret_cast<double2 *>(out);

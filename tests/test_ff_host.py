@@ -237,3 +237,49 @@ def test_float_pair_functions_against_long_double():
     bars = [2e-13, 2e-13, 5e-13, 5e-13] + [1e-13] * 6
     for name, got, bar in zip(names, w, bars):
         assert got <= bar, f"{name}: {got:.3g} > {bar:g}"
+
+
+WIDEN_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <cfloat>
+#include <cstring>
+#include "phs_ff.h"
+static bool same(double a, double b) { return (a != a && b != b) || a == b; }
+int main() {
+  long n = 0, bad = 0;
+  // every exponent and sign with significands at their ends, and infinities and NaN
+  const uint32_t fr[] = {0u, 1u, 2u, 0x3fffffu, 0x400000u, 0x555555u, 0x7ffffeu, 0x7fffffu};
+  for (uint32_t top = 0; top < 512; top++)
+    for (uint32_t f : fr) {
+      const float v = ff_bitsf(top << 23 | f);
+      const double want = std::fabs(v) < FLT_MIN ? 0.0 : (double)v;
+      if (!same(ff_widen(v), want)) bad++;
+      // a pair: the sum of the two, rounded once (any exponents, signs and order)
+      for (uint32_t t2 = 0; t2 < 512; t2 += 3) {
+        const float w = ff_bitsf(t2 << 23 | (f ^ 0x2aaaaau));
+        const double sum = want + (std::fabs(w) < FLT_MIN ? 0.0 : (double)w);
+        if (!same(ff_to_double_int(ff_make(v, w)), sum)) bad++;
+        n++;
+      }
+    }
+  std::printf("%ld %ld\n", n, bad);
+  return 0;
+}
+"""
+
+
+def test_widening_of_floats_is_exact():
+    try:
+        subprocess.run(["g++", "--version"], check=True, capture_output=True)
+    except (OSError, subprocess.CalledProcessError):
+        pytest.skip("g++ not available")
+    with tempfile.TemporaryDirectory() as d:
+        src, exe = os.path.join(d, "w.cpp"), os.path.join(d, "w")
+        with open(src, "w") as fh:
+            fh.write(WIDEN_DRIVER)
+        subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=c++17", "-I", CSRC, src, "-o", exe],
+                       check=True)
+        n, bad = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
+    assert int(n) > 600_000
+    assert int(bad) == 0
