@@ -394,10 +394,7 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
       PhsChildFF &G = F.child[j];
-      G.internal = C.internal;
-      G.out_index = C.out_index;
-      G.map_id = C.map_id;
-      G.x_msq = C.x_msq;
+      F.child_code[j] = C.internal | C.map_id << 1 | (C.x_msq & 0xff) << 8 | (C.out_index & 0xff) << 16;
       G.msq_leaf = split(C.msq_leaf);
       G.m_leaf = split(C.m_leaf);
       G.m2 = split(C.m * C.m);
@@ -418,21 +415,16 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
       if (C.internal && (C.map_id == PHS_MAP_STEP_E || C.map_id == PHS_MAP_STEP_H)) out.exact_only = 1;
     }
     if (V.friend_sign) out.exact_only = 1;
-    F.x_phi = V.x_phi;
-    F.x_ct = V.x_ct;
-    F.ct_class = V.ct_class;
-    F.carry = V.carry;
-    F.push = V.push;
-    F.self_root = V.self_root;
-    F.massless = V.massless;
-    F.kind = V.kind;
+    F.code = V.x_phi | V.x_ct << 8 | V.ct_class << 16 | V.self_root << 17 | V.massless << 18 |
+             V.kind << 20 | (V.carry + 1) << 23 | (V.push + 1) << 25;
     F.b0 = split(V.b0);
     F.b1 = split(V.b1);
     PhsTestVisit &P = out.test[v];
     for (int j = 0; j < 2; j++) {
       const PhsChildFF &G = F.child[j];
+      const PhsChild &C = V.child[j];
       PhsTestChild &Q = P.child[j];
-      switch (G.map_id) {
+      switch (C.map_id) {
         case PHS_MAP_NO:
           Q.c[0] = G.msq_min.hi;
           Q.c[1] = G.msq_max.hi;
@@ -451,8 +443,8 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
           Q.c[2] = G.msq_min.hi;
           Q.c[3] = G.msq_max.hi;
       }
-      Q.m = G.internal ? G.m_max.hi : G.m_leaf.hi;
-      Q.code = (G.internal ? 1 : 0) | (G.map_id & 127) << 1 | (G.x_msq & 255) << 8;
+      Q.m = C.internal ? G.m_max.hi : G.m_leaf.hi;
+      Q.code = (C.internal ? 1 : 0) | (C.map_id & 127) << 1 | (C.x_msq & 255) << 8;
     }
     P.child[0].code |= (V.push + 1) << 16 | (V.carry + 1) << 18 | (V.self_root ? 1 : 0) << 20;
   }

@@ -20,8 +20,9 @@
 // thousand instructions a warp); a sin/cos table of 256 entries with a shorter series, exact
 // leading differences in roots and quotients, conversions through the integer-to-float unit,
 // and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 322 us, a constant's pair in one
-// load (PhsFF) to 304 us, outputs widened with integers (ff_to_double_int) to 267 us.  The error
-// of the momenta went from 2.1e-14 to 1.0e-14.  What waits on global loads (18 % of the stalls) is
+// load (PhsFF) to 304 us, outputs widened with integers (ff_to_double_int) to 270 us, a visit's
+// integers in one load (PhsVisitFF) to 263 us.  The error of the momenta went from 2.1e-14 to
+// 1.0e-14.  What waits on global loads (18 % of the stalls) is
 // the program's constants: prefetches of the x rows changed nothing, and the program staged in
 // shared memory gave tt 1 % and cost the 64-channel batch 2 %.  Five or six blocks a SM (96, 80
 // registers, spills) and the mappings of both daughters unrolled were slower.
@@ -72,7 +73,7 @@ struct ChildVar {
 __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C) {
   return {ld(C.a1), ld(C.a2), ld(C.u1), ld(C.msq_max), ld(C.m_max)};
 }
-__device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChild &C64,
+__device__ __forceinline__ ChildVar child_var(int map_id, const PhsChildFF &C, const PhsChild &C64,
                                               double sqrts, double m_tot, double inv_s) {
   double a0, a1, a2, mn, mx, mmax;
   child_constants(fx_regs(), C64, sqrts, m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
@@ -81,7 +82,7 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChil
   r.a2 = ff_from_double_int(a2);
   r.msq_max = ff_from_double_int(mx);
   r.m_max = ff_from_double_int(mmax);
-  if (C.map_id == PHS_MAP_SCHANNEL) {
+  if (map_id == PHS_MAP_SCHANNEL) {
     r.a1 = ff_from_double_int(a1 - a0);
     // pi/2 - a1: exact for a1 >= pi/4 (the only case that uses it), then pi/2's low part
     r.u1 = ff_from_double_int((1.5707963267948966 - a1) + 6.123233995736766e-17);
@@ -97,13 +98,13 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChil
 // a1 = atan(u) = pi/2 - atan(1/u) and atan(w) = w - w^3/3 + w^5/5 for w = 1/u (the next term
 // is below 2^-72 of pi/2, as in phs_math.h); pi/2 - a1 is that series itself.  Other maps
 // and smaller u take the FP64 constants.  sqrts, inv_s: the event's sqrt(s) and 1/s.
-__device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChild &C64, ff sqrts,
+__device__ __forceinline__ ChildVar child_var(int map_id, const PhsChildFF &C, const PhsChild &C64, ff sqrts,
                                               ff inv_s, ff m_tot, double sqrts64, double m_tot64) {
-  if (C.map_id == PHS_MAP_NO || C.map_id == PHS_MAP_SCHANNEL) {
+  if (map_id == PHS_MAP_NO || map_id == PHS_MAP_SCHANNEL) {
     ChildVar r;
     r.m_max = ff_add(ff_sub(sqrts, m_tot), ld(C.m_min));
     r.msq_max = ff_sqr(r.m_max);
-    if (C.map_id == PHS_MAP_NO) {
+    if (map_id == PHS_MAP_NO) {
       r.a1 = ff_sub(r.msq_max, ld(C.msq_min));
       r.a2 = ff_mul(r.a1, inv_s);
       r.u1 = ff_from_float(0.0f);
@@ -120,7 +121,7 @@ __device__ __forceinline__ ChildVar child_var(const PhsChildFF &C, const PhsChil
     }
   }
   const double s64 = dmul(sqrts64, sqrts64);
-  return child_var(C, C64, sqrts64, m_tot64, 1.0 / s64);
+  return child_var(map_id, C, C64, sqrts64, m_tot64, 1.0 / s64);
 }
 
 // 1 - x: on the FP64 pipe (uniform beams, where it is mostly idle), or with integer operations.
@@ -134,10 +135,10 @@ __device__ __forceinline__ ff one_minus(double x) {
 // x arrives as a float-float pair truncated from the double, so x < 0.5 is decided on its
 // high part exactly as the reference decides it on the double.
 template <bool INT>
-__device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &cv, double xd,
+__device__ __forceinline__ bool map_msq_ff(int map_id, const PhsChildFF &C, const ChildVar &cv, double xd,
                                            const FFTables &T, ff &msq, ff &f) {
   const ff x = ff_from_double_int(xd);
-  switch (C.map_id) {
+  switch (map_id) {
     case PHS_MAP_NO:
       msq = ff_add(ld(C.msq_min), ff_mul(x, ff_sub(cv.msq_max, ld(C.msq_min))));
       f = ff_from_float(1.0f);
@@ -167,7 +168,7 @@ __device__ __forceinline__ bool map_msq_ff(const PhsChildFF &C, const ChildVar &
     case PHS_MAP_UCHANNEL: {
       // one exponential for all five: the t/u-channel maps take x >= 0.5 from the other
       // end, with the argument and the sum selected per lane
-      const bool upper = (C.map_id == PHS_MAP_TCHANNEL || C.map_id == PHS_MAP_UCHANNEL) && !(x.hi < 0.5f);
+      const bool upper = (map_id == PHS_MAP_TCHANNEL || map_id == PHS_MAP_UCHANNEL) && !(x.hi < 0.5f);
       const ff msq1 = ff_mul(ld(C.a0), ff_exp(ff_mul(upper ? one_minus<INT>(xd) : x, cv.a1), T));
       msq = upper ? ff_add(ff_sub(ld(C.a0), msq1), cv.msq_max)
                   : ff_add(ff_sub(msq1, ld(C.a0)), ld(C.msq_min));
@@ -263,6 +264,9 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisitFF &V = ch.visit[v];
+    const int4 head = *reinterpret_cast<const int4 *>(&V.code);   // (code, child_code)
+    const int code = head.x;
+    const bool self_root = code >> 17 & 1;
     ff cmsq[2] = {ld(V.child[0].msq_leaf), ld(V.child[1].msq_leaf)};
     ff cm[2] = {ld(V.child[0].m_leaf), ld(V.child[1].m_leaf)};
     bool exact = false;
@@ -270,15 +274,16 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 #pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChildFF &C = V.child[j];
-      if (!C.internal) continue;
+      const int cc = j == 0 ? head.y : head.z, map_id = cc >> 1 & 15;
+      if (!(cc & 1)) continue;
       ff f = one, mq = zero;
       const ChildVar cv = PER_EVENT
-          ? child_var(C, a.channels[seg.channel].visit[v].child[j], sqrts_f, inv_s_f, ld(ch.m_tot),
+          ? child_var(map_id, C, a.channels[seg.channel].visit[v].child[j], sqrts_f, inv_s_f, ld(ch.m_tot),
                       sqrts64, a.channels[seg.channel].m_tot)
           : child_var(C);
-      if (!map_msq_ff<PER_EVENT>(C, cv, xrow_at(xe, C.x_msq, seg.x_stride), T, mq, f)) exact = true;
+      if (!map_msq_ff<PER_EVENT>(map_id, C, cv, xrow_at(xe, cc >> 8 & 0xff, seg.x_stride), T, mq, f)) exact = true;
       if (PER_EVENT) factor = ff_mul(factor, cv.a2);
-      if (C.map_id != PHS_MAP_NO) factor = ff_mul(factor, f);
+      if (map_id != PHS_MAP_NO) factor = ff_mul(factor, f);
       if (msq_near_zero(mq, s_scale)) exact = true;
       if (mq.hi < 0.0f) {  // the reference takes sqrt of a negative: not ok
         ok = false;
@@ -300,12 +305,12 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
     }
     if (exact) return false;
     // the test's lower bound m > m1 + m2, likewise
-    const int massless = V.massless;
+    const int massless = code >> 18 & 3;
     const ff msum = massless == 0 ? ff_add(cm[0], cm[1]) : massless == 3 ? zero : ffsel(massless & 1, cm[1], cm[0]);
     const ff dlo = massless == 3 ? m_b : ff_sub(m_b, msum);
     if (near_zero(dlo, m_b.hi)) return false;
     ok = ok && dlo.hi > 0.0f;
-    int kind = V.kind;
+    int kind = code >> 20 & 7;
     if (lab)
       kind = kind == PHS_KIND_ROOT ? PHS_KIND_ROOT_LAB
              : kind == PHS_KIND_FIRST ? PHS_KIND_FIRST_LAB
@@ -318,7 +323,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       pc = ce0 = ce1 = ff_half(m_b);
       if (!pair && m_b.hi > 0.0f) rm = ff_recip_fast(m_b);   // n_out = 2
     } else {
-      rm = !PER_EVENT && V.self_root ? ld(ch.inv_sqrts) : (m_b.hi > 0.0f ? ff_recip_fast(m_b) : zero);
+      rm = !PER_EVENT && self_root ? ld(ch.inv_sqrts) : (m_b.hi > 0.0f ? ff_recip_fast(m_b) : zero);
       ff sl;
       if (massless != 0) {
         sl = ff_mul(dlo, ff_add(m_b, msum));               // m^2 - m_j^2
@@ -346,9 +351,9 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 
     // the decay angles
     StepFF t;
-    ff_sincos2pi(ff_from_double_int(xrow_at(xe, V.x_phi, seg.x_stride)), T, t.sp, t.cp);
-    const double xctd = xrow_at(xe, V.x_ct, seg.x_stride);
-    if (V.ct_class == PHS_CT_COLLINEAR) {
+    ff_sincos2pi(ff_from_double_int(xrow_at(xe, code & 0xff, seg.x_stride)), T, t.sp, t.cp);
+    const double xctd = xrow_at(xe, code >> 8 & 0xff, seg.x_stride);
+    if (code >> 16 & 1) {   // PHS_CT_COLLINEAR
       const ff xct = ff_from_double_int(xctd);
       ff b0 = ld(V.b0), b1 = ld(V.b1), fct;
       if (PER_EVENT) {
@@ -420,11 +425,11 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
           qb[r] = ff_dot2_add_raw(l0, qb0, l3, qb3, ff_neg(w));
         }
       }
-      put_momentum_ff(out, V.child[0].out_index, ch.n_out, qa);
-      put_momentum_ff(out, V.child[1].out_index, ch.n_out, qb);
+      put_momentum_ff(out, head.y >> 16, ch.n_out, qa);
+      put_momentum_ff(out, head.z >> 16, ch.n_out, qb);
     } else {
       // rotation + boost of the visited branch (friend steps take the exact path)
-      if (!V.self_root) {
+      if (!self_root) {
         t.bg = ff_mul(p_b, rm);
         t.ga = ff_mul(E_b, rm);
       }
@@ -462,19 +467,20 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       }
       // leaf momenta L_new (E, 0, 0, +-p) (a loop that is not unrolled, as in phs_event_f64)
 #pragma unroll 1
-      for (int j = V.child[0].internal ? (V.child[1].internal ? 2 : 1) : 0; j < 2; j++) {
-        const PhsChildFF &C = V.child[j];
-        if (C.internal) break;
+      for (int j = head.y & 1 ? (head.z & 1 ? 2 : 1) : 0; j < 2; j++) {
+        const int cc = j == 0 ? head.y : head.z;
+        if (cc & 1) break;
         const ff E = ffsel(j == 0, ce0, ce1), pj = j == 0 ? pc : ff_neg(pc);
         ff q[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) q[r] = ff_dot2_raw(L[4 * r], E, L[4 * r + 3], pj);
-        put_momentum_ff(out, C.out_index, ch.n_out, q);
+        put_momentum_ff(out, cc >> 16, ch.n_out, q);
       }
     }
 
-    if (V.push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
-      const bool j0 = V.push == 0;
+    const int push = (code >> 25 & 3) - 1, carry = (code >> 23 & 3) - 1;
+    if (push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
+      const bool j0 = push == 0;
 #pragma unroll
       for (int i = 0; i < 16; i++) fstack_store(fst, sp, i, L[i]);
       fstack_store(fst, sp, 16, ffsel(j0, cmsq[0], cmsq[1]));
@@ -483,8 +489,8 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       fstack_store(fst, sp, 19, ffsel(j0, ce0, ce1));
       sp++;
     }
-    if (V.carry >= 0) {
-      const bool j0 = V.carry == 0;
+    if (carry >= 0) {
+      const bool j0 = carry == 0;
       msq_b = ffsel(j0, cmsq[0], cmsq[1]);
       m_b = ffsel(j0, cm[0], cm[1]);
       p_b = j0 ? pc : ff_neg(pc);

@@ -141,12 +141,11 @@ struct PhsSegment {
 // ------------------------------------------------------------------------------------
 // Float-float form of a channel program, for the FP32-pipe kernel: every constant is a
 // pair of floats hi + lo (about 48 bits).  Built on the host from PhsChannel.
-struct alignas(8) PhsFF {  // (a pair is one load: two took 17 of 322 us for 1e6 tt events)
+struct alignas(8) PhsFF {  // (a pair is one load: two took 18 of 322 us for 1e6 tt events)
   float hi, lo;
 };
 
 struct PhsChildFF {
-  int32_t internal, out_index, map_id, x_msq;
   PhsFF msq_leaf, m_leaf;
   PhsFF m2, mw;       // Breit-Wigner: m^2 and m*w
   PhsFF a0, a1, a2;   // mapping constants; Breit-Wigner keeps a1 - a0 in a1
@@ -156,10 +155,13 @@ struct PhsChildFF {
   PhsFF inv_mw;       // Breit-Wigner: 1 / (m w) (per-event a1)
 };
 
-struct PhsVisitFF {
+// The visit's integers (as in PhsVisit and PhsChild) in one 16-byte load: x_phi | x_ct << 8 |
+// ct_class << 16 | self_root << 17 | massless << 18 | kind << 20 | (carry + 1) << 23 |
+// (push + 1) << 25, and per child internal | map_id << 1 | x_msq << 8 | out_index << 16.
+// (A load each, they took 7 of 270 us for 1e6 tt events, 17 of 219 for 5e5 with their own beams.)
+struct alignas(16) PhsVisitFF {
+  int32_t code, child_code[2], pad;
   PhsChildFF child[2];
-  int32_t x_phi, x_ct, ct_class, carry, push, self_root;
-  int32_t massless, kind;  // as in PhsVisit
   PhsFF b0, b1;
 };
 
