@@ -282,6 +282,15 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
     }
   }
   out.n_visits = v;
+  for (int u = 0; u < v; u++) {
+    PhsVisit &V = out.visit[u];
+    V.code = V.x_phi | V.x_ct << 8 | V.ct_class << 16 | V.self_root << 17 | V.massless << 18 |
+             V.kind << 20 | (V.carry + 1) << 23 | (V.push + 1) << 25;
+    for (int j = 0; j < 2; j++) {
+      const PhsChild &C = V.child[j];
+      V.child_code[j] = C.internal | C.map_id << 1 | (C.x_msq & 0xff) << 8 | (C.out_index & 0xff) << 16;
+    }
+  }
   {
     // the visit of each internal daughter: the next one (carry), or the one after the pop
     std::vector<std::pair<int, int>> pushed;
@@ -394,7 +403,6 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
       PhsChildFF &G = F.child[j];
-      F.child_code[j] = C.internal | C.map_id << 1 | (C.x_msq & 0xff) << 8 | (C.out_index & 0xff) << 16;
       G.msq_leaf = split(C.msq_leaf);
       G.m_leaf = split(C.m_leaf);
       G.m2 = split(C.m * C.m);
@@ -415,8 +423,8 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
       if (C.internal && (C.map_id == PHS_MAP_STEP_E || C.map_id == PHS_MAP_STEP_H)) out.exact_only = 1;
     }
     if (V.friend_sign) out.exact_only = 1;
-    F.code = V.x_phi | V.x_ct << 8 | V.ct_class << 16 | V.self_root << 17 | V.massless << 18 |
-             V.kind << 20 | (V.carry + 1) << 23 | (V.push + 1) << 25;
+    F.code = V.code;
+    for (int j = 0; j < 2; j++) F.child_code[j] = V.child_code[j];
     F.b0 = split(V.b0);
     F.b1 = split(V.b1);
     PhsTestVisit &P = out.test[v];

@@ -449,20 +449,23 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
+    const int4 head = *reinterpret_cast<const int4 *>(&V.code);   // (code, child_code)
+    const int code = head.x;
     double cmsq[2] = {V.child[0].msq_leaf, V.child[1].msq_leaf}, cm[2] = {V.child[0].m_leaf, V.child[1].m_leaf};
     // (not unrolled: the mapping code of one daughter serves both)
 #pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
-      if (C.internal) {
+      const int cc = j == 0 ? head.y : head.z, map_id = cc >> 1 & 15;
+      if (cc & 1) {
         double mq, mj;
         double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
         if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
         double f, aux;
-        map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
+        map_msq(k, map_id, xrow_at(xe, cc >> 8 & 0xff, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
                 mq, f, aux);
-        if (PER_EVENT && C.map_id != PHS_MAP_STEP_E && C.map_id != PHS_MAP_STEP_H) factor = fx_mul(k, factor, a2);
-        if (C.map_id != PHS_MAP_NO) factor = fx_mul(k, factor, f);
+        if (PER_EVENT && map_id != PHS_MAP_STEP_E && map_id != PHS_MAP_STEP_H) factor = fx_mul(k, factor, a2);
+        if (map_id != PHS_MAP_NO) factor = fx_mul(k, factor, f);
         mj = fx_sqrt(mq, k);
         ok = ok && !fx_gt(mj, mmax);   // NaN fails at the daughter's own visit
         if (j == 0) {
@@ -475,7 +478,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
       }
     }
     // Kallen function and kinematic test at the visited branch (phs_cpu.cpp:218-233)
-    const int massless = V.massless;
+    const int massless = code >> 18 & 3;
     double sl;
     ok = kallen_ok(k, massless, msq_b, m_b, cmsq, cm, sl) && ok;
     // one reciprocal of m serves p_decay = sqrt(lda)/(2m), sqrt(lda)/m^2, bg, gamma and the
@@ -484,7 +487,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
     // Two massless daughters share m equally, their sqrt(lda)/m^2 is 1, and as the last
     // visit of their line nothing else needs 1/m.  sqrt(lda)/m^2 is kept halved, the powers
     // of two put back at the end.
-    int kind = V.kind;
+    int kind = code >> 20 & 7;
     if (lab)
       kind = kind == PHS_KIND_ROOT ? PHS_KIND_ROOT_LAB
              : kind == PHS_KIND_FIRST ? PHS_KIND_FIRST_LAB
@@ -496,7 +499,7 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
       if (!pair) rm = fx_hi(m_b) - 1u < 0x7fefffffu ? fx_rcp(m_b, k) : 0.0;   // a friend's, or n_out = 2
     } else {
       double hm;
-      if (!PER_EVENT && V.self_root) {
+      if (!PER_EVENT && (code >> 17 & 1)) {
         rm = ch.inv_sqrts;
         hm = fx_scale(rm, -1);
       } else {
@@ -518,15 +521,15 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
 
     // the decay angles
     Step t;
-    sincos2pi(xrow_at(xe, V.x_phi, seg.x_stride), t.sp, t.cp);
+    sincos2pi(xrow_at(xe, code & 0xff, seg.x_stride), t.sp, t.cp);
     double b0 = V.b0, b1 = V.b1;
-    if (PER_EVENT && V.ct_class == PHS_CT_COLLINEAR) {
+    if (PER_EVENT && (code >> 16 & 1) == PHS_CT_COLLINEAR) {
       b0 = dmul(V.m, V.m) / s;
       b1 = log(dadd(b0, 1.0) / b0);
     }
     double fct;
-    map_ct(k, V.ct_class, xrow_at(xe, V.x_ct, seg.x_stride), b0, b1, t.ct, t.st, fct);
-    if (V.ct_class == PHS_CT_COLLINEAR) factor = fx_mul(k, factor, fct);   // the uniform map's factor is 1
+    map_ct(k, (code >> 16 & 1), xrow_at(xe, code >> 8 & 0xff, seg.x_stride), b0, b1, t.ct, t.st, fct);
+    if ((code >> 16 & 1) == PHS_CT_COLLINEAR) factor = fx_mul(k, factor, fct);   // the uniform map's factor is 1
 
     if (pair) {
       // two outgoing daughters: (E, 0, 0, +-p) rotated by (theta, phi), boosted along z by
@@ -569,11 +572,11 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
           qb[r] = fma(l0, qb0, fma(l3, qb3, -w));
         }
       }
-      put_momentum(out, V.child[0].out_index, ch.n_out, qa[0], qa[1], qa[2], qa[3]);
-      put_momentum(out, V.child[1].out_index, ch.n_out, qb[0], qb[1], qb[2], qb[3]);
+      put_momentum(out, head.y >> 16, ch.n_out, qa[0], qa[1], qa[2], qa[3]);
+      put_momentum(out, head.z >> 16, ch.n_out, qb[0], qb[1], qb[2], qb[3]);
     } else {
       // rotation + boost of the visited branch (phs_cpu.cpp:299-330)
-      if (!V.self_root) {
+      if (!(code >> 17 & 1)) {
         t.bg = fx_mul(k, p_b, rm);
         t.ga = fx_mul(k, E_b, rm);
       }
@@ -619,21 +622,22 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
       // leaf momenta: L_new * (E, 0, 0, +-p) (phs_cpu.cpp:286-291).  (A loop that is not
       // unrolled: the compiler would issue the FP64 instructions of an absent leaf too.)
 #pragma unroll 1
-      for (int j = V.child[0].internal ? (V.child[1].internal ? 2 : 1) : 0; j < 2; j++) {
-        const PhsChild &C = V.child[j];
-        if (C.internal) break;
+      for (int j = head.y & 1 ? (head.z & 1 ? 2 : 1) : 0; j < 2; j++) {
+        const int cc = j == 0 ? head.y : head.z;
+        if (cc & 1) break;
         const double E = j == 0 ? ce0 : ce1, pj = j == 0 ? pc : fx_neg(pc);
         double q[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) q[r] = fma(L[4 * r], E, fx_mul(k, L[4 * r + 3], pj));
-        put_momentum(out, C.out_index, ch.n_out, q[0], q[1], q[2], q[3]);
+        put_momentum(out, cc >> 16, ch.n_out, q[0], q[1], q[2], q[3]);
       }
     }
 
     // next frame: push one internal child, carry the other (or pop)
     // (selects instead of indexing keep the child values in registers)
-    if (V.push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
-      const bool j0 = V.push == 0;
+    const int push = (code >> 25 & 3) - 1, carry = (code >> 23 & 3) - 1;
+    if (push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
+      const bool j0 = push == 0;
 #pragma unroll
       for (int i = 0; i < 16; i++) stack_store<BLOCK>(smem, sp, i, L[i]);
       stack_store<BLOCK>(smem, sp, 16, j0 ? cmsq[0] : cmsq[1]);
@@ -642,8 +646,8 @@ __device__ __forceinline__ void phs_event_f64(const PhsLaunch &a, const FxRegs &
       stack_store<BLOCK>(smem, sp, 19, j0 ? ce0 : ce1);
       sp++;
     }
-    if (V.carry >= 0) {
-      const bool j0 = V.carry == 0;
+    if (carry >= 0) {
+      const bool j0 = carry == 0;
       msq_b = j0 ? cmsq[0] : cmsq[1];
       m_b = j0 ? cm[0] : cm[1];
       p_b = j0 ? pc : fx_neg(pc);
@@ -697,17 +701,20 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
     const PhsVisit &V = ch.visit[v];
+    const int4 head = *reinterpret_cast<const int4 *>(&V.code);   // (code, child_code)
+    const int code = head.x;
     double cmsq[2] = {V.child[0].msq_leaf, V.child[1].msq_leaf}, cm[2] = {V.child[0].m_leaf, V.child[1].m_leaf};
     // (not unrolled: the mapping code of one daughter serves both)
 #pragma unroll 1
     for (int j = 0; j < 2; j++) {
       const PhsChild &C = V.child[j];
-      if (C.internal) {
+      const int cc = j == 0 ? head.y : head.z, map_id = cc >> 1 & 15;
+      if (cc & 1) {
         double mq, mj;
         double a0 = C.a0, a1 = C.a1, a2 = C.a2, mn = C.msq_min, mx = C.msq_max, mmax = C.m_max;
         if (PER_EVENT) child_constants(k, C, sqrts, ch.m_tot, inv_s, a0, a1, a2, mn, mx, mmax);
         double f, aux;
-        map_msq(k, C.map_id, xrow_at(xe, C.x_msq, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
+        map_msq(k, map_id, xrow_at(xe, cc >> 8 & 0xff, seg.x_stride), s, C.m, C.w, mn, mx, a0, a1, a2,
                 mq, f, aux);
         mj = fx_sqrt(mq, k);
         ok = ok && !fx_gt(mj, mmax);
@@ -721,15 +728,16 @@ __device__ __forceinline__ bool phs_ok_f64(const PhsLaunch &a, const FxRegs &k,
       }
     }
     double sl;
-    ok = kallen_ok(k, V.massless, msq_b, m_b, cmsq, cm, sl) && ok;
-    if (V.push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
-      const bool j0 = V.push == 0;
+    ok = kallen_ok(k, code >> 18 & 3, msq_b, m_b, cmsq, cm, sl) && ok;
+    const int push = (code >> 25 & 3) - 1, carry = (code >> 23 & 3) - 1;
+    if (push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
+      const bool j0 = push == 0;
       stack_store<BLOCK>(smem, sp, 16, j0 ? cmsq[0] : cmsq[1]);
       stack_store<BLOCK>(smem, sp, 17, j0 ? cm[0] : cm[1]);
       sp++;
     }
-    if (V.carry >= 0) {
-      const bool j0 = V.carry == 0;
+    if (carry >= 0) {
+      const bool j0 = carry == 0;
       msq_b = j0 ? cmsq[0] : cmsq[1];
       m_b = j0 ? cm[0] : cm[1];
     } else if (sp > 0) {

@@ -66,7 +66,14 @@ struct PhsChild {
   double inv_da;      //   1 / (a1 - a0) at the handle's sqrt(s) (the inverse map's divisors)
 };
 
-struct PhsVisit {
+// The integers that the forward walks read come packed in one 16-byte load: code = x_phi | x_ct << 8
+// | ct_class << 16 | self_root << 17 | massless << 18 | kind << 20 | (carry + 1) << 23 |
+// (push + 1) << 25, child_code = internal | map_id << 1 | x_msq << 8 | out_index << 16.  (A load
+// each, some twelve a visit: 1e6 tt events in FP32 pairs 270 -> 263 us, 5e5 with their own beams 219
+// -> 203; in FP64 3e5 12-particle events 224 -> 217, 2^22 events over 64 channels 578 -> 571, 1e7 tt
+// events 5200 -> 5179.)
+struct alignas(16) PhsVisit {
+  int32_t code, child_code[2], pad;
   PhsChild child[2];  // child[0] = daughters1 (+p_decay), child[1] = daughters2 (-p_decay)
   int32_t x_phi;      // index of the phi x
   int32_t x_ct;       // index of the cos(theta) x
@@ -155,10 +162,7 @@ struct PhsChildFF {
   PhsFF inv_mw;       // Breit-Wigner: 1 / (m w) (per-event a1)
 };
 
-// The visit's integers (as in PhsVisit and PhsChild) in one 16-byte load: x_phi | x_ct << 8 |
-// ct_class << 16 | self_root << 17 | massless << 18 | kind << 20 | (carry + 1) << 23 |
-// (push + 1) << 25, and per child internal | map_id << 1 | x_msq << 8 | out_index << 16.
-// (A load each, they took 7 of 270 us for 1e6 tt events, 17 of 219 for 5e5 with their own beams.)
+// code, child_code: as in PhsVisit.
 struct alignas(16) PhsVisitFF {
   int32_t code, child_code[2], pad;
   PhsChildFF child[2];
