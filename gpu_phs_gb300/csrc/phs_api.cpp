@@ -335,7 +335,7 @@ bool wide_serves(const PhsLaunch &a, int tiles_per_visit) {
 
 int launch_ff_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int device, int depth,
                     int64_t n_events, cudaStream_t st) {
-  if (!pinned && wide_serves(a, PHS_WIDE_TILES / 2)) {   // (2e4 tt events: 25 us in pairs, 29 wide)
+  if (!pinned && wide_serves(a, a.max_visits > PHS_WIDE_FF_VISITS ? PHS_WIDE_TILES : PHS_WIDE_TILES_FF)) {
     CUDA_TRY(phs_launch_forward_f64(a, 0, PHS_F64_WIDE, st));
     return PHS_OK;
   }

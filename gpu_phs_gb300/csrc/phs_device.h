@@ -59,9 +59,14 @@ struct PhsLaunch {
 #define PHS_F64_VARIANTS_PER_EVENT 5
 #define PHS_F64_WIDE 9
 // Tiles a visit of the largest tree up to which the wide form is the faster one (us a call, wide
-// against one pass / split: 3 visits 1e4 events 12.4 / 14.5, 2e4 18.6 / 18.5, 4e4 27 / 21; 5 visits
-// 2e4 29 / 33, 4e4 45 / 38; 11 visits 4e4 92 / 95, 1.6e5 287 / 268).
-#define PHS_WIDE_TILES 160
+// against one pass: 5 visits 1.6e4 events 18.8 / 22.6, 2.4e4 30.2 / 28.4; 11 visits 3.2e4 66.6 /
+// 73.6, 4.8e4 97.5 / 92.8).  FP32 pairs: 80 up to 5 visits (3 visits 8e3 10.3 / 10.3; 5 visits 1.2e4
+// 15.4 / 16.7, 1.6e4 18.8 / 16.9), where few launches meet an undecided event; larger trees mostly
+// wait for the FP64 walk of one, and the line is FP64's (7 visits 1.6e4 25 / 47, 2.4e4 34 / 50; 11
+// visits 2.4e4 58 / 85, 4.8e4 97 / 92).
+#define PHS_WIDE_TILES 128
+#define PHS_WIDE_TILES_FF 80
+#define PHS_WIDE_FF_VISITS 5
 cudaError_t phs_launch_forward_f64(const PhsLaunch &a, int n_blocks, int variant,
                                    cudaStream_t stream);
 int phs_forward_blocks_per_sm(int stack_depth, bool per_event, int variant);
