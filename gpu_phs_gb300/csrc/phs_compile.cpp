@@ -393,7 +393,9 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
   out.s = split(in.sqrts * in.sqrts);
   out.lab_bg = split(in.lab_bg);
   out.lab_gamma = split(in.lab_gamma);
-  out.f0 = split(in.f0);
+  int e = 0;
+  out.f0 = split(2.0 * std::frexp(in.f0, &e));
+  out.f0_exp = e - 1;
   out.inv_sqrts = split(in.inv_sqrts);
   out.m_tot = split(in.m_tot);
   out.volume = in.volume;
@@ -421,6 +423,12 @@ void channel_to_ff(const PhsChannel &in, PhsChannelFF &out) {
         G.u1 = split_ld(half_pi - (long double)C.a1);
       }
       if (C.internal && (C.map_id == PHS_MAP_STEP_E || C.map_id == PHS_MAP_STEP_H)) out.exact_only = 1;
+      // the factor of an exponential map runs from a0 to a0 exp(a1): between 1e-12 and 1e17 (in
+      // GeV^2: any real process) two of them and a Kallen term stay in the floats' range.  (A
+      // Breit-Wigner's 1 + tan^2 z stays below 6e13: nearer to pi/2 the walk takes FP64.)
+      if (C.internal && C.map_id != PHS_MAP_NO && C.map_id != PHS_MAP_SCHANNEL &&
+          !(C.a0 >= 1e-12 && C.a0 * std::exp(C.a1) <= 1e17))
+        out.exact_only = 1;
     }
     if (V.friend_sign) out.exact_only = 1;
     F.code = V.code;

@@ -308,11 +308,11 @@ FF_FN ff ff_one_minus_double_int(double x) {
 }
 
 // A float as a double with integer operations: exact (infinities and NaN too), but 0 for zeros of
-// either sign and below 2^-126.
-FF_FN double ff_widen(float f) {
+// either sign and below 2^-126.  Times 2^e for a finite f, e2 = e 2^20.
+FF_FN double ff_widen(float f, int e2 = 0) {
   const uint32_t b = ff_fbits(f), m = b & 0x7fffffffu;
   if (m < 0x00800000u) return 0.0;
-  const uint32_t h = ((m >> 3) + 0x38000000u) | (m >= 0x7f800000u ? 0x7ff00000u : 0u);
+  const uint32_t h = ((m >> 3) + (0x38000000u + (uint32_t)e2)) | (m >= 0x7f800000u ? 0x7ff00000u : 0u);
   return ff_bitsd((uint64_t)((b & 0x80000000u) | h) << 32 | (uint32_t)(b << 29));
 }
 // hi + lo as a double, normalized or not.  A float-to-double conversion holds the FP64 pipe as long
@@ -322,6 +322,20 @@ FF_FN double ff_widen(float f) {
 // beams from 238 to 221 us (there the addition was in integers as well, behind a normalization:
 // for uniform beams that gave 302).
 FF_FN double ff_to_double_int(ff a) { return ff_widen(a.hi) + ff_widen(a.lo); }
+
+// f 2^e with f's high part put back into [1, 2), for |f| < 2^127: a product of many factors that
+// stays in the floats' range whatever their sizes.
+FF_FN void ff_renorm(ff &f, int &e) {
+  const uint32_t b = ff_fbits(f.hi) & 0x7f800000u;
+  const float scale = ff_bitsf(0x7f000000u - b);   // 2^(127 - exponent field), exact on both parts
+  f = ff_make(f_mul(f.hi, scale), f_mul(f.lo, scale));
+  e += (int)(b >> 23) - 127;
+}
+// f 2^e as a double (finite f; the exponent goes into the widened parts, which then stay normal).
+FF_FN double ff_to_double_scaled(ff f, int e) {
+  if (e < -800 || e > 800) return ldexp(ff_to_double_int(f), e);
+  return ff_widen(f.hi, e * 1048576) + ff_widen(f.lo, e * 1048576);
+}
 
 // ------------------------------------------------------------------ elementary functions
 // Cody-Waite splits (three floats summing to the constant to ~2^-72 relative).

@@ -184,10 +184,14 @@ struct alignas(16) PhsTestVisit {
 };
 struct PhsChannelFF {
   int32_t n_out, n_visits;
-  int32_t exact_only;  // 1: STEP_E/STEP_H mappings or a friend boost: FP64 path
+  int32_t exact_only;  // 1: STEP_E/STEP_H mappings, a friend boost, constants out of the floats'
+                       // range: FP64 path
   int32_t lab;
   PhsFF sqrts, s, lab_bg, lab_gamma;
-  PhsFF f0, inv_sqrts;  // as in PhsChannel
+  PhsFF inv_sqrts;    // as in PhsChannel
+  PhsFF f0;           // PhsChannel::f0 as f0 2^f0_exp, f0 in [1, 2): n narrow resonances have
+  int32_t f0_exp;     // (pi m Gamma / s)^n, below the floats' range for the larger trees
+  int32_t pad;
   PhsFF m_tot;        // the sum of all outgoing masses (per-event m_max)
   double volume;
   PhsVisitFF visit[PHS_MAX_VISITS];
