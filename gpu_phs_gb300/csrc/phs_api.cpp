@@ -329,13 +329,15 @@ int attach_pass_buffers(Segments &S, PhsLaunch &a) {
 
 // Few tiles: the time is one walk's latency, which the wide form shortens (the FP64 kernels'
 // bits, which meet the FP32-pair precision's bar too).
-bool wide_serves(const PhsLaunch &a, int tiles_per_visit) {
-  return !a.friends && a.n_tiles <= (int64_t)tiles_per_visit * a.max_visits;
+bool wide_serves(const PhsLaunch &a, int64_t n_tiles, int tiles_per_visit) {
+  return !a.friends && n_tiles <= (int64_t)tiles_per_visit * a.max_visits;
 }
 
+// call_tiles: the tiles of the whole API call, which choose between the wide form and the pairs:
+// the chunks of a host call have one arithmetic, the device call's over the same events.
 int launch_ff_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int device, int depth,
-                    int64_t n_events, cudaStream_t st) {
-  if (!pinned && wide_serves(a, a.max_visits > PHS_WIDE_FF_VISITS ? PHS_WIDE_TILES : PHS_WIDE_TILES_FF)) {
+                    int64_t n_events, int64_t call_tiles, cudaStream_t st) {
+  if (!pinned && wide_serves(a, call_tiles, a.max_visits > PHS_WIDE_FF_VISITS ? PHS_WIDE_TILES : PHS_WIDE_TILES_FF)) {
     CUDA_TRY(phs_launch_forward_f64(a, 0, PHS_F64_WIDE, st));
     return PHS_OK;
   }
@@ -365,7 +367,7 @@ int launch_ff_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int dev
 int launch_f64_tuned(int &variant, bool pinned, Segments &S, PhsLaunch a, int device, int depth,
                      int64_t n_events, cudaStream_t st) {
   const bool per_event = a.E1 != nullptr;
-  if (!pinned && wide_serves(a, PHS_WIDE_TILES)) {
+  if (!pinned && wide_serves(a, a.n_tiles, PHS_WIDE_TILES)) {
     CUDA_TRY(phs_launch_forward_f64(a, 0, PHS_F64_WIDE, st));
     return PHS_OK;
   }
@@ -794,7 +796,7 @@ static int check_counts(const int64_t *counts, int n_channels, int64_t n_events)
 static int launch_process(phs_process_t h, Segments &S, int64_t n_events, const int64_t *counts,
                           int64_t ev0, const double *x, double *p, double *f, double *v,
                           uint8_t *ok, const double *E1, const double *E2, int64_t fstride,
-                          bool whizard_cols, cudaStream_t stream) {
+                          bool whizard_cols, cudaStream_t stream, int64_t call_tiles = 0) {
   int64_t one = n_events;
   const int64_t *cnt = counts ? counts : &one;
   int rc = build_segments(S, cnt, h->p.n_channels, h->lay, ev0, 0, 0, whizard_cols);
@@ -821,7 +823,7 @@ static int launch_process(phs_process_t h, Segments &S, int64_t n_events, const 
   if (a.n_tiles == 0) return PHS_OK;
   if (h->precision == PHS_PRECISION_F32X2)
     return launch_ff_tuned(h->ff_variant_ev[E1 != nullptr], h->ff_pinned, S, a, h->device, h->stack_depth,
-                           n_events, stream);
+                           n_events, call_tiles ? call_tiles : a.n_tiles, stream);
   return launch_f64_tuned(h->f64_variant[E1 != nullptr], h->pinned, S, a, h->device, h->stack_depth, n_events,
                           stream);
 }
@@ -1071,7 +1073,11 @@ extern "C" int phs_generate_host(phs_process_t h, int64_t n_events, const int64_
     }
     std::vector<int64_t> cnt(nch, 0), prefix(nch + 1, 0);
     if (counts) std::copy(counts, counts + nch, cnt.begin()); else cnt[0] = n_events;
-    for (int c = 0; c < nch; c++) prefix[c + 1] = prefix[c] + cnt[c];
+    int64_t call_tiles = 0;
+    for (int c = 0; c < nch; c++) {
+      prefix[c + 1] = prefix[c] + cnt[c];
+      call_tiles += (cnt[c] + 31) / 32;
+    }
     int k = 0;
     int64_t e0 = 0;
     for (const int64_t n : host_chunks(n_events, chunk)) {
@@ -1087,7 +1093,7 @@ extern "C" int phs_generate_host(phs_process_t h, int64_t n_events, const int64_
                                cudaMemcpyHostToDevice, st));
       int rc = launch_process(h, h->pseg[s], n, cc.data(), 0, h->bx[s].as<double>(),
                               h->bp[s].as<double>(), h->bf[s].as<double>(), h->bv[s].as<double>(),
-                              h->bo[s].as<uint8_t>(), nullptr, nullptr, 1, false, st);
+                              h->bo[s].as<uint8_t>(), nullptr, nullptr, 1, false, st, call_tiles);
       if (rc) return rc;
       CUDA_TRY(cudaMemcpyAsync(p + e0 * 4 * n_out, h->bp[s].ptr, n * 4 * n_out * sizeof(double),
                                cudaMemcpyDeviceToHost, st));
@@ -1232,7 +1238,7 @@ extern "C" int phs_batch_generate_device(phs_batch_t b, const int64_t *counts, c
     if (a.n_tiles == 0) return PHS_OK;
     if (b->precision == PHS_PRECISION_F32X2)
       return launch_ff_tuned(b->ff_variant, b->ff_pinned, b->segs, a, b->device, b->stack_depth, n_events,
-                             (cudaStream_t)stream);
+                             a.n_tiles, (cudaStream_t)stream);
     return launch_f64_tuned(b->f64_variant, b->pinned, b->segs, a, b->device, b->stack_depth, n_events,
                             (cudaStream_t)stream);
   });

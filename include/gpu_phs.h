@@ -55,7 +55,8 @@ extern "C" {
 #define PHS_PRECISION_F64 0   /* IEEE FP64 throughout (default) */
 #define PHS_PRECISION_F32X2 1 /* float-float pairs on the FP32 pipe (~48 bits); events within
                                  1e-5 of a kinematic limit are recomputed in FP64, so ok flags
-                                 stay bit-exact */
+                                 stay bit-exact.  Calls of few events (see
+                                 phs_process_set_precision) run in FP64 */
 
 typedef struct phs_process *phs_process_t;
 typedef struct phs_batch *phs_batch_t;
@@ -119,8 +120,13 @@ int phs_process_set_beams(phs_process_t proc, double E1, double E2);
  * afterwards keep their own setting): PHS_PRECISION_F64 or PHS_PRECISION_F32X2.  With
  * per-event beams (phs_generate_beams_device) F32X2 evaluates the constants that depend on
  * sqrt(s) per event in FP64 and walks in float-float, or runs the FP64 compacting kernel
- * where the autotuner finds that faster (few events passing).  No counterpart in the
- * reference (FP64 only). */
+ * where the autotuner finds that faster (few events passing).  With F32X2 a call of few events
+ * runs in FP64, which is the faster form there: up to 80 32-event tiles a visit (n_out - 1 visits,
+ * each channel's events in tiles of their own) for n_out <= 6 and 128 beyond, no friend boosts,
+ * the variant not pinned.  The other calls run in pairs, with the same bits in every form, so an
+ * event's bits depend on which side of that line its call lies (they agree to 1e-7 or better); a
+ * host call gives the device call's bits.  Pin the variant (phs_process_set_variants) for the same
+ * bits at any size.  No counterpart in the reference (FP64 only). */
 int phs_process_set_precision(phs_process_t proc, int precision);
 
 /* The autotuned kernel variants of the handle's uniform-beam launches, or -1 before the

@@ -86,3 +86,21 @@ def test_factor_of_many_narrow_resonances(torch, name, beams):
         print(f"{name} {beams} variant {variant}: ok {int(sel.sum())}, factor {ferr:.2e}, momenta {perr:.2e}")
         assert ferr <= TOL, ferr
         assert perr <= TOL, perr
+
+
+@pytest.mark.parametrize("n_out, n", [(6, 810_000), (6, 12_000), (8, 77_924), (8, 20_000), (8, 28_700)])
+def test_host_call_has_the_device_call_s_form(torch, n_out, n):
+    """A host call's chunks (16384 events, then growing, a short last one) take the form of the whole
+    call: the device call's bits, where a chunk alone would be small enough for the FP64 wide form
+    too.  (28 700 events in three channels: 897 or 898 tiles of 7 visits, just beyond the line.)"""
+    from gpu_phs_gb300.api import PhaseSpace
+    proc = P.nested_resonances(n_out)
+    counts = np.array([n - 2 * (n // 3), n // 3, n // 3], np.int64)
+    x = torch.from_numpy(uniform_x(19, n, proc.n_x)).pin_memory()
+    ps = PhaseSpace(proc, 500.0, 500.0)
+    ps.set_precision(1)
+    h = ps.generate_host(x, counts)
+    d = ps.generate(x.cuda(), counts)
+    torch.cuda.synchronize()
+    for a, b in ((h.p, d.p), (h.factor, d.factor), (h.volume, d.volume), (h.ok, d.ok)):
+        assert torch.equal(a, b.cpu())
