@@ -1,10 +1,14 @@
 """The FP32-pair kernels with their form pinned (a small launch that is not pinned takes the wide
-FP64 form)."""
+FP64 form), and the FP64 one-pass kernel pinned at the sizes of the small fixtures."""
 import numpy as np
 import pytest
 
+from conftest import (REFCPU_FIXTURES, all_maps_process, assert_within_conditioning, counts_of, golden,
+                      load_process, wide_beams)
 from gpu_phs_gb300 import processes as P
 from gpu_phs_gb300.philox import uniform_x
+from oracle import oracle
+from test_gpu_ff import check
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +108,100 @@ def test_host_call_has_the_device_call_s_form(torch, n_out, n):
     torch.cuda.synchronize()
     for a, b in ((h.p, d.p), (h.factor, d.factor), (h.volume, d.volume), (h.ok, d.ok)):
         assert torch.equal(a, b.cpu())
+
+
+def generate(torch, proc, x, sqrts, counts=None, precision=1, variant=0, beams=None):
+    from gpu_phs_gb300.api import PhaseSpace
+    ps = PhaseSpace(proc, sqrts / 2, sqrts / 2)
+    ps.set_precision(precision)
+    ps.set_variants(*((variant, -1) if precision else (-1, variant)))
+    xd = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    if beams is None:
+        ev = ps.generate(xd, counts)
+    else:
+        ev = ps.generate_beams(xd, *(torch.from_numpy(b).cuda() for b in beams), counts)
+    torch.cuda.synchronize()
+    return [t.cpu().numpy() for t in (ev.p, ev.factor, ev.volume, ev.ok)]
+
+
+@pytest.mark.parametrize("precision, variant", [(0, 0)] + [(1, v) for v in FF_FORMS])
+@pytest.mark.parametrize("name", REFCPU_FIXTURES)
+def test_reference_fixtures_pinned(torch, name, precision, variant):
+    z = golden(f"refcpu_{name}")
+    proc = load_process(z)
+    sq = float(z["sqrts"][0])
+    x = uniform_x(int(z["seed"][0]), len(z["ok"]), proc.n_x)
+    got = generate(torch, proc, x, sq, counts_of(z["channel"], proc.n_channels), precision, variant)
+    check(got, z["p"], z["factor"], z["volume"], z["ok"], sq, 1e-12 if precision == 0 else TOL)
+
+
+@pytest.mark.parametrize("precision, variant", [(0, 0)] + [(1, v) for v in FF_FORMS])
+@pytest.mark.parametrize("n_out", [10, 12])
+def test_largest_trees_pinned(torch, n_out, precision, variant):
+    proc = P.nested_resonances(n_out)
+    counts = np.array([3000, 1, 2999], np.int64)
+    x = uniform_x(41, int(counts.sum()), proc.n_x)
+    r = oracle.Oracle(proc, 1000.0).generate(x, np.repeat(np.arange(3), counts).astype(np.int32))
+    got = generate(torch, proc, x, 1000.0, counts, precision, variant)
+    check(got, r.p, r.factor, r.volume, r.ok, 1000.0, 1e-12 if precision == 0 else TOL)
+
+
+@pytest.mark.parametrize("variant", FF_FORMS)
+def test_batch_pinned(torch, variant):
+    from gpu_phs_gb300.api import Batch, PhaseSpace
+    rng = np.random.default_rng(21)
+    procs = [P.random_process(rng, n_out, 1, 1000.0) for n_out in (3, 8, 5, 4, 7, 6)]
+    batch = Batch([PhaseSpace(p, 500.0, 500.0) for p in procs])
+    batch.set_precision(1)
+    batch.set_variants(variant, -1)
+    counts = np.array([37, 1000, 64, 333, 95, 2048], np.int64)
+    po = batch.offsets(counts)[1]
+    xs = [uniform_x(30 + i, int(c), p.n_x) for i, (p, c) in enumerate(zip(procs, counts))]
+    xflat = torch.from_numpy(np.concatenate([a.reshape(-1) for a in xs])).cuda()
+    p, f, v, ok = (t.cpu().numpy() for t in batch.generate(xflat, counts))
+    e = np.concatenate([[0], np.cumsum(counts)])
+    for i, proc in enumerate(procs):
+        r = oracle.Oracle(proc, 1000.0).generate(xs[i])
+        k = slice(e[i], e[i + 1])
+        check((p[po[i]:po[i + 1]].reshape(-1, proc.n_out, 4), f[k], v[k], ok[k]), r.p, r.factor, r.volume, r.ok,
+              1000.0)
+
+
+@pytest.mark.parametrize("beams", ["uniform", "mid", "wide"])
+@pytest.mark.parametrize("n_out", [4, 7, 8])
+def test_every_mapping_pinned(torch, n_out, beams):
+    """The pair kernels on every mapping kind, uniform and per-event beams, at the bar of
+    test_gpu_parity.test_every_mapping_uniform_beams."""
+    proc = all_maps_process(100 + n_out, n_out, 8)
+    n = 20_000
+    counts = np.full(8, n // 8, np.int64)
+    ch = np.repeat(np.arange(8), counts).astype(np.int32)
+    x = uniform_x((700 if beams == "uniform" else 200) + n_out, n, proc.n_x)
+    E = None
+    if beams == "mid":
+        rng = np.random.default_rng(n_out)
+        E = rng.uniform(300.0, 700.0, n), rng.uniform(300.0, 700.0, n)
+    elif beams == "wide":
+        E = wide_beams(n, 1000.0, 7)
+    E1, E2 = E or (None, None)
+    sq = np.full(n, 1000.0) if E is None else 2.0 * np.sqrt(E1 * E2)
+    o = oracle.Oracle(proc, 1000.0)
+    r = o.generate(x, ch, E1=E1, E2=E2)
+    for variant in FF_FORMS if E is None else [0, 1]:
+        p, f, v, ok = generate(torch, proc, x, 1000.0, counts, 1, variant, E)
+        assert_within_conditioning(p, f, ok, o, x, r, sq, E1, E2, TOL, 1024, channels=ch)
+        assert (np.abs(v - r.volume) / r.volume).max() < 1e-15
+
+
+@pytest.mark.parametrize("n_out, per_visit", [(6, 80), (7, 128)])
+def test_line_between_the_wide_form_and_the_pairs(torch, n_out, per_visit):
+    """Just below the line an unpinned call has the FP64 kernel's bits, just above it the pairs'."""
+    proc = P.nested_resonances(n_out).subset([0])
+    line = per_visit * (n_out - 1)
+    for tiles, precision in ((line, 0), (line + 1, 1)):
+        n = 32 * tiles - 5
+        x = uniform_x(8, n, proc.n_x)
+        got = generate(torch, proc, x, 1000.0, variant=-1)
+        want = generate(torch, proc, x, 1000.0, precision=precision)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
