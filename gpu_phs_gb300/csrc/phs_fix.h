@@ -64,6 +64,8 @@ FX_FN float fx_rsqrt_est(float a) { return rsqrtf(a); }
 FX_FN float fx_rcp_est(float a) { return __fdividef(1.0f, a); }
 FX_FN float fx_fmaf(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 FX_FN float fx_mulf(float a, float b) { return __fmul_rn(a, b); }
+FX_FN float fx_minf(float a, float b) { return fminf(a, b); }
+FX_FN float fx_maxf(float a, float b) { return fmaxf(a, b); }
 FX_FN int fx_rint32(float a) { return __float2int_rn(a); }
 FX_FN uint32_t fx_trunc_u32(float a) { return __float2uint_rz(a); }
 FX_FN double fx_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -82,6 +84,8 @@ FX_FN float fx_rsqrt_est(float a) { return 1.0f / sqrtf(a); }
 FX_FN float fx_rcp_est(float a) { return 1.0f / a; }
 FX_FN float fx_fmaf(float a, float b, float c) { return fmaf(a, b, c); }
 FX_FN float fx_mulf(float a, float b) { return a * b; }
+FX_FN float fx_minf(float a, float b) { return a < b ? a : b; }
+FX_FN float fx_maxf(float a, float b) { return a > b ? a : b; }
 FX_FN int fx_rint32(float a) { return (int)lrintf(a); }
 FX_FN uint32_t fx_trunc_u32(float a) { return (uint32_t)a; }
 FX_FN double fx_fma(double a, double b, double c) { return fma(a, b, c); }
@@ -114,12 +118,14 @@ FX_RARE double fx_lib_sin(double x) { return sin(x); }
 FX_RARE double fx_lib_cos(double x) { return cos(x); }
 
 // ------------------------------------------------------------ square root and reciprocal
-// y0 + c (y0 in [0.5, 1), |c| < 2^-22) as a double: y0's bits widened, c added in units of
-// y0's last place.
+// y0 + c (y0 in [0.5, 1), |c| < 2^-21) as a double: y0's bits widened, c added in units of twice
+// its last place.  (With an estimate 2 ulps off and the operand's low bits |c| reaches 1.1 2^-22.
+// The callers clamp their estimates to [0.5, 1): the true value lies there, but an estimate within
+// its 2 ulps may not, and in the binade below c would count half.)
 FX_FN uint64_t fx_seed(float y0, float c) {
   const uint32_t b = fx_fbits(y0);
   const uint64_t d = (uint64_t)((b >> 3) + ((1023u - 127u) << 20)) << 32 | (uint64_t)(b << 29);
-  return d + (uint64_t)(int64_t)fx_rint32(fx_mulf(c, 0x1p53f));
+  return d + 2 * (uint64_t)(int64_t)fx_rint32(fx_mulf(c, 0x1p52f));
 }
 
 // 1/sqrt(x) to about 2^-45 for a normal x > 0; the bits of a double.
@@ -129,7 +135,7 @@ FX_FN uint64_t fx_rsqrt_seed(double x) {
   const float mh = fx_float(((127u + even) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
   const float ml = fx_mulf((float)(lo & 0x1fffffffu), even ? 0x1p-51f : 0x1p-52f);
   float y0 = fx_rsqrt_est(mh);
-  y0 = y0 < 0x1.fffffep-1f ? y0 : 0x1.fffffep-1f;
+  y0 = fx_minf(fx_maxf(y0, 0.5f), 0x1.fffffep-1f);
   const float p = fx_mulf(y0, y0), pl = fx_fmaf(y0, y0, -p);
   float e = fx_fmaf(-mh, p, 1.0f);             // 1 - m y0^2
   e = fx_fmaf(-mh, pl, e);
@@ -161,7 +167,7 @@ FX_FN double fx_rcp(double x, const FxRegs &k = FxRegs{-0.0, 1.0}) {
   const float mh = fx_float((127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
   const float ml = fx_mulf((float)(lo & 0x1fffffffu), 0x1p-52f);
   float y0 = fx_rcp_est(mh);
-  y0 = y0 < 0x1.fffffep-1f ? y0 : 0x1.fffffep-1f;
+  y0 = fx_minf(fx_maxf(y0, 0.5f), 0x1.fffffep-1f);
   float e = fx_fmaf(-mh, y0, 1.0f);
   e = fx_fmaf(-ml, y0, e);
   const float c = fx_mulf(y0, fx_fmaf(e, e, e));

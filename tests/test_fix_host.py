@@ -255,3 +255,51 @@ def test_sincos_at_simple_fractions(tmp_path):
                    check=True)
     worst = float(subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout)
     assert worst <= 2.0 ** -58
+
+
+SEED_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <initializer_list>
+#include "phs_fix.h"
+typedef long double Q;
+static double ulp(double a) { return std::nextafter(a, INFINITY) - a; }
+int main() {
+  // mantissas next to 1, 2 and 4, where the estimate changes its binade, and in between
+  double rcp = 0, root = 0;
+  auto one = [&](double x) {
+    const double r = fx_rcp(x), s = fx_sqrt(x);
+    rcp = std::fmax(rcp, std::fabs((double)((Q)r - 1.0L / (Q)x)) / ulp(1.0 / x));
+    root = std::fmax(root, std::fabs((double)((Q)s - sqrtl((Q)x))) / ulp(std::sqrt(x)));
+  };
+  for (double c : {1.0, 2.0, 4.0, 0.25, 1024.0})
+    for (int i = 0; i < 60000; i++) {
+      one(c + i * c * 0x1p-36 + (i % 7) * ulp(c));
+      one(c - i * c * 0x1p-36 - (1 + i % 5) * ulp(c / 2));
+    }
+  for (int i = 0; i < 400000; i++) one(1 + i * 7.5e-6);
+  std::printf("%.6f %.6f\n", rcp, root);
+}
+"""
+
+
+@pytest.mark.parametrize("ulps", [-2, -1, 0, 1, 2])
+def test_seeds_of_any_estimate_within_two_ulps(tmp_path, ulps):
+    """The device's reciprocal and reciprocal root estimates are within 2 ulps: with any such
+    estimate (the host's, moved) the reciprocal stays within an ulp and the root within half of one
+    and a little."""
+    try:
+        subprocess.run(["g++", "--version"], check=True, capture_output=True)
+    except (OSError, subprocess.CalledProcessError):
+        pytest.skip("g++ not available")
+    head = open(os.path.join(CSRC, "phs_fix.h")).read()
+    for body in ("1.0f / sqrtf(a)", "1.0f / a"):
+        assert head.count(f"return {body}; }}") == 1
+        head = head.replace(f"return {body}; }}", f"return fx_float(fx_fbits({body}) + ({ulps})); }}")
+    (tmp_path / "phs_fix.h").write_text(head)
+    (tmp_path / "s.cpp").write_text(SEED_DRIVER)
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=gnu++17", "-I", str(tmp_path), str(tmp_path / "s.cpp"),
+                    "-o", str(tmp_path / "s")], check=True)
+    rcp, root = map(float, subprocess.run([str(tmp_path / "s")], check=True, capture_output=True, text=True).stdout.split())
+    assert rcp <= 1.001
+    assert root <= 0.501
