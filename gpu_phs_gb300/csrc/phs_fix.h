@@ -182,10 +182,14 @@ FX_FN double fx_quot(double a, double b, double r, const FxRegs &k) {
   const double q = fx_mul(k, a, r);
   return fx_fma(fx_fma(-q, b, a), r, q);
 }
-// b such that fx_quot serves a / b: normal, positive, and neither huge nor tiny.
-FX_FN bool fx_quot_serves(double b) { return fx_hi(b) - 0x04000000u < 0x78000000u; }
+// b and a such that fx_quot serves a / b: b normal, positive, neither huge nor tiny; a neither
+// huge nor infinite (the residual of an infinite quotient is no number).
+FX_FN bool fx_quot_serves(double b) { return fx_hi(b) - 0x20b00000u < 0x3e800000u; }   // 2^-500 .. 2^500
+FX_FN bool fx_quot_serves(double a, double b) {
+  return fx_quot_serves(b) && (fx_hi(a) & 0x7fffffffu) < 0x5f300000u;
+}
 FX_FN double fx_div(double a, double b, const FxRegs &k) {
-  if (!fx_quot_serves(b)) return fx_lib_div(a, b);
+  if (!fx_quot_serves(a, b)) return fx_lib_div(a, b);
   return fx_quot(a, b, fx_rcp(b, k), k);
 }
 

@@ -303,3 +303,43 @@ def test_seeds_of_any_estimate_within_two_ulps(tmp_path, ulps):
     rcp, root = map(float, subprocess.run([str(tmp_path / "s")], check=True, capture_output=True, text=True).stdout.split())
     assert rcp <= 1.001
     assert root <= 0.501
+
+
+QUOTIENT_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <random>
+#include "phs_fix.h"
+static bool same(double a, double b) { return (a != a && b != b) || a == b; }
+int main() {
+  const FxRegs k{-0.0, 1.0};
+  std::mt19937_64 g(3);
+  std::uniform_real_distribution<double> U(1, 2);
+  const double a[] = {0.0, INFINITY, -INFINITY, NAN, 1.7e308, -1.7e308, 1e300, 0x1p499, 0x1p500, 1.0, -3.0, 0x1p-400};
+  long n = 0, bad = 0;
+  for (int e = -1022; e <= 1023; e++)
+    for (int i = 0; i < 40; i++)
+      for (double s : a) {
+        const double b = std::ldexp(U(g), e), x = i ? s * U(g) : s;
+        const double q = fx_div(x, b, k), w = x / b;
+        bad += !(same(q, w) || (std::fabs(w) < 0x1p-960 && std::fabs(q - w) <= 0x1p-1012));
+        n++;
+      }
+  std::printf("%ld %ld\n", n, bad);
+}
+"""
+
+
+def test_quotients_of_infinite_and_huge_numerators(tmp_path):
+    """A logarithm of 0 over a constant is -inf, and what overflows is infinite: fx_div is the
+    division's value for every numerator and denominator."""
+    try:
+        subprocess.run(["g++", "--version"], check=True, capture_output=True)
+    except (OSError, subprocess.CalledProcessError):
+        pytest.skip("g++ not available")
+    (tmp_path / "q.cpp").write_text(QUOTIENT_DRIVER)
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=gnu++17", "-I", CSRC, str(tmp_path / "q.cpp"), "-o",
+                    str(tmp_path / "q")], check=True)
+    n, bad = subprocess.run([str(tmp_path / "q")], check=True, capture_output=True, text=True).stdout.split()
+    assert int(n) > 900_000
+    assert int(bad) == 0
