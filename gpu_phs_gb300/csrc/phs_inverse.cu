@@ -272,7 +272,7 @@ __device__ void inverse_geometry(const FxRegs &k, const PhsChannel &ch, const In
       qz = add(add(add(mul(G[12], q0[0]), mul(G[13], q0[1])), mul(G[14], q0[2])), mul(G[15], q0[3]));
     }
     double phi = fx_atan2(qy, qx);
-    if ((int32_t)fx_hi(phi) < 0) phi = add(phi, 2.0 * PHS_PI);
+    if (fx_bits(phi) > 0x8000000000000000ull) phi = add(phi, 2.0 * PHS_PI);   // below 0 (-0 is not)
     geo[(PHS_INV_GEO * v + 3) * PHS_INV_BLOCK] = mul(phi, 1.0 / (2.0 * PHS_PI));   // x_phi
     const double ct = fx_div(qz, fx_sqrt(add(add(mul(qx, qx), mul(qy, qy)), mul(qz, qz)), k), k);
     geo[(PHS_INV_GEO * v + 2) * PHS_INV_BLOCK] = ct;
