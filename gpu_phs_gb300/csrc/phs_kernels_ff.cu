@@ -33,6 +33,7 @@
 #include "phs_device.h"
 #include "phs_event_f64.cuh"  // the compacting loop and rot_z_onto
 #include "phs_ff.h"
+#include "phs_pretest.h"
 #include "phs_program.h"
 
 #define PHS_FF_STATE 40   // floats per saved frame: L[16], msq, m, p, E as pairs
@@ -532,55 +533,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 // the reference's own sums and bounds), so such an event fails the reference's test too.
 // Its outputs are written here.  Every other event goes to pass B, whose float-float /
 // FP64 walk decides its flag exactly.  Returns false for a failed event.
-//
-// Against those 64 epsilons (3.8e-6), per unit of the magnitudes: the angle of the tangent is
-// within 5e-7 (x, the constants, product and sum, rounded to nearest, of magnitudes up to pi),
-// the hardware sine and cosine within 2^-21.4 and 2^-21.2 (|w| <= pi/4), so tan or cot within
-// 1.3e-6 (1 + tan^2); the hardware exponential within 2 + 1.2 |y| epsilons, its argument within
-// 3 epsilons of |y|.  Square roots and quotients approximate to 2 epsilons, inside the 1e-6.
-#define PHS_F32_EPS_BOUND (64.0f * 5.9604645e-8f)
-// A double to the nearest float (ties away) with integer operations: the conversion unit for
-// doubles takes 16 cycles of an SM a warp.  Below 2^-126: 0; for |d| < 2^128.
-__device__ __forceinline__ float f32_of(double d) {
-  const uint64_t b = fx_bits(d) + 0x10000000ull;
-  const uint32_t hw = (uint32_t)(b >> 32), mag = hw & 0x7fffffffu;
-  return mag < (897u << 20) ? 0.0f
-                            : fx_float((hw & 0x80000000u) | ((mag - (896u << 20)) << 3) | ((uint32_t)b >> 29));
-}
-
-// c0..c5: the packed constants of PhsTestChild.
-__device__ __forceinline__ float msq_f32(int map_id, float4 c, float c4, float c5, double xd,
-                                         float &e) {
-  const float x = f32_of(xd), k = PHS_F32_EPS_BOUND;
-  switch (map_id) {
-    case PHS_MAP_NO:
-      e = k * (fabsf(c.x) + fabsf(c.y));
-      return c.x + x * (c.y - c.x);
-    case PHS_MAP_SCHANNEL: {
-      // one tangent per lane, of z or of pi/2 -+ z (selected, not branched: lanes of a warp
-      // take different sides)
-      const float z = c.x + x * c.y;  // c.y holds a1 - a0
-      const bool hi_side = z > 0.78539816f, lo_side = z < -0.78539816f, cot = hi_side || lo_side;
-      const float w = hi_side ? c.w + (1.0f - x) * c.y : (lo_side ? c.z + x * c.y : z);
-      const float sw = __sinf(w), cw = __cosf(w);
-      const float q = __fdividef(cot ? cw : sw, cot ? sw : cw), t = lo_side ? -q : q;
-      e = k * (fabsf(c4) + fabsf(c5) * (1.0f + t * t));
-      return c4 + c5 * t;
-    }
-    case PHS_MAP_COLLINEAR:
-    case PHS_MAP_INFRARED:
-    case PHS_MAP_RADIATION:
-    case PHS_MAP_TCHANNEL:
-    case PHS_MAP_UCHANNEL: {
-      const bool upper = (map_id == PHS_MAP_TCHANNEL || map_id == PHS_MAP_UCHANNEL) && !(xd < 0.5);
-      const float y = (upper ? 1.0f - x : x) * c.y, em = __expf(y) - 1.0f;
-      e = k * (fabsf(upper ? c.w : c.z) + fabsf(c.x) * (em + 1.0f) * (1.0f + fabsf(y)));
-      return upper ? c.w - c.x * em : c.x * em + c.z;
-    }
-  }
-  e = INFINITY;
-  return 0.0f;
-}
+// (msq_f32, phs_pretest.h; square roots approximate to 2 epsilons, inside the 1e-6.)
 
 // The exact FP64 walk of one event.  It shares the float-float frame stack's memory (slots of 8 bytes, 20 a
 // frame: a thread uses one walk at a time, and no slot of one thread overlaps another's).
@@ -740,7 +693,7 @@ __device__ __forceinline__ bool phs_ok_f32(const PhsLaunch &a, const PhsSegment 
       } else {
         float e;
         const int xi = (code >> 8) & 255;
-        const float msq = msq_f32((code >> 1) & 127, A[j], B[j].x, B[j].y,
+        const float msq = msq_f32((code >> 1) & 127, A[j].x, A[j].y, A[j].z, A[j].w, B[j].x, B[j].y,
                                   phs_in(xi, seg.x_stride, PHS_CHK_X) ? ld_x_narrow(xe + xi) : 0.0, e);
         fails = fails || msq + e < 0.0f;                // negative for certain: not ok
         lo[j] = sqrt_approx(fmaxf(msq - e, 0.0f)) * dn;       // NaN bounds decide nothing
