@@ -1041,8 +1041,15 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
 // eighth of 512 Ki events, left gaps after every chunk, and calls of less than 1.4e6 events ran
 // in one or two chunks.  Measured, tt events: 6e4 174 -> 145 us, 3e5 671 -> 458 us, 1.5e6 1.93 -> 1.88
 // ms, where the link takes 1.67 ms for the copies both ways alone.)
-static std::vector<int64_t> host_chunks(int64_t n, int64_t chunk) {
+// tune: the variant is not chosen yet: a first chunk of kTuneEvents events, which times the
+// variants while no other chunk is in flight (a call of 789 000 events or fewer has no other chunk
+// that large, and would run untuned however often it is repeated).
+static std::vector<int64_t> host_chunks(int64_t n, int64_t chunk, bool tune) {
   std::vector<int64_t> out;
+  if (tune && chunk >= kTuneEvents) {
+    out.push_back(kTuneEvents);
+    n -= kTuneEvents;
+  }
   for (int64_t c = 1 << 14; n > 0; c = std::min(c + c / 2, chunk)) {
     out.push_back(std::min(std::min(c, chunk), n));
     n -= out.back();
@@ -1080,7 +1087,8 @@ extern "C" int phs_generate_host(phs_process_t h, int64_t n_events, const int64_
     }
     int k = 0;
     int64_t e0 = 0;
-    for (const int64_t n : host_chunks(n_events, chunk)) {
+    const bool tune = (h->precision == PHS_PRECISION_F32X2 ? h->ff_variant_ev : h->f64_variant)[0] < 0;
+    for (const int64_t n : host_chunks(n_events, chunk, tune)) {
       const int s = k++ % phs_process::kStreams;
       cudaStream_t st = h->streams[s];
       // this chunk's per-channel counts
