@@ -1020,14 +1020,18 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
   a.group_lo = (int32_t)(std::upper_bound(gb.begin(), gb.end(), a.order_lo) - gb.begin()) - 1;
   a.group_hi = (int32_t)(std::lower_bound(gb.begin(), gb.end(), a.order_hi) - gb.begin());
   if (a.order_lo >= a.order_hi) return PHS_OK;
-  // events per block: long tiles fill the warps with ok events, short ones give blocks to
-  // every SM; halved until the grid is four times what is resident (measured for 2e5 events x
-  // 16 channels: 2.79 ms, 2.85 at eight times)
+  // events per block: the launch's (event, shape) pairs over as few full waves of resident blocks as
+  // tiles of PHS_INV_TILE events allow.  Long tiles fill the warps with ok events (a block's last
+  // warp of them is half empty), and a wave that is not full leaves SMs idle.  (Tiles halved until
+  // there were four waves had 8 ok events a block for 4e4 events of one 12-particle shape, 12 % of
+  // them ok: 704 us, 270 so.)
   const int64_t resident = (int64_t)sm_count(h->device) *
                            phs_inverse_blocks_per_sm(a.n_out, a.stack_depth, a.max_visits,
                                                      E1 != nullptr, cache, !a.lab);
-  a.tile = PHS_INV_TILE;
-  while (a.tile > 64 && (n_events + a.tile - 1) / a.tile * (a.group_hi - a.group_lo) < 4 * resident) a.tile /= 2;
+  const int64_t groups = a.group_hi - a.group_lo, chunks = (n_events + PHS_INV_CHUNK - 1) / PHS_INV_CHUNK;
+  const int64_t waves = std::max<int64_t>(1, (n_events * groups + resident * PHS_INV_TILE - 1) / (resident * PHS_INV_TILE));
+  const int64_t per_group = std::max<int64_t>(1, waves * resident / groups);
+  a.tile = (int32_t)std::min<int64_t>(PHS_INV_TILE, (chunks + per_group - 1) / per_group * PHS_INV_CHUNK);
   CUDA_TRY(phs_launch_inverse(a, st));
   return PHS_OK;
 }

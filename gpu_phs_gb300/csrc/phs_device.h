@@ -143,9 +143,11 @@ void phs_adjoint_sizes(int max_visits, int max_pops, int stack_depth, bool frien
 #define PHS_ADJ_BLOCK_HOST 64
 
 // Inverse map (phs_inverse.cu): for every event and every channel, the x row and factor
-// that channel assigns to the event's momenta.  Threads per block: with ~84 doubles of shared
-// memory per thread, 64-thread blocks keep 5 blocks (10 warps) resident per SM where
-// 128-thread blocks keep 2 (8 warps).
+// that channel assigns to the event's momenta.  Threads per block: four warps, so that a block's
+// shared memory (98 KB for 6 particles with the mapping cache, 193 KB for 12 without) leaves 1 to 3
+// blocks, 4 to 12 warps, on an SM.  With 11 and 12 particles the cache (PHS_INV_CACHE) fits blocks
+// of 64 threads alone; those, with it, take as long (12 particles, 8 channels of one shape, 2e5
+// events: 0.84 ms either way).
 #define PHS_INV_BLOCK 128
 struct PhsInvLaunch {
   const PhsChannel *channels;  // device, per channel (uniform-beam constants)
@@ -168,7 +170,7 @@ struct PhsInvLaunch {
   // this launch inverts the channels at group_order positions [order_lo, order_hi) (all:
   // 0, n_channels), which lie in the groups [group_lo, group_hi)
   int32_t order_lo, order_hi, group_lo, group_hi;
-  int32_t tile;                // events per block (a multiple of 32, at most PHS_INV_TILE)
+  int32_t tile;                // events per block (a multiple of PHS_INV_CHUNK, at most PHS_INV_TILE)
   int64_t n_events;
   int64_t x_ch_stride;         // rows per channel in x_out (n_events, or more for a launch
                                // over a range of the events of a longer array)
@@ -177,6 +179,7 @@ struct PhsInvLaunch {
 };
 cudaError_t phs_launch_inverse(const PhsInvLaunch &a, cudaStream_t stream);
 #define PHS_INV_TILE 1024
+#define PHS_INV_CHUNK 64   // consecutive events; a block's chunks lie a grid apart
 // cache: the per-visit mapping results that channels of a shape reuse (a.group_reuse set);
 // phs_inverse_fits_cache tells whether the block's shared memory holds them.  lab_rows:
 // uniform beams without a lab boost, where the kernel reads the outgoing momenta from p

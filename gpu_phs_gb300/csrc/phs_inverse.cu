@@ -396,18 +396,21 @@ __device__ double inverse_maps(const FxRegs &k, const PhsChannel &ch, double sqr
 }
 
 // One block: `tile` events and the channels of one tree shape (in the launch's slice of the
-// group order).  It writes their outputs that need no arithmetic, gathers the tile's ok events
-// and walks them, a warp 32 at a time.  What bounds the kernel is the FP64 pipe; events are ok
-// in very different shares from channel to channel, so blocks are many and short and the
-// hardware's block scheduler spreads them.  (Persistent blocks that each took 64 events through
-// every channel left most SMs idle: 40 000 ok events of 2e5 are 600 such walks.)
+// group order).  It gathers the tile's ok events and walks them, a warp 32 at a time, and writes
+// the outputs that need no arithmetic.  What bounds the kernel is the FP64 pipe; events are ok in
+// very different shares from channel to channel, so a tile is chunks of PHS_INV_CHUNK events spread
+// evenly over all of them, and blocks differ little.  (Contiguous tiles: 2e5 events of 16 channels 2.60
+// ms, 2.47 so; 2e5 of 16 channels of 8 particles 1.26 -> 1.04.  Persistent blocks that each took 64
+// events through every channel left most SMs idle: 40 000 ok events of 2e5 are 600 such walks.)
+// The other outputs are written beside the walks: ahead of them, with one block on an SM, 2e5
+// events of 8 channels of 12 particles, 12 % of them ok, took 1.08 ms instead of 0.92.
 // LAB_ROWS: no lab boost (uniform beams with E1 = E2): the outgoing momenta are read from p
 // instead of staged in shared memory (InvMomenta).
 template <bool PER_EVENT, bool LAB_ROWS>
 __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
     phs_inverse_kernel(const __grid_constant__ PhsInvLaunch a) {
   static_assert(!(PER_EVENT && LAB_ROWS), "per-event beams stage their CM momenta");
-  constexpr int kWarps = PHS_INV_BLOCK / 32;
+  constexpr int kWarps = PHS_INV_BLOCK / 32, kChunk = PHS_INV_CHUNK;
   extern __shared__ double sm[];
   const FxRegs k = fx_regs();
   double *pm = sm;  // [4 (n_out - 1), or 4 (2 n_out - 1) with staging][block]
@@ -416,16 +419,19 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
   double *cache = a.group_reuse ? geo + (size_t)PHS_INV_GEO * a.max_visits * PHS_INV_BLOCK
                                 : nullptr;  // per-visit mapping results
   __shared__ uint16_t listed[PHS_INV_TILE];  // the tile's ok events
-  __shared__ int warp_ok[kWarps];
+  __shared__ int warp_ok[kWarps], next_work;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n_groups = a.group_hi - a.group_lo;
-  const int64_t n_items = (a.n_events + a.tile - 1) / a.tile * n_groups;
+  const int64_t per_group = (a.n_events + a.tile - 1) / a.tile, n_items = per_group * n_groups;
+  const int64_t n_chunks = (a.n_events + kChunk - 1) / kChunk;
   const bool has_own = a.x_own != nullptr;
 
   for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int g = a.group_lo + (int)(item % n_groups);
-    const int64_t e0 = item / n_groups * a.tile;
-    const int n_ev = (int)min((int64_t)a.tile, a.n_events - e0);
+    // the block's chunks: first, first + per_group, ..  (entry j: chunk j / kChunk of them)
+    const int64_t first = item / n_groups;
+    const int n_ch = (int)((n_chunks - first + per_group - 1) / per_group);
+    const auto event = [&](int j) { return ((int64_t)(j / kChunk) * per_group + first) * kChunk + j % kChunk; };
     const int gb = a.group_begin[g], ge = a.group_begin[g + 1];
     const int lo = max(gb, a.order_lo), hi = min(ge, a.order_hi);
     // checked build: the group's entries, its shape's program, the regions sized for it and
@@ -434,56 +440,23 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
         !phs_in(a.group_order[gb], a.n_channels, PHS_CHK_CHANNEL) ||
         !phs_in(a.channels[a.group_order[gb]].n_visits - 1, a.max_visits, PHS_CHK_VISITS) ||
         !phs_in(a.channels[a.group_order[gb]].n_out - 1, a.n_out, PHS_CHK_SLOT) ||
-        !phs_in(n_ev - 1, PHS_INV_TILE, PHS_CHK_SLOT) || !phs_in(e0 + n_ev - 1, a.x_ch_stride, PHS_CHK_INV))
+        !phs_in(n_ch * kChunk - 1, PHS_INV_TILE, PHS_CHK_SLOT) ||
+        !phs_in(min(event(n_ch * kChunk - 1), a.n_events - 1), a.x_ch_stride, PHS_CHK_INV))
       continue;
 
-    // 1. per channel: the outputs that need no arithmetic (the generating channel's own x and
-    // factor, x padding beyond a channel's n_x_used, zeros for ok = false events); rows of
-    // consecutive events are contiguous
-    for (int i = lo; i < hi; i++) {
-      const int c = a.group_order[i];
-      if (!phs_in(c, a.n_channels, PHS_CHK_CHANNEL)) continue;
-      // the generating channel of an event: the last c with ch_begin[c] <= event
-      const int64_t own0 = a.ch_begin[c] - e0;
-      const int64_t own1 = (c + 1 < a.n_channels ? a.ch_begin[c + 1] : a.n_events) - e0;
-      const int n_used = a.channels[c].n_x_used;
-      double *xr = a.x_out + ((int64_t)c * a.x_ch_stride + e0) * a.n_x;
-      const double *xo = has_own ? a.x_own + e0 * a.n_x : nullptr;
-      int ev = tid / a.n_x, kx = tid - ev * a.n_x;
-      const int dev = PHS_INV_BLOCK / a.n_x, dkx = PHS_INV_BLOCK - dev * a.n_x;
-      for (int j = tid; j < n_ev * a.n_x; j += PHS_INV_BLOCK) {
-        const bool own = has_own && ev >= own0 && ev < own1;
-        if (own || kx >= n_used)
-          xr[j] = xo ? xo[j] : 0.0;
-        else if (a.ok && !a.ok[e0 + ev])
-          xr[j] = 0.0;
-        ev += dev;
-        kx += dkx;
-        if (kx >= a.n_x) {
-          kx -= a.n_x;
-          ev++;
-        }
-      }
-      for (int j = tid; j < n_ev; j += PHS_INV_BLOCK) {
-        double *fo = a.all_factors + (e0 + j) * a.n_channels + c;
-        if (has_own && j >= own0 && j < own1)
-          *fo = a.factor_own ? a.factor_own[e0 + j] : 0.0;
-        else if (a.ok && !a.ok[e0 + j])
-          *fo = 0.0;
-      }
-    }
-
-    // 2. the ok events, listed in order: the inversions run in full warps (an FP64 instruction
+    // 1. the ok events, listed in order: the inversions run in full warps (an FP64 instruction
     // costs the pipe the same whatever the number of active lanes).  A shape's only channel
     // does not invert the events that it generated.
     const bool skip_own = has_own && hi - lo == 1;
     const int c0 = a.group_order[lo];
-    const int64_t skip0 = skip_own ? a.ch_begin[c0] - e0 : 0;
-    const int64_t skip1 = skip_own ? (c0 + 1 < a.n_channels ? a.ch_begin[c0 + 1] : a.n_events) - e0 : 0;
+    const int64_t skip0 = skip_own ? a.ch_begin[c0] : 0;
+    const int64_t skip1 = skip_own ? (c0 + 1 < a.n_channels ? a.ch_begin[c0 + 1] : a.n_events) : 0;
     int n_list = 0;  // block-uniform
-    for (int base = 0; base < n_ev; base += PHS_INV_BLOCK) {
+    if (tid == 0) next_work = 0;   // (read after the barriers below)
+    for (int base = 0; base < n_ch * kChunk; base += PHS_INV_BLOCK) {
       const int j = base + tid;
-      const bool take = j < n_ev && (!a.ok || a.ok[e0 + j]) && !(j >= skip0 && j < skip1);
+      const int64_t e = event(j);
+      const bool take = j < n_ch * kChunk && e < a.n_events && (!a.ok || a.ok[e]) && !(e >= skip0 && e < skip1);
       const unsigned m = __ballot_sync(0xffffffffu, take);
       if (lane == 0) warp_ok[wid] = __popc(m);
       __syncthreads();
@@ -498,12 +471,55 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
       __syncthreads();  // warp_ok is read, the entries are written
     }
 
-    // 3. the geometry once per event, then the mappings of each channel of the shape
-    for (int at = wid * 32; at < n_list; at += PHS_INV_BLOCK) {
-      const int slot = at + lane;
-      if (slot < n_list && phs_in(listed[slot], n_ev, PHS_CHK_SLOT)) {
-        const int j = listed[slot];
-        const int64_t e = e0 + j;
+    // 2. the warps take what there is to do from a counter: first walks of 32 listed events (the
+    // geometry once per event, then the mappings of each channel of the shape), then pieces of the
+    // outputs that need no arithmetic, so that warps without a walk write beside those with one
+    const int n_walks = (n_list + 31) / 32, n_work = n_walks + n_ch * (hi - lo);
+    for (;;) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&next_work, 1);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at >= n_work) break;
+      if (at >= n_walks) {
+        // per channel the generating channel's own x and factor, x padding beyond a channel's
+        // n_x_used, zeros for ok = false events; rows of consecutive events are contiguous
+        const int i = lo + (at - n_walks) / n_ch;
+        const int c = a.group_order[i];
+        if (!phs_in(c, a.n_channels, PHS_CHK_CHANNEL)) continue;
+        const int64_t ep = event((at - n_walks) % n_ch * kChunk);
+        const int n_p = (int)min((int64_t)kChunk, a.n_events - ep);
+        const int64_t own0 = a.ch_begin[c] - ep;
+        const int64_t own1 = (c + 1 < a.n_channels ? a.ch_begin[c + 1] : a.n_events) - ep;
+        const int n_used = a.channels[c].n_x_used;
+        double *xr = a.x_out + ((int64_t)c * a.x_ch_stride + ep) * a.n_x;
+        const double *xo = has_own ? a.x_own + ep * a.n_x : nullptr;
+        int ev = lane / a.n_x, kx = lane - ev * a.n_x;
+        const int dev = 32 / a.n_x, dkx = 32 - dev * a.n_x;
+        for (int j = lane; j < n_p * a.n_x; j += 32) {
+          const bool own = has_own && ev >= own0 && ev < own1;
+          if (own || kx >= n_used)
+            xr[j] = xo ? xo[j] : 0.0;
+          else if (a.ok && !a.ok[ep + ev])
+            xr[j] = 0.0;
+          ev += dev;
+          kx += dkx;
+          if (kx >= a.n_x) {
+            kx -= a.n_x;
+            ev++;
+          }
+        }
+        for (int j = lane; j < n_p; j += 32) {
+          double *fo = a.all_factors + (ep + j) * a.n_channels + c;
+          if (has_own && j >= own0 && j < own1)
+            *fo = a.factor_own ? a.factor_own[ep + j] : 0.0;
+          else if (a.ok && !a.ok[ep + j])
+            *fo = 0.0;
+        }
+        continue;
+      }
+      const int slot = at * 32 + lane;
+      if (slot < n_list && phs_in(event(listed[slot]), a.n_events, PHS_CHK_SLOT)) {
+        const int64_t e = event(listed[slot]);
         const PhsChannel &ch0 = a.channels[0];
         double sqrts = ch0.sqrts, lab_bg = ch0.lab ? ch0.lab_bg : 0.0;
         double lab_ga = ch0.lab ? ch0.lab_gamma : 1.0;
@@ -546,7 +562,7 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
         }
       }
     }
-    __syncthreads();  // the list is read
+    __syncthreads();  // the list is read, the counter was
   }
 }
 
