@@ -544,34 +544,43 @@ __device__ __forceinline__ void exact_event(const PhsLaunch &a, const PhsSegment
 }
 
 // Events that the float-float walk cannot decide (about 0.1 %, and all of a channel without a
-// float-float form) wait in a queue per warp and take the exact FP64 walk 32 at a time, or as
-// many as there are when the warp goes on to another segment or ends.  (A kernel behind the
-// walk for all of them took 35 to 50 us more a call, the latency of one FP64 walk and of two
-// launches.)
+// float-float form) wait in a queue per warp and take the exact FP64 walk 32 at a time, the last ones
+// of a warp together.  (A kernel behind the walk for all of them took 35 to 50 us more a call, the
+// latency of one FP64 walk and of two launches.)  The 32 may be of several segments, their lanes then
+// walking different programs: a warp's next tile is mostly of another segment, and a walk for each
+// segment's few events took 1e6 events of 10 channels with beams of their own 1161 us (5 particles;
+// 8: 1456) where this takes 687 (1136); 2^24 events over 64 channels 1534 -> 1526.
 template <bool PER_EVENT>
 struct ExactQueue {
-  int32_t *slots;   // 64, in shared memory
+  uint32_t *slots;  // 64, in shared memory: events by their place in the launch's tiles
   double *stack;
-  int n = 0, seg = 0;   // warp-uniform
+  int n = 0;        // warp-uniform
   __device__ __forceinline__ void flush(const PhsLaunch &a, const PhsSegment *segs, int least) {
     const int lane = threadIdx.x & 31;
     while (n >= least && n > 0) {
       const int take = n < 32 ? n : 32;
       __syncwarp();
-      const int32_t l = lane < take && phs_in(n - take + lane, 64, PHS_CHK_QUEUE) ? slots[n - take + lane] : -1;
+      const bool mine = lane < take && phs_in(n - take + lane, 64, PHS_CHK_QUEUE);
+      const int64_t at = mine ? slots[n - take + lane] : 0;
       __syncwarp();
       n -= take;
-      if (l >= 0) exact_event<PER_EVENT>(a, segs[seg], l, stack);
+      if (mine) {
+        int lo = 0, hi = a.n_segments - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (segs[mid].tile_begin <= at >> 5) lo = mid; else hi = mid - 1;
+        }
+        exact_event<PER_EVENT>(a, segs[lo], at - segs[lo].tile_begin * 32, stack);
+      }
       __syncwarp();
     }
   }
-  // Collective: the lanes with `want` queue event `local` of segment si (at most 31 wait, of si).
-  __device__ __forceinline__ void push(bool want, int si, int64_t local) {
+  // Collective: the lanes with `want` queue event `local` of segment sg (at most 31 wait).
+  __device__ __forceinline__ void push(bool want, const PhsSegment &sg, int64_t local) {
     const unsigned m = __ballot_sync(0xffffffffu, want);
     const int slot = n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
-    if (want && phs_in(slot, 64, PHS_CHK_QUEUE)) slots[slot] = (int32_t)local;
+    if (want && phs_in(slot, 64, PHS_CHK_QUEUE)) slots[slot] = (uint32_t)(sg.tile_begin * 32 + local);
     n += __popc(m);
-    seg = si;
   }
 };
 
@@ -777,7 +786,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
     phs_forward_ff_kernel(const __grid_constant__ PhsLaunch a) {
   static_assert(!(COMPACT && PER_EVENT), "the FP32 pre-test needs uniform beams");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int32_t exact_slots[PHS_FWD_BLOCK / 32][64];
+  __shared__ uint32_t exact_slots[PHS_FWD_BLOCK / 32][64];
   FFTables &T = *reinterpret_cast<FFTables *>(smem_raw);
   float *fst = reinterpret_cast<float *>(smem_raw + sizeof(FFTables));
   ExactQueue<PER_EVENT> exact{exact_slots[threadIdx.x >> 5], reinterpret_cast<double *>(fst)};
@@ -801,9 +810,9 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
           write_failed_event(a, sg, loc);
           return false;
         },
-        [&](int si, const PhsSegment &sg, int64_t loc) {
-          exact.flush(a, segs, si == exact.seg ? 32 : 1);
-          exact.push(loc >= 0 && !phs_event_ff(a, sg, loc, T, fst), si, loc);
+        [&](int, const PhsSegment &sg, int64_t loc) {
+          exact.flush(a, segs, 32);
+          exact.push(loc >= 0 && !phs_event_ff(a, sg, loc, T, fst), sg, loc);
         });
   } else {
     // (one call site of the exact walk, ahead of each tile: its code is large)
@@ -814,11 +823,11 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
         int mid = (lo + hi + 1) >> 1;
         if (segs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
       }
-      exact.flush(a, segs, more && lo == exact.seg ? 32 : 1);
+      exact.flush(a, segs, more ? 32 : 1);
       if (!more) break;
       const PhsSegment seg = segs[lo];
       const int64_t local = (tile - seg.tile_begin) * 32 + lane;
-      exact.push(local < seg.ev_count && !phs_event_ff<PER_EVENT>(a, seg, local, T, fst), lo, local);
+      exact.push(local < seg.ev_count && !phs_event_ff<PER_EVENT>(a, seg, local, T, fst), seg, local);
     }
   }
   if constexpr (COMPACT) exact.flush(a, segs, 1);
@@ -932,7 +941,7 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
   float *fst = reinterpret_cast<float *>(smem_raw + sizeof(FFTables));
   fill_ff_tables(T);
   __syncthreads();
-  __shared__ int32_t exact_slots[PHS_FWD_BLOCK / 32][64];
+  __shared__ uint32_t exact_slots[PHS_FWD_BLOCK / 32][64];
   ExactQueue<false> exact{exact_slots[threadIdx.x >> 5], reinterpret_cast<double *>(fst)};
   const int lane = threadIdx.x & 31;
   const PhsSegment *segs = a.n_segments <= PHS_INLINE_SEGS ? a.seg_inline : a.segments;
@@ -950,14 +959,14 @@ __global__ void __launch_bounds__(PHS_FWD_BLOCK, MIN_BLOCKS)
       if (pass_tile[mid] <= t) lo = mid; else hi = mid - 1;
     }
     // (one call site of the exact walk, ahead of each claim: its code is large)
-    exact.flush(a, segs, t < n_claims && lo == exact.seg ? 32 : 1);
+    exact.flush(a, segs, t < n_claims ? 32 : 1);
     if (t >= n_claims) break;
     const PhsSegment &seg = segs[lo];
     const int64_t idx = (t - pass_tile[lo]) * 32 + lane;
     const bool valid = idx < (int64_t)a.pass_count[lo] && phs_in(idx, seg.ev_count, PHS_CHK_QUEUE) &&
                        phs_in(seg.tile_begin * 32 + idx, a.n_tiles * 32, PHS_CHK_QUEUE);
     const int64_t local = valid ? a.pass_queue[seg.tile_begin * 32 + idx] : 0;
-    exact.push(valid && !phs_event_ff(a, seg, local, T, fst), lo, local);
+    exact.push(valid && !phs_event_ff(a, seg, local, T, fst), seg, local);
   }
 }
 

@@ -205,3 +205,32 @@ def test_line_between_the_wide_form_and_the_pairs(torch, n_out, per_visit):
         want = generate(torch, proc, x, 1000.0, precision=precision)
         for a, b in zip(got, want):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("variant", FF_FORMS)
+def test_exact_events_of_many_small_segments(torch, variant):
+    """A warp's exact FP64 walk takes events of any segments together: channels of 3 to 8 particles with
+    a STEP map each (no float-float form) and 1 to 7 events give the FP64 kernel's bits."""
+    from gpu_phs_gb300.api import Batch, PhaseSpace
+    rng = np.random.default_rng(77)
+    procs = []
+    for i in range(90):
+        p = P.random_process(rng, 3 + i % 6, 1, 1000.0)
+        p.map_ids = p.map_ids.copy()
+        # the largest branch below the root
+        code = max((c for c in (p.d1[0, 2 ** p.n_out - 2], p.d2[0, 2 ** p.n_out - 2]) if p.has_children[0, c - 1]))
+        p.map_ids[0, code - 1] = P.MAP_STEP_E if i % 2 else P.MAP_STEP_H
+        p.map_masses[0, code - 1], p.map_widths[0, code - 1] = 300.0, 30.0
+        procs.append(p)
+    counts = np.array([1 + i % 7 for i in range(len(procs))], np.int64)
+    spaces = [PhaseSpace(p, 500.0, 500.0) for p in procs]
+    size = int(sum(p.n_x * int(c) for p, c in zip(procs, counts)))
+    x = torch.rand(size, dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    plain, pairs = Batch(spaces), Batch(spaces)
+    plain.set_variants(-1, 0)
+    pairs.set_precision(1)
+    pairs.set_variants(variant, -1)
+    want, got = plain.generate(x, counts), pairs.generate(x, counts)
+    assert 20 < int(want[3].sum()) < len(want[3])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
