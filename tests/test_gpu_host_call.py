@@ -36,3 +36,22 @@ def test_a_call_of_many_events_chooses_the_variant(torch, n, precision):
     for e in (h, h2):
         for a, b in ((e.p, d.p), (e.factor, d.factor), (e.volume, d.volume), (e.ok, d.ok)):
             assert torch.equal(a, b.cpu())
+
+
+@pytest.mark.parametrize("pinned", ["none", "all", "p", "factor"])
+@pytest.mark.parametrize("n", [1000, 40_000, 600_001])
+def test_pinned_and_pageable_outputs(torch, n, pinned):
+    """Pinned outputs take small chunks first, pageable ones the largest: the same results."""
+    from gpu_phs_gb300.api import Events, PhaseSpace
+    proc = P.tt()
+    x = torch.from_numpy(uniform_x(5, n, proc.n_x)).pin_memory()
+    ps = PhaseSpace(proc, 500.0, 500.0)
+    d = ps.generate(x.cuda())
+    out = []
+    for name, shape, dtype in (("p", (n, proc.n_out, 4), torch.float64), ("factor", (n,), torch.float64),
+                               ("volume", (n,), torch.float64), ("ok", (n,), torch.uint8)):
+        t = torch.full(shape, 7, dtype=dtype)
+        out.append(t.pin_memory() if pinned in ("all", name) else t)
+    h = ps.generate_host(x, out=Events(*out))
+    for a, b in ((h.p, d.p), (h.factor, d.factor), (h.volume, d.volume), (h.ok, d.ok)):
+        assert torch.equal(a, b.cpu())
