@@ -278,14 +278,10 @@ __device__ void child_constants(const FxRegs &k, const PhsChild &C, double sqrts
 __device__ __noinline__ double lib_sinpi(double x) { return sinpi(x); }
 __device__ __noinline__ double lib_cospi(double x) { return cospi(x); }
 
-// sin and cos of 2 pi x for a phi mapping's x: in fixed point for 0 <= x < 1 (absolute
-// error 2^-60), else the library's.
+// sin and cos of 2 pi x for a phi mapping's x: in fixed point for 0 <= x < 1, else the library's.
 __device__ __forceinline__ void sincos2pi(double x, double &s, double &c) {
   if (fx_hi(x) < 0x3ff00000u) {
-    int64_t si, ci;
-    fx_sincos2pi_q62(fx_q64(x), si, ci);
-    s = fx_from_q62(si);
-    c = fx_from_q62(ci);
+    fx_sincos2pi(x, s, c);
   } else {
     s = lib_sinpi(2.0 * x);
     c = lib_cospi(2.0 * x);

@@ -343,3 +343,76 @@ def test_quotients_of_infinite_and_huge_numerators(tmp_path):
     n, bad = subprocess.run([str(tmp_path / "q")], check=True, capture_output=True, text=True).stdout.split()
     assert int(n) > 900_000
     assert int(bad) == 0
+
+
+SINCOS_DRIVER = r"""
+#include <cstdio>
+#include <cmath>
+#include <random>
+#include "phs_fix.h"
+typedef long double Q;
+static const Q PI = 3.14159265358979323846264338327950288L;
+static double err(double got, Q want) {
+  if (want == 0) return got != 0;
+  const double a = std::fabs((double)want);
+  return std::fabs((double)((Q)got - want)) / (std::nextafter(a, INFINITY) - a);
+}
+int main() {
+  std::mt19937_64 g(9);
+  std::uniform_real_distribution<double> U(0, 1);
+  double turns = 0, small = 0, radians = 0;
+  long n = 0;
+  for (int i = 0; i < 1500000; i++) {
+    double x;
+    switch (i % 4) {
+      case 0: x = U(g); break;
+      case 1: x = std::ldexp(U(g), -(int)(U(g) * 900)); break;
+      default: x = 0.25 * (i % 5) + (U(g) - 0.5) * std::ldexp(1.0, -(int)(U(g) * 50));
+    }
+    double s, c;
+    if (x >= 0 && x < 1) {
+      // the residual from the nearest quarter turn is exact
+      const double k = std::rint(4 * x);
+      const Q r = ((Q)x - (Q)k / 4) * 2 * PI, sr = sinl(r), cr = cosl(r);
+      const int q = (int)k & 3;
+      fx_sincos2pi(x, s, c);
+      turns = std::fmax(turns, err(s, q == 0 ? sr : q == 1 ? cr : q == 2 ? -sr : -cr));
+      turns = std::fmax(turns, err(c, q == 0 ? cr : q == 1 ? -sr : q == 2 ? -cr : sr));
+      n++;
+    }
+    if (x < 0x1p-9 && x >= 0) {
+      fx_sincos(x, s, c);
+      small = std::fmax(small, std::fmax(err(s, sinl((Q)x)), err(c, cosl((Q)x))));
+    }
+    const double phi = U(g) * 2 * M_PI;
+    fx_sincos(phi, s, c);
+    radians = std::fmax(radians, std::fabs((double)((Q)s - sinl((Q)phi))) - 0.52 * (std::nextafter(std::fabs(s), 9.0) - std::fabs(s)));
+  }
+  int bad = 0;
+  for (int k = 0; k < 4; k++) {   // quarter turns are exact, zeros positive
+    double s, c;
+    fx_sincos2pi(0.25 * k, s, c);
+    bad += s != (k == 1) - (k == 3) || c != (k == 0) - (k == 2) || (s == 0 && std::signbit(s)) || (c == 0 && std::signbit(c));
+  }
+  std::printf("%ld %.4f %.4f %.3e %d\n", n, turns, small, radians, bad);
+}
+"""
+
+
+def test_sin_and_cos_keep_their_relative_accuracy(tmp_path):
+    """sin and cos of 2 pi x within 1.2 ulp of themselves (2^-61 absolute where they are 2^-9, half an
+    ulp for the rounding) for x down to 2^-900 and to 2^-50 from a quarter turn; the sine of radians
+    below 2^-9 within 0.52 ulp, elsewhere within half an ulp and 2^-58."""
+    try:
+        subprocess.run(["g++", "--version"], check=True, capture_output=True)
+    except (OSError, subprocess.CalledProcessError):
+        pytest.skip("g++ not available")
+    (tmp_path / "s.cpp").write_text(SINCOS_DRIVER)
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=gnu++17", "-I", CSRC, str(tmp_path / "s.cpp"), "-o",
+                    str(tmp_path / "s")], check=True)
+    n, turns, small, radians, bad = subprocess.run([str(tmp_path / "s")], check=True, capture_output=True,
+                                                   text=True).stdout.split()
+    assert int(n) > 1_000_000
+    assert float(turns) <= 1.2 and float(small) <= 0.525
+    assert float(radians) <= 2.0 ** -58
+    assert int(bad) == 0
