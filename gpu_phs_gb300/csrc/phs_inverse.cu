@@ -395,6 +395,12 @@ __device__ double inverse_maps(const FxRegs &k, const PhsChannel &ch, double sqr
   return factor;
 }
 
+// The block's shared memory beside the dynamic one (phs_inverse_smem_bytes).
+struct InvShared {
+  uint16_t listed[PHS_INV_TILE];  // the tile's ok events
+  int warp_ok[PHS_INV_BLOCK / 32], next_work;
+};
+
 // One block: `tile` events and the channels of one tree shape (in the launch's slice of the
 // group order).  It gathers the tile's ok events and walks them, a warp 32 at a time, and writes
 // the outputs that need no arithmetic.  What bounds the kernel is the FP64 pipe; events are ok in
@@ -418,8 +424,7 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
   double *geo = stk + (size_t)PHS_INV_STATE * a.stack_depth * PHS_INV_BLOCK;  // per-visit geometry
   double *cache = a.group_reuse ? geo + (size_t)PHS_INV_GEO * a.max_visits * PHS_INV_BLOCK
                                 : nullptr;  // per-visit mapping results
-  __shared__ uint16_t listed[PHS_INV_TILE];  // the tile's ok events
-  __shared__ int warp_ok[kWarps], next_work;
+  __shared__ InvShared sh;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n_groups = a.group_hi - a.group_lo;
   const int64_t per_group = (a.n_events + a.tile - 1) / a.tile, n_items = per_group * n_groups;
@@ -452,21 +457,21 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
     const int64_t skip0 = skip_own ? a.ch_begin[c0] : 0;
     const int64_t skip1 = skip_own ? (c0 + 1 < a.n_channels ? a.ch_begin[c0 + 1] : a.n_events) : 0;
     int n_list = 0;  // block-uniform
-    if (tid == 0) next_work = 0;   // (read after the barriers below)
+    if (tid == 0) sh.next_work = 0;   // (read after the barriers below)
     for (int base = 0; base < n_ch * kChunk; base += PHS_INV_BLOCK) {
       const int j = base + tid;
       const int64_t e = event(j);
       const bool take = j < n_ch * kChunk && e < a.n_events && (!a.ok || a.ok[e]) && !(e >= skip0 && e < skip1);
       const unsigned m = __ballot_sync(0xffffffffu, take);
-      if (lane == 0) warp_ok[wid] = __popc(m);
+      if (lane == 0) sh.warp_ok[wid] = __popc(m);
       __syncthreads();
       int before = n_list, total = 0;
       for (int w = 0; w < kWarps; w++) {
-        if (w < wid) before += warp_ok[w];
-        total += warp_ok[w];
+        if (w < wid) before += sh.warp_ok[w];
+        total += sh.warp_ok[w];
       }
       const int d = before + __popc(m & ((1u << lane) - 1u));
-      if (take && phs_in(d, PHS_INV_TILE, PHS_CHK_SLOT)) listed[d] = (uint16_t)j;
+      if (take && phs_in(d, PHS_INV_TILE, PHS_CHK_SLOT)) sh.listed[d] = (uint16_t)j;
       n_list += total;
       __syncthreads();  // warp_ok is read, the entries are written
     }
@@ -477,7 +482,7 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
     const int n_walks = (n_list + 31) / 32, n_work = n_walks + n_ch * (hi - lo);
     for (;;) {
       int at = 0;
-      if (lane == 0) at = atomicAdd(&next_work, 1);
+      if (lane == 0) at = atomicAdd(&sh.next_work, 1);
       at = __shfl_sync(0xffffffffu, at, 0);
       if (at >= n_work) break;
       if (at >= n_walks) {
@@ -518,8 +523,8 @@ __global__ void __launch_bounds__(PHS_INV_BLOCK, 3)
         continue;
       }
       const int slot = at * 32 + lane;
-      if (slot < n_list && phs_in(event(listed[slot]), a.n_events, PHS_CHK_SLOT)) {
-        const int64_t e = event(listed[slot]);
+      if (slot < n_list && phs_in(event(sh.listed[slot]), a.n_events, PHS_CHK_SLOT)) {
+        const int64_t e = event(sh.listed[slot]);
         const PhsChannel &ch0 = a.channels[0];
         double sqrts = ch0.sqrts, lab_bg = ch0.lab ? ch0.lab_bg : 0.0;
         double lab_ga = ch0.lab ? ch0.lab_gamma : 1.0;
@@ -578,7 +583,7 @@ bool phs_inverse_fits_cache(int n_out, int stack_depth, int max_visits) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return phs_inverse_smem_bytes(n_out, stack_depth, max_visits, true, false) <= (size_t)optin;
+  return phs_inverse_smem_bytes(n_out, stack_depth, max_visits, true, false) + sizeof(InvShared) <= (size_t)optin;
 }
 
 static const void *inverse_kernel(bool per_event, bool lab_rows) {
