@@ -163,18 +163,28 @@ struct ChanLayout {  // per launched channel: shape of its x and p rows
   int x_stride;
 };
 
+int sm_count(int device) {
+  static int cached[64] = {0};
+  if (device >= 0 && device < 64 && cached[device]) return cached[device];
+  int n = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+  if (n <= 0) n = 1;
+  if (device >= 0 && device < 64) cached[device] = n;
+  return n;
+}
+
 int build_segments(Segments &S, const int64_t *counts, int n_channels,
-                   const std::vector<ChanLayout> &lay, int64_t ev0, int64_t x0, int64_t p0,
+                   const std::vector<ChanLayout> &lay, int device, int64_t ev0, int64_t x0, int64_t p0,
                    bool whizard_cols) {
   S.host.clear();
   // tiles per work chunk: long chunks append to the pre-test's queues with fewer atomics, short
-  // ones share the work evenly over its resident warps (152 SMs x 32): at least 8 chunks a warp,
+  // ones share the work evenly over its resident warps (32 an SM): at least 8 chunks a warp,
   // or single tiles.  With 8 tiles always, 3e5 events left three warps of four idle: 12-particle
   // trees 264 us (226 so), 3e5 events over 64 channels 107 (82), 2^22 610 (582).
   int64_t total = 0;
   for (int c = 0; c < n_channels; c++) total += counts[c] > 0 ? counts[c] : 0;
   S.chunk_tiles = PHS_CHUNK_TILES;
-  while (S.chunk_tiles > 1 && total / 32 < (int64_t)S.chunk_tiles * 8 * 4864) S.chunk_tiles /= 2;
+  while (S.chunk_tiles > 1 && total / 32 < (int64_t)S.chunk_tiles * 8 * 32 * sm_count(device)) S.chunk_tiles /= 2;
   int64_t ev = ev0, x = x0, p = p0, tile = 0, chunk = 0;
   for (int c = 0; c < n_channels; c++) {
     const int64_t n = counts[c];
@@ -238,16 +248,6 @@ int attach_segments(Segments &S, PhsLaunch &a, cudaStream_t stream) {
   }
   a.segments = S.dev.as<PhsSegment>();
   return PHS_OK;
-}
-
-int sm_count(int device) {
-  static int cached[64] = {0};
-  if (device >= 0 && device < 64 && cached[device]) return cached[device];
-  int n = 0;
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
-  if (n <= 0) n = 1;
-  if (device >= 0 && device < 64) cached[device] = n;
-  return n;
 }
 
 int grid_for(int64_t n_tiles, int device, int stack_depth, bool per_event, int variant) {
@@ -799,7 +799,7 @@ static int launch_process(phs_process_t h, Segments &S, int64_t n_events, const 
                           bool whizard_cols, cudaStream_t stream, int64_t call_tiles = 0) {
   int64_t one = n_events;
   const int64_t *cnt = counts ? counts : &one;
-  int rc = build_segments(S, cnt, h->p.n_channels, h->lay, ev0, 0, 0, whizard_cols);
+  int rc = build_segments(S, cnt, h->p.n_channels, h->lay, h->device, ev0, 0, 0, whizard_cols);
   if (rc) return rc;
   PhsLaunch a;
   memset(&a, 0, sizeof a);
@@ -886,7 +886,7 @@ extern "C" int phs_adjoint_device(phs_process_t h, int64_t n_events, const int64
       return fail(PHS_ERR_INVALID_ARG, "null data pointer");
     DeviceGuard g(h->device);
     int64_t one = n_events;
-    int rc = build_segments(h->segs, counts ? counts : &one, h->p.n_channels, h->lay, 0, 0, 0, false);
+    int rc = build_segments(h->segs, counts ? counts : &one, h->p.n_channels, h->lay, h->device, 0, 0, 0, false);
     if (rc) return rc;
     PhsLaunch a;
     memset(&a, 0, sizeof a);
@@ -1248,7 +1248,7 @@ extern "C" int phs_batch_generate_device(phs_batch_t b, const int64_t *counts, c
     if (int rc = check_counts(counts, n, n_events)) return rc;
     if (int rc = check_ptrs(n_events, x, p, f, v, ok)) return rc;
     DeviceGuard g(b->device);
-    int rc = build_segments(b->segs, counts, n, b->lay, 0, 0, 0, false);
+    int rc = build_segments(b->segs, counts, n, b->lay, b->device, 0, 0, 0, false);
     if (rc) return rc;
     PhsLaunch a;
     memset(&a, 0, sizeof a);
@@ -1367,7 +1367,7 @@ extern "C" int phs_generate_device_noalloc(phs_process_t h, double E1, double E2
     std::vector<ChanLayout> lay(P.n_channels, ChanLayout{P.n_out, P.n_x});
     int64_t one = n_events;
     Segments S;
-    int rc = build_segments(S, counts ? counts : &one, P.n_channels, lay, 0, 0, 0, false);
+    int rc = build_segments(S, counts ? counts : &one, P.n_channels, lay, h->device, 0, 0, 0, false);
     if (rc) return rc;
     PhsLaunch a;
     memset(&a, 0, sizeof a);
