@@ -490,7 +490,7 @@ def measure_variants(torch, steps: int, warmup: int, x_tt, out_tt, ms_tt64, pin=
         "hbm_gbs": (wbytes + rbytes) / t_inv * 1e-6,
         "algorithmic_bytes_per_step": wbytes + rbytes,
         "ok_fraction": ev.ok.double().mean().item(),
-        "launch": "one persistent kernel: 64 events per block at a time, every channel per event"}
+        "launch": "one kernel, a block per tile of events and tree shape"}
     # the CPU path beside it: the reference has no CPU inverse (its inverse is GPU code,
     # phs.cu:1499-1554), so the oracle's restatement of that algorithm runs, on the first
     # ns events (each channel's first ns / n_channels), checked element by element
@@ -822,8 +822,8 @@ def run_ours(args):
         e2e = {"value": statistics.median(windows), "unit": "events/s",
                "h2d_bytes_per_step": n * proc.n_x * 8,
                "d2h_bytes_per_step": n * (32 * proc.n_out + 8 + 1),
-               "path": "phs_generate_host (C ABI), pinned host buffers, 512 Ki-event chunks on 3 "
-                       "streams; volumes (one constant per channel) written on the host",
+               "path": "phs_generate_host (C ABI), pinned host buffers, chunks of 16 Ki events "
+                       "growing by half to 512 Ki on 3 streams; volumes (one constant per channel) written on the host",
                "steps": e2e_steps, "windows": windows,
                "windowing": "median of three windows of `steps` calls each"}
         if world == 1:

@@ -28,8 +28,9 @@ def _stream(stream) -> Optional[int]:
     import torch
     if stream is not None:
         return stream.cuda_stream
-    # the current stream's handle without a Stream object (0.3 us instead of 3)
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the current stream's handle without a Stream object (0.3 us instead of 3), where torch has it
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
 
 
 @dataclass

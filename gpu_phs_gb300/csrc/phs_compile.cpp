@@ -238,8 +238,6 @@ int compile_channel(const Process &p, int c, double sqrts, PhsChannel &out, Chan
     V.b0 = b[0];
     V.b1 = b[1];
     V.m = p.map_m[mx(cur)];
-    V.self_m_min = m_min;
-    V.self_m_max = m_max;
     V.self_root = cur == R;
     V.parent_root = cur != R && (kid(R, 0) == cur || kid(R, 1) == cur);
     // friends (extract_boost_origins, phs.cu:268-292): code 2^n_out pairs the branch with

@@ -36,15 +36,11 @@ FF_FN float f_add(float a, float b) { return __fadd_rn(a, b); }
 FF_FN float f_sub(float a, float b) { return __fsub_rn(a, b); }
 FF_FN float f_mul(float a, float b) { return __fmul_rn(a, b); }
 FF_FN float f_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-FF_FN float f_sqrt(float a) { return __fsqrt_rn(a); }
-FF_FN float f_div(float a, float b) { return __fdiv_rn(a, b); }
 #else
 FF_FN float f_add(float a, float b) { volatile float r = a + b; return r; }
 FF_FN float f_sub(float a, float b) { volatile float r = a - b; return r; }
 FF_FN float f_mul(float a, float b) { volatile float r = a * b; return r; }
 FF_FN float f_fma(float a, float b, float c) { return fmaf(a, b, c); }
-FF_FN float f_sqrt(float a) { return sqrtf(a); }
-FF_FN float f_div(float a, float b) { volatile float r = a / b; return r; }
 #endif
 
 FF_FN ff ff_make(float hi, float lo) { ff r; r.hi = hi; r.lo = lo; return r; }
@@ -100,34 +96,10 @@ FF_FN ff ff_mul_f(ff a, float b) {
   return fast_two_sum(p.hi, e);
 }
 
-// a*b + c
-FF_FN ff ff_fma(ff a, ff b, ff c) { return ff_add(ff_mul(a, b), c); }
-
 FF_FN ff ff_sqr(ff a) {
   ff p = two_prod(a.hi, a.hi);
   float e = f_fma(f_add(a.hi, a.hi), a.lo, p.lo);
   return fast_two_sum(p.hi, e);
-}
-
-FF_FN ff ff_div(ff a, ff b) {
-  float q1 = f_div(a.hi, b.hi);
-  ff r = ff_sub(a, ff_mul_f(b, q1));
-  float q2 = f_div(r.hi, b.hi);
-  ff q = fast_two_sum(q1, q2);
-  r = ff_sub(a, ff_mul(b, q));
-  float q3 = f_div(r.hi, b.hi);
-  return ff_add_f(q, q3);
-}
-
-FF_FN ff ff_recip(ff b) { return ff_div(ff_from_float(1.0f), b); }
-
-// sqrt(a), a >= 0; one Newton step on the float square root, residual in float-float.
-FF_FN ff ff_sqrt(ff a) {
-  if (!(a.hi > 0.0f)) return ff_make(a.hi == 0.0f ? 0.0f : f_sqrt(a.hi), 0.0f);
-  float y = f_sqrt(a.hi);
-  ff r = ff_sub(a, two_prod(y, y));
-  float c = f_div(r.hi, f_add(y, y));
-  return fast_two_sum(y, c);
 }
 
 #if defined(__CUDA_ARCH__)
@@ -212,31 +184,6 @@ FF_FN ff ff_dot3(ff a0, ff b0, ff a1, ff b1, ff a2, ff b2) {
   return fast_two_sum(s.hi, f_add(e, s.lo));
 }
 
-FF_FN ff ff_dot4(ff a0, ff b0, ff a1, ff b1, ff a2, ff b2, ff a3, ff b3) {
-  const ff p0 = two_prod(a0.hi, b0.hi), p1 = two_prod(a1.hi, b1.hi);
-  const ff p2 = two_prod(a2.hi, b2.hi), p3 = two_prod(a3.hi, b3.hi);
-  float e = f_fma(a0.hi, b0.lo, f_fma(a0.lo, b0.hi, p0.lo));
-  e = f_add(e, f_fma(a1.hi, b1.lo, f_fma(a1.lo, b1.hi, p1.lo)));
-  e = f_add(e, f_fma(a2.hi, b2.lo, f_fma(a2.lo, b2.hi, p2.lo)));
-  e = f_add(e, f_fma(a3.hi, b3.lo, f_fma(a3.lo, b3.hi, p3.lo)));
-  ff s = two_sum(p0.hi, p1.hi);
-  e = f_add(e, s.lo);
-  s = two_sum(s.hi, p2.hi);
-  e = f_add(e, s.lo);
-  s = two_sum(s.hi, p3.hi);
-  return fast_two_sum(s.hi, f_add(e, s.lo));
-}
-
-FF_FN bool ff_gt(ff a, ff b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
-FF_FN float ff_to_float(ff a) { return f_add(a.hi, a.lo); }
-
-// Double -> float-float, truncated to 48 bits (the pair holds 48).
-FF_FN ff ff_from_double(double d) {
-  float hi = (float)d;
-  float lo = (float)(d - (double)hi);
-  return ff_make(hi, lo);
-}
-
 #if defined(__CUDA_ARCH__)
 FF_FN uint64_t ff_dbits(double d) { return (uint64_t)__double_as_longlong(d); }
 FF_FN double ff_bitsd(uint64_t b) { return __longlong_as_double((long long)b); }
@@ -251,7 +198,7 @@ FF_FN float ff_bitsf(uint32_t b) { float f; memcpy(&f, &b, 4); return f; }
 FF_FN int ff_clz(uint32_t v) { return v ? __builtin_clz(v) : 32; }
 #endif
 
-// The same conversions without FP64 instructions: the significand's upper 24 bits are the high
+// Double -> float-float (48 bits) without FP64 instructions: the significand's upper 24 bits are the high
 // part's, the 29 bits below it are converted as an integer and scaled (rounded to 24 bits).  The
 // high part is truncated, so for 0 <= d < 1 the order against 0.5 is kept exactly (d < 0.5 iff
 // hi < 0.5f).  Values below 2^-103 in magnitude (or non-finite) are not handled: their low part
@@ -351,15 +298,14 @@ FF_FN double ff_to_double_scaled(ff f, int e) {
 #define FF_PI_HI 3.1415927410125732f
 #define FF_PI_LO -8.7422776573475858e-08f
 
-// Tables (built on the host, phs_ff_tables in phs_kernels_ff.cu):
+// Tables (built per block in shared memory, fill_ff_tables in phs_kernels_ff.cu; on the host,
+// ff_fill_tables):
 //   trig[k] = {sin(k pi/128).hi, .lo, cos(k pi/128).hi, .lo}, k = 0..255
 //   exp2[j] = {2^(j/32).hi, .lo}, j = 0..31
 struct FFTables {
   float4 trig[256];
   float2 exp2[32];
 };
-
-FF_FN ff ff_pi() { return ff_make(FF_PI_HI, FF_PI_LO); }
 
 // sin and cos of k pi/128 + f for |f| <= pi/256 (radians): sin f = f - f^3/6 + f^5/120 (the
 // cubic term as a pair: tan next to 0 and cot next to pi/2 keep their relative accuracy) and
@@ -408,13 +354,6 @@ FF_FN ff ff_tan(ff z, const FFTables &T) {
   ff s, c;
   ff_sincos(z, T, s, c);
   return ff_div_fast(s, c);
-}
-
-// cot(u) = 1/tan(u) for 0 < |u| <= pi/2.
-FF_FN ff ff_cot(ff u, const FFTables &T) {
-  ff s, c;
-  ff_sincos(u, T, s, c);
-  return ff_div_fast(c, s);
 }
 
 // exp(y), |y| < 80.

@@ -83,8 +83,6 @@ struct alignas(16) PhsVisit {
   int32_t push;       // child pushed on the stack after this visit (0/1), -1: none
   double b0, b1;      // collinear cos(theta) constants at the handle's sqrt(s)
   double m;           // the visited branch's mapping mass (per-event b0 = m^2/s)
-  double self_m_min;  // the visited branch's m_min (per-event m_max)
-  double self_m_max;  // the visited branch's ok-test bound at the handle's sqrt(s)
   int32_t self_root;  // 1 for the root visit
   int32_t both_leaves;  // 1 when neither child is internal (only L columns 0,3 needed)
   int32_t friend_sign;  // 0, or the beam (+1: along +z, -1: along -z) that the visited
