@@ -271,16 +271,22 @@ FF_FN double ff_widen(float f, int e2 = 0) {
 FF_FN double ff_to_double_int(ff a) { return ff_widen(a.hi) + ff_widen(a.lo); }
 
 // f 2^e with f's high part put back into [1, 2), for |f| < 2^127: a product of many factors that
-// stays in the floats' range whatever their sizes.
-FF_FN void ff_renorm(ff &f, int &e) {
+// stays in the floats' range whatever their sizes.  e counts in units of `unit`.
+FF_FN void ff_renorm(ff &f, int &e, int unit) {
   const uint32_t b = ff_fbits(f.hi) & 0x7f800000u;
   const float scale = ff_bitsf(0x7f000000u - b);   // 2^(127 - exponent field), exact on both parts
   f = ff_make(f_mul(f.hi, scale), f_mul(f.lo, scale));
-  e += (int)(b >> 23) - 127;
+  e += ((int)(b >> 23) - 127) * unit;
 }
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+double ff_rare_ldexp(double d, int e) { return ldexp(d, e); }
 // f 2^e as a double (finite f; the exponent goes into the widened parts, which then stay normal).
 FF_FN double ff_to_double_scaled(ff f, int e) {
-  if (e < -800 || e > 800) return ldexp(ff_to_double_int(f), e);
+  if (e < -800 || e > 800) return ff_rare_ldexp(ff_to_double_int(f), e);
   return ff_widen(f.hi, e * 1048576) + ff_widen(f.lo, e * 1048576);
 }
 

@@ -21,7 +21,8 @@
 // leading differences in roots and quotients, conversions through the integer-to-float unit,
 // and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 322 us, a constant's pair in one
 // load (PhsFF) to 304 us, outputs widened with integers (ff_to_double_int) to 270 us, a visit's
-// integers in one load (PhsVisitFF) to 263 us.  The error of the momenta went from 2.1e-14 to
+// integers in one load (PhsVisitFF) to 263 us (259 now, with the undecided events' walks shared by
+// segments and the factor's exponent).  The error of the momenta went from 2.1e-14 to
 // 1.0e-14.  What waits on global loads (18 % of the stalls) is
 // the program's constants: prefetches of the x rows changed nothing, and the program staged in
 // shared memory gave tt 1 % and cost the 64-channel batch 2 %.  Five or six blocks a SM (96, 80
@@ -235,14 +236,13 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
   // beams: the channel's, or this event's (phs_event_f64's expressions)
   ff sqrts_f = ld(ch.sqrts), s_f = ld(ch.s), lab_bg = ld(ch.lab_bg), lab_ga = ld(ch.lab_gamma);
   const bool lab = PER_EVENT || ch.lab != 0;
-  double sqrts64 = 0.0, s64 = 0.0;
+  double sqrts64 = 0.0;
   ff inv_s_f = zero;
   if (PER_EVENT) {
     // the beams in float-float; sqrt(s) in FP64 as well for the volume, the collinear
     // cos(theta) constants and the maps whose constants stay FP64
     const double E1 = a.E1[ev], E2 = a.E2[ev];
     sqrts64 = dmul(2.0, sqrt(dmul(E1, E2)));
-    s64 = dmul(sqrts64, sqrts64);
     const ff e1 = ff_from_double_int(E1), e2 = ff_from_double_int(E2);
     const ff r = ff_sqrt_fast(ff_mul(e1, e2));
     sqrts_f = ff_twice(r);
@@ -258,12 +258,13 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
 #pragma unroll
   for (int i = 0; i < 16; i++) L[i] = zero;
   ff msq_b = s_f, m_b = sqrts_f, p_b = zero, E_b = sqrts_f;
-  // the factor, times 2^fe: its terms run from mappings' constants of 1e-11 each to tan^2 z of 1e13,
-  // so the pair is put back into [1, 2) once a visit (1e6 tt events 259.5 -> 261.2 us)
+  // the factor, times 2^(fe >> 2): its terms run from mappings' constants of 1e-11 each to tan^2 z of
+  // 1e13, so the pair is put back into [1, 2) once a visit.  fe & 3 is the number of saved frames (two
+  // registers for them spill: 2e6 tt events with their own beams 770 us, 751 so; 1e6 with uniform
+  // ones 257.9, 259.0 without the exponent)
   ff factor = PER_EVENT ? one : ld(ch.f0);
-  int fe = PER_EVENT ? 0 : ch.f0_exp;
+  int fe = PER_EVENT ? 0 : ch.f0_exp * 4;
   bool ok = true;
-  int sp = 0;
 
   const int n_visits = ch.n_visits;
   for (int v = 0; v < n_visits; v++) {
@@ -342,7 +343,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       const ff slrm = ff_mul(sl, rm);
       pc = ff_half(slrm);                                  // sqrt(lambda) / (2 m)
       factor = ff_mul(factor, ff_mul(slrm, rm));           // sqrt(lambda) / m^2
-      ff_renorm(factor, fe);
+      ff_renorm(factor, fe, 4);
       if (massless == 0) {
         const ff dc = ff_sub(cmsq[0], cmsq[1]), hm = ff_half(rm);
         ce0 = ff_mul(ff_add(msq_b, dc), hm);
@@ -363,7 +364,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       ff b0 = ld(V.b0), b1 = ld(V.b1), fct;
       if (PER_EVENT) {
         const double m = a.channels[seg.channel].visit[v].m;
-        const double b0d = dmul(m, m) / s64;
+        const double b0d = dmul(m, m) / dmul(sqrts64, sqrts64);
         b0 = ff_from_double_int(b0d);
         b1 = ff_from_double_int(log(dadd(b0d, 1.0) / b0d));
       }
@@ -380,7 +381,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
         fct = zero;
       }
       factor = ff_mul(factor, fct);   // the uniform map's is 1
-      ff_renorm(factor, fe);
+      ff_renorm(factor, fe, 4);
     } else {
       // ct = 2x - 1, st = sqrt(2(1 - x) 2x) = 2 sqrt((1-x) x)
       if (PER_EVENT) {
@@ -485,6 +486,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
     }
 
     const int push = (code >> 25 & 3) - 1, carry = (code >> 23 & 3) - 1;
+    const int sp = fe & 3;
     if (push >= 0 && phs_in(sp, a.stack_depth, PHS_CHK_STACK)) {
       const bool j0 = push == 0;
 #pragma unroll
@@ -493,7 +495,7 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       fstack_store(fst, sp, 17, ffsel(j0, cm[0], cm[1]));
       fstack_store(fst, sp, 18, j0 ? pc : ff_neg(pc));
       fstack_store(fst, sp, 19, ffsel(j0, ce0, ce1));
-      sp++;
+      fe++;
     }
     if (carry >= 0) {
       const bool j0 = carry == 0;
@@ -502,18 +504,18 @@ __device__ __forceinline__ bool phs_event_ff(const PhsLaunch &a, const PhsSegmen
       p_b = j0 ? pc : ff_neg(pc);
       E_b = ffsel(j0, ce0, ce1);
     } else if (sp > 0) {
-      sp--;
+      fe--;
 #pragma unroll
-      for (int i = 0; i < 16; i++) L[i] = fstack_load(fst, sp, i);
-      msq_b = fstack_load(fst, sp, 16);
-      m_b = fstack_load(fst, sp, 17);
-      p_b = fstack_load(fst, sp, 18);
-      E_b = fstack_load(fst, sp, 19);
+      for (int i = 0; i < 16; i++) L[i] = fstack_load(fst, sp - 1, i);
+      msq_b = fstack_load(fst, sp - 1, 16);
+      m_b = fstack_load(fst, sp - 1, 17);
+      p_b = fstack_load(fst, sp - 1, 18);
+      E_b = fstack_load(fst, sp - 1, 19);
     }
   }
 
   a.volume[ev] = PER_EVENT ? channel_volume(a.channels[seg.channel], sqrts64) : ch.volume;
-  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? ff_to_double_scaled(factor, fe) : 0.0;
+  a.factor[ev * a.factor_stride + seg.factor_col] = ok ? ff_to_double_scaled(factor, fe >> 2) : 0.0;
   a.ok[ev] = ok ? 1 : 0;
   if (!ok) {
     double2 *o = reinterpret_cast<double2 *>(out);
