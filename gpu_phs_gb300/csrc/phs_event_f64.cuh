@@ -20,9 +20,9 @@
 //     predicated instructions, which take their turn on the FP64 pipe all the same.
 // A tt event takes 302 FP64 instructions (445 before, 81 of them predicated off), the pipe is
 // 91 % busy.  Against the library's functions and the plain product of matrices: 1e7 tt events
-// 13.84 -> 8.29 (functions) -> 5.18 ms; 3e6 events of the 13 TeV caterpillar 0.346 -> 0.225,
-// 2^22 events over 64 channels 1.10 -> 0.57, 5e5 tt events with their own beams 0.936 -> 0.413,
-// 3e5 12-particle events 0.502 -> 0.215 ms (the first, second and last of these four with the
+// 13.84 -> 8.29 (functions) -> 5.21 ms; 3e6 events of the 13 TeV caterpillar 0.346 -> 0.225,
+// 2^22 events over 64 channels 1.10 -> 0.57, 5e5 tt events with their own beams 0.936 -> 0.416,
+// 3e5 12-particle events 0.502 -> 0.216 ms (the first, second and last of these four with the
 // pre-test's own changes).
 // Momenta are nearer the exact map (median error of tt 3.1e-16 -> 2.2e-16 of the energy, against
 // an 80-bit evaluation).

@@ -329,8 +329,8 @@ FX_FN uint64_t fx_div_q62(uint64_t n, uint64_t d) {
   return q + (uint64_t)(((int64_t)r * (int64_t)(uint32_t)(Y >> 33)) >> 29);
 }
 
-// tan(z) for |z| < pi/2 as doubles: within 0.51 ulp above pi/4 and for 2^-10 < |z|; below,
-// within 2^-62 absolute.  z and, above pi/4, pi/2 - |z| are reduced exactly.
+// tan(z) for |z| < pi/2 as doubles: within 0.51 ulp.  z and, above pi/4, pi/2 - |z| are reduced
+// exactly and stay normalized.
 FX_FN double fx_tan(double z) {
   const uint32_t zh = fx_hi(z);
   const int be = (int)((zh >> 20) & 0x7ffu);                      // <= 1023

@@ -17,8 +17,8 @@
 // constants (the same bits), and what is rare is called rather than inlined: four warps of a
 // block walk the same program, but different blocks do not, and with twice the code the
 // instruction fetches took a sixth of the time.  2e5 events of 16 channels (6 particles):
-// 6.09 -> 2.60 ms (FP64 pipe 79 % busy; 3.45 ms with 64-thread blocks and the rare code
-// inlined, 4.0 ms with 32-thread blocks).
+// 6.09 -> 2.47 ms (before tiles were spread over the call 2.60; 3.45 with 64-thread blocks and the
+// rare code inlined, 4.0 with 32-thread blocks).
 //
 // At a visit of branch b, with Gp and (theta, phi) the frame and angles of b's parent:
 //   G   = [R_f^-1] B_z(-bg_b) R_y(-theta) R_z(-phi) Gp   b's rest frame, z along its flight

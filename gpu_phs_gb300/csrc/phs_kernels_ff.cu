@@ -21,7 +21,7 @@
 // leading differences in roots and quotients, conversions through the integer-to-float unit,
 // and 1 - x, 2x - 1 and x (1 - x) on the FP64 pipe took it to 322 us, a constant's pair in one
 // load (PhsFF) to 304 us, outputs widened with integers (ff_to_double_int) to 270 us, a visit's
-// integers in one load (PhsVisitFF) to 263 us (259 now, with the undecided events' walks shared by
+// integers in one load (PhsVisitFF) to 263 us (258 now, with the undecided events' walks shared by
 // segments and the factor's exponent).  The error of the momenta went from 2.1e-14 to
 // 1.0e-14.  What waits on global loads (18 % of the stalls) is
 // the program's constants: prefetches of the x rows changed nothing, and the program staged in
@@ -554,7 +554,8 @@ __device__ __forceinline__ void exact_event(const PhsLaunch &a, const PhsSegment
 // 8: 1456) where this takes 687 (1136); 2^24 events over 64 channels 1534 -> 1526.
 template <bool PER_EVENT>
 struct ExactQueue {
-  uint32_t *slots;  // 64, in shared memory: events by their place in the launch's tiles
+  uint32_t *slots;  // 64, in shared memory: events by their place in the launch's tiles (32 a tile;
+                    // below 2^32: an event takes 97 bytes of device memory and more)
   double *stack;
   int n = 0;        // warp-uniform
   __device__ __forceinline__ void flush(const PhsLaunch &a, const PhsSegment *segs, int least) {
