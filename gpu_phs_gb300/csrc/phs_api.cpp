@@ -1020,18 +1020,27 @@ static int inverse_launch(phs_process_t h, int64_t n_events, const int64_t *d_ch
   a.group_lo = (int32_t)(std::upper_bound(gb.begin(), gb.end(), a.order_lo) - gb.begin()) - 1;
   a.group_hi = (int32_t)(std::lower_bound(gb.begin(), gb.end(), a.order_hi) - gb.begin());
   if (a.order_lo >= a.order_hi) return PHS_OK;
-  // events per block: the launch's (event, shape) pairs over as few full waves of resident blocks as
-  // tiles of PHS_INV_TILE events allow.  Long tiles fill the warps with ok events (a block's last
+  // events per block: the launch's (event, shape) pairs over few full waves of resident blocks, in
+  // tiles of PHS_INV_TILE events at most.  Long tiles fill the warps with ok events (a block's last
   // warp of them is half empty), and a wave that is not full leaves SMs idle.  (Tiles halved until
   // there were four waves had 8 ok events a block for 4e4 events of one 12-particle shape, 12 % of
-  // them ok: 704 us, 270 so.)
-  const int64_t resident = (int64_t)sm_count(h->device) *
-                           phs_inverse_blocks_per_sm(a.n_out, a.stack_depth, a.max_visits,
-                                                     E1 != nullptr, cache, !a.lab);
+  // them ok: 704 us, 270 in one wave.)  Shapes differ in their channels and their depth, and so in
+  // the time of their blocks: with several shapes and several blocks a SM, at least three waves
+  // even that out.  (One / three waves, us: 42145 4-particle events of 7 shapes, 86 % ok, 307 / 262;
+  // 20902 5-particle events of 2 shapes, 68 % ok, 62 / 55; with few ok events one wave would do, as
+  // 20000 8-particle events of 4 shapes, 11 % ok, 96 / 158, but their number is not known here.)
+  const int per_sm = phs_inverse_blocks_per_sm(a.n_out, a.stack_depth, a.max_visits, E1 != nullptr, cache, !a.lab);
+  const int64_t resident = (int64_t)sm_count(h->device) * per_sm;
   const int64_t groups = a.group_hi - a.group_lo, chunks = (n_events + PHS_INV_CHUNK - 1) / PHS_INV_CHUNK;
-  const int64_t waves = std::max<int64_t>(1, (n_events * groups + resident * PHS_INV_TILE - 1) / (resident * PHS_INV_TILE));
-  const int64_t per_group = std::max<int64_t>(1, waves * resident / groups);
-  a.tile = (int32_t)std::min<int64_t>(PHS_INV_TILE, (chunks + per_group - 1) / per_group * PHS_INV_CHUNK);
+  int64_t waves = std::max<int64_t>(groups > 1 && per_sm > 1 ? 3 : 1,
+                                    n_events * groups / (resident * PHS_INV_TILE));
+  int64_t block_chunks = 0;
+  for (;; waves++) {
+    const int64_t per_group = std::max<int64_t>(1, waves * resident / groups);
+    block_chunks = (chunks + per_group - 1) / per_group;
+    if (block_chunks * PHS_INV_CHUNK <= PHS_INV_TILE) break;
+  }
+  a.tile = (int32_t)(block_chunks * PHS_INV_CHUNK);
   CUDA_TRY(phs_launch_inverse(a, st));
   return PHS_OK;
 }
